@@ -104,6 +104,37 @@ def test_diffus_and_ghosts_bitwise():
     np.testing.assert_array_equal(_host(d_dff), dff)
 
 
+# edges of the 16 x 8 tile of small grids and the 32 x 16 tile of grids above
+# 3 * 152 * 512 (diffusion) and 9 * 152 * 512 cells (advection)
+@pytest.mark.parametrize("scheme", ["weno5", "quick", "fromm"])
+@pytest.mark.parametrize("shape", [(16, 8), (17, 9), (15, 7), (3, 130), (569, 547), (863, 833)])
+@pytest.mark.parametrize("bcs", [("periodic", "closed"), ("closed", "periodic")])
+def test_stencil_tiles_bitwise(scheme, shape, bcs):
+    Nz, Nx = shape
+    xBC, zBC = bcs
+    rng = np.random.default_rng(Nz + Nx)
+    f = rng.random((Nz, Nx)) + rng.standard_normal((Nz, Nx)) ** 3
+    k = rng.random((Nz, Nx)) + 0.5
+    u, w = rng.standard_normal((Nz, Nx + 1)), rng.standard_normal((Nz + 1, Nx))
+    u[rng.random(u.shape) < 0.05] = 0.0
+    if scheme != "weno5":      # what is not finite takes the reference's full formula
+        f[Nz // 2, Nx // 2], f[0, 1] = np.inf, np.nan
+    d = [torch.zeros(s, dtype=torch.float64, device="cuda") for s in ((Nx, Nz), (Nx + 1, Nz + 2), (Nx + 2, Nz + 1))]
+    with np.errstate(all="ignore"):
+        ref = O.advect_centered_with_flux(f, u, w, 0.37, scheme, xBC, zBC)
+    xc.advect_centered_with_flux(*d, _dev(f), _dev(u), _dev(w), 0.37, scheme, xBC, zBC)
+    torch.cuda.synchronize()
+    for got, want in zip(d, ref):
+        np.testing.assert_array_equal(_host(got), want)
+    f = rng.random((Nz, Nx))
+    ref = O.diffus_centered_with_flux(f, k, 0.3)
+    xc.diffus_with_flux(*d, _dev(O.embed_halo(f, 1, "closed", "periodic")), _dev(O.embed_halo(k, 1, "closed", "periodic")),
+                        0.3)
+    torch.cuda.synchronize()
+    for got, want in zip(d, ref):
+        np.testing.assert_array_equal(_host(got), want)
+
+
 def test_ghosts_halo3_both_closed():
     Nz, Nx, g = 9, 6, 3
     f = np.random.default_rng(1).random((Nz, Nx))

@@ -292,13 +292,11 @@ constexpr int kWeno5OneDiv = 105;
 inline int advect_scheme(int scheme, const xc_params& p) {
   return scheme == XC_WENO5 && p.weno_weights == 1 ? kWeno5OneDiv : scheme;
 }
+// pad: qx_int, qz_int view the interior of arrays with the reference's padding
+// (one row above and below, one column left and right), which is filled too
 int stencil_advect_flux(const double* f, int ldf, bool halod, int Nz, int Nx, int scheme,
                         int xBC, int zBC, CView u, CView w, double h,
-                        DView adv, DView qx_int, DView qz_int, cudaStream_t s);
-int stencil_diffus_flux(const double* f, const double* k, int ld, bool halod, int Nz, int Nx,
-                        int xBC, int zBC, double h, DView dff, DView qx_int, DView qz_int,
-                        cudaStream_t s);
-int pad_face_fluxes(DView qx, DView qz, int Nz, int Nx, int xBC, int zBC, cudaStream_t s);
+                        DView adv, DView qx_int, DView qz_int, cudaStream_t s, bool pad = false);
 int scheme_halo(int scheme);
 
 int phsevo_impl(xc_ctx* c, int scheme, const double coefs[6], double dt, double alpha);

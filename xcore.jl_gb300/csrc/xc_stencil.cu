@@ -10,13 +10,35 @@
 // Compiled with -fmad=false so no multiply-add is contracted (Julia does not
 // contract either); with identical inputs the results are bitwise equal to
 // the reference arithmetic.
+//
+// What bounds it: sm_103a's FP64 unit takes one warp instruction per 64 cycles
+// and sub-partition, so the stencils cost their FP64 instructions and little
+// else.  Products by 2, 4 and 1/4 are exact and go into the following sum as an
+// FMA (the same rounding, one instruction instead of two), quotients run on
+// the integer pipe (xc_fp64.cuh), signs are tested on the bits.  WENO5 in the
+// reference's form takes 60 FP64 instructions per face instead of 110: 237 us
+// for one 1024^2 field with its fluxes instead of 443; QUICK 7.3 us at 400^2 instead of 21.
+#include "xc_fp64.cuh"
 #include "xc_internal.cuh"
 
 namespace {
 
-constexpr int TZ = 32;        // tile rows (z, contiguous in memory)
-constexpr int TX = 16;        // tile columns (x)
-constexpr int NT = 256;       // threads per CTA
+// Tiles: TZ rows (z, contiguous in memory) x TX columns (x), NT threads.  One
+// thread evaluates one face at a time and the x and z faces of a tile are one
+// index space, so that a small tile's faces (280 of 16 x 8) are one round of
+// its threads: the time of a small grid is that round.  The larger tile
+// evaluates 2.09 faces per cell instead of 2.19 and reads less halo, but its
+// last wave is emptier.  Measured, small against large tile, WENO5: 7.0 / 22.4
+// us at 100^2, 42 / 54 at 400^2, 117 / 120 at 700^2, 171 / 171 at 850^2, 239 /
+// 237 at 1024^2, 513 / 498 at 1500^2; diffusion, which is read and write: 7.6
+// / 8.2 at 400^2, 11.1 / 10.4 at 512^2, 39 / 31 at 1024^2.  The lines lie at
+// nine and at three waves of the larger tile (152 of 512 cells each).
+template <int Z, int X, int T> struct TileShape {
+  static constexpr int TZ = Z, TX = X, NT = T;
+};
+using SmallTile = TileShape<16, 8, 288>;
+using LargeTile = TileShape<32, 16, 256>;
+constexpr long long kSmallAdvect = 9LL * kNumSMs * 512, kSmallDiffus = 3LL * kNumSMs * 512;
 
 // ---------------------------------------------------------------------------
 // face reconstructions (advect.jl:35-53, 216-229, 275-283)
@@ -25,51 +47,50 @@ __device__ __forceinline__ double weno5_poly(double fmm, double fm, double fc, d
                                              double fpp) {
   const double sixth = 1.0 / 6.0, quarter = 0.25, c1312 = 13.0 / 12.0;
   const double eps_val = XC_EPS;
-  double p1 = sixth * ((2.0 * fmm - 7.0 * fm) + 11.0 * fc);
-  double p2 = sixth * ((-fm + 5.0 * fc) + 2.0 * fp);
-  double p3 = sixth * ((2.0 * fc + 5.0 * fp) - fpp);
-  double t = (fmm - 2.0 * fm) + fc, s = (fmm - 4.0 * fm) + 3.0 * fc;
-  double b1 = c1312 * (t * t) + quarter * (s * s);
-  t = (fm - 2.0 * fc) + fp;
+  const double p1 = sixth * (__fma_rn(2.0, fmm, -(7.0 * fm)) + 11.0 * fc);
+  const double p2 = sixth * __fma_rn(2.0, fp, 5.0 * fc - fm);
+  const double p3 = sixth * (__fma_rn(2.0, fc, 5.0 * fp) - fpp);
+  double t = __fma_rn(-2.0, fm, fmm) + fc, s = __fma_rn(-4.0, fm, fmm) + 3.0 * fc;
+  const double b1 = __fma_rn(quarter, s * s, c1312 * (t * t));
+  t = __fma_rn(-2.0, fc, fm) + fp;
   s = fm - fp;
-  double b2 = c1312 * (t * t) + quarter * (s * s);
-  t = (fc - 2.0 * fp) + fpp;
-  s = (3.0 * fc - 4.0 * fp) + fpp;
-  double b3 = c1312 * (t * t) + quarter * (s * s);
-  double e1 = b1 + eps_val, e2 = b2 + eps_val, e3 = b3 + eps_val;
-  double w1 = 0.1 / (e1 * e1);
-  double w2 = 0.6 / (e2 * e2);
-  double w3 = 0.3 / (e3 * e3);
-  return ((w1 * p1 + w2 * p2) + w3 * p3) / ((w1 + w2) + w3);
+  const double b2 = __fma_rn(quarter, s * s, c1312 * (t * t));
+  t = __fma_rn(-2.0, fp, fc) + fpp;
+  s = __fma_rn(-4.0, fp, 3.0 * fc) + fpp;
+  const double b3 = __fma_rn(quarter, s * s, c1312 * (t * t));
+  const double e1 = b1 + eps_val, e2 = b2 + eps_val, e3 = b3 + eps_val;
+  const double w1 = xc_div(0.1, e1 * e1);
+  const double w2 = xc_div(0.6, e2 * e2);
+  const double w3 = xc_div(0.3, e3 * e3);
+  return xc_div((w1 * p1 + w2 * p2) + w3 * p3, (w1 + w2) + w3);
 }
 
 // The same reconstruction with the weights over a common denominator: with
 // q_k = (eps + b_k)^2 the weights d_k / q_k are proportional to
-// n_1 = d_1 q_2 q_3, n_2 = d_2 q_1 q_3, n_3 = d_3 q_1 q_2, so the weighted
-// mean needs one division instead of four (an FP64 division costs about ten
-// times a multiply on this GPU).  Each q_k lies in [eps^2, (eps + b_k)^2]:
-// the products stay normal and finite for fields below about 1e70.  The
-// polynomials and smoothness indicators use fused multiply-adds (about 60
-// FP64 instructions per reconstruction instead of 78; within a few ulps).
+// n_1 = q_2 q_3, n_2 = 6 q_1 q_3, n_3 = 3 q_1 q_2, so the weighted mean needs
+// one division instead of four.  Each q_k lies in [eps^2, (eps + b_k)^2]: the
+// products stay normal and finite for fields below about 1e70.  The
+// smoothness indicators are taken four times as large (a power of two, which
+// leaves the weights as they are) and the common factor 1/6 of the three
+// polynomials is applied once: 46 FP64 instructions per reconstruction
+// (within a few ulps).
 __device__ __forceinline__ double weno5_poly_onediv(double fmm, double fm, double fc, double fp,
                                                     double fpp) {
-  const double sixth = 1.0 / 6.0, quarter = 0.25, c1312 = 13.0 / 12.0;
-  const double eps_val = XC_EPS;
-  const double p1 = sixth * __fma_rn(11.0, fc, __fma_rn(-7.0, fm, 2.0 * fmm));
-  const double p2 = sixth * __fma_rn(2.0, fp, __fma_rn(5.0, fc, -fm));
-  const double p3 = sixth * (__fma_rn(2.0, fc, 5.0 * fp) - fpp);
+  const double c133 = 4.0 * (13.0 / 12.0), eps4 = 4.0 * XC_EPS;
+  const double p1 = __fma_rn(11.0, fc, __fma_rn(-7.0, fm, 2.0 * fmm));
+  const double p2 = __fma_rn(2.0, fp, __fma_rn(5.0, fc, -fm));
+  const double p3 = __fma_rn(2.0, fc, __fma_rn(5.0, fp, -fpp));
   double t = __fma_rn(-2.0, fm, fmm) + fc, s = __fma_rn(3.0, fc, __fma_rn(-4.0, fm, fmm));
-  const double b1 = __fma_rn(c1312 * t, t, quarter * (s * s));
+  const double e1 = __fma_rn(c133 * t, t, s * s) + eps4;
   t = __fma_rn(-2.0, fc, fm) + fp;
   s = fm - fp;
-  const double b2 = __fma_rn(c1312 * t, t, quarter * (s * s));
+  const double e2 = __fma_rn(c133 * t, t, s * s) + eps4;
   t = __fma_rn(-2.0, fp, fc) + fpp;
-  s = __fma_rn(3.0, fc, -4.0 * fp) + fpp;
-  const double b3 = __fma_rn(c1312 * t, t, quarter * (s * s));
-  const double e1 = b1 + eps_val, e2 = b2 + eps_val, e3 = b3 + eps_val;
+  s = __fma_rn(3.0, fc, __fma_rn(-4.0, fp, fpp));
+  const double e3 = __fma_rn(c133 * t, t, s * s) + eps4;
   const double q1 = e1 * e1, q2 = e2 * e2, q3 = e3 * e3;
-  const double n1 = 0.1 * (q2 * q3), n2 = 0.6 * (q1 * q3), n3 = 0.3 * (q1 * q2);
-  return __fma_rn(n1, p1, __fma_rn(n2, p2, n3 * p3)) / ((n1 + n2) + n3);
+  const double n1 = q2 * q3, n2 = 6.0 * (q1 * q3), n3 = 3.0 * (q1 * q2);
+  return (1.0 / 6.0) * xc_div(__fma_rn(n1, p1, __fma_rn(n2, p2, n3 * p3)), (n1 + n2) + n3);
 }
 
 __device__ __forceinline__ double weno3_poly(double fm, double fc, double fp) {
@@ -77,9 +98,9 @@ __device__ __forceinline__ double weno3_poly(double fm, double fc, double fp) {
   double p1 = half * (fc + fp);
   double p2 = half * (3.0 * fc - fm);
   double d1 = fp - fc, d2 = fc - fm;
-  double w1 = (1.0 / 3.0) / (d1 * d1 + eps_val);
-  double w2 = (2.0 / 3.0) / (d2 * d2 + eps_val);
-  return (w1 * p1 + w2 * p2) / (w1 + w2);
+  double w1 = xc_div(1.0 / 3.0, d1 * d1 + eps_val);
+  double w2 = xc_div(2.0 / 3.0, d2 * d2 + eps_val);
+  return xc_div(w1 * p1 + w2 * p2, w1 + w2);
 }
 
 __device__ __forceinline__ double tvd_flux(double fm, double fc, double fp, double vm, double vp) {
@@ -92,6 +113,11 @@ __device__ __forceinline__ double tvd_flux(double fm, double fc, double fp, doub
 
 __device__ __forceinline__ double vpos(double v) { return (v + fabs(v)) * 0.5; }
 __device__ __forceinline__ double vneg(double v) { return (v - fabs(v)) * 0.5; }
+__device__ __forceinline__ bool sign_bit(double v) { return __double2hiint(v) < 0; }
+__device__ __forceinline__ bool zero_bits(double v) {
+  return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0;
+}
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
 // Flux through the face between cells s2 and s3 of the six-cell window
 // s0..s5, with face velocity v (and the neighbouring faces' vl, vr for TVD).
@@ -103,31 +129,40 @@ __device__ __forceinline__ double face_flux(double s0, double s1, double s2, dou
     return v * (s2 + s3) * 0.5;
   } else if (S == XC_UPWD1) {
     return vpos(v) * s2 + vneg(v) * s3;
-  } else if (S == XC_QUICK) {
+  } else if (S == XC_QUICK || S == XC_FROMM) {
+    // vpos(v) pos + vneg(v) neg with only the upwind value formed: the other
+    // term is a zero, which changes no value -- unless its factor is not
+    // finite, so a window with an infinity or NaN takes the whole formula.
     const double sixth = 1.0 / 6.0;
-    double pos = sixth * ((2.0 * s3 + 5.0 * s2) - s1);
-    double neg = sixth * ((2.0 * s2 + 5.0 * s3) - s4);
-    return vpos(v) * pos + vneg(v) * neg;
-  } else if (S == XC_FROMM) {
-    double pos = s2 + 0.25 * (s3 - s1);
-    double neg = s3 + 0.25 * (s2 - s4);
+    if (finite_bits(s1) && finite_bits(s2) && finite_bits(s3) && finite_bits(s4) && finite_bits(v)) {
+      const bool up = !sign_bit(v);
+      const double a1 = up ? s1 : s4, a2 = up ? s2 : s3, a3 = up ? s3 : s2;
+      return v * (S == XC_QUICK ? sixth * (__fma_rn(2.0, a3, 5.0 * a2) - a1) : __fma_rn(0.25, a3 - a1, a2));
+    }
+    double pos, neg;
+    if (S == XC_QUICK) {
+      pos = sixth * ((2.0 * s3 + 5.0 * s2) - s1);
+      neg = sixth * ((2.0 * s2 + 5.0 * s3) - s4);
+    } else {
+      pos = s2 + 0.25 * (s3 - s1);
+      neg = s3 + 0.25 * (s2 - s4);
+    }
     return vpos(v) * pos + vneg(v) * neg;
   } else if (S == XC_WENO3 || S == XC_WENO5 || S == kWeno5OneDiv) {
     // vpos(v) pos + vneg(v) neg has one weight exactly zero: only the upwind
     // reconstruction is evaluated.  The dropped term is (+0) x (finite) = +-0,
     // which changes no value (at most the sign of a zero result); v = +-0
-    // gives 0 and a NaN v stays NaN, as in the full formula.
+    // gives 0 and a NaN v stays NaN, as in the full formula.  The other weight
+    // is v itself.
     // The mirrored stencil is selected first, so a warp with faces of both
     // signs still evaluates one polynomial per face.
-    const bool up = v > 0.0;
+    const bool up = !sign_bit(v);
     const double a0 = up ? s0 : s5, a1 = up ? s1 : s4, a2 = up ? s2 : s3, a3 = up ? s3 : s2,
                  a4 = up ? s4 : s1;
     const double p = S == XC_WENO5        ? weno5_poly(a0, a1, a2, a3, a4)
                      : S == kWeno5OneDiv ? weno5_poly_onediv(a0, a1, a2, a3, a4)
                                          : weno3_poly(a1, a2, a3);
-    if (up) return vpos(v) * p;
-    if (v < 0.0) return vneg(v) * p;
-    return v * 0.0;
+    return zero_bits(v) ? v : v * p;
   } else {  // XC_TVDIM
     double cpos = vpos(v), cneg = vneg(v);
     double pos = tvd_flux(s1, s2, s3, vpos(vl), cpos);
@@ -157,22 +192,60 @@ __device__ __forceinline__ int map_face(int k, int n, int bc) {
 }
 
 // ---------------------------------------------------------------------------
-// advection tile kernel
-// f: interior (Nz, Nx) field read through the BC map, or (HALOD) the caller's
-// halo'd (Nz+2G, Nx+2G) array.  u (Nz, Nx+1) x-face velocities, w (Nz+1, Nx)
-// z-face velocities (for HALOD tvdim: the padded (Nz, Nx+3) / (Nz+3, Nx)).
-// Outputs (any may be null): adv (Nz, Nx), qx_int (Nz, Nx+1), qz_int (Nz+1, Nx).
+// face-flux arrays with the reference's padding: qx is (Nz+2, Nx+1) and its
+// rows 0 and Nz+1 copy the last and first interior row (periodic z) or the
+// neighbouring one (closed); qz is (Nz+1, Nx+2), its columns 0 and Nx+1
+// likewise in x (advect.jl:779-795, diffus.jl:194-208).  `qx`, `qz` view the
+// unpadded faces; the thread that has a face's flux writes its copies too.
 // ---------------------------------------------------------------------------
-template <int S, bool HALOD>
-__global__ void __launch_bounds__(NT) advect_tile_kernel(
-    const double* __restrict__ f, int ldf, int Nz, int Nx, int xBC, int zBC,
-    CView u, CView w, double invh, DView adv, DView qx, DView qz) {
-  XC_PDL_WAIT();
-  constexpr int G = Halo<S>::G;
-  constexpr int HZ = TZ + 2 * G, HX = TX + 2 * G;
-  __shared__ double sf[HX][HZ];
-  __shared__ double sqx[TX + 1][TZ];
-  __shared__ double sqz[TX][TZ + 1];
+__device__ __forceinline__ void put_qx(DView qx, int j, int i, double q, int Nz, int zBC, bool pad) {
+  double* p = qx.p + (size_t)i * (size_t)qx.ld + j;
+  *p = q;
+  if (pad) {
+    const bool per = zBC == XC_PERIODIC && Nz > 1;
+    if (j == (per ? Nz - 1 : 0)) *(p - j - 1) = q;
+    if (j == (per ? 0 : Nz - 1)) *(p - j + Nz) = q;
+  }
+}
+__device__ __forceinline__ void put_qz(DView qz, int j, int i, double q, int Nx, int xBC, bool pad) {
+  double* p = qz.p + (size_t)i * (size_t)qz.ld + j;
+  *p = q;
+  if (pad) {
+    const bool per = xBC == XC_PERIODIC && Nx > 1;
+    if (i == (per ? Nx - 1 : 0)) *(qz.p + j - qz.ld) = q;
+    if (i == (per ? 0 : Nx - 1)) *(qz.p + j + (size_t)Nx * (size_t)qz.ld) = q;
+  }
+}
+
+// One field's advection or diffusion: f the interior (Nz, Nx) field read
+// through the BC map or, halo'd, the caller's (Nz+2G, Nx+2G) array.  u
+// (Nz, Nx+1) x-face velocities, w (Nz+1, Nx) z-face velocities (halo'd tvdim:
+// the padded (Nz, Nx+3) / (Nz+3, Nx)); k1 (times k2 when given) diffusivity.
+// Outputs (any may be null): out (Nz, Nx), qx (Nz, Nx+1), qz (Nz+1, Nx).
+struct FluxArgs {
+  const double* f;
+  int ld;
+  CView u, w;
+  const double *k1, *k2;
+  DView out, qx, qz;
+};
+
+template <class T, int G> struct TileSmem {
+  static constexpr int HZ = T::TZ + 2 * G, HX = T::TX + 2 * G;
+  static constexpr int NXF = T::TZ * (T::TX + 1), NZF = (T::TZ + 1) * T::TX;   // x faces, then z faces
+  double f[HX * HZ];
+  double q[NXF + NZF];
+};
+
+// ---------------------------------------------------------------------------
+// advection of one tile
+// ---------------------------------------------------------------------------
+template <class T, int S, bool HALOD>
+__device__ __forceinline__ void advect_tile(TileSmem<T, Halo<S>::G>& sm, const FluxArgs& a, int Nz, int Nx, int xBC,
+                                            int zBC, double invh, bool pad) {
+  constexpr int G = Halo<S>::G, TZ = T::TZ, TX = T::TX, NT = T::NT;
+  using M = TileSmem<T, G>;
+  constexpr int HZ = M::HZ, HX = M::HX;
   const int j0 = blockIdx.x * TZ, i0 = blockIdx.y * TX;
   const int tid = threadIdx.x;
 
@@ -182,179 +255,158 @@ __global__ void __launch_bounds__(NT) advect_tile_kernel(
     double v = 0.0;
     if (HALOD) {
       int hj = j + G, hi = i + G;
-      if (hj < Nz + 2 * G && hi < Nx + 2 * G) v = f[(size_t)hi * ldf + hj];
+      if (hj < Nz + 2 * G && hi < Nx + 2 * G) v = a.f[(size_t)hi * a.ld + hj];
     } else {
-      v = f[(size_t)map_bc(i, Nx, xBC) * ldf + map_bc(j, Nz, zBC)];
+      v = a.f[(size_t)map_bc(i, Nx, xBC) * a.ld + map_bc(j, Nz, zBC)];
     }
-    sf[ii][jj] = v;
+    sm.f[idx] = v;
   }
   __syncthreads();
 
-  // x-faces: rows j0..j0+TZ-1, faces i0..i0+TX
-  for (int idx = tid; idx < TZ * (TX + 1); idx += NT) {
-    int jj = idx % TZ, ii = idx / TZ;
-    int j = j0 + jj, i = i0 + ii;
+  for (int idx = tid; idx < M::NXF + M::NZF; idx += NT) {
+    const bool xf = idx < M::NXF;
+    const int k = xf ? idx : idx - M::NXF;
+    const int ii = xf ? k / TZ : k / (TZ + 1), jj = k - ii * (xf ? TZ : TZ + 1);
+    const int j = j0 + jj, i = i0 + ii;
     double q = 0.0;
-    if (j < Nz && i <= Nx) {
-      double uv = AT(u, j, HALOD && S == XC_TVDIM ? i + 1 : i);
-      double ul = 0.0, ur = 0.0;
+    // x face i sits between cells i-1 and i, z face j between j-1 and j
+    if (xf ? (j < Nz && i <= Nx) : (j <= Nz && i < Nx)) {
+      double v, vl = 0.0, vr = 0.0;
       if (S == XC_TVDIM) {
-        if (HALOD) {
-          ul = AT(u, j, i);
-          ur = AT(u, j, i + 2);
+        if (xf) {
+          v = AT(a.u, j, HALOD ? i + 1 : i);
+          vl = AT(a.u, j, HALOD ? i : map_face(i - 1, Nx, xBC));
+          vr = AT(a.u, j, HALOD ? i + 2 : map_face(i + 1, Nx, xBC));
         } else {
-          ul = AT(u, j, map_face(i - 1, Nx, xBC));
-          ur = AT(u, j, map_face(i + 1, Nx, xBC));
+          v = AT(a.w, HALOD ? j + 1 : j, i);
+          vl = AT(a.w, HALOD ? j : map_face(j - 1, Nz, zBC), i);
+          vr = AT(a.w, HALOD ? j + 2 : map_face(j + 1, Nz, zBC), i);
         }
+      } else {
+        v = xf ? AT(a.u, j, i) : AT(a.w, j, i);
       }
-      // face i sits between cells i-1 and i -> tile columns ii+G-1 and ii+G
-      const int c = ii + G, r = jj + G;
-      double s0 = (G >= 3) ? sf[c - 3][r] : 0.0;
-      double s1 = (G >= 2) ? sf[c - 2][r] : 0.0;
-      double s4 = (G >= 2) ? sf[c + 1][r] : 0.0;
-      double s5 = (G >= 3) ? sf[c + 2][r] : 0.0;
-      q = face_flux<S>(s0, s1, sf[c - 1][r], sf[c][r], s4, s5, uv, ul, ur);
-      if (qx.p && (ii < TX || i == Nx)) AT(qx, j, i) = q;
-    }
-    sqx[ii][jj] = q;
-  }
-  // z-faces: faces j0..j0+TZ, columns i0..i0+TX-1
-  for (int idx = tid; idx < (TZ + 1) * TX; idx += NT) {
-    int jj = idx % (TZ + 1), ii = idx / (TZ + 1);
-    int j = j0 + jj, i = i0 + ii;
-    double q = 0.0;
-    if (j <= Nz && i < Nx) {
-      double wv = AT(w, HALOD && S == XC_TVDIM ? j + 1 : j, i);
-      double wt = 0.0, wb = 0.0;
-      if (S == XC_TVDIM) {
-        if (HALOD) {
-          wt = AT(w, j, i);
-          wb = AT(w, j + 2, i);
-        } else {
-          wt = AT(w, map_face(j - 1, Nz, zBC), i);
-          wb = AT(w, map_face(j + 1, Nz, zBC), i);
-        }
+      const int st = xf ? HZ : 1;
+      const double* c = sm.f + (ii + G) * HZ + jj + G;
+      const double s0 = (G >= 3) ? c[-3 * st] : 0.0;
+      const double s1 = (G >= 2) ? c[-2 * st] : 0.0;
+      const double s4 = (G >= 2) ? c[st] : 0.0;
+      const double s5 = (G >= 3) ? c[2 * st] : 0.0;
+      q = face_flux<S>(s0, s1, c[-st], c[0], s4, s5, v, vl, vr);
+      // the last tile of each axis also writes the closing face
+      if (xf) {
+        if (a.qx.p && (ii < TX || i == Nx)) put_qx(a.qx, j, i, q, Nz, zBC, pad);
+      } else {
+        if (a.qz.p && (jj < TZ || j == Nz)) put_qz(a.qz, j, i, q, Nx, xBC, pad);
       }
-      const int c = ii + G, r = jj + G;
-      double s0 = (G >= 3) ? sf[c][r - 3] : 0.0;
-      double s1 = (G >= 2) ? sf[c][r - 2] : 0.0;
-      double s4 = (G >= 2) ? sf[c][r + 1] : 0.0;
-      double s5 = (G >= 3) ? sf[c][r + 2] : 0.0;
-      q = face_flux<S>(s0, s1, sf[c][r - 1], sf[c][r], s4, s5, wv, wt, wb);
-      if (qz.p && (jj < TZ || j == Nz)) AT(qz, j, i) = q;
     }
-    sqz[ii][jj] = q;
+    sm.q[idx] = q;
   }
-  if (!adv.p) return;
+  if (!a.out.p) return;
   __syncthreads();
+  const double* qz = sm.q + M::NXF;
   for (int idx = tid; idx < TZ * TX; idx += NT) {
     int jj = idx % TZ, ii = idx / TZ;
     int j = j0 + jj, i = i0 + ii;
     if (j < Nz && i < Nx)
-      AT(adv, j, i) = (((sqx[ii + 1][jj] - sqx[ii][jj]) + sqz[ii][jj + 1]) - sqz[ii][jj]) * invh;
+      AT(a.out, j, i) = (((sm.q[idx + TZ] - sm.q[idx]) + qz[ii * (TZ + 1) + jj + 1]) - qz[ii * (TZ + 1) + jj]) * invh;
   }
 }
 
-// ---------------------------------------------------------------------------
-// diffusion tile kernel (diffus.jl:9-31, 68-91); k = k1 (* k2 when given)
-// ---------------------------------------------------------------------------
-template <bool HALOD>
-__global__ void __launch_bounds__(NT) diffus_tile_kernel(
-    const double* __restrict__ f, const double* __restrict__ k1, const double* __restrict__ k2,
-    int ld, int Nz, int Nx, int xBC, int zBC, double invh, DView dff, DView qx, DView qz) {
+template <class T, int S, bool HALOD>
+__global__ void __launch_bounds__(T::NT) advect_tile_kernel(FluxArgs a, int Nz, int Nx, int xBC, int zBC, double invh,
+                                                            bool pad) {
   XC_PDL_WAIT();
-  constexpr int G = 1;
-  constexpr int HZ = TZ + 2 * G, HX = TX + 2 * G;
-  __shared__ double sf[HX][HZ];
-  __shared__ double sk[HX][HZ];
+  __shared__ TileSmem<T, Halo<S>::G> sm;
+  advect_tile<T, S, HALOD>(sm, a, Nz, Nx, xBC, zBC, invh, pad);
+}
+
+// ---------------------------------------------------------------------------
+// diffusion of one tile (diffus.jl:9-31, 68-91).  A face's product
+// (k_L + k_R)(f_R - f_L) is formed once: the divergence takes it from both
+// sides, and the face flux -(k_L + k_R)/2 (f_R - f_L)/h is the same product
+// halved and negated, which is exact (subnormal products aside, far below any
+// flux).  12 FP64 instructions per cell instead of 28.
+// ---------------------------------------------------------------------------
+template <class T, bool HALOD>
+__device__ __forceinline__ void diffus_tile(TileSmem<T, 1>& sm, double* sk, const FluxArgs& a, int Nz, int Nx, int xBC,
+                                            int zBC, double invh, bool pad) {
+  constexpr int TZ = T::TZ, TX = T::TX, NT = T::NT;
+  using M = TileSmem<T, 1>;
+  constexpr int HZ = M::HZ, HX = M::HX;
   const int j0 = blockIdx.x * TZ, i0 = blockIdx.y * TX;
   const int tid = threadIdx.x;
   for (int idx = tid; idx < HZ * HX; idx += NT) {
     int jj = idx % HZ, ii = idx / HZ;
-    int j = j0 - G + jj, i = i0 - G + ii;
+    int j = j0 - 1 + jj, i = i0 - 1 + ii;
     double fv = 0.0, kv = 0.0;
-    if (HALOD) {
-      int hj = j + G, hi = i + G;
-      if (hj < Nz + 2 && hi < Nx + 2) {
-        size_t o = (size_t)hi * ld + hj;
-        fv = f[o];
-        kv = k1[o];
-        if (k2) kv = kv * k2[o];
-      }
-    } else {
-      size_t o = (size_t)map_bc(i, Nx, xBC) * ld + map_bc(j, Nz, zBC);
-      fv = f[o];
-      kv = k1[o];
-      if (k2) kv = kv * k2[o];
+    size_t o = (size_t)(i + 1) * a.ld + (j + 1);
+    bool in = i <= Nx && j <= Nz;
+    if (!HALOD) {
+      o = (size_t)map_bc(i, Nx, xBC) * a.ld + map_bc(j, Nz, zBC);
+      in = true;
     }
-    sf[ii][jj] = fv;
-    sk[ii][jj] = kv;
+    if (in) {
+      fv = a.f[o];
+      kv = a.k1[o];
+      if (a.k2) kv = kv * a.k2[o];
+    }
+    sm.f[idx] = fv;
+    sk[idx] = kv;
   }
   __syncthreads();
-  const double half = 0.5;
-  const double invh2 = invh * invh;
-  if (dff.p) {
-    for (int idx = tid; idx < TZ * TX; idx += NT) {
-      int jj = idx % TZ, ii = idx / TZ;
-      int j = j0 + jj, i = i0 + ii;
-      if (j < Nz && i < Nx) {
-        int c = ii + 1, r = jj + 1;
-        double fc = sf[c][r], kc = sk[c][r];
-        double fxr = (sk[c + 1][r] + kc) * (sf[c + 1][r] - fc);
-        double fxl = (kc + sk[c - 1][r]) * (fc - sf[c - 1][r]);
-        double fzb = (sk[c][r + 1] + kc) * (sf[c][r + 1] - fc);
-        double fzt = (kc + sk[c][r - 1]) * (fc - sf[c][r - 1]);
-        AT(dff, j, i) = (half * invh2) * (((fxr - fxl) + fzb) - fzt);
-      }
+  const double mhalf_invh = -0.5 * invh;
+  for (int idx = tid; idx < M::NXF + M::NZF; idx += NT) {
+    const bool xf = idx < M::NXF;
+    const int k = xf ? idx : idx - M::NXF;
+    const int ii = xf ? k / TZ : k / (TZ + 1), jj = k - ii * (xf ? TZ : TZ + 1);
+    const int j = j0 + jj, i = i0 + ii;
+    const int c = (ii + 1) * HZ + jj + 1, b = c - (xf ? HZ : 1);
+    const double q = (sk[c] + sk[b]) * (sm.f[c] - sm.f[b]);
+    sm.q[idx] = q;
+    if (xf) {
+      if (a.qx.p && j < Nz && i <= Nx && (ii < TX || i == Nx))
+        put_qx(a.qx, j, i, q * mhalf_invh, Nz, zBC, pad);
+    } else {
+      if (a.qz.p && j <= Nz && i < Nx && (jj < TZ || j == Nz))
+        put_qz(a.qz, j, i, q * mhalf_invh, Nx, xBC, pad);
     }
   }
-  if (qx.p) {
-    for (int idx = tid; idx < TZ * (TX + 1); idx += NT) {
-      int jj = idx % TZ, ii = idx / TZ;
-      int j = j0 + jj, i = i0 + ii;
-      if (j < Nz && i <= Nx && (ii < TX || i == Nx)) {
-        int c = ii + 1, r = jj + 1;
-        double fL = sf[c - 1][r], fR = sf[c][r], kL = sk[c - 1][r], kR = sk[c][r];
-        AT(qx, j, i) = (((-(kL + kR)) * half) * (fR - fL)) * invh;
-      }
-    }
-  }
-  if (qz.p) {
-    for (int idx = tid; idx < (TZ + 1) * TX; idx += NT) {
-      int jj = idx % (TZ + 1), ii = idx / (TZ + 1);
-      int j = j0 + jj, i = i0 + ii;
-      if (j <= Nz && i < Nx && (jj < TZ || j == Nz)) {
-        int c = ii + 1, r = jj + 1;
-        double fT = sf[c][r - 1], fB = sf[c][r], kT = sk[c][r - 1], kB = sk[c][r];
-        AT(qz, j, i) = (((-(kT + kB)) * half) * (fB - fT)) * invh;
-      }
-    }
+  if (!a.out.p) return;
+  __syncthreads();
+  const double* qz = sm.q + M::NXF;
+  const double hih2 = 0.5 * (invh * invh);
+  for (int idx = tid; idx < TZ * TX; idx += NT) {
+    int jj = idx % TZ, ii = idx / TZ;
+    int j = j0 + jj, i = i0 + ii;
+    if (j < Nz && i < Nx)
+      AT(a.out, j, i) =
+          hih2 * (((sm.q[idx + TZ] - sm.q[idx]) + qz[ii * (TZ + 1) + jj + 1]) - qz[ii * (TZ + 1) + jj]);
   }
 }
 
-// MATLAB-sized boundary rows/cols of the face-flux arrays (advect.jl:779-795,
-// diffus.jl:194-208): qz cols 0 / Nx+1 and qx rows 0 / Nz+1.
-__global__ void pad_fluxes_kernel(DView qx, DView qz, int Nz, int Nx, int xBC, int zBC) {
+template <class T, bool HALOD>
+__global__ void __launch_bounds__(T::NT) diffus_tile_kernel(FluxArgs a, int Nz, int Nx, int xBC, int zBC, double invh,
+                                                            bool pad) {
   XC_PDL_WAIT();
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < Nz + 1) {   // qz (Nz+1, Nx+2)
-    if (xBC == XC_PERIODIC && Nx > 1) {
-      AT(qz, t, 0) = AT(qz, t, Nx);
-      AT(qz, t, Nx + 1) = AT(qz, t, 1);
-    } else {
-      AT(qz, t, 0) = AT(qz, t, 1);
-      AT(qz, t, Nx + 1) = AT(qz, t, Nx);
-    }
-  }
-  if (t < Nx + 1) {   // qx (Nz+2, Nx+1)
-    if (zBC == XC_PERIODIC && Nz > 1) {
-      AT(qx, 0, t) = AT(qx, Nz, t);
-      AT(qx, Nz + 1, t) = AT(qx, 1, t);
-    } else {
-      AT(qx, 0, t) = AT(qx, 1, t);
-      AT(qx, Nz + 1, t) = AT(qx, Nz, t);
-    }
-  }
+  __shared__ TileSmem<T, 1> sm;
+  __shared__ double sk[TileSmem<T, 1>::HX * TileSmem<T, 1>::HZ];
+  diffus_tile<T, HALOD>(sm, sk, a, Nz, Nx, xBC, zBC, invh, pad);
+}
+
+// the three stencils of phsevo! side by side in one launch (blockIdx.z: the
+// advection of X, of M, the diffusion of chi): they are independent, and a
+// small grid's tiles of all three fill the GPU better than one after another
+struct PhsevoFluxes { FluxArgs a[3]; };
+template <class T, int S>
+__global__ void __launch_bounds__(T::NT) phsevo_flux_kernel(PhsevoFluxes p, int Nz, int Nx, int xBC, int zBC,
+                                                            double invh) {
+  XC_PDL_WAIT();
+  constexpr int G = Halo<S>::G;
+  struct Diff { TileSmem<T, 1> t; double sk[TileSmem<T, 1>::HX * TileSmem<T, 1>::HZ]; };
+  union Smem { TileSmem<T, G> adv; Diff dif; };
+  __shared__ Smem sm;
+  if (blockIdx.z < 2) advect_tile<T, S, false>(sm.adv, p.a[blockIdx.z], Nz, Nx, xBC, zBC, invh, true);
+  else diffus_tile<T, false>(sm.dif.t, sm.dif.sk, p.a[2], Nz, Nx, xBC, zBC, invh, true);
 }
 
 // ghost ring of a halo'd array (ghosts.jl:18-51; for N >= halo the x-then-z
@@ -390,7 +442,7 @@ __global__ void phsevo_tail_kernel(int Nz, int Nx, double a1, double a2, double 
     double Xc = AT(X, j, i);
     double res = ((a1 * Xc - a2 * AT(Xo, j, i)) - a3 * AT(Xoo, j, i)) -
                  (((b1 * dxdt + b2 * AT(dXdto, j, i)) + b3 * AT(dXdtoo, j, i)) * dt);
-    double upd = ((-alpha) * res) / a1;
+    double upd = xc_div((-alpha) * res, a1);
     double Xn = Xc + upd;
     double r = AT(rho, j, i);
     double lo = r * XC_EPS, hi = r * (1.0 - XC_EPS);
@@ -398,22 +450,55 @@ __global__ void phsevo_tail_kernel(int Nz, int Nx, double a1, double a2, double 
     AT(X, j, i) = Xn;
     double Mn = r - Xn;
     AT(M, j, i) = Mn;
-    AT(x, j, i) = Xn / r;
-    AT(m, j, i) = Mn / r;
+    AT(x, j, i) = xc_div(Xn, r);
+    AT(m, j, i) = xc_div(Mn, r);
   });
 }
 
+template <class T>
+dim3 tile_grid(int Nz, int Nx, int nz = 1) {
+  return dim3((Nz + T::TZ - 1) / T::TZ, (Nx + T::TX - 1) / T::TX, nz);
+}
+
+template <class T, int S>
+void launch_advect_tile(const FluxArgs& a, bool halod, int Nz, int Nx, int xBC, int zBC, double invh, bool pad,
+                        cudaStream_t s) {
+  if (halod)
+    xc_launch(advect_tile_kernel<T, S, true>, tile_grid<T>(Nz, Nx), T::NT, 0, s, a, Nz, Nx, xBC, zBC, invh, pad);
+  else
+    xc_launch(advect_tile_kernel<T, S, false>, tile_grid<T>(Nz, Nx), T::NT, 0, s, a, Nz, Nx, xBC, zBC, invh, pad);
+}
+
 template <int S>
-int launch_advect(const double* f, int ldf, bool halod, int Nz, int Nx, int xBC, int zBC, CView u,
-                  CView w, double invh, DView adv, DView qx, DView qz, cudaStream_t s) {
-  // the last tile of each axis also writes the closing face (index Nz / Nx)
-  dim3 grid((Nz + TZ - 1) / TZ, (Nx + TX - 1) / TX);
-  if (halod) {
-    xc_launch(advect_tile_kernel<S, true>, grid, NT, 0, s, f, ldf, Nz, Nx, xBC, zBC, u, w, invh, adv, qx, qz);
-  } else {
-    xc_launch(advect_tile_kernel<S, false>, grid, NT, 0, s, f, ldf, Nz, Nx, xBC, zBC, u, w, invh, adv, qx, qz);
-  }
+int launch_advect(const FluxArgs& a, bool halod, int Nz, int Nx, int xBC, int zBC, double invh, bool pad,
+                  cudaStream_t s) {
+  if ((long long)Nz * Nx <= kSmallAdvect)
+    launch_advect_tile<SmallTile, S>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+  else
+    launch_advect_tile<LargeTile, S>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
   XC_LAUNCH_CHECK();
+  return XC_OK;
+}
+
+template <int S>
+int launch_phsevo_fluxes(const PhsevoFluxes& p, int Nz, int Nx, int xBC, int zBC, double invh, cudaStream_t s) {
+  if ((long long)Nz * Nx <= kSmallAdvect)
+    xc_launch(phsevo_flux_kernel<SmallTile, S>, tile_grid<SmallTile>(Nz, Nx, 3), SmallTile::NT, 0, s, p, Nz, Nx, xBC,
+              zBC, invh);
+  else
+    xc_launch(phsevo_flux_kernel<LargeTile, S>, tile_grid<LargeTile>(Nz, Nx, 3), LargeTile::NT, 0, s, p, Nz, Nx, xBC,
+              zBC, invh);
+  XC_LAUNCH_CHECK();
+  return XC_OK;
+}
+
+int check_advect(int scheme, int Nz, int Nx) {
+  int g = scheme_halo(scheme);
+  if (g < 0) { xc_set_error("advect: unsupported scheme %d", scheme); return XC_BAD_ARG; }
+  if (Nz < g || Nx < g) {
+    xc_set_error("advect: grid %dx%d smaller than the scheme halo %d", Nz, Nx, g);
+    return XC_BAD_ARG;
+  }
   return XC_OK;
 }
 
@@ -430,50 +515,33 @@ int scheme_halo(int scheme) {
 
 int stencil_advect_flux(const double* f, int ldf, bool halod, int Nz, int Nx, int scheme, int xBC,
                         int zBC, CView u, CView w, double h, DView adv, DView qx_int,
-                        DView qz_int, cudaStream_t s) {
-  int g = scheme_halo(scheme);
-  if (g < 0) { xc_set_error("advect: unsupported scheme %d", scheme); return XC_BAD_ARG; }
-  if (Nz < g || Nx < g) {
-    xc_set_error("advect: grid %dx%d smaller than the scheme halo %d", Nz, Nx, g);
-    return XC_BAD_ARG;
-  }
+                        DView qz_int, cudaStream_t s, bool pad) {
+  XC_TRY(check_advect(scheme, Nz, Nx));
   double invh = 1.0 / h;
+  const FluxArgs a{f, ldf, u, w, nullptr, nullptr, adv, qx_int, qz_int};
   switch (scheme) {
-    case XC_CENTR: return launch_advect<XC_CENTR>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
-    case XC_UPWD1: return launch_advect<XC_UPWD1>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
-    case XC_QUICK: return launch_advect<XC_QUICK>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
-    case XC_FROMM: return launch_advect<XC_FROMM>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
-    case XC_WENO3: return launch_advect<XC_WENO3>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
-    case XC_WENO5: return launch_advect<XC_WENO5>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
-    case kWeno5OneDiv:
-      return launch_advect<kWeno5OneDiv>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
-    default: return launch_advect<XC_TVDIM>(f, ldf, halod, Nz, Nx, xBC, zBC, u, w, invh, adv, qx_int, qz_int, s);
+    case XC_CENTR: return launch_advect<XC_CENTR>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+    case XC_UPWD1: return launch_advect<XC_UPWD1>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+    case XC_QUICK: return launch_advect<XC_QUICK>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+    case XC_FROMM: return launch_advect<XC_FROMM>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+    case XC_WENO3: return launch_advect<XC_WENO3>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+    case XC_WENO5: return launch_advect<XC_WENO5>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+    case kWeno5OneDiv: return launch_advect<kWeno5OneDiv>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
+    default: return launch_advect<XC_TVDIM>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
   }
 }
 
-static int diffus_launch(const double* f, const double* k1, const double* k2, int ld, bool halod,
-                         int Nz, int Nx, int xBC, int zBC, double h, DView dff, DView qx, DView qz,
-                         cudaStream_t s) {
-  dim3 grid((Nz + TZ - 1) / TZ, (Nx + TX - 1) / TX);
-  double invh = 1.0 / h;
-  if (halod) {
-    xc_launch(diffus_tile_kernel<true>, grid, NT, 0, s, f, k1, k2, ld, Nz, Nx, xBC, zBC, invh, dff, qx, qz);
-  } else {
-    xc_launch(diffus_tile_kernel<false>, grid, NT, 0, s, f, k1, k2, ld, Nz, Nx, xBC, zBC, invh, dff, qx, qz);
-  }
-  XC_LAUNCH_CHECK();
-  return XC_OK;
-}
-
-int stencil_diffus_flux(const double* f, const double* k, int ld, bool halod, int Nz, int Nx,
-                        int xBC, int zBC, double h, DView dff, DView qx_int, DView qz_int,
-                        cudaStream_t s) {
-  return diffus_launch(f, k, nullptr, ld, halod, Nz, Nx, xBC, zBC, h, dff, qx_int, qz_int, s);
-}
-
-int pad_face_fluxes(DView qx, DView qz, int Nz, int Nx, int xBC, int zBC, cudaStream_t s) {
-  int n = (Nz > Nx ? Nz : Nx) + 1;
-  xc_launch(pad_fluxes_kernel, (n + 255) / 256, 256, 0, s, qx, qz, Nz, Nx, xBC, zBC);
+// diffusion of a halo'd field
+static int diffus_launch(const double* f, const double* k, int ld, int Nz, int Nx, int xBC, int zBC, double h,
+                         DView dff, DView qx, DView qz, bool pad, cudaStream_t s) {
+  const FluxArgs a{f, ld, CView{nullptr, 0}, CView{nullptr, 0}, k, nullptr, dff, qx, qz};
+  const double invh = 1.0 / h;
+  if ((long long)Nz * Nx <= kSmallDiffus)
+    xc_launch(diffus_tile_kernel<SmallTile, true>, tile_grid<SmallTile>(Nz, Nx), SmallTile::NT, 0, s, a, Nz, Nx, xBC,
+              zBC, invh, pad);
+  else
+    xc_launch(diffus_tile_kernel<LargeTile, true>, tile_grid<LargeTile>(Nz, Nx), LargeTile::NT, 0, s, a, Nz, Nx, xBC,
+              zBC, invh, pad);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
@@ -491,16 +559,26 @@ int phsevo_impl(xc_ctx* c, int scheme, const double coefs[6], double dt, double 
   auto qz_int = [&](int id) { DView q = F(c, id); return DView{q.p + q.ld, q.ld}; };
   DView X = F(c, FLD_X), M = F(c, FLD_M);
   scheme = advect_scheme(scheme, c->p);
-  XC_TRY(stencil_advect_flux(X.p, X.ld, false, Nz, Nx, scheme, xBC, zBC, Ux_face, Wx_face, h,
-                             F(c, FLD_advn_X), qx_int(FLD_qx_advn_X), qz_int(FLD_qz_advn_X), s));
-  XC_TRY(stencil_advect_flux(M.p, M.ld, false, Nz, Nx, scheme, xBC, zBC, Um_face, Wm_face, h,
-                             F(c, FLD_advn_M), qx_int(FLD_qx_advn_M), qz_int(FLD_qz_advn_M), s));
-  // diffusion of chi with k = X .* kx (phsevo.jl:192-194)
-  XC_TRY(diffus_launch(F(c, FLD_chi).p, X.p, F(c, FLD_kx).p, Nz, false, Nz, Nx, xBC, zBC, h,
-                       F(c, FLD_dffn_X), qx_int(FLD_qx_dffn_X), qz_int(FLD_qz_dffn_X), s));
-  XC_TRY(pad_face_fluxes(F(c, FLD_qx_advn_X), F(c, FLD_qz_advn_X), Nz, Nx, xBC, zBC, s));
-  XC_TRY(pad_face_fluxes(F(c, FLD_qx_advn_M), F(c, FLD_qz_advn_M), Nz, Nx, xBC, zBC, s));
-  XC_TRY(pad_face_fluxes(F(c, FLD_qx_dffn_X), F(c, FLD_qz_dffn_X), Nz, Nx, xBC, zBC, s));
+  XC_TRY(check_advect(scheme, Nz, Nx));
+  const CView none{nullptr, 0};
+  PhsevoFluxes pf{{{X.p, X.ld, Ux_face, Wx_face, nullptr, nullptr, F(c, FLD_advn_X), qx_int(FLD_qx_advn_X),
+                    qz_int(FLD_qz_advn_X)},
+                   {M.p, M.ld, Um_face, Wm_face, nullptr, nullptr, F(c, FLD_advn_M), qx_int(FLD_qx_advn_M),
+                    qz_int(FLD_qz_advn_M)},
+                   // diffusion of chi with k = X .* kx (phsevo.jl:192-194)
+                   {F(c, FLD_chi).p, Nz, none, none, X.p, F(c, FLD_kx).p, F(c, FLD_dffn_X), qx_int(FLD_qx_dffn_X),
+                    qz_int(FLD_qz_dffn_X)}}};
+  const double invh = 1.0 / h;
+  switch (scheme) {
+    case XC_CENTR: XC_TRY(launch_phsevo_fluxes<XC_CENTR>(pf, Nz, Nx, xBC, zBC, invh, s)); break;
+    case XC_UPWD1: XC_TRY(launch_phsevo_fluxes<XC_UPWD1>(pf, Nz, Nx, xBC, zBC, invh, s)); break;
+    case XC_QUICK: XC_TRY(launch_phsevo_fluxes<XC_QUICK>(pf, Nz, Nx, xBC, zBC, invh, s)); break;
+    case XC_FROMM: XC_TRY(launch_phsevo_fluxes<XC_FROMM>(pf, Nz, Nx, xBC, zBC, invh, s)); break;
+    case XC_WENO3: XC_TRY(launch_phsevo_fluxes<XC_WENO3>(pf, Nz, Nx, xBC, zBC, invh, s)); break;
+    case XC_WENO5: XC_TRY(launch_phsevo_fluxes<XC_WENO5>(pf, Nz, Nx, xBC, zBC, invh, s)); break;
+    case kWeno5OneDiv: XC_TRY(launch_phsevo_fluxes<kWeno5OneDiv>(pf, Nz, Nx, xBC, zBC, invh, s)); break;
+    default: XC_TRY(launch_phsevo_fluxes<XC_TVDIM>(pf, Nz, Nx, xBC, zBC, invh, s));
+  }
   dim3 blk(32, 8);
   xc_launch(phsevo_tail_kernel, dim3(persistent_grid((const void*)phsevo_tail_kernel, Nz, Nx)), blk, 0, s, Nz, Nx,
       coefs[0], coefs[1], coefs[2], coefs[3],
@@ -552,10 +630,8 @@ extern "C" int xc_advect_with_flux(double* adv, double* qx, double* qz, const do
   }
   cudaStream_t s = (cudaStream_t)stream;
   CView uv{u, Nz}, wv{w, scheme == XC_TVDIM ? Nz + 3 : Nz + 1};
-  DView qxv{qx, Nz + 2}, qzv{qz, Nz + 1};
-  XC_TRY(stencil_advect_flux(f_halo, Nz + 2 * g, true, Nz, Nx, scheme, xBC, zBC, uv, wv, h,
-                             DView{adv, Nz}, DView{qx + 1, Nz + 2}, DView{qz + (Nz + 1), Nz + 1}, s));
-  return pad_face_fluxes(qxv, qzv, Nz, Nx, xBC, zBC, s);
+  return stencil_advect_flux(f_halo, Nz + 2 * g, true, Nz, Nx, scheme, xBC, zBC, uv, wv, h, DView{adv, Nz},
+                             DView{qx + 1, Nz + 2}, DView{qz + (Nz + 1), Nz + 1}, s, true);
 }
 
 extern "C" int xc_advect_centered_with_flux(double* adv, double* qx, double* qz, const double* f,
@@ -570,10 +646,7 @@ extern "C" int xc_advect_centered_with_flux(double* adv, double* qx, double* qz,
   cudaStream_t s = (cudaStream_t)stream;
   CView uv{u, Nz}, wv{w, Nz + 1};
   DView qxi{qx ? qx + 1 : nullptr, Nz + 2}, qzi{qz ? qz + (Nz + 1) : nullptr, Nz + 1};
-  XC_TRY(stencil_advect_flux(f, Nz, false, Nz, Nx, scheme, xBC, zBC, uv, wv, h, DView{adv, Nz},
-                             qxi, qzi, s));
-  if (qx) return pad_face_fluxes(DView{qx, Nz + 2}, DView{qz, Nz + 1}, Nz, Nx, xBC, zBC, s);
-  return XC_OK;
+  return stencil_advect_flux(f, Nz, false, Nz, Nx, scheme, xBC, zBC, uv, wv, h, DView{adv, Nz}, qxi, qzi, s, true);
 }
 
 extern "C" int xc_diffus(double* dff, const double* f_halo, const double* k_halo, int Nz, int Nx,
@@ -582,8 +655,8 @@ extern "C" int xc_diffus(double* dff, const double* f_halo, const double* k_halo
     xc_set_error("xc_diffus: bad arguments");
     return XC_BAD_ARG;
   }
-  return diffus_launch(f_halo, k_halo, nullptr, Nz + 2, true, Nz, Nx, XC_PERIODIC, XC_CLOSED, h,
-                       DView{dff, Nz}, DView{nullptr, 0}, DView{nullptr, 0}, (cudaStream_t)stream);
+  return diffus_launch(f_halo, k_halo, Nz + 2, Nz, Nx, XC_PERIODIC, XC_CLOSED, h, DView{dff, Nz}, DView{nullptr, 0},
+                       DView{nullptr, 0}, false, (cudaStream_t)stream);
 }
 
 extern "C" int xc_diffus_with_flux(double* dff, double* qx, double* qz, const double* f_halo,
@@ -593,8 +666,6 @@ extern "C" int xc_diffus_with_flux(double* dff, double* qx, double* qz, const do
     xc_set_error("xc_diffus_with_flux: bad arguments");
     return XC_BAD_ARG;
   }
-  cudaStream_t s = (cudaStream_t)stream;
-  XC_TRY(diffus_launch(f_halo, k_halo, nullptr, Nz + 2, true, Nz, Nx, xBC, zBC, h, DView{dff, Nz},
-                       DView{qx + 1, Nz + 2}, DView{qz + (Nz + 1), Nz + 1}, s));
-  return pad_face_fluxes(DView{qx, Nz + 2}, DView{qz, Nz + 1}, Nz, Nx, xBC, zBC, s);
+  return diffus_launch(f_halo, k_halo, Nz + 2, Nz, Nx, xBC, zBC, h, DView{dff, Nz}, DView{qx + 1, Nz + 2},
+                       DView{qz + (Nz + 1), Nz + 1}, true, (cudaStream_t)stream);
 }
