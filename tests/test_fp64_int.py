@@ -1,7 +1,9 @@
-"""The integer-pipe FP64 quotient and square root (csrc/xc_fp64.cuh), compiled
-for the host, against the processor's own: the same bits for every pair of
-operands, with the seeds moved by the error the device's approximations may
-have (and the wider one of their emulation here)."""
+"""The integer-pipe FP64 functions (csrc/xc_fp64.cuh), compiled for the host.
+
+The quotient, the square root, the scalings and the comparisons against the
+processor's own: the same bits for every operand, with the seeds moved by the
+error the device's approximations may have (and the wider one of their
+emulation here).  The exponential and the logarithm against long double."""
 import os
 import shutil
 import subprocess
@@ -53,13 +55,49 @@ int main() {
       check(x, 0.1 + (double)(i % 97));
     }
   }
+  auto same = [&](double a, double b) { if (xc_bits(a) != xc_bits(b) && !(a != a && b != b)) ++bad; };
+  for (long i = 0; i < 1000000; ++i) {
+    double x = xc_from_bits(g());
+    if (i % 2) x = xc_from_bits((g() % (6ull << 52)) | (g() & (1ull << 63)));      // subnormals and their neighbours
+    if (i < 13) x = special[i];
+    same(xc_half(x), x * 0.5); same(xc_scale2<-2>(x), x * 0.25); same(xc_scale2<1>(x), x * 2.0);
+    const double lo = 1e-16, hi = 1.0 - 1e-16;
+    same(xc_clamp_pos(x, lo, hi), x > hi ? hi : (x < lo ? lo : x));
+    same(xc_max_pos(x, lo), x != x ? x : (x > lo ? x : lo));
+    same(xc_max0(x), x != x ? x : (x > 0 ? x : 0.0));
+    if (xc_ge_pos(x, 1e-8) != (x >= 1e-8) || xc_isnan(x) != (x != x)) ++bad;
+  }
+  // exp: half an ulp plus the fixed point's error, which grows with |x| as the
+  // 64-bit log2(e) does (2^-64 of x log2(e), 2^-53 being half an ulp at worst)
+  std::uniform_real_distribution<double> U(-1.0, 1.0);
+  const double scale[] = {1e-9, 5e-5, 7e-5, 0.02, 1.0, 64.0, 707.0};
+  for (long i = 0; i < 3000000; ++i) {
+    const double sc = scale[i % 7], x = U(g) * sc, e = xc_exp(x);
+    const long double t = expl((long double)x);
+    int k;
+    std::frexp((double)t, &k);
+    const double err = (double)(fabsl((long double)e - t) / ldexpl(1.0L, k - 53));
+    if (!(err <= 0.504 + std::fabs(x) * 1.45 * 0.0005)) { if (bad++ < 9) std::printf("exp %a: %g ulp\n", x, err); }
+  }
+  for (double x : {0.0, -0.0, 5e-324, -1e-300, 1e-17, -5e-17, 709.0, 710.0, -746.0, 1.0 / 0.0, -1.0 / 0.0, 0.0 / 0.0})
+    same(xc_exp(x), std::exp(x));
+  // log2 to 2^-54 of one, the powers built on it to 2e-15 (c times twice that, half an ulp)
+  for (long i = 0; i < 3000000; ++i) {
+    double x = std::exp(U(g) * 36.5);
+    if (i & 1) x = 1.0 - std::fabs(U(g)) * 1e-9;
+    if (!xc_log2_ok(x) || fabsl((long double)xc_log2_fixed(x) - log2l((long double)x) * 0x1p57L) > 8) ++bad;
+    const double c = i % 3 ? 1 / 2.09 : 1 / 0.37, B = 0.63;
+    const long double t = powl((long double)x / B, (long double)c);
+    const double r = xc_exp2_product((uint64_t)(c * 0x1p58), xc_log2_fixed(x) - xc_log2_fixed(B));
+    if (!(fabsl(r - t) <= 2e-15L * t)) ++bad;
+  }
   std::printf("bad %ld\n", bad);
   return bad != 0;
 }
 """
 
 
-def test_quotient_and_root_have_the_processors_bits(tmp_path):
+def test_integer_functions_against_the_processor(tmp_path):
     gxx = shutil.which("g++")
     if gxx is None:
         pytest.skip("g++ not available")

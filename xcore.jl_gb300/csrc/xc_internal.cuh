@@ -13,6 +13,7 @@
 #include <string>
 
 #include "xcore_gb300.h"
+#include "xc_fp64.cuh"
 
 // ---------------------------------------------------------------------------
 // field registry: name, shape code, element size.  Shape codes follow the
@@ -234,22 +235,14 @@ unsigned persistent_grid(const void* kernel, int rows, int cols);
 // min(0.0, -0.0) is -0.0 whatever the argument order (a plain a > b ? a : b
 // returns the second argument for two zeros).  Either result is independent
 // of the order in which a reduction combines its values.
-__host__ __device__ __forceinline__ bool jsignbit(double a) {
-#ifdef __CUDA_ARCH__
-  return __double_as_longlong(a) < 0;
-#else
-  return std::signbit(a);
-#endif
-}
+// Compared as integers: an FP64 comparison takes an FP64 slot.
 __host__ __device__ __forceinline__ double jmax(double a, double b) {
-  if (a > b) return a;
-  if (b > a) return b;
-  return (a != a || b != b) ? a + b : (jsignbit(a) ? b : a);
+  if (xc_isnan(a)) return a;
+  return xc_isnan(b) || xc_order(b) > xc_order(a) ? b : a;
 }
 __host__ __device__ __forceinline__ double jmin(double a, double b) {
-  if (a < b) return a;
-  if (b < a) return b;
-  return (a != a || b != b) ? a + b : (jsignbit(a) ? a : b);
+  if (xc_isnan(a)) return a;
+  return xc_isnan(b) || xc_order(b) < xc_order(a) ? b : a;
 }
 
 // deterministic reductions (xc_reduce.cu): CTA partials, combined in a fixed

