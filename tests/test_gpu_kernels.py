@@ -225,6 +225,24 @@ def test_noise_filter_sizes(shape):
     assert_fields(ds, st, ["xiew", "xieu", "xixw", "xixu", "xisw", "xisu", "xie", "xix", "xis"], tol=1e-12)
 
 
+# direct filter passes: sigma 2 h (24 neighbours: 49 and 50 columns are the
+# first that fit, 48 take the FFT), 2.6 h (31 neighbours), 3 h (FFT); grids at
+# the edges of the 64 x 4, 32 x 8 and staggered 32 x 8 tiles, rows 31 and 63
+# being those whose last ghost row begins a tile
+@pytest.mark.parametrize("cells, shape", [(3, (64, 49)), (3, (31, 50)), (3, (63, 48)), (3, (65, 64)), (4.2, (64, 63)),
+                                          (4.2, (33, 65)), (5, (40, 72)), (1, (31, 33))])
+def test_noise_direct_and_fft_filter(cells, shape):
+    N, Nx = shape
+    h = 10.0 / N
+    par, g, sc, ns, st, dt, rng = realistic_state(N=N, Nx=Nx, steps=0, L0=cells * h, l0=cells * h)
+    ds = device_state(par, g, sc, st)
+    re, rs = rng.standard_normal((g.Nz, g.Nx)), rng.standard_normal((g.Nz, g.Nx))
+    O.noise(st, g, par, sc, ns, dt, True, re, rs)
+    ds.noise(dt, True, re, rs)
+    assert_fields(ds, st, ["psie", "psix", "psis", "xiew", "xieu", "xixw", "xixu", "xisw", "xisu", "xie", "xix", "xis"],
+                  tol=1e-12)
+
+
 def test_dt_resnorm_sums():
     par, g, sc, ns, st, dt, rng = realistic_state()
     ds = device_state(par, g, sc, st)

@@ -17,6 +17,17 @@
 // Two real lines are packed into one complex FFT (real kernel => the real and
 // imaginary parts stay separate).  Mathematically this is the reference
 // operator; the FFTs are hand-written radix-2 shared-memory transforms.
+//
+// Where the filter is well resolved its kernel is short: for s >= 2 h the
+// spectrum falls below 2^-56 before the Nyquist wavenumber, so c[d] is the
+// Gaussian exp(-(d h / 2 s)^2) itself (to that accuracy), and beyond R = 24
+// (s = 2 h, the correlation length of three cells of every configuration) all
+// its values together are below 2^-54 of its sum.  Both passes are then direct
+// sums of 2 R + 1 terms: 49 FP64 instructions per cell and pass on a
+// processor bound by its FP64 unit, against 60 (x, power of two) and 90 (z) of
+// the FFTs, and up to three times that where the padding to a power of two
+// doubles a line (a pass of 1024^2 in 94 us instead of 228 and 124, one of
+// 300 x 231 in 7 instead of 105).  Longer kernels (R > 32) and unresolved ones take the FFT.
 #include <cmath>
 #include <complex>
 #include <mutex>
@@ -70,10 +81,19 @@ struct LineFilter {      // one 1-D convolution pass
   double2* tw;           // device, M/2 twiddles exp(-2 pi i k / M)
 };
 
+constexpr int kMaxRadius = 32;
+struct DirectFilter {    // one 1-D convolution pass as a direct sum
+  int R;                 // largest lag (0: none, the FFT serves this pass)
+  int period;            // lags wrap around at this length; cells beyond the line's end are zero
+  double tap[kMaxRadius + 1];
+};
+
 struct NoisePlan {
   int padL0, padl0;
   double fL, fl;
   LineFilter ze, xe, zs, xs;   // e: sigma = L0h, pad = padL0; s: sigma = l0h, pad = padl0
+  DirectFilter dz[2], dx[2];   // e, s
+  bool direct;                 // all four passes are short: no FFT plans are built
 };
 
 namespace {
@@ -119,6 +139,24 @@ int build_line_filter(LineFilter& lf, int L, int period, double h, double sigma,
   XC_CUDA_TRY(cudaMemcpy(lf.khat, khat.data(), sizeof(double) * lf.M, cudaMemcpyHostToDevice));
   XC_CUDA_TRY(cudaMemcpy(lf.tw, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice));
   return XC_OK;
+}
+
+// the direct form of a pass over lines of period n, or R = 0
+void build_direct(DirectFilter& f, int n, double h, double sigma) {
+  f.R = 0;
+  f.period = n;
+  const double s = sigma / h;
+  if (!(s >= 1.99 && s <= 4.0)) return;
+  auto gauss = [&](int d) { return std::exp(-(double)d * d / (4.0 * s * s)) / (2.0 * s * std::sqrt(M_PI)); };
+  int R = 1;
+  for (; R <= kMaxRadius; ++R) {
+    double tail = 0.0;
+    for (int d = R + 1; d < R + 64; ++d) tail += 2.0 * gauss(d);
+    if (tail <= 0x1p-54) break;
+  }
+  if (R > kMaxRadius || 2 * R + 1 > n) return;
+  f.R = R;
+  for (int d = 0; d <= R; ++d) f.tap[d] = gauss(d);
 }
 
 void free_line_filter(LineFilter& lf) {
@@ -244,6 +282,46 @@ int run_line_filter(const LineFilter& lf, CView in, DView out, int rows, int col
   return XC_OK;
 }
 
+// Direct passes over the three noise fields side by side (blockIdx.z), an
+// output per thread: a tile of 64 x 4 cells along z or 32 x 8 across x, with
+// its 2 R neighbours on the line in shared memory.  The FP64 unit bounds it
+// (2 R + 1 instructions of 64 cycles a warp and sub-partition); the tile's
+// repeated reads come from L2.
+struct DirectPass {
+  CView in[3];
+  DView out[3];
+  DirectFilter f[2];       // of fields 0, 1 and of field 2
+};
+template <int AXIS>
+__global__ void __launch_bounds__(256) direct_filter_kernel(const __grid_constant__ DirectPass p, int Nz, int Nx) {
+  XC_PDL_WAIT();
+  constexpr int BZ = AXIS == 0 ? 64 : 32, BX = AXIS == 0 ? 4 : 8;
+  constexpr int LZ = AXIS == 0 ? BZ + 2 * kMaxRadius : BZ, LX = AXIS == 0 ? BX : BX + 2 * kMaxRadius;
+  __shared__ double x[LX][LZ];
+  const DirectFilter& f = p.f[blockIdx.z == 2 ? 1 : 0];
+  const CView in = p.in[blockIdx.z];
+  const int R = f.R, n = f.period;
+  const int j0 = blockIdx.x * BZ, i0 = blockIdx.y * BX;
+  const int nz = AXIS == 0 ? BZ + 2 * R : BZ, nx = AXIS == 0 ? BX : BX + 2 * R;
+  for (int k = threadIdx.x; k < nz * nx; k += 256) {
+    const int ii = k / nz, jj = k - ii * nz;
+    int j = j0 + jj - (AXIS == 0 ? R : 0), i = i0 + ii - (AXIS == 1 ? R : 0);
+    int& q = AXIS == 0 ? j : i;
+    if (q < 0) q += n;
+    else if (q >= n) q -= n;               // beyond n + R only in front of cells outside the grid
+    x[ii][jj] = j < Nz && i < Nx ? AT(in, j, i) : 0.0;
+  }
+  __syncthreads();
+  const int jj = threadIdx.x % BZ, ii = threadIdx.x / BZ, j = j0 + jj, i = i0 + ii;
+  if (j >= Nz || i >= Nx) return;
+  const double* c = AXIS == 0 ? &x[ii][jj + R] : &x[ii + R][jj];
+  constexpr int st = AXIS == 0 ? 1 : LZ;
+  double acc = 0.0;                        // from the smallest terms inwards
+#pragma unroll 4
+  for (int d = R; d > 0; --d) acc = __fma_rn(f.tap[d], c[-d * st] + c[d * st], acc);
+  AT(p.out[blockIdx.z], j, i) = __fma_rn(f.tap[0], c[0], acc);
+}
+
 // OU update (noise.jl:160-183), one thread per cell
 __global__ void ou_kernel(int Nz, int Nx, double Xi, double L0h, double i2L0h, double i2l0h, double txi0,
                           double dt, double cdt, double fL, double fl, CView V, CView vx, CView fReL, CView ke, CView chi,
@@ -256,101 +334,140 @@ __global__ void ou_kernel(int Nz, int Nx, double Xi, double L0h, double i2L0h, d
     // the same values up to rounding (these fields carry the 1e-12 tolerance):
     // 1/tau_e = 2 (V + eps) / L0h and 1/tau_s = 2 (vx + eps) / l0h as
     // products, and tau' = 1 / (1/tau + c) + dt with c = 1 / (100 dt) entering
-    // only as -dt / tau' = -dt u / (1 + dt u), u = 1/tau + c.  An FP64 division
-    // costs about ten FP64 instructions on this GPU's narrow FP64 pipe.
+    // only as -dt / tau' = -dt u / (1 + dt u), u = 1/tau + c.  Those five, the
+    // roots and the exponentials run on the integer pipe: 45 FP64 instructions
+    // per cell are left of 183 (bound by the FP64 unit, 375 -> 105 us at 1024^2).
     const double ve = AT(V, j, i) + XC_EPS, vs = AT(vx, j, i) + XC_EPS;
-    const double taue = L0h / (2.0 * ve);
+    const double taue = xc_div(L0h, xc_scale2<1>(ve));
     const double itaue = ve * i2L0h, itaus = vs * i2l0h;   // i2L0h = 2 / L0h, i2l0h = 2 / l0h
-    double St = txi0 / (taue + XC_EPS);
+    double St = xc_div(txi0, taue + XC_EPS);
     double fr = AT(fReL, j, i), k = AT(ke, j, i), ch = AT(chi, j, i);
-    double sge = Xi * sqrt(jmax(0.0, (fr * k) * itaue));
-    double sgx = Xi * sqrt(jmax(0.0, ((((ch * fr) * k) * itaue) * St) / (1.0 + St * St)));
-    double sgs = Xi * sqrt(jmax(0.0, (ch * AT(ks, j, i)) * itaus));
-    const double ue = itaue + cdt, us = itaus + cdt;   // cdt = 1 / (100 dt)
-    double Fte = exp(((-dt) * ue) / (1.0 + dt * ue)), Fts = exp(((-dt) * us) / (1.0 + dt * us));
-    double ae = sqrt(jmax(0.0, 1.0 - Fte * Fte)), as = sqrt(jmax(0.0, 1.0 - Fts * Fts));
-    double r1 = AT(re, j, i), r2 = AT(rs, j, i);
-    AT(psie, j, i) = Fte * AT(psieo, j, i) + ((ae * sge) * fL) * r1;
-    AT(psix, j, i) = Fte * AT(psixo, j, i) + ((ae * sgx) * fL) * r1;
-    AT(psis, j, i) = Fts * AT(psiso, j, i) + ((as * sgs) * fl) * r2;
+    double sge = Xi * xc_sqrt(xc_max0((fr * k) * itaue));
+    double sgx = Xi * xc_sqrt(xc_max0(xc_div((((ch * fr) * k) * itaue) * St, 1.0 + St * St)));
+    double sgs = Xi * xc_sqrt(xc_max0((ch * AT(ks, j, i)) * itaus));
+    const double due = dt * (itaue + cdt), dus = dt * (itaus + cdt);   // cdt = 1 / (100 dt)
+    double Fte = xc_exp(xc_div(-due, 1.0 + due)), Fts = xc_exp(xc_div(-dus, 1.0 + dus));
+    double ae = xc_sqrt(xc_max0(1.0 - Fte * Fte)), as = xc_sqrt(xc_max0(1.0 - Fts * Fts));
+    const double re1 = (ae * fL) * AT(re, j, i), rs1 = (as * fl) * AT(rs, j, i);
+    AT(psie, j, i) = Fte * AT(psieo, j, i) + sge * re1;
+    AT(psix, j, i) = Fte * AT(psixo, j, i) + sgx * re1;
+    AT(psis, j, i) = Fts * AT(psiso, j, i) + sgs * rs1;
   });
 }
 
-// re-standardise to the raw mean/std (noise.jl:261-267); st = {raw mean,
-// raw sum sq dev, flt mean, flt sum sq dev} per field
-// (the two standard deviations, the same for every cell, are formed once per
-// block by the same operations)
-// (the ratio raw std / filtered std, the same for every cell, is formed once
-// per block: the per-cell FP64 division of (v - mean) raw / flt becomes a
-// product, within the 1e-12 tolerance of these fields)
-__global__ void rescale_kernel(int Nz, int Nx, DView f0, DView f1, DView f2, const double* st) {
-  XC_PDL_WAIT();
-  __shared__ double ratio[3];
-  __shared__ int use[3];
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const double nm1 = (double)Nz * (double)Nx - 1.0;
-    for (int q = 0; q < 3; ++q) {
-      const double raw_std = sqrt(st[4 * q + 1] / nm1), flt_std = sqrt(st[4 * q + 3] / nm1);
-      use[q] = flt_std > XC_EPS;
-      ratio[q] = raw_std / flt_std;
-    }
-  }
-  __syncthreads();
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (j >= Nz || i >= Nx) return;
-  DView fs[3] = {f0, f1, f2};
-  for (int q = 0; q < 3; ++q) {
-    const double* s = st + 4 * q;
-    if (use[q]) {
-      double v = AT(fs[q], j, i);
-      AT(fs[q], j, i) = ((v - s[2]) * ratio[q]) + s[0];
-    }
-  }
+// The filtered fields are re-standardised to the raw mean and std
+// (noise.jl:261-267; st = {raw mean, raw sum sq dev, filtered mean, filtered
+// sum sq dev} per field) where the staggered differences below read them:
+// the ratio raw std / filtered std, the same for every cell, is formed once
+// per block, and (v - mean) raw / flt becomes a product, within the 1e-12
+// tolerance of these fields.
+struct Standard {
+  double mean[3], ratio[3], raw[3];
+  int use[3];
+};
+__device__ __forceinline__ double standardised(const Standard& n, int q, double v) {
+  return n.use[q] ? (v - n.mean[q]) * n.ratio[q] + n.raw[q] : v;
 }
 
+// grid.icz / grid.icx extension (closed z, periodic x: noise.jl:143-144)
 __device__ __forceinline__ int icz_c(int j, int Nz) { return j == 0 ? 0 : (j == Nz + 1 ? Nz - 1 : j - 1); }
 __device__ __forceinline__ int icx_p(int i, int Nx) { return i == 0 ? Nx - 1 : (i == Nx + 1 ? 0 : i - 1); }
 
-// grid.icz / grid.icx extension (closed z, periodic x: noise.jl:143-144)
-__device__ __forceinline__ double ext(CView f, int a, int b, int Nz, int Nx) {
-  return AT(f, icz_c(a, Nz), icx_p(b, Nx));
-}
-__device__ __forceinline__ double corner_avg(CView pe, int j, int i, int Nz, int Nx) {
-  return (((ext(pe, j, i, Nz, Nx) + ext(pe, j, i + 1, Nz, Nx)) + ext(pe, j + 1, i, Nz, Nx)) +
-          ext(pe, j + 1, i + 1, Nz, Nx)) / 4.0;
-}
-
-// staggered noise fluxes (noise.jl:195-220), one thread per (j, i) of (Nz+2, Nx+2)
 // exp(y) where only 1 - exp(y) is used: below y = -38, exp(y) < 3.2e-17 is
 // under half an ulp of 1 (2^-54), so 1 - exp(y) rounds to exactly 1.0 and
-// the exponential -- some twenty FP64 instructions -- is skipped without
-// changing a bit (the crystal-fraction taper, a / 1e-4 with a >= 0.004)
-__device__ __forceinline__ double exp_tail(double y) { return y < -38.0 ? 0.0 : exp(y); }
+// the exponential is skipped without changing a bit (the crystal-fraction
+// taper, a / 1e-4 with a >= 0.004)
+__device__ __forceinline__ double exp_tail(double y) { return y < -38.0 ? 0.0 : xc_exp(y); }
+__device__ __forceinline__ double taper(double a, double b) {
+  return (1.0 - exp_tail(xc_div(-a, 1e-4))) * (1.0 - exp_tail(xc_div(-xc_max0(b - 0.4), 0.05)));
+}
 
-__global__ void stagger_kernel(int Nz, int Nx, CView pe, CView px, CView ps, CView chiw,
-                               CView muw, CView chiu, CView muu, DView xieu, DView xiew,
-                               DView xixu, DView xixw, DView xisu, DView xisw) {
+// staggered noise fluxes (noise.jl:195-220), one thread per (j, i) of
+// (Nz+2, Nx+2), in tiles of 32 x 8.  The standardised fields of the extended
+// grid (cells j, j+1 by i, i+1; corners need one more on the low side for the
+// ghost rows and columns, which repeat and wrap) are formed once per tile in
+// shared memory, and so is each corner's average.  22 FP64 instructions per
+// cell instead of 106, and no pass of its own for the re-standardisation:
+// 214 + 74 -> 100 us at 1024^2.
+constexpr int SZ = 32, SX = 8;
+__global__ void __launch_bounds__(256) stagger_kernel(int Nz, int Nx, CView pe, CView px, CView ps, const double* st,
+                                                      CView chiw, CView muw, CView chiu, CView muu, DView xieu,
+                                                      DView xiew, DView xixu, DView xixw, DView xisu, DView xisw) {
   XC_PDL_WAIT();
-  for_tiles(Nz + 2, Nx + 2, [&](int j, int i) {
-    if (j > Nz + 1 || i > Nx + 1) return;
-    if (i <= Nx) {   // (Nz+2, Nx+1): xieu = xieu_int[icz, :], xixu, xisu
-      int jj = icz_c(j, Nz);
-      AT(xieu, j, i) = corner_avg(pe, jj + 1, i, Nz, Nx) - corner_avg(pe, jj, i, Nz, Nx);
-      double a = AT(chiu, j, i), b = AT(muu, j, i);
-      double tap = (1.0 - exp_tail((-a) / 1e-4)) * (1.0 - exp_tail((-jmax(0.0, b - 0.4)) / 0.05));
-      AT(xixu, j, i) = (-(ext(px, j, i + 1, Nz, Nx) - ext(px, j, i, Nz, Nx))) * tap;
-      AT(xisu, j, i) = (-(ext(ps, j, i + 1, Nz, Nx) - ext(ps, j, i, Nz, Nx))) * tap;
+  __shared__ Standard norm;
+  // e: psi_e on the extended rows j0-2 .. j0+32 and columns i0-1 .. i0+8; c: the
+  // averages of the corners there; sx, ss: psi_x, psi_s from row j0, column i0
+  __shared__ double e[SX + 2][SZ + 3], c[SX + 1][SZ + 2], sx[SX + 1][SZ + 1], ss[SX + 1][SZ + 1];
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  if (tid < 3) {
+    const double nm1 = (double)Nz * (double)Nx - 1.0;
+    const double* s = st + 4 * tid;
+    const double raw_std = sqrt(s[1] / nm1), flt_std = sqrt(s[3] / nm1);
+    norm.use[tid] = !(flt_std <= XC_EPS);   // a NaN anywhere makes the whole field NaN, as the 2-D FFT does
+    norm.ratio[tid] = raw_std / flt_std;
+    norm.mean[tid] = s[2];
+    norm.raw[tid] = s[0];
+  }
+  __syncthreads();
+  const int nbx = (Nz + 2 + SZ - 1) / SZ, nt = nbx * ((Nx + 2 + SX - 1) / SX);
+  for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+    const int j0 = (t % nbx) * SZ, i0 = (t / nbx) * SX;
+    // the extended index a stands for cell icz(a) / icx(a); the corner (b, d)
+    // averages the cells b, b+1 by d, d+1.  Ghost row j of xieu takes the
+    // corners of cell row icz(j): Nz-1 for row Nz+1, two before it, which may
+    // be the tile's first.
+    for (int k = tid; k < (SX + 2) * (SZ + 3); k += 256) {
+      const int ii = k / (SZ + 3), jj = k - ii * (SZ + 3);
+      const int a = j0 - 2 + jj, b = i0 - 1 + ii;
+      if (a >= 0 && a <= Nz + 1 && b >= 0 && b <= Nx + 1) {
+        const int cj = icz_c(a, Nz), ci = icx_p(b, Nx);
+        e[ii][jj] = standardised(norm, 0, AT(pe, cj, ci));
+        if (ii >= 1 && jj >= 2) {
+          sx[ii - 1][jj - 2] = standardised(norm, 1, AT(px, cj, ci));
+          ss[ii - 1][jj - 2] = standardised(norm, 2, AT(ps, cj, ci));
+        }
+      }
     }
-    if (j <= Nz) {   // (Nz+1, Nx+2): xiew = xiew_int[:, icx], xixw, xisw
-      int ii = icx_p(i, Nx);
-      AT(xiew, j, i) = -(corner_avg(pe, j, ii + 1, Nz, Nx) - corner_avg(pe, j, ii, Nz, Nx));
-      double a = AT(chiw, j, i), b = AT(muw, j, i);
-      double tap = (1.0 - exp_tail((-a) / 1e-4)) * (1.0 - exp_tail((-jmax(0.0, b - 0.4)) / 0.05));
-      AT(xixw, j, i) = (-(ext(px, j + 1, i, Nz, Nx) - ext(px, j, i, Nz, Nx))) * tap;
-      AT(xisw, j, i) = (-(ext(ps, j + 1, i, Nz, Nx) - ext(ps, j, i, Nz, Nx))) * tap;
+    __syncthreads();
+    for (int k = tid; k < (SX + 1) * (SZ + 2); k += 256) {
+      const int ii = k / (SZ + 2), jj = k - ii * (SZ + 2);
+      const int a = j0 - 2 + jj, b = i0 - 1 + ii;
+      if (a >= 0 && a <= Nz && b >= 0 && b <= Nx)
+        c[ii][jj] = xc_scale2<-2>(((e[ii][jj] + e[ii + 1][jj]) + e[ii][jj + 1]) + e[ii + 1][jj + 1]);
     }
-  });
+    __syncthreads();
+    const int jj = threadIdx.x, ii = threadIdx.y, j = j0 + jj, i = i0 + ii;
+    if (j <= Nz + 1 && i <= Nx + 1) {
+      if (i <= Nx) {   // (Nz+2, Nx+1): xieu = xieu_int[icz, :], xixu, xisu
+        const int r = icz_c(j, Nz) - j0 + 2;       // corner rows r, r + 1 of the tile
+        AT(xieu, j, i) = c[ii + 1][r + 1] - c[ii + 1][r];
+        const double tap = taper(AT(chiu, j, i), AT(muu, j, i));
+        AT(xixu, j, i) = (-(sx[ii + 1][jj] - sx[ii][jj])) * tap;
+        AT(xisu, j, i) = (-(ss[ii + 1][jj] - ss[ii][jj])) * tap;
+      }
+      if (j <= Nz) {   // (Nz+1, Nx+2): xiew = xiew_int[:, icx], xixw, xisw
+        const int d = icx_p(i, Nx) - i0 + 1;
+        double hi, lo;
+        if (d >= 0 && d < SX) {
+          hi = c[d + 1][jj + 2];
+          lo = c[d][jj + 2];
+        } else {       // the wrapped ghost columns: another tile's corners
+          const int ix = icx_p(i, Nx);
+          auto corner = [&](int b) {
+            auto ex = [&](int a, int q) { return standardised(norm, 0, AT(pe, icz_c(a, Nz), icx_p(q, Nx))); };
+            return xc_scale2<-2>(((ex(j, b) + ex(j, b + 1)) + ex(j + 1, b)) + ex(j + 1, b + 1));
+          };
+          hi = corner(ix + 1);
+          lo = corner(ix);
+        }
+        AT(xiew, j, i) = -(hi - lo);
+        const double tap = taper(AT(chiw, j, i), AT(muw, j, i));
+        AT(xixw, j, i) = (-(sx[ii][jj + 1] - sx[ii][jj])) * tap;
+        AT(xisw, j, i) = (-(ss[ii][jj + 1] - ss[ii][jj])) * tap;
+      }
+    }
+    __syncthreads();
+  }
 }
 
 // speed magnitudes (noise.jl:223-236)
@@ -359,15 +476,15 @@ __global__ void speeds_kernel(int Nz, int Nx, CView xisw, CView xisu, CView xixw
   XC_PDL_WAIT();
   for_tiles(Nz, Nx, [&](int j, int i) {
     if (j >= Nz || i >= Nx) return;
-    double wz = (AT(xisw, j, i + 1) + AT(xisw, j + 1, i + 1)) / 2.0;
-    double wx = (AT(xisu, j + 1, i) + AT(xisu, j + 1, i + 1)) / 2.0;
-    AT(xis, j, i) = sqrt(wz * wz + wx * wx);
-    wz = (AT(xixw, j, i + 1) + AT(xixw, j + 1, i + 1)) / 2.0;
-    wx = (AT(xixu, j + 1, i) + AT(xixu, j + 1, i + 1)) / 2.0;
-    AT(xix, j, i) = sqrt(wz * wz + wx * wx);
-    wz = (AT(xiew, j, i + 1) + AT(xiew, j + 1, i + 1)) / 2.0;
-    wx = (AT(xieu, j + 1, i) + AT(xieu, j + 1, i + 1)) / 2.0;
-    AT(xie, j, i) = sqrt(wz * wz + wx * wx);
+    double wz = xc_half(AT(xisw, j, i + 1) + AT(xisw, j + 1, i + 1));
+    double wx = xc_half(AT(xisu, j + 1, i) + AT(xisu, j + 1, i + 1));
+    AT(xis, j, i) = xc_sqrt(wz * wz + wx * wx);
+    wz = xc_half(AT(xixw, j, i + 1) + AT(xixw, j + 1, i + 1));
+    wx = xc_half(AT(xixu, j + 1, i) + AT(xixu, j + 1, i + 1));
+    AT(xix, j, i) = xc_sqrt(wz * wz + wx * wx);
+    wz = xc_half(AT(xiew, j, i + 1) + AT(xiew, j + 1, i + 1));
+    wx = xc_half(AT(xieu, j + 1, i) + AT(xieu, j + 1, i + 1));
+    AT(xie, j, i) = xc_sqrt(wz * wz + wx * wx);
   });
 }
 
@@ -382,6 +499,12 @@ int noise_plan_create(xc_ctx* c) {
   np->fL = 2.0 / std::sqrt(1.0 - std::exp(-(h * h) / (2.0 * (L0h * L0h))));
   np->fl = 2.0 / std::sqrt(1.0 - std::exp(-(h * h) / (2.0 * (l0h * l0h))));
   const int Nz = c->Nz, Nx = c->Nx;
+  build_direct(np->dz[0], Nz + np->padL0, h, L0h);
+  build_direct(np->dx[0], Nx, h, L0h);
+  build_direct(np->dz[1], Nz + np->padl0, h, l0h);
+  build_direct(np->dx[1], Nx, h, l0h);
+  np->direct = np->dz[0].R && np->dx[0].R && np->dz[1].R && np->dx[1].R;
+  if (np->direct) return XC_OK;
   XC_TRY(build_line_filter(np->ze, Nz, Nz + np->padL0, h, L0h, false));
   XC_TRY(build_line_filter(np->xe, Nx, Nx, h, L0h, true));
   XC_TRY(build_line_filter(np->zs, Nz, Nz + np->padl0, h, l0h, false));
@@ -427,9 +550,28 @@ int noise_impl(xc_ctx* c, double dt, int first_iter, const double* re, const dou
   const LineFilter* xf[3] = {&np->xe, &np->xe, &np->xs};
   double* st = c->dscal + SC_NOISE_STATS;
   const double n = (double)Nz * (double)Nx;
-  for (int q = 0; q < 3; ++q) {
-    XC_TRY(run_line_filter(*zf[q], CF(c, src[q]), mid, Nz, Nx, 0, s));
-    XC_TRY(run_line_filter(*xf[q], CView{mid.p, Nz}, flt[q], Nz, Nx, 1, s));
+  if (np->direct) {
+    // the z passes go to the speed fields, which the last kernel overwrites
+    DirectPass pz, px;
+    const int mids[3] = {FLD_xie, FLD_xix, FLD_xis};
+    for (int q = 0; q < 3; ++q) {
+      pz.in[q] = CF(c, src[q]);
+      pz.out[q] = F(c, mids[q]);
+      px.in[q] = CF(c, mids[q]);
+      px.out[q] = flt[q];
+    }
+    for (int q = 0; q < 2; ++q) {
+      pz.f[q] = np->dz[q];
+      px.f[q] = np->dx[q];
+    }
+    xc_launch(direct_filter_kernel<0>, dim3((Nz + 63) / 64, (Nx + 3) / 4, 3), 256, 0, s, pz, Nz, Nx);
+    xc_launch(direct_filter_kernel<1>, dim3((Nz + 31) / 32, (Nx + 7) / 8, 3), 256, 0, s, px, Nz, Nx);
+    XC_LAUNCH_CHECK();
+  } else {
+    for (int q = 0; q < 3; ++q) {
+      XC_TRY(run_line_filter(*zf[q], CF(c, src[q]), mid, Nz, Nx, 0, s));
+      XC_TRY(run_line_filter(*xf[q], CView{mid.p, Nz}, flt[q], Nz, Nx, 1, s));
+    }
   }
   // the six means in one launch, then the six centred sums of squares
   // (mean and corrected std of noise.jl:261-264)
@@ -443,11 +585,9 @@ int noise_impl(xc_ctx* c, double dt, int first_iter, const double* re, const dou
   }
   XC_TRY(reduce_batch(c, means, 6, s, partials));
   XC_TRY(reduce_batch(c, devs, 6, s, partials));
-  xc_launch(rescale_kernel, grid2d(Nz, Nx, blk), blk, 0, s, Nz, Nx, flt[0], flt[1], flt[2], st);
-  XC_LAUNCH_CHECK();
   xc_launch(stagger_kernel, dim3(persistent_grid((const void*)stagger_kernel, Nz + 2, Nx + 2)), blk, 0, s, Nz, Nx,
       CView{flt[0].p, Nz},
-      CView{flt[1].p, Nz}, CView{flt[2].p, Nz}, CF(c, FLD_chiw),
+      CView{flt[1].p, Nz}, CView{flt[2].p, Nz}, st, CF(c, FLD_chiw),
       CF(c, FLD_muw), CF(c, FLD_chiu), CF(c, FLD_muu), F(c, FLD_xieu), F(c, FLD_xiew),
       F(c, FLD_xixu), F(c, FLD_xixw), F(c, FLD_xisu), F(c, FLD_xisw));
   XC_LAUNCH_CHECK();
@@ -469,7 +609,18 @@ int noise_bench_zpass(xc_ctx* c, int iters, double out[4]) {
   int st = XC_OK;
   for (int it = -1; it < iters && st == XC_OK; ++it) {
     if (it == 0) cudaEventRecord(e0, c->stream);
-    st = run_line_filter(np->ze, CF(c, FLD_psie), DView{c->tmp[5], Nz}, Nz, Nx, 0, c->stream);
+    if (np->direct) {
+      DirectPass p;
+      for (int q = 0; q < 3; ++q) {
+        p.in[q] = CF(c, FLD_psie);
+        p.out[q] = DView{c->tmp[5], Nz};
+      }
+      p.f[0] = p.f[1] = np->dz[0];
+      xc_launch(direct_filter_kernel<0>, dim3((Nz + 63) / 64, (Nx + 3) / 4, 1), 256, 0, c->stream, p, Nz, Nx);
+      XC_LAUNCH_CHECK();
+    } else {
+      st = run_line_filter(np->ze, CF(c, FLD_psie), DView{c->tmp[5], Nz}, Nz, Nx, 0, c->stream);
+    }
   }
   cudaEventRecord(e1, c->stream);
   cudaEventSynchronize(e1);
@@ -481,7 +632,8 @@ int noise_bench_zpass(xc_ctx* c, int iters, double out[4]) {
   const double M = np->ze.M, logM = np->ze.logM;
   out[0] = ms / iters;
   out[1] = 16.0 * Nz * (double)Nx;                   // read psi, write the filtered field
-  out[2] = (double)((Nx + 1) / 2) * 2.0 * 5.0 * M * logM;   // forward + inverse complex FFT per line pair
+  // 2 R + 1 multiply-adds per cell, or forward + inverse complex FFT per line pair
+  out[2] = np->direct ? 2.0 * (2 * np->dz[0].R + 1) * Nz * (double)Nx : (double)((Nx + 1) / 2) * 2.0 * 5.0 * M * logM;
   out[3] = (double)Nz * Nx;
   return XC_OK;
 }
