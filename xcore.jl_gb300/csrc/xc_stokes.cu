@@ -1127,6 +1127,244 @@ __device__ void dense_apply_cta(const T* __restrict__ inv, int n, const T* b, T*
   __syncthreads();
 }
 
+// ---- direct solve of a larger coarsest level (wide inverse) -----------------
+// Grid sides with an odd factor leave a coarsest level of up to some thousand
+// unknowns (25 x 25 cells of a 100^2 or 400^2 grid: 1404).  Hundreds of Jacobi
+// sweeps by one CTA took 2.7 ms (FP64) or 0.5 ms (FP32) of every V-cycle
+// there.  Instead the level's matrix, its rows scaled by their diagonal, is
+// inverted in FP32 once per solve by blocked Gauss-Jordan elimination over the
+// whole GPU (32 columns a launch, partial pivoting inside the diagonal
+// block), and a coarse solve is a matrix-vector product.  The FP64 hierarchy
+// adds one step of refinement with the level's FP64 rows, which leaves an
+// error of the order of 1e-8 where the sweeps left some per cent.  One known
+// vector is solved back after the inversion: if it is off by more than 1e-2
+// (a matrix too ill conditioned for FP32, or a pivot of a block that vanishes),
+// *ok stays 0 and the sweeps serve the level as before.
+constexpr int kWideMax = 2048;       // most unknowns (16 MiB of inverse)
+constexpr int kWideCta = 320;        // most unknowns of a product inside a one-CTA V-cycle
+struct WideInverse {
+  const float* inv;                  // np x np, row-major
+  int np;                            // unknowns rounded up to 32
+};
+
+// M = diag^-1 A; row r of column c is the level's row r applied to the unit
+// vector e_c, which starts at `unit` + n - c (2 n elements, a one at n)
+template <typename T>
+__global__ void wide_form_vel_kernel(Geo g, OpConst k, VOp<T> op, const T* unit, int n, int np, float* M, float* dinv,
+                                     int* bad) {
+  XC_PDL_WAIT();
+  const int r = blockIdx.x * 32 + threadIdx.x, c = blockIdx.y * 8 + threadIdx.y;
+  if (r >= np || c >= np) return;
+  float v = r == c ? 1.0f : 0.0f;
+  if (r < n && c < n) {
+    const T* xv = unit + n - c;
+    T d, a;
+    if (r < g.NW) {
+      a = vel_row_w<T, false>(g, k, op, xv, xv + g.NW, nullptr, r, r % (g.Nz + 1), r / (g.Nz + 1), &d);
+    } else {
+      const int u = r - g.NW;
+      a = vel_row_u<T, false>(g, k, op, xv, xv + g.NW, nullptr, u, u % (g.Nz + 2), u / (g.Nz + 2), &d);
+    }
+    v = (float)(a / d);
+    if (c == 0) {
+      dinv[r] = (float)((T)1 / d);
+      if (!(d > (T)0)) *bad = 1;
+    }
+  } else if (c == 0) {
+    dinv[r] = 1.0f;
+  }
+  M[(size_t)r * np + c] = v;
+}
+
+// the 32 x 32 block D -> D^-1 by one warp (lane = row, implicit row pivoting);
+// returns false on a pivot below 1e-6
+__device__ __forceinline__ bool warp_invert32(float (*D)[33], float* prow, int lane) {
+  float a[32], e[32];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    a[c] = D[lane][c];
+    e[c] = lane == c ? 1.0f : 0.0f;
+  }
+  bool used = false, good = true;
+  int mine = 0;
+#pragma unroll
+  for (int p = 0; p < 32; ++p) {
+    // the largest entry of the column among the rows not used yet (its five
+    // lowest bits give way to the lane)
+    const unsigned key = used ? 0u : ((__float_as_uint(fabsf(a[p])) & ~31u) | (31u - lane));
+    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+    const int q = 31 - (int)(top & 31u);
+    good = good && (top & ~31u) > __float_as_uint(1e-6f) && (top & ~31u) < 0x7f800000u;
+    if (lane == q) {
+      const float ip = 1.0f / a[p];
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        if (c > p) { a[c] *= ip; prow[c] = a[c]; }
+        e[c] *= ip;
+        prow[32 + c] = e[c];
+      }
+      used = true;
+      mine = p;
+    }
+    __syncwarp();
+    if (lane != q) {
+      const float f = a[p];
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        if (c > p) a[c] -= f * prow[c];
+        e[c] -= f * prow[32 + c];
+      }
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int c = 0; c < 32; ++c) D[mine][c] = e[c];
+  return good;
+}
+
+// step k of the in-place inversion, src -> dst, a 64 x 64 tile per CTA:
+// R = D^-1 [A_k* with its own block replaced by I]; row block k becomes R, the
+// others A_i* - A_ik R with A_ik taken out of the base.  Every CTA inverts D
+// for itself (one warp, while the others load), so a step is one launch.
+__global__ void __launch_bounds__(256) wide_step_kernel(const float* __restrict__ src, float* dst, int np, int k,
+                                                        int* bad) {
+  XC_PDL_WAIT();
+  __shared__ float D[32][33], prow[64];
+  __shared__ float raw[32][64], R[32][64], C[64][33];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64, k0 = 32 * k;
+  if (warp == 0) {
+    for (int r = 0; r < 32; ++r) D[r][lane] = src[(size_t)(k0 + r) * np + k0 + lane];
+    __syncwarp();
+    if (!warp_invert32(D, prow, lane) && lane == 0) *bad = 1;
+  } else {
+    for (int e = tid - 32; e < 32 * 64; e += 224) {
+      const int r = e >> 6, c = c0 + (e & 63);
+      raw[r][e & 63] = c >= k0 && c < k0 + 32 ? (c - k0 == r ? 1.0f : 0.0f)
+                                              : (c < np ? src[(size_t)(k0 + r) * np + c] : 0.0f);
+    }
+    for (int e = tid - 32; e < 64 * 32; e += 224) {
+      const int r = e >> 5, c = e & 31;
+      C[r][c] = r0 + r < np ? src[(size_t)(r0 + r) * np + k0 + c] : 0.0f;
+    }
+  }
+  __syncthreads();
+  {
+    const int c = tid & 63, rb = tid >> 6;     // rows rb, rb + 4, ...
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) {
+      const float x = raw[q][c];
+#pragma unroll
+      for (int m = 0; m < 8; ++m) acc[m] += D[rb + 4 * m][q] * x;
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) R[rb + 4 * m][c] = acc[m];
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  float acc[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int r = r0 + ty * 4 + a, c = c0 + tx + 16 * b;
+      acc[a][b] = r < np && c < np && !(c >= k0 && c < k0 + 32) ? src[(size_t)r * np + c] : 0.0f;
+    }
+#pragma unroll 8
+  for (int q = 0; q < 32; ++q) {
+    float x[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) x[b] = R[q][tx + 16 * b];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const float f = C[ty * 4 + a][q];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b] -= f * x[b];
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int r = r0 + ty * 4 + a, c = c0 + tx + 16 * b;
+      if (r >= np || c >= np) continue;
+      const bool prow_block = r >= k0 && r < k0 + 32;
+      dst[(size_t)r * np + c] = prow_block ? R[r - k0][tx + 16 * b] : acc[a][b];
+    }
+}
+
+// A^-1 = M^-1 diag^-1: column c scaled by 1 / d_c
+__global__ void wide_scale_kernel(float* M, int np, const float* __restrict__ dinv) {
+  XC_PDL_WAIT();
+  const int c = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
+  if (c < np && r < np) M[(size_t)r * np + c] *= dinv[c];
+}
+
+// x = inv b, or x += inv b: a warp per row
+template <typename T>
+__device__ __forceinline__ float wide_row(const WideInverse& w, int n, const T* b, int r, int lane) {
+  const float* a = w.inv + (size_t)r * w.np;
+  float s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+  int c = lane;
+  for (; c + 96 < n; c += 128) {
+    s0 += a[c] * (float)b[c];
+    s1 += a[c + 32] * (float)b[c + 32];
+    s2 += a[c + 64] * (float)b[c + 64];
+    s3 += a[c + 96] * (float)b[c + 96];
+  }
+  for (; c < n; c += 32) s0 += a[c] * (float)b[c];
+  float s = (s0 + s1) + (s2 + s3);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) wide_apply_kernel(WideInverse w, int n, const T* __restrict__ b, T* x, int add) {
+  XC_PDL_WAIT();
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= n) return;
+  const float s = wide_row<T>(w, n, b, r, lane);
+  if (lane == 0) x[r] = add ? x[r] + (T)s : (T)s;
+}
+
+// the known vector of the check, +-1 in a scattered pattern, and the zero
+// right-hand side that makes the residual kernel return -A y
+template <typename T>
+__global__ void wide_probe_kernel(int n, T* y, T* zero) {
+  XC_PDL_WAIT();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  y[t] = ((unsigned)t * 2654435761u) >> 31 ? (T)1 : (T)-1;
+  zero[t] = (T)0;
+}
+// *ok = 1 where x = inv (-A y) is -y to 1e-2 and no step failed (one CTA); vel:
+// also not where the uniform-U mode is unlifted (see vel_coarse_cta)
+template <typename T>
+__global__ void __launch_bounds__(1024) wide_check_kernel(int n, const T* __restrict__ x, const T* __restrict__ y,
+                                                          const int* bad, int* ok, Geo g, OpConst k, VOp<T> op,
+                                                          int vel) {
+  XC_PDL_WAIT();
+  __shared__ double red[32];
+  bool good = true;
+  for (int t = threadIdx.x; t < n; t += blockDim.x) good = good && fabs((float)(x[t] + y[t])) <= 1e-2f;
+  bool null_mode = false;
+  if (vel && k.top_cnv == -1 && k.bot_cnv == -1 && !k.mms) {
+    double si = 0, sd = 0;
+    for (int u = threadIdx.x; u < g.NU; u += blockDim.x) {
+      const int j = u % (g.Nz + 2);
+      if (j >= 1 && j <= g.Nz) {
+        si += (double)vel_inertia_u<T>(g, op, u);
+        sd += (double)vel_diag<T>(g, k, op, g.NW + u);
+      }
+    }
+    si = cta_sum(si, red);
+    sd = cta_sum(sd, red);
+    null_mode = si <= 1e-6 * sd;
+  }
+  const int all = __syncthreads_and(good);
+  if (threadIdx.x == 0) *ok = all && !*bad && !null_mode ? 1 : 0;
+}
+
 // many damped-Jacobi sweeps on the coarsest velocity level, by one whole CTA.
 // With free slip at top and bottom (top_cnv = bot_cnv = -1) and periodic x, a
 // uniform U shift is a null mode of the viscous rows; where inertia does not
@@ -1135,10 +1373,27 @@ __device__ void dense_apply_cta(const T* __restrict__ inv, int n, const T* b, T*
 // coarse correction and left to the pinned fine level and the Krylov method.
 template <typename T>
 __device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op, T* x, T* x2, const T* b,
-                               int sweeps, T omega, const T* inv = nullptr, const int* inv_ok = nullptr) {
+                               int sweeps, T omega, const T* inv, const int* inv_ok, const WideInverse& wide) {
   const long long n = (long long)g.NW + g.NU;
   if (inv && *inv_ok) {
     dense_apply_cta<T>(inv, (int)n, b, x);
+    return;
+  }
+  if (wide.inv && *inv_ok) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int pass = 0; pass < (kFly<T> ? 1 : 2); ++pass) {
+      const T* rhs = b;
+      if (pass == 1) {       // one step of refinement in FP64, the residual in x2
+        for (long long t = threadIdx.x; t < n; t += blockDim.x) vel_residual_at<T>(g, k, op, x, b, x2, t);
+        __syncthreads();
+        rhs = x2;
+      }
+      for (int r = warp; r < n; r += nw) {
+        const float v = wide_row<T>(wide, (int)n, rhs, r, lane);
+        if (lane == 0) x[r] = pass == 1 ? x[r] + (T)v : (T)v;
+      }
+      __syncthreads();
+    }
     return;
   }
   for (long long t = threadIdx.x; t < n; t += blockDim.x) x[t] = 0;
@@ -1176,9 +1431,10 @@ __device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op,
 }
 template <typename T>
 __global__ void vel_coarse_kernel(Geo g, OpConst k, VOp<T> op, T* x, T* x2, const T* __restrict__ b, int sweeps,
-                                  T omega, const T* inv, const int* inv_ok) {
+                                  T omega, const T* inv, const int* inv_ok, WideInverse wide, const int* solved) {
   XC_PDL_WAIT();
-  vel_coarse_cta<T>(g, k, op, x, x2, b, sweeps, omega, inv, inv_ok);
+  if (solved && *solved) return;     // by the launches of the wide inverse before this one
+  vel_coarse_cta<T>(g, k, op, x, x2, b, sweeps, omega, inv, inv_ok, wide);
 }
 
 // the inverse of the coarsest velocity level (NW + NU <= kDenseMax), one CTA
@@ -1419,11 +1675,28 @@ __global__ void p_coarsen_kernel(int Nzc, int Nxc, const T* __restrict__ kx, con
 
 template <typename T>
 __device__ void p_coarse_cta(int Nz, int Nx, const T* __restrict__ kx, const T* __restrict__ kz, int pin,
-                             T dpin, T* x, T* x2, const T* b, int sweeps, T omega, const T* inv = nullptr,
-                             const int* inv_ok = nullptr) {
+                             T dpin, T* x, T* x2, const T* b, int sweeps, T omega, const T* inv,
+                             const int* inv_ok, const WideInverse& wide) {
   const int n = Nz * Nx;
   if (inv && *inv_ok) {
     dense_apply_cta<T>(inv, n, b, x);
+    return;
+  }
+  if (wide.inv && *inv_ok) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int pass = 0; pass < (kFly<T> ? 1 : 2); ++pass) {
+      const T* rhs = b;
+      if (pass == 1) {
+        for (int t = threadIdx.x; t < n; t += blockDim.x) p_residual_at<T>(Nz, Nx, kx, kz, pin, dpin, x, b, x2, t);
+        __syncthreads();
+        rhs = x2;
+      }
+      for (int r = warp; r < n; r += nw) {
+        const float v = wide_row<T>(wide, n, rhs, r, lane);
+        if (lane == 0) x[r] = pass == 1 ? x[r] + (T)v : (T)v;
+      }
+      __syncthreads();
+    }
     return;
   }
   for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = 0;
@@ -1446,9 +1719,32 @@ __device__ void p_coarse_cta(int Nz, int Nx, const T* __restrict__ kx, const T* 
 template <typename T>
 __global__ void p_coarse_kernel(int Nz, int Nx, const T* __restrict__ kx, const T* __restrict__ kz, int pin,
                                 T dpin, T* x, T* x2, const T* __restrict__ b, int sweeps, T omega, const T* inv,
-                                const int* inv_ok) {
+                                const int* inv_ok, WideInverse wide, const int* solved) {
   XC_PDL_WAIT();
-  p_coarse_cta<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega, inv, inv_ok);
+  if (solved && *solved) return;
+  p_coarse_cta<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega, inv, inv_ok, wide);
+}
+
+// diag^-1 L of a coarsest pressure level, as wide_form_vel_kernel
+template <typename T>
+__global__ void wide_form_p_kernel(int Nz, int Nx, const T* __restrict__ kx, const T* __restrict__ kz, int pin, T dpin,
+                                   const T* unit, int np, float* M, float* dinv, int* bad) {
+  XC_PDL_WAIT();
+  const int r = blockIdx.x * 32 + threadIdx.x, c = blockIdx.y * 8 + threadIdx.y, n = Nz * Nx;
+  if (r >= np || c >= np) return;
+  float v = r == c ? 1.0f : 0.0f;
+  if (r < n && c < n) {
+    T d;
+    const T a = p_apply_at<T>(Nz, Nx, kx, kz, pin, dpin, unit + n - c, r % Nz, r / Nz, &d);
+    v = (float)(a / d);
+    if (c == 0) {
+      dinv[r] = (float)((T)1 / d);
+      if (!(d > (T)0)) *bad = 1;
+    }
+  } else if (c == 0) {
+    dinv[r] = 1.0f;
+  }
+  M[(size_t)r * np + c] = v;
 }
 
 // the inverse of the coarsest pressure level (Nz Nx <= kDenseMax), one CTA
@@ -1568,7 +1864,7 @@ constexpr size_t kStageMaxBytes = 160 * 1024;
 // before and after each coarse correction, the coarsest solved directly
 template <typename T>
 __device__ void vel_vcycle_cta(const VelLevels<T>& L, const OpConst& kf, int l0, int lc, int nu, T om, int csweeps,
-                               const T* inv, const int* inv_ok) {
+                               const T* inv, const int* inv_ok, const WideInverse& wide) {
   for (int l = l0; l < lc; ++l) {
     const OpConst k = level_const(kf, l);
     const Geo& g = L.g[l];
@@ -1582,7 +1878,8 @@ __device__ void vel_vcycle_cta(const VelLevels<T>& L, const OpConst& kf, int l0,
     for (long long t = threadIdx.x; t < nc; t += blockDim.x) vel_restrict_at<T>(g, c, L.r[l], L.b[l + 1], t);
     __syncthreads();
   }
-  vel_coarse_cta<T>(L.g[lc], level_const(kf, lc), L.op[lc], L.x[lc], L.x2[lc], L.b[lc], csweeps, om, inv, inv_ok);
+  vel_coarse_cta<T>(L.g[lc], level_const(kf, lc), L.op[lc], L.x[lc], L.x2[lc], L.b[lc], csweeps, om, inv, inv_ok,
+                    wide);
   for (int l = lc - 1; l >= l0; --l) {
     const OpConst k = level_const(kf, l);
     const Geo& g = L.g[l];
@@ -1596,7 +1893,7 @@ __device__ void vel_vcycle_cta(const VelLevels<T>& L, const OpConst& kf, int l0,
 template <typename T>
 __global__ void __launch_bounds__(1024) vel_vcycle_small_kernel(VelLevels<T> Lg, OpConst kf, int l0, int lc, int nu,
                                                                 T om, int csweeps, int staged, const T* inv,
-                                                                const int* inv_ok) {
+                                                                const int* inv_ok, WideInverse wide) {
   XC_PDL_WAIT();
   extern __shared__ __align__(16) unsigned char xc_stage[];
   __shared__ VelLevels<T> L;
@@ -1642,7 +1939,7 @@ __global__ void __launch_bounds__(1024) vel_vcycle_small_kernel(VelLevels<T> Lg,
     cta_copy<T>(L.b[l0], Lg.b[l0], (long long)L.g[l0].NW + L.g[l0].NU);
     __syncthreads();
   }
-  vel_vcycle_cta<T>(L, kf, l0, lc, nu, om, csweeps, inv, inv_ok);
+  vel_vcycle_cta<T>(L, kf, l0, lc, nu, om, csweeps, inv, inv_ok, wide);
   if (staged) cta_copy<T>(Lg.x[l0], L.x[l0], (long long)L.g[l0].NW + L.g[l0].NU);
 }
 
@@ -1701,7 +1998,7 @@ __device__ void vel_smooth_cluster(const Geo& g, const OpConst& k, const VOp<T>&
 template <typename T>
 __global__ void __launch_bounds__(1024) vel_vcycle_cluster_kernel(VelLevels<T> Lg, OpConst kf, int l0, int ls, int lc,
                                                                   int nu, int nu_post, T om, int csweeps,
-                                                                  const T* inv, const int* inv_ok) {
+                                                                  const T* inv, const int* inv_ok, WideInverse wide) {
   XC_PDL_WAIT();
   __shared__ VelLevels<T> L;
   if (threadIdx.x == 0) L = Lg;
@@ -1721,7 +2018,7 @@ __global__ void __launch_bounds__(1024) vel_vcycle_cluster_kernel(VelLevels<T> L
     for (long long t = t0; t < nc; t += ts) vel_restrict_at<T>(g, c, L.r[l], L.b[l + 1], t);
     cluster_barrier();
   }
-  if (rank == 0) vel_vcycle_cta<T>(L, kf, ls, lc, nu, om, csweeps, inv, inv_ok);
+  if (rank == 0) vel_vcycle_cta<T>(L, kf, ls, lc, nu, om, csweeps, inv, inv_ok, wide);
   cluster_barrier();
   for (int l = ls - 1; l >= l0; --l) {
     const OpConst k = level_const(kf, l);
@@ -1782,7 +2079,7 @@ __host__ __device__ inline long long p_stage_elems(const int* Nzs, const int* Nx
 template <typename T>
 __global__ void __launch_bounds__(1024) p_vcycle_small_kernel(PLevels<T> Lg, int l0, int lc, int nu, T om,
                                                               int csweeps, int staged, const T* inv,
-                                                              const int* inv_ok) {
+                                                              const int* inv_ok, WideInverse wide) {
   XC_PDL_WAIT();
   extern __shared__ __align__(16) unsigned char xc_stage[];
   __shared__ PLevels<T> L;
@@ -1822,7 +2119,7 @@ __global__ void __launch_bounds__(1024) p_vcycle_small_kernel(PLevels<T> Lg, int
     __syncthreads();
   }
   p_coarse_cta<T>(L.Nz[lc], L.Nx[lc], L.kx[lc], L.kz[lc], L.pin[lc], L.dpin[lc], L.x[lc], L.x2[lc], L.b[lc],
-                  csweeps, om, inv, inv_ok);
+                  csweeps, om, inv, inv_ok, wide);
   for (int l = lc - 1; l >= l0; --l) {
     const int n = L.Nz[l] * L.Nx[l];
     for (int t = threadIdx.x; t < n; t += blockDim.x) p_prolong_at<T>(L.Nz[l + 1], L.Nx[l + 1], L.x[l + 1], L.x[l], t);
@@ -2397,6 +2694,14 @@ struct Hier {
   T* pinv;
   int* dok;
   bool vdirect, pdirect;
+  // wide inverses of larger coarsest levels (dok serves them too); scratch:
+  // the second matrix of the elimination, 1 / diagonals, the unit vectors and
+  // the failure flag
+  float *vwide, *pwide, *wscratch, *wdinv;
+  T* wunit;
+  int* wbad;
+  int vwide_np, pwide_np;      // allocated sizes
+  bool vwide_on, pwide_on;     // in use by the current solve
   T* cp;          // DM coefficient planes (fine level)
   T* scl;         // scaling vector
   T* etarho;      // eta/rho on interior cells
@@ -2558,6 +2863,7 @@ void free_hier(Hier<T>& H) {
   cudaFree(H.kr); cudaFree(H.cp); cudaFree(H.scl); cudaFree(H.etarho); cudaFree(H.V); cudaFree(H.Z);
   cudaFree(H.w); cudaFree(H.t); cudaFree(H.y); cudaFree(H.rv); cudaFree(H.rin);
   cudaFree(H.vinv); cudaFree(H.pinv); cudaFree(H.dok);
+  cudaFree(H.vwide); cudaFree(H.pwide); cudaFree(H.wscratch); cudaFree(H.wdinv); cudaFree(H.wunit); cudaFree(H.wbad);
   H.nv = H.np_lv = 0;
 }
 
@@ -2608,6 +2914,16 @@ void launch_sweep(const SolveCfg& cfg, const Geo& g, const OpConst& k, const VOp
     }
   }
   pdl(PDL_ON, vel_sweep2d_kernel<T, MODE>, grid2(g), blk2(), s, g, k, op, xi, b, out, om, dscl);
+}
+
+template <typename T>
+WideInverse vel_wide(const Hier<T>& H, int lc) {
+  const int n = H.vg[lc].NW + H.vg[lc].NU;
+  return H.vwide_on ? WideInverse{H.vwide, (n + 31) / 32 * 32} : WideInverse{nullptr, 0};
+}
+template <typename T>
+WideInverse p_wide(const Hier<T>& H, int lc) {
+  return H.pwide_on ? WideInverse{H.pwide, (H.pNz[lc] * H.pNx[lc] + 31) / 32 * 32} : WideInverse{nullptr, 0};
 }
 
 // CTAs per cluster of the cluster V-cycle (16 where the device schedules
@@ -2681,15 +2997,18 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
       lcfg.numAttrs = PDL_ON ? 2 : 1;
       XC_CUDA_TRY(cudaLaunchKernelEx(&lcfg, vel_vcycle_cluster_kernel<T>, L, kf, l, ls, lc, cfg.nu, cfg.nu_post, om,
                                      coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx),
-                                     (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok));
+                                     (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok, vel_wide(H, lc)));
       xc_count_launch();
       XC_LAUNCH_CHECK();
       return XC_OK;
     }
   }
-  if (!vel_coarsest(H, cfg, l) && (long long)g.Nz * g.Nx <= cfg.small_cells) {
-    int lc = l;
-    while (!vel_coarsest(H, cfg, lc)) ++lc;
+  int lc_small = l;
+  while (!vel_coarsest(H, cfg, lc_small)) ++lc_small;
+  // a wide product of many unknowns belongs to the whole GPU, not to one CTA
+  const bool grid_coarse = H.vwide_on && H.vg[lc_small].NW + H.vg[lc_small].NU > kWideCta;
+  if (!vel_coarsest(H, cfg, l) && (long long)g.Nz * g.Nx <= cfg.small_cells && !grid_coarse) {
+    const int lc = lc_small;
     VelLevels<T> L;
     for (int q = 0; q <= lc; ++q) {
       L.g[q] = H.vg[q]; L.op[q] = vop(H, q);
@@ -2698,14 +3017,25 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
     const size_t bytes = sizeof(T) * (size_t)vel_stage_elems<T>(H.vg, l, lc);
     const int staged = cfg.stage_small && bytes <= kStageMaxBytes;
     pdl_smem(PDL_ON, vel_vcycle_small_kernel<T>, 1, coarse_threads(n), staged ? bytes : 0, s, L, kf, l, lc, cfg.nu,
-             om, coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx), staged, H.vdirect ? H.vinv : nullptr, H.dok);
+             om, coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx), staged, H.vdirect ? H.vinv : nullptr, H.dok,
+             vel_wide(H, lc));
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
   if (vel_coarsest(H, cfg, l)) {
+    const int* solved = nullptr;
+    if (H.vwide_on && n > kWideCta) {
+      const WideInverse wi = vel_wide(H, l);
+      pdl(PDL_ON, wide_apply_kernel<T>, nblk(n, 8), 256, s, wi, (int)n, (const T*)H.vb[l], H.vx[l], 0);
+      if (!kFly<T>) {
+        launch_sweep<T, 2>(cfg, g, k, vop(H, l), H.vx[l], H.vb[l], H.vr[l], om, (const T*)nullptr, s);
+        pdl(PDL_ON, wide_apply_kernel<T>, nblk(n, 8), 256, s, wi, (int)n, (const T*)H.vr[l], H.vx[l], 1);
+      }
+      solved = H.dok;
+    }
     pdl(PDL_ON, vel_coarse_kernel<T>, 1, coarse_threads(n), s, g, k, vop(H, l), H.vx[l], H.vx2[l], H.vb[l],
-                                                        coarse_sweeps(cfg, g.Nz, g.Nx), om,
-                                                        (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok);
+        coarse_sweeps(cfg, g.Nz, g.Nx), om, (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok,
+        solved ? WideInverse{nullptr, 0} : vel_wide(H, l), solved);
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
@@ -2753,9 +3083,11 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
   const int Nz = H.pNz[l], Nx = H.pNx[l], n = Nz * Nx;
   const T om = (T)cfg.omega_p;
   *res = H.px[l];
-  if (!p_coarsest(H, cfg, l) && (long long)n <= cfg.small_cells) {
-    int lc = l;
-    while (!p_coarsest(H, cfg, lc)) ++lc;
+  int lc_small = l;
+  while (!p_coarsest(H, cfg, lc_small)) ++lc_small;
+  const bool grid_coarse = H.pwide_on && H.pNz[lc_small] * H.pNx[lc_small] > kWideCta;
+  if (!p_coarsest(H, cfg, l) && (long long)n <= cfg.small_cells && !grid_coarse) {
+    const int lc = lc_small;
     PLevels<T> L;
     for (int q = 0; q <= lc; ++q) {
       L.Nz[q] = H.pNz[q]; L.Nx[q] = H.pNx[q]; L.pin[q] = H.ppin[q]; L.dpin[q] = H.pdpin[q];
@@ -2765,14 +3097,26 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
     const size_t bytes = sizeof(T) * (size_t)p_stage_elems<T>(H.pNz, H.pNx, l, lc);
     const int staged = cfg.stage_small && bytes <= kStageMaxBytes;
     pdl_smem(PDL_ON, p_vcycle_small_kernel<T>, 1, coarse_threads(n), staged ? bytes : 0, s, L, l, lc, cfg.nu_p, om,
-             coarse_sweeps(cfg, H.pNz[lc], H.pNx[lc]), staged, H.pdirect ? H.pinv : nullptr, H.dok + 1);
+             coarse_sweeps(cfg, H.pNz[lc], H.pNx[lc]), staged, H.pdirect ? H.pinv : nullptr, H.dok + 1,
+             p_wide(H, lc));
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
   if (p_coarsest(H, cfg, l)) {
+    const int* solved = nullptr;
+    if (H.pwide_on && n > kWideCta) {
+      const WideInverse wi = p_wide(H, l);
+      pdl(PDL_ON, wide_apply_kernel<T>, nblk(n, 8), 256, s, wi, n, (const T*)H.pb[l], H.px[l], 0);
+      if (!kFly<T>) {
+        pdl(PDL_ON, p_residual_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], H.px[l],
+            H.pb[l], H.pr[l]);
+        pdl(PDL_ON, wide_apply_kernel<T>, nblk(n, 8), 256, s, wi, n, (const T*)H.pr[l], H.px[l], 1);
+      }
+      solved = H.dok + 1;
+    }
     pdl(PDL_ON, p_coarse_kernel<T>, 1, coarse_threads(n), s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], H.px[l],
-                                                      H.px2[l], H.pb[l], coarse_sweeps(cfg, Nz, Nx), om,
-                                                      (const T*)(H.pdirect ? H.pinv : nullptr), (const int*)(H.dok + 1));
+        H.px2[l], H.pb[l], coarse_sweeps(cfg, Nz, Nx), om, (const T*)(H.pdirect ? H.pinv : nullptr),
+        (const int*)(H.dok + 1), solved ? WideInverse{nullptr, 0} : p_wide(H, l), solved);
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
@@ -3594,6 +3938,76 @@ int fgmres_outer(StokesWork* w, const OpConst& k, const SolveCfg& cfg, const Sol
 // build the operator coefficients and both multigrid hierarchies for one solve
 // (mg = false: the fine-level operator only -- the FP64 hierarchy of a mixed
 // solve, whose multigrid is not used)
+// the wide inverses of the coarsest levels lv, lp (those that are on)
+template <typename T>
+int wide_inverses(Hier<T>& H, const OpConst& k, const SolveCfg& cfg, int lv, int lp, cudaStream_t s) {
+  const Geo& g = H.vg[lv];
+  const int nv = H.vwide_on ? g.NW + g.NU : 0, np = H.pwide_on ? H.pNz[lp] * H.pNx[lp] : 0;
+  const int vnp = (nv + 31) / 32 * 32, pnp = (np + 31) / 32 * 32;
+  if (vnp > H.vwide_np || pnp > H.pwide_np) {
+    // first use, or another option chose a larger coarsest level: the
+    // captured steps hold the old addresses
+    XC_CUDA_TRY(cudaStreamSynchronize(s));
+    for (int e = 0; e < 2; ++e) drop_graphs(H, e);
+    const int a = std::max(vnp, H.vwide_np), b = std::max(pnp, H.pwide_np), m = std::max(a, b);
+    cudaFree(H.vwide); cudaFree(H.pwide); cudaFree(H.wscratch); cudaFree(H.wdinv); cudaFree(H.wunit); cudaFree(H.wbad);
+    H.vwide = H.pwide = H.wscratch = H.wdinv = nullptr;
+    H.wunit = nullptr;
+    H.wbad = nullptr;
+    H.vwide_np = H.pwide_np = 0;
+    if (a) XC_CUDA_TRY(cudaMalloc(&H.vwide, sizeof(float) * a * a));
+    if (b) XC_CUDA_TRY(cudaMalloc(&H.pwide, sizeof(float) * b * b));
+    XC_CUDA_TRY(cudaMalloc(&H.wscratch, sizeof(float) * m * m));
+    XC_CUDA_TRY(cudaMalloc(&H.wdinv, sizeof(float) * m));
+    XC_CUDA_TRY(cudaMalloc(&H.wunit, sizeof(T) * (2 * m + 1)));
+    XC_CUDA_TRY(cudaMalloc(&H.wbad, sizeof(int) * 2));
+    H.vwide_np = a;
+    H.pwide_np = b;
+  }
+  const T one = (T)1;
+  XC_CUDA_TRY(cudaMemsetAsync(H.wbad, 0, sizeof(int) * 2, s));
+  for (int q = 0; q < 2; ++q) {
+    const int n = q ? np : nv, m = q ? pnp : vnp;
+    if (!n) continue;
+    const int steps = m / 32;
+    float* a = q ? H.pwide : H.vwide;
+    float* src = steps % 2 ? H.wscratch : a;        // so that the last step lands in a
+    float* dst = steps % 2 ? a : H.wscratch;
+    XC_CUDA_TRY(cudaMemsetAsync(H.wunit, 0, sizeof(T) * (2 * n + 1), s));
+    XC_CUDA_TRY(cudaMemcpyAsync(H.wunit + n, &one, sizeof(T), cudaMemcpyHostToDevice, s));
+    const dim3 fg((m + 31) / 32, (m + 7) / 8), b2 = blk2();
+    int* bad = H.wbad + q;
+    if (q)
+      pdl(PDL_ON, wide_form_p_kernel<T>, fg, b2, s, H.pNz[lp], H.pNx[lp], (const T*)H.kx[lp], (const T*)H.kz[lp],
+          H.ppin[lp], H.pdpin[lp], (const T*)H.wunit, m, src, H.wdinv, bad);
+    else
+      pdl(PDL_ON, wide_form_vel_kernel<T>, fg, b2, s, g, level_const(k, lv), vop(H, lv), (const T*)H.wunit, n, m, src,
+          H.wdinv, bad);
+    for (int st = 0; st < steps; ++st) {
+      pdl(PDL_ON, wide_step_kernel, dim3((m + 63) / 64, (m + 63) / 64), 256, s, (const float*)src, dst, m, st, bad);
+      std::swap(src, dst);
+    }
+    pdl(PDL_ON, wide_scale_kernel, fg, b2, s, a, m, (const float*)H.wdinv);
+    // x = inv (-A y) against y
+    T* y = q ? H.px2[lp] : H.vx2[lv];
+    T* zero = q ? H.pb[lp] : H.vb[lv];
+    T* r = q ? H.pr[lp] : H.vr[lv];
+    T* x = q ? H.px[lp] : H.vx[lv];
+    pdl(PDL_ON, wide_probe_kernel<T>, nblk(n), 256, s, n, y, zero);
+    if (q)
+      pdl(PDL_ON, p_residual_kernel<T>, nblk(n), 256, s, H.pNz[lp], H.pNx[lp], (const T*)H.kx[lp], (const T*)H.kz[lp],
+          H.ppin[lp], H.pdpin[lp], (const T*)y, (const T*)zero, r);
+    else
+      pdl(PDL_ON, vel_sweep2d_kernel<T, 2>, grid2(g), b2, s, g, level_const(k, lv), vop(H, lv), (const T*)y,
+          (const T*)zero, r, (T)cfg.omega_v, (const T*)nullptr);
+    pdl(PDL_ON, wide_apply_kernel<T>, nblk(n, 8), 256, s, WideInverse{a, m}, n, (const T*)r, x, 0);
+    pdl(PDL_ON, wide_check_kernel<T>, 1, 1024, s, n, (const T*)x, (const T*)y, (const int*)bad, H.dok + q, g,
+        level_const(k, lv), vop(H, lv), q ? 0 : 1);
+    XC_LAUNCH_CHECK();
+  }
+  return XC_OK;
+}
+
 template <typename T>
 int setup_hier(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, xc_ctx* c, cudaStream_t s,
                bool mg = true) {
@@ -3649,8 +4063,28 @@ int setup_hier(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg,
   int lv = 0, lp = 0;
   while (!vel_coarsest(H, cfg, lv)) ++lv;
   while (!p_coarsest(H, cfg, lp)) ++lp;
-  H.vdirect = cfg.direct_coarse && (long long)H.vg[lv].NW + H.vg[lv].NU <= kDenseMax;
-  H.pdirect = cfg.direct_coarse && (long long)H.pNz[lp] * H.pNx[lp] <= kDenseMax;
+  const long long nv = (long long)H.vg[lv].NW + H.vg[lv].NU, np = (long long)H.pNz[lp] * H.pNx[lp];
+  // FP64 levels of at most kDenseMax unknowns keep their FP64 inverse by one
+  // CTA; all others up to kWideMax take the wide one, the FP32 ones however
+  // small (60 unknowns: 25 us of launches instead of 129 us in one CTA).  The
+  // inertia-free limit of the manufactured solution stays with its sweeps.
+  H.vdirect = cfg.direct_coarse && nv <= kDenseMax && (!kFly<T> || k.mms);
+  H.pdirect = cfg.direct_coarse && np <= kDenseMax && (!kFly<T> || k.mms);
+  // And where a coarsest pressure level is too large for its dense inverse,
+  // its sweeps must determine the pressure's slowest mode, the constant lifted
+  // by the pin alone, well enough that both ways end in the same digits: with
+  // k = dt / h^2 the mode decays as (1 - omega / (4 n k))^sweeps, c being that
+  // exponent at the scales' first time step.  Measured over 60 grids, P of the
+  // two ways differs by at most 2.5e-10 for c >= 0.01 (FP64 to a residual of
+  // 1e-12; the 100^2 box: c = 0.011, a step in 15 ms instead of 233) and c >=
+  // 0.0125 (mixed to 1e-13), but by 1e-9 to 2e-8 below, all of it the sweeps'
+  // error: there the results stay those of the sweeps.
+  const double k0 = c->p.dt0 / (w->g.h * w->g.h);
+  const double sweeps_c = coarse_sweeps(cfg, H.pNz[lp], H.pNx[lp]) * cfg.omega_p / (4.0 * (double)np * k0);
+  const bool wide = cfg.direct_coarse && !k.mms && (np <= kDenseMax || sweeps_c >= (kFly<T> ? 0.0125 : 0.01));
+  H.vwide_on = wide && !H.vdirect && nv <= kWideMax;
+  H.pwide_on = wide && !H.pdirect && np <= kWideMax;
+  if (H.vwide_on || H.pwide_on) XC_TRY(wide_inverses<T>(H, k, cfg, lv, lp, s));
   if (H.vdirect) {
     vel_dense_inv_kernel<T><<<1, 256, 0, s>>>(H.vg[lv], level_const(k, lv), vop(H, lv), H.vinv, H.dok);
     xc_count_launch();
