@@ -94,3 +94,28 @@ def test_conv3x3_rejects_untileable_shapes():
     assert rc == xc.XC_BAD_ARG
     rc = xc.lib().xc_nn_conv3x3(_p(x), _p(w), None, _p(y), None, 1, 8, 128, 24, 16, 0, None)
     assert rc == xc.XC_BAD_ARG
+
+
+# every pair of widths (pixels by TMA from 64 channels on, by copies below;
+# weights resident or in the ring; one to four groups of taps) over enough tiles
+# that each CTA's rings wrap; 512 tiles, and 30 of 16-pixel rows
+@pytest.mark.parametrize("Cin", [16, 32, 64, 128])
+@pytest.mark.parametrize("Cout", [16, 32, 64, 128])
+@pytest.mark.parametrize("B, H, W", [(4, 128, 128), (3, 80, 16)])
+def test_conv3x3_and_wgrad_all_widths(Cin, Cout, B, H, W):
+    x, w, bias = _operands(B, H, W, Cin, Cout, seed=Cin + 2 * Cout + H)
+    y32 = torch.full((B, H, W, Cout), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    rc = xc.lib().xc_nn_conv3x3(_p(x), _p(w), _p(bias), None, _p(y32), B, H, W, Cin, Cout, 1, None)
+    assert rc == xc.XC_OK, xc.lib().xc_last_error()
+    ref = _torch_conv(x, w, bias, 1)
+    assert _rel(y32, ref) <= 1e-5
+    assert float((y32 - ref).abs().max()) <= 1e-4 * float(ref.abs().max())
+    dy = torch.randn((B, H, W, Cout), generator=torch.Generator(device="cuda").manual_seed(Cin), device="cuda") \
+        .to(torch.bfloat16)
+    dw = torch.full((Cout, 9, Cin), float("nan"), device="cuda")
+    rc = xc.lib().xc_nn_conv3x3_wgrad(_p(x), _p(dy), _p(dw), B, H, W, Cin, Cout, None)
+    assert rc == xc.XC_OK, xc.lib().xc_last_error()
+    ref = torch.nn.grad.conv2d_weight(x.float().permute(0, 3, 1, 2), (Cout, Cin, 3, 3),
+                                      dy.float().permute(0, 3, 1, 2), padding=1)
+    assert _rel(dw, ref.permute(0, 2, 3, 1).reshape(Cout, 9, Cin)) <= 1e-4

@@ -16,6 +16,7 @@
 // runs on the tcgen05 kernel of xc_nn_conv.cu; the data gradient of a
 // convolution is the forward convolution of dY with the flipped, transposed
 // weights, its weight gradient the tcgen05 wgrad GEMM.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -57,6 +58,7 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 
 // y[b][h][w][:] = mean of x over the 2x2 block (x is 2h x 2w)
 __global__ void pool2_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, int B, int h, int w, int C) {
+  XC_PDL_WAIT();
   const long long nv = (long long)B * h * w * (C / 8);
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= nv) return;
@@ -81,6 +83,7 @@ __global__ void pool2_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, i
 // u[b][Y][X] = t[b][Y/2][X/2] + skip[b][Y][X]  (u is H x W, t is H/2 x W/2)
 __global__ void up_add_kernel(const bf16* __restrict__ t, const bf16* __restrict__ skip, bf16* __restrict__ u,
                               int B, int H, int W, int C) {
+  XC_PDL_WAIT();
   const long long nv = (long long)B * H * W * (C / 8);
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= nv) return;
@@ -96,20 +99,9 @@ __global__ void up_add_kernel(const bf16* __restrict__ t, const bf16* __restrict
   reinterpret_cast<uint4*>(u)[i] = pack8(a);
 }
 
-// d = y > 0 ? d : 0 (ReLU backward from the stored post-activation y)
-__global__ void relu_mask_kernel(bf16* __restrict__ d, const bf16* __restrict__ y, long long nv) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  float a[8], b[8];
-  unpack8(reinterpret_cast<const uint4*>(d)[i], a);
-  unpack8(reinterpret_cast<const uint4*>(y)[i], b);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) a[j] = b[j] > 0.0f ? a[j] : 0.0f;
-  reinterpret_cast<uint4*>(d)[i] = pack8(a);
-}
-
 // dt[b][y][x] = sum of du over the 2x2 block (upsampling backward)
 __global__ void up_back_kernel(const bf16* __restrict__ du, bf16* __restrict__ dt, int B, int h, int w, int C) {
+  XC_PDL_WAIT();
   const long long nv = (long long)B * h * w * (C / 8);
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= nv) return;
@@ -129,9 +121,11 @@ __global__ void up_back_kernel(const bf16* __restrict__ du, bf16* __restrict__ d
   reinterpret_cast<uint4*>(dt)[t] = pack8(acc);
 }
 
-// dx[b][Y][X] = dskip[b][Y][X] + dp[b][Y/2][X/2] / 4  (pooling backward + skip)
+// dx[b][Y][X] = dskip[b][Y][X] + dp[b][Y/2][X/2] / 4 where y > 0, else 0
+// (pooling backward + skip, then the ReLU's backward from its stored output y)
 __global__ void pool_back_add_kernel(const bf16* __restrict__ dskip, const bf16* __restrict__ dp,
-                                     bf16* __restrict__ dx, int B, int H, int W, int C) {
+                                     const bf16* __restrict__ y, bf16* __restrict__ dx, int B, int H, int W, int C) {
+  XC_PDL_WAIT();
   const long long nv = (long long)B * H * W * (C / 8);
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= nv) return;
@@ -139,36 +133,20 @@ __global__ void pool_back_add_kernel(const bf16* __restrict__ dskip, const bf16*
   const long long p = i / (C / 8);
   const int X = (int)(p % W), Y = (int)((p / W) % H), b = (int)(p / ((long long)W * H));
   const size_t src = (((size_t)b * (H / 2) + Y / 2) * (W / 2) + X / 2) * (C / 8) + cv;
-  float a[8], s[8];
+  float a[8], s[8], o[8];
   unpack8(reinterpret_cast<const uint4*>(dp)[src], a);
   unpack8(reinterpret_cast<const uint4*>(dskip)[i], s);
+  unpack8(reinterpret_cast<const uint4*>(y)[i], o);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) a[j] = s[j] + 0.25f * a[j];
+  for (int j = 0; j < 8; ++j) a[j] = o[j] > 0.0f ? s[j] + 0.25f * a[j] : 0.0f;
   reinterpret_cast<uint4*>(dx)[i] = pack8(a);
-}
-
-// per-channel partial sums of d over pixel stripes (bias gradient, pass 1)
-constexpr int kBiasBlocks = 256;
-__global__ void bias_partial_kernel(const bf16* __restrict__ d, long long npix, int C, float* __restrict__ part) {
-  // thread c of the block sums channel c over pixels blockIdx.x, + gridDim.x, ...
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    float s = 0.0f;
-    for (long long p = blockIdx.x; p < npix; p += gridDim.x) s += __bfloat162float(d[p * C + c]);
-    part[(size_t)blockIdx.x * C + c] = s;
-  }
-}
-__global__ void bias_final_kernel(const float* __restrict__ part, int nb, int C, float* db, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float s = 0.0f;
-  for (int k = 0; k < nb; ++k) s += part[(size_t)k * C + c];
-  db[c] = accumulate ? db[c] + s : s;
 }
 
 // BF16 copies of the FP32 master weights: w16 [Cout][9][Cin] and the flipped,
 // transposed wf16 [Cin][9][Cout] with wf[ci][t][co] = w[co][8 - t][ci]
 __global__ void weights_bf16_kernel(const float* __restrict__ w, bf16* __restrict__ w16, bf16* __restrict__ wf16,
                                     int Cin, int Cout) {
+  XC_PDL_WAIT();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 9 * Cin * Cout) return;
   const int ci = i % Cin, t = (i / Cin) % 9, co = i / (9 * Cin);
@@ -181,6 +159,7 @@ __global__ void weights_bf16_kernel(const float* __restrict__ w, bf16* __restric
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, long long n, float lr, float b1, float b2, float c1, float c2,
                             float eps) {
+  XC_PDL_WAIT();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -193,6 +172,7 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
 
 // input pack: FP32 [npix][kInCh] -> BF16 [npix][16] (zero padded)
 __global__ void pack_input_kernel(const float* __restrict__ in, bf16* __restrict__ x, long long npix, int cin) {
+  XC_PDL_WAIT();
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= npix) return;
   float f[8];
@@ -211,6 +191,7 @@ __global__ void pack_input_kernel(const float* __restrict__ in, bf16* __restrict
 // BF16 (channels >= cout get zero gradient)
 __global__ void mse_kernel(const float* __restrict__ out, const float* __restrict__ target, int cout,
                            long long npix, float inv_n, bf16* __restrict__ dout, float* __restrict__ part) {
+  XC_PDL_WAIT();
   __shared__ float sh[256];
   float acc = 0.0f;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npix;
@@ -238,17 +219,23 @@ __global__ void mse_kernel(const float* __restrict__ out, const float* __restric
   }
   if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
-__global__ void sum_final_kernel(const float* __restrict__ part, int n, float scale, float* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float s = 0.0f;
-    for (int k = 0; k < n; ++k) s += part[k];
-    *out = s * scale;
+// the block partials in order: 256 loads at once, then a fixed tree
+__global__ void __launch_bounds__(256) sum_final_kernel(const float* __restrict__ part, float scale, float* out) {
+  XC_PDL_WAIT();
+  __shared__ float sh[256];
+  sh[threadIdx.x] = part[threadIdx.x];
+  __syncthreads();
+  for (int s = 128; s > 0; s >>= 1) {
+    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+    __syncthreads();
   }
+  if (threadIdx.x == 0) *out = sh[0] * scale;
 }
 
 // output unpack: FP32 [npix][16] -> [npix][cout]
 __global__ void unpack_output_kernel(const float* __restrict__ o16, float* __restrict__ out, long long npix,
                                      int cout) {
+  XC_PDL_WAIT();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= npix * cout) return;
   const long long p = i / cout;
@@ -280,11 +267,9 @@ struct xc_nn {
   float* out16;       // FP32 [npix0][16]
   bf16* gl[4][3];     // three gradient buffers per level, sized for the level's widest tensor
   float* partial;     // wgrad scratch
-  int partial_blocks;
-  float* bias_part;
   float* loss_part;
   float* loss;
-  int* err;
+  ErrFlag err;
   std::vector<void*> allocs;
   cudaStream_t stream;
 };
@@ -305,60 +290,48 @@ long long npix(const xc_nn* n, int level) { return (long long)n->B * (n->H >> le
 int conv(xc_nn* n, int L, const bf16* x, bf16* y, float* y32, cudaStream_t s) {
   const int lev = kSpec[L][2];
   return nn_conv3x3_fwd(x, n->w16[L], n->params + n->boff[L], y, y32, n->B, n->H >> lev, n->W >> lev, kSpec[L][0],
-                        kSpec[L][1], kSpec[L][3], n->err, s);
+                        kSpec[L][1], kSpec[L][3], n->err.dev, s);
 }
 
-// data gradient of layer L: dx = conv(dy, flipped weights), no bias
-int conv_dgrad(xc_nn* n, int L, const bf16* dy, bf16* dx, cudaStream_t s) {
+// data gradient of layer L: dx = conv(dy, flipped weights), no bias; with y
+// (the ReLU output dx is the gradient of) the ReLU's backward too
+int conv_dgrad(xc_nn* n, int L, const bf16* dy, bf16* dx, const bf16* y, cudaStream_t s) {
   const int lev = kSpec[L][2];
   return nn_conv3x3_fwd(dy, n->wf16[L], nullptr, dx, nullptr, n->B, n->H >> lev, n->W >> lev, kSpec[L][1],
-                        kSpec[L][0], 0, n->err, s);
+                        kSpec[L][0], 0, n->err.dev, s, y);
 }
 
 int conv_wgrad(xc_nn* n, int L, const bf16* x, const bf16* dy, cudaStream_t s) {
   const int lev = kSpec[L][2];
-  const int H = n->H >> lev, W = n->W >> lev;
-  XC_TRY(nn_conv3x3_wgrad(x, dy, n->grads + n->woff[L], n->partial, n->partial_blocks, n->B, H, W, kSpec[L][0],
-                          kSpec[L][1], 1.0f, 0, n->err, s));
-  const int C = kSpec[L][1];
-  bias_partial_kernel<<<kBiasBlocks, 128, 0, s>>>(dy, npix(n, lev), C, n->bias_part); xc_count_launch();
-  bias_final_kernel<<<1, 128, 0, s>>>(n->bias_part, kBiasBlocks, C, n->grads + n->boff[L], 0); xc_count_launch();
-  XC_LAUNCH_CHECK();
-  return XC_OK;
+  return nn_conv3x3_wgrad(x, dy, n->grads + n->woff[L], n->grads + n->boff[L], n->partial, n->B, n->H >> lev,
+                          n->W >> lev, kSpec[L][0], kSpec[L][1], 1.0f, 0, n->err.dev, s);
 }
 
 int pool(xc_nn* n, int lev_out, const bf16* x, bf16* y, int C, cudaStream_t s) {
   const long long nv = npix(n, lev_out) * (C / 8);
-  pool2_kernel<<<nblk(nv), 256, 0, s>>>(x, y, n->B, n->H >> lev_out, n->W >> lev_out, C); xc_count_launch();
+  xc_launch(pool2_kernel, nblk(nv), 256, 0, s, x, y, n->B, n->H >> lev_out, n->W >> lev_out, C);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
 
 int up_add(xc_nn* n, int lev_out, const bf16* t, const bf16* skip, bf16* u, int C, cudaStream_t s) {
   const long long nv = npix(n, lev_out) * (C / 8);
-  up_add_kernel<<<nblk(nv), 256, 0, s>>>(t, skip, u, n->B, n->H >> lev_out, n->W >> lev_out, C); xc_count_launch();
-  XC_LAUNCH_CHECK();
-  return XC_OK;
-}
-
-int relu_mask(xc_nn* n, int lev, bf16* d, const bf16* y, int C, cudaStream_t s) {
-  const long long nv = npix(n, lev) * (C / 8);
-  relu_mask_kernel<<<nblk(nv), 256, 0, s>>>(d, y, nv); xc_count_launch();
+  xc_launch(up_add_kernel, nblk(nv), 256, 0, s, t, skip, u, n->B, n->H >> lev_out, n->W >> lev_out, C);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
 
 int up_back(xc_nn* n, int lev_out, const bf16* du, bf16* dt, int C, cudaStream_t s) {
   const long long nv = npix(n, lev_out) * (C / 8);
-  up_back_kernel<<<nblk(nv), 256, 0, s>>>(du, dt, n->B, n->H >> lev_out, n->W >> lev_out, C); xc_count_launch();
+  xc_launch(up_back_kernel, nblk(nv), 256, 0, s, du, dt, n->B, n->H >> lev_out, n->W >> lev_out, C);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
 
-int pool_back_add(xc_nn* n, int lev_out, const bf16* dskip, const bf16* dp, bf16* dx, int C, cudaStream_t s) {
+int pool_back_add(xc_nn* n, int lev_out, const bf16* dskip, const bf16* dp, const bf16* y, bf16* dx, int C,
+                  cudaStream_t s) {
   const long long nv = npix(n, lev_out) * (C / 8);
-  pool_back_add_kernel<<<nblk(nv), 256, 0, s>>>(dskip, dp, dx, n->B, n->H >> lev_out, n->W >> lev_out, C);
-  xc_count_launch();
+  xc_launch(pool_back_add_kernel, nblk(nv), 256, 0, s, dskip, dp, y, dx, n->B, n->H >> lev_out, n->W >> lev_out, C);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
@@ -366,9 +339,8 @@ int pool_back_add(xc_nn* n, int lev_out, const bf16* dskip, const bf16* dp, bf16
 int refresh_bf16(xc_nn* n, cudaStream_t s) {
   for (int L = 0; L < kLayers; ++L) {
     const int ne = 9 * kSpec[L][0] * kSpec[L][1];
-    weights_bf16_kernel<<<nblk(ne), 256, 0, s>>>(n->params + n->woff[L], n->w16[L], n->wf16[L], kSpec[L][0],
+    xc_launch(weights_bf16_kernel, nblk(ne), 256, 0, s, n->params + n->woff[L], n->w16[L], n->wf16[L], kSpec[L][0],
                                                   kSpec[L][1]);
-    xc_count_launch();
   }
   XC_LAUNCH_CHECK();
   return XC_OK;
@@ -376,7 +348,7 @@ int refresh_bf16(xc_nn* n, cudaStream_t s) {
 
 int forward(xc_nn* n, const float* in, cudaStream_t s) {
   const long long p0 = npix(n, 0);
-  pack_input_kernel<<<nblk(p0), 256, 0, s>>>(in, n->in0, p0, n->in_ch); xc_count_launch();
+  xc_launch(pack_input_kernel, nblk(p0), 256, 0, s, in, n->in0, p0, n->in_ch);
   XC_LAUNCH_CHECK();
   XC_TRY(conv(n, C0A, n->in0, n->a0, nullptr, s));
   XC_TRY(conv(n, C0B, n->a0, n->x0, nullptr, s));
@@ -410,50 +382,39 @@ int backward(xc_nn* n, cudaStream_t s) {
   bf16** G3 = n->gl[3];
   // level 0 output
   XC_TRY(conv_wgrad(n, COUT, n->y0, G0[0], s));
-  XC_TRY(conv_dgrad(n, COUT, G0[0], G0[1], s));          // d y0
-  XC_TRY(relu_mask(n, 0, G0[1], n->y0, 16, s));
+  XC_TRY(conv_dgrad(n, COUT, G0[0], G0[1], n->y0, s));   // d y0
   XC_TRY(conv_wgrad(n, C0D, n->u0, G0[1], s));
-  XC_TRY(conv_dgrad(n, C0D, G0[1], G0[2], s));          // d u0 = d x0 (skip part)
+  XC_TRY(conv_dgrad(n, C0D, G0[1], G0[2], nullptr, s)); // d u0 = d x0 (skip part)
   XC_TRY(up_back(n, 1, G0[2], G1[0], 16, s));           // d t1
   XC_TRY(conv_wgrad(n, C1U, n->y1, G1[0], s));
-  XC_TRY(conv_dgrad(n, C1U, G1[0], G1[1], s));          // d y1 (32 ch)
-  XC_TRY(relu_mask(n, 1, G1[1], n->y1, 32, s));
+  XC_TRY(conv_dgrad(n, C1U, G1[0], G1[1], n->y1, s));   // d y1 (32 ch)
   XC_TRY(conv_wgrad(n, C1D, n->u1, G1[1], s));
-  XC_TRY(conv_dgrad(n, C1D, G1[1], G1[2], s));          // d u1 = d x1 (skip part)
+  XC_TRY(conv_dgrad(n, C1D, G1[1], G1[2], nullptr, s)); // d u1 = d x1 (skip part)
   XC_TRY(up_back(n, 2, G1[2], G2[0], 32, s));           // d t2
   XC_TRY(conv_wgrad(n, C2U, n->y2, G2[0], s));
-  XC_TRY(conv_dgrad(n, C2U, G2[0], G2[1], s));          // d y2 (64)
-  XC_TRY(relu_mask(n, 2, G2[1], n->y2, 64, s));
+  XC_TRY(conv_dgrad(n, C2U, G2[0], G2[1], n->y2, s));   // d y2 (64)
   XC_TRY(conv_wgrad(n, C2D, n->u2, G2[1], s));
-  XC_TRY(conv_dgrad(n, C2D, G2[1], G2[2], s));          // d u2 = d x2 (skip part)
+  XC_TRY(conv_dgrad(n, C2D, G2[1], G2[2], nullptr, s)); // d u2 = d x2 (skip part)
   XC_TRY(up_back(n, 3, G2[2], G3[0], 64, s));           // d t3
   XC_TRY(conv_wgrad(n, C3U, n->x3, G3[0], s));
-  XC_TRY(conv_dgrad(n, C3U, G3[0], G3[1], s));          // d x3 (128)
-  XC_TRY(relu_mask(n, 3, G3[1], n->x3, 128, s));
+  XC_TRY(conv_dgrad(n, C3U, G3[0], G3[1], n->x3, s));   // d x3 (128)
   XC_TRY(conv_wgrad(n, C3B, n->a3, G3[1], s));
-  XC_TRY(conv_dgrad(n, C3B, G3[1], G3[2], s));          // d a3
-  XC_TRY(relu_mask(n, 3, G3[2], n->a3, 128, s));
+  XC_TRY(conv_dgrad(n, C3B, G3[1], G3[2], n->a3, s));   // d a3
   XC_TRY(conv_wgrad(n, C3A, n->p3, G3[2], s));
-  XC_TRY(conv_dgrad(n, C3A, G3[2], G3[0], s));          // d p3 (64)
-  XC_TRY(pool_back_add(n, 2, G2[2], G3[0], G2[0], 64, s));   // d x2
-  XC_TRY(relu_mask(n, 2, G2[0], n->x2, 64, s));
+  XC_TRY(conv_dgrad(n, C3A, G3[2], G3[0], nullptr, s)); // d p3 (64)
+  XC_TRY(pool_back_add(n, 2, G2[2], G3[0], n->x2, G2[0], 64, s));   // d x2
   XC_TRY(conv_wgrad(n, C2B, n->a2, G2[0], s));
-  XC_TRY(conv_dgrad(n, C2B, G2[0], G2[1], s));          // d a2
-  XC_TRY(relu_mask(n, 2, G2[1], n->a2, 64, s));
+  XC_TRY(conv_dgrad(n, C2B, G2[0], G2[1], n->a2, s));   // d a2
   XC_TRY(conv_wgrad(n, C2A, n->p2, G2[1], s));
-  XC_TRY(conv_dgrad(n, C2A, G2[1], G2[2], s));          // d p2 (32)
-  XC_TRY(pool_back_add(n, 1, G1[2], G2[2], G1[0], 32, s));   // d x1
-  XC_TRY(relu_mask(n, 1, G1[0], n->x1, 32, s));
+  XC_TRY(conv_dgrad(n, C2A, G2[1], G2[2], nullptr, s)); // d p2 (32)
+  XC_TRY(pool_back_add(n, 1, G1[2], G2[2], n->x1, G1[0], 32, s));   // d x1
   XC_TRY(conv_wgrad(n, C1B, n->a1, G1[0], s));
-  XC_TRY(conv_dgrad(n, C1B, G1[0], G1[1], s));          // d a1
-  XC_TRY(relu_mask(n, 1, G1[1], n->a1, 32, s));
+  XC_TRY(conv_dgrad(n, C1B, G1[0], G1[1], n->a1, s));   // d a1
   XC_TRY(conv_wgrad(n, C1A, n->p1, G1[1], s));
-  XC_TRY(conv_dgrad(n, C1A, G1[1], G1[2], s));          // d p1 (16)
-  XC_TRY(pool_back_add(n, 0, G0[2], G1[2], G0[0], 16, s));   // d x0
-  XC_TRY(relu_mask(n, 0, G0[0], n->x0, 16, s));
+  XC_TRY(conv_dgrad(n, C1A, G1[1], G1[2], nullptr, s)); // d p1 (16)
+  XC_TRY(pool_back_add(n, 0, G0[2], G1[2], n->x0, G0[0], 16, s));   // d x0
   XC_TRY(conv_wgrad(n, C0B, n->a0, G0[0], s));
-  XC_TRY(conv_dgrad(n, C0B, G0[0], G0[1], s));          // d a0
-  XC_TRY(relu_mask(n, 0, G0[1], n->a0, 16, s));
+  XC_TRY(conv_dgrad(n, C0B, G0[0], G0[1], n->a0, s));   // d a0
   XC_TRY(conv_wgrad(n, C0A, n->in0, G0[1], s));
   return XC_OK;
 }
@@ -461,22 +422,13 @@ int backward(xc_nn* n, cudaStream_t s) {
 int loss_and_dout(xc_nn* n, const float* target, cudaStream_t s) {
   const long long p0 = npix(n, 0);
   const float inv_n = 1.0f / (float)p0;
-  mse_kernel<<<256, 256, 0, s>>>(n->out16, target, n->out_ch, p0, inv_n, n->gl[0][0], n->loss_part); xc_count_launch();
-  sum_final_kernel<<<1, 32, 0, s>>>(n->loss_part, 256, inv_n, n->loss); xc_count_launch();
+  xc_launch(mse_kernel, 256, 256, 0, s, n->out16, target, n->out_ch, p0, inv_n, n->gl[0][0], n->loss_part);
+  xc_launch(sum_final_kernel, 1, 256, 0, s, n->loss_part, inv_n, n->loss);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
 
-int check_err(xc_nn* n, cudaStream_t s, const char* what) {
-  int h = 0;
-  XC_CUDA_TRY(cudaMemcpyAsync(&h, n->err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  XC_CUDA_TRY(cudaStreamSynchronize(s));
-  if (h) {
-    xc_set_error("%s: a bounded wait inside a convolution kernel ran out (code %d)", what, h);
-    return XC_TIMEOUT;
-  }
-  return XC_OK;
-}
+int check_err(xc_nn* n, cudaStream_t s, const char* what) { return n->err.check(s, what); }
 
 // He-normal initial weights from a host generator (splitmix64 + Box-Muller),
 // zero biases; the output layer starts small
@@ -567,12 +519,13 @@ extern "C" int xc_nn_create(int H, int W, int batch, int in_ch, int out_ch, unsi
   const int widest[4] = {16, 32, 64, 128};
   for (int l = 0; l < 4; ++l)
     for (int k = 0; k < 3; ++k) NN_ALLOC(n->gl[l][k], p[l] * widest[l]);
-  n->partial_blocks = 2 * kNumSMs / 9 + 1;
-  NN_ALLOC(n->partial, (size_t)n->partial_blocks * 9 * 128 * 128);
-  NN_ALLOC(n->bias_part, (size_t)kBiasBlocks * 128);
+  long long scratch = 0;
+  for (int L = 0; L < kLayers; ++L)
+    scratch = std::max(scratch, nn_wgrad_scratch(batch, H >> kSpec[L][2], W >> kSpec[L][2], kSpec[L][0], kSpec[L][1]));
+  NN_ALLOC(n->partial, scratch);
   NN_ALLOC(n->loss_part, 256);
   NN_ALLOC(n->loss, 1);
-  NN_ALLOC(n->err, 1);
+  if ((st = n->err.init()) != XC_OK) return fail(st);
 #undef NN_ALLOC
   cudaStream_t s = n->stream;
   std::vector<float> h;
@@ -580,8 +533,7 @@ extern "C" int xc_nn_create(int H, int W, int batch, int in_ch, int out_ch, unsi
   if (cudaMemcpyAsync(n->params, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice, s) != cudaSuccess ||
       cudaMemsetAsync(n->m1, 0, sizeof(float) * off, s) != cudaSuccess ||
       cudaMemsetAsync(n->m2, 0, sizeof(float) * off, s) != cudaSuccess ||
-      cudaMemsetAsync(n->grads, 0, sizeof(float) * off, s) != cudaSuccess ||
-      cudaMemsetAsync(n->err, 0, sizeof(int), s) != cudaSuccess) {
+      cudaMemsetAsync(n->grads, 0, sizeof(float) * off, s) != cudaSuccess) {
     xc_set_error("xc_nn_create: initialisation copy failed");
     return fail(XC_CUDA);
   }
@@ -642,7 +594,7 @@ extern "C" int xc_nn_forward(xc_nn* n, const float* in, float* out, void* stream
   cudaStream_t s = stream ? (cudaStream_t)stream : n->stream;
   XC_TRY(forward(n, in, s));
   const long long p0 = npix(n, 0);
-  unpack_output_kernel<<<nblk(p0 * n->out_ch), 256, 0, s>>>(n->out16, out, p0, n->out_ch); xc_count_launch();
+  xc_launch(unpack_output_kernel, nblk(p0 * n->out_ch), 256, 0, s, n->out16, out, p0, n->out_ch);
   XC_LAUNCH_CHECK();
   return check_err(n, s, "xc_nn_forward");
 }
@@ -667,9 +619,8 @@ extern "C" int xc_nn_train_step(xc_nn* n, const float* in, const float* target, 
   ++n->adam_t;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.0f - std::pow(b1, (float)n->adam_t), c2 = 1.0f - std::pow(b2, (float)n->adam_t);
-  adam_kernel<<<nblk(n->nparams), 256, 0, s>>>(n->params, n->grads, n->m1, n->m2, n->nparams, lr, b1, b2, c1, c2,
+  xc_launch(adam_kernel, nblk(n->nparams), 256, 0, s, n->params, n->grads, n->m1, n->m2, n->nparams, lr, b1, b2, c1, c2,
                                                1e-8f);
-  xc_count_launch();
   XC_LAUNCH_CHECK();
   XC_TRY(refresh_bf16(n, s));
   if (loss) XC_CUDA_TRY(cudaMemcpyAsync(loss, n->loss, sizeof(float), cudaMemcpyDeviceToHost, s));

@@ -53,6 +53,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 // TMA: tiled tensor loads into shared memory, completion counted in bytes on
 // an mbarrier (the tensor map lives in kernel parameter space)
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, int c0, int c1, int c2,
@@ -120,6 +124,20 @@ __device__ __forceinline__ void fence_async_shared() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// 16-byte asynchronous copies by the CTA's threads (zeros where !in)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(__cvta_generic_to_global(src)),
+               "r"(in ? 16 : 0)
+               : "memory");
+}
+// one arrival on the mbarrier once this thread's copies so far have landed (it
+// counts against the barrier's expected arrivals); the thread that hands the
+// data to the tensor core executes fence_async_shared() after its wait
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // layout codes of the shared-memory descriptor (bits 61..63)
 constexpr uint32_t kLayoutSW128 = 2, kLayoutSW64 = 4, kLayoutSW32 = 6;
 
@@ -135,24 +153,31 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t sbo_bytes,
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46) | ((uint64_t)layout << 61);
 }
 
+// the same for an MN-major operand: rows of `layout`'s width along M (or N),
+// one row per K index.  The swizzled unit is 8 such rows; the leading byte
+// offset steps to the next row-width of M (or N), the stride byte offset to
+// the next 8 K indices
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes,
+                                                 uint32_t layout) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46) | ((uint64_t)layout << 61);
+}
+
 // instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, M x N
-__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+// K-major (or both MN-major, mn = 1), M x N
+__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N, uint32_t mn = 0) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (mn << 15) | (mn << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
 __host__ __device__ constexpr uint32_t tmem_cols_for(uint32_t n) {
   return n <= 32 ? 32u : (n <= 64 ? 64u : (n <= 128 ? 128u : (n <= 256 ? 256u : 512u)));
 }
 
-// byte offset of element (row, k) inside a K-major swizzled tile whose rows
-// hold row_bytes (32, 64 or 128) bytes of 16-bit elements
-__device__ __forceinline__ uint32_t swz_offset(uint32_t row, uint32_t k, uint32_t row_bytes) {
-  const uint32_t byte = k * 2u;
-  const uint32_t chunk = byte >> 4;
-  const uint32_t mask = (row_bytes >> 4) - 1u;             // chunk bits of one row
-  const uint32_t phase = (row * row_bytes) >> 7;           // address bits 7.. of the row start
-  return row * row_bytes + (((chunk ^ phase) & mask) << 4) + (byte & 15u);
+// byte offset of 16-byte chunk c of row `row` in a swizzled tile of RB-byte
+// rows (RB = 32, 64 or 128): what a TMA load with that swizzle would write
+template <uint32_t RB>
+__device__ __forceinline__ uint32_t swz_chunk(uint32_t row, uint32_t c) {
+  return row * RB + ((c ^ (((row * RB) >> 7) & (RB / 16u - 1u))) << 4);
 }
 
 }  // namespace xcnn
