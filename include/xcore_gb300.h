@@ -122,14 +122,13 @@ typedef struct xc_solver_opts {
                               1 FP64 FGMRES whose preconditioner is the FP32 inner solve (measured
                               4% slower at 1024^2: the inner solves' corrections are nearly
                               independent, so keeping them gains no iterations) */
-  int fused_pressure_cells; /* pressure-multigrid levels of at most this many cells fuse the first
-                               sweep, residual and restriction (descent) and the prolongation and
-                               first post sweep (ascent) into one launch each; larger levels launch
-                               each operation (same results either way; default and -1: none,
-                               measured no faster) */
-  int stage_small_levels;  /* 1: the one-CTA V-cycles of the small levels stage them in shared
-                              memory instead of reading global memory (same results; measured
-                              1.5% slower at 1024^2) */
+  int fused_pressure_cells; /* pressure-multigrid levels run the first sweep, residual and
+                               restriction (descent) and the prolongation and first post sweep
+                               (ascent) as one launch each, from shared-memory tiles; levels of at
+                               most this many cells form every neighbour's value from global memory
+                               instead (same results either way; default and -1: none) */
+  int stage_small_levels;  /* no longer chooses anything: the one-CTA V-cycles of the small levels run
+                              from shared memory wherever they fit it (same results) */
   int jacobi_coarse;       /* 1: Jacobi sweeps (coarse_sweeps) on the coarsest levels even where they
                               have at most 64 unknowns, which by default are solved with their
                               dense inverse (formed and inverted on the device once per solve) */

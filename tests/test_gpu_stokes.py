@@ -366,3 +366,46 @@ def test_cluster_vcycle_matches_the_per_level_launches(N):
     assert abs(ia["iterations"] - ib["iterations"]) <= 1, (ia, ib)
     for a, b in zip(fa, fb):
         assert np.abs(a - b).max() <= 1e-7 * np.abs(a).max()
+
+
+@pytest.mark.parametrize("shape,kw", [
+    ((48, 40), {}),                                  # 24x20 | 12x10, 6x5: wide coarsest inside one CTA
+    ((64, 64), dict(smooth_sweeps=2, post_sweeps=2)),  # 32x32 | 16x16 .. 4x4: both iterates, dense coarsest
+    ((16, 256), {}),                                 # 8x128 | 4x64, 2x32, 1x16: long levels
+    ((64, 64), dict(jacobi_coarse=True)),            # coarsest level by sweeps in registers
+    ((200, 200), dict(jacobi_coarse=True)),          # 25x25 by one CTA
+])
+def test_staged_vcycle_gives_the_generic_results(shape, kw):
+    """The velocity levels of at most 256 cells run from shared memory with a thread per row; under cluster_cells the
+    cluster's first CTA runs them with the generic per-unknown bodies on global memory.  The operations and their
+    order are the same, so the solutions are equal bit for bit."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=shape[0], Nx=shape[1], steps=1)
+    coefs = O.time_coefs("bd2im", 2)
+    out = []
+    for cc in (0, 1 << 20):
+        ds = device_state(par, g, sc, st)
+        info = ds.fluidmech(coefs, dt, solver="mixed", rtol=1e-9, maxit=600, cluster_cells=cc, **kw)
+        out.append((info["iterations"], [ds[k] for k in ("W", "U", "P")]))
+        ds.close()
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("shape", [(66, 34), (128, 128), (130, 128)])
+@pytest.mark.parametrize("bc", [{}, dict(open_cnv=True)])
+def test_small_level_kernels_give_the_tiled_results(shape, bc):
+    """Levels of at most 128^2 cells run their FP32 sweeps with a thread per row, larger ones with a thread per
+    position; the tiled kernel serves both alike with the same operations: equal bits on either side of the limit."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=shape[0], Nx=shape[1], steps=1)
+    coefs = O.time_coefs("bd2im", 2)
+    out = []
+    for tiled in (False, True):
+        ds = xc.State(product_params(par), grid=xc.Grid(Nx=g.Nx, Nz=g.Nz, h=g.h, D=g.D, L=g.L), scales=sc, **bc)
+        upload_all(ds, st)
+        info = ds.fluidmech(coefs, dt, solver="mixed", rtol=1e-9, maxit=2000, tiled_sweep=tiled)
+        out.append((info["iterations"], [ds[k] for k in ("W", "U", "P")]))
+        ds.close()
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)

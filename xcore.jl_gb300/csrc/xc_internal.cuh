@@ -113,8 +113,14 @@ inline void xc_count_launch() {
 // waits there for the grid before it on the stream to finish and flush its
 // memory (a no-op when launched without the attribute), so it may be launched
 // with programmatic stream serialization -- scheduled while the previous
-// kernel drains instead of after it, hiding the launch gap.
+// kernel drains instead of after it, hiding the launch gap.  A unit that defines
+// XC_PDL_EARLY lets the grid after it be scheduled as soon as this one is past
+// its own wait, rather than when its blocks have ended.
+#ifdef XC_PDL_EARLY
+#define XC_PDL_WAIT() asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory")
+#else
 #define XC_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
+#endif
 
 // launch with programmatic stream serialization (the kernel must begin with
 // XC_PDL_WAIT()), counted like a plain launch

@@ -27,6 +27,12 @@
 #include <utility>
 #include <vector>
 
+// The solver's launches are short and follow one another: each grid may be
+// scheduled while the one before it runs (64^2 step 8110 -> 7882 us, 512^2 solve
+// 6829 -> 6194 us, 1024^2 step 50.5 -> 48.2 ms).  The stencil, update and noise
+// units' launches are longer and lose by it: the next grid's blocks take up
+// residency early (100^2 WENO5 call 7.0 -> 9.3 us).
+#define XC_PDL_EARLY
 #include "xc_internal.cuh"
 #include "xc_nn.cuh"
 
@@ -229,9 +235,15 @@ __device__ __forceinline__ T sdiv(T r, T d) {
   if constexpr (kFly<T>) return __fdividef(r, d);
   else return r / d;
 }
-// rounded products and sums the compiler may not contract into FMAs: the
-// pressure multigrid forms the same values in its fused and split kernels,
-// whose inlined contexts would otherwise contract differently
+// the same quotient, the FP64 one on the integer pipe
+template <typename T>
+__device__ __forceinline__ T rdiv(T r, T d) {
+  if constexpr (kFly<T>) return __fdividef(r, d);
+  else return xc_div(r, d);
+}
+// rounded products, sums and fused products: the multigrid forms the same
+// values in its fused, staged and split kernels, whose inlined contexts the
+// compiler would otherwise contract differently
 template <typename T>
 __device__ __forceinline__ T mul_rn(T a, T b) {
   if constexpr (kFly<T>) return __fmul_rn(a, b);
@@ -241,6 +253,11 @@ template <typename T>
 __device__ __forceinline__ T add_rn(T a, T b) {
   if constexpr (kFly<T>) return __fadd_rn(a, b);
   else return __dadd_rn(a, b);
+}
+template <typename T>
+__device__ __forceinline__ T fma_rn(T a, T b, T c) {
+  if constexpr (kFly<T>) return __fmaf_rn(a, b, c);
+  else return __fma_rn(a, b, c);
 }
 
 // dw / du and the FP32 viscosity copies of one level (terms as vel_coef_kernel)
@@ -290,16 +307,17 @@ struct RowW { T d, c1, c2, c3, c4, c5, c6, c7, c8; };
 template <typename T>
 __device__ __forceinline__ RowW<T> fly_row(T C1, T C2, T P1, T P2, T extra, T ih2) {
   const T c23 = (T)(2.0 / 3.0), c13 = (T)(1.0 / 3.0), hf = (T)0.5;
+  const T hC1 = mul_rn<T>(hf, C1), hC2 = mul_rn<T>(hf, C2);
   RowW<T> w;
-  w.d = extra + (c23 * (P1 + P2) * ih2 + hf * (C1 + C2) * ih2);
-  w.c1 = -c23 * P1 * ih2;
-  w.c2 = -c23 * P2 * ih2;
-  w.c3 = -hf * C1 * ih2;
-  w.c4 = -hf * C2 * ih2;
-  w.c5 = -(hf * C1 - c13 * P1) * ih2;
-  w.c6 = +(hf * C1 - c13 * P2) * ih2;
-  w.c7 = +(hf * C2 - c13 * P1) * ih2;
-  w.c8 = -(hf * C2 - c13 * P2) * ih2;
+  w.d = add_rn<T>(extra, fma_rn<T>(mul_rn<T>(hf, add_rn<T>(C1, C2)), ih2, mul_rn<T>(mul_rn<T>(c23, add_rn<T>(P1, P2)), ih2)));
+  w.c1 = mul_rn<T>(mul_rn<T>(-c23, P1), ih2);
+  w.c2 = mul_rn<T>(mul_rn<T>(-c23, P2), ih2);
+  w.c3 = -mul_rn<T>(hC1, ih2);
+  w.c4 = -mul_rn<T>(hC2, ih2);
+  w.c5 = -mul_rn<T>(fma_rn<T>(-c13, P1, hC1), ih2);
+  w.c6 = mul_rn<T>(fma_rn<T>(-c13, P2, hC1), ih2);
+  w.c7 = mul_rn<T>(fma_rn<T>(-c13, P1, hC2), ih2);
+  w.c8 = -mul_rn<T>(fma_rn<T>(-c13, P2, hC2), ih2);
   return w;
 }
 template <typename T>
@@ -338,45 +356,79 @@ __device__ __forceinline__ RowW<T> u_row(const Geo& g, const VOp<T>& op, long lo
 // W row t = (j, i) and U row u = (j, i) of A x, with the row's diagonal in *dg
 // (boundary rows: their exact-row value).  FULL adds the pressure gradient GG p
 // of the fine level (fluidmech.jl:343-356).
-template <typename T, bool FULL>
-__device__ __forceinline__ T vel_row_w(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xw,
-                                       const T* xu, const T* xp, long long t, int j, int i, T* dg) {
+// interior rows from their weights (pw at W(j, i), pu at U(j, i-1)) ...
+template <typename T>
+__device__ __forceinline__ T vel_dot_w(const RowW<T>& c, const T* pw, const T* pu, int lw, int lu) {
+  T s = fma_rn<T>(c.d, pw[0], mul_rn<T>(c.c1, pw[-1]));
+  s = fma_rn<T>(c.c2, pw[1], s);
+  s = fma_rn<T>(c.c3, pw[-lw], s);
+  s = fma_rn<T>(c.c4, pw[lw], s);
+  s = fma_rn<T>(c.c5, pu[0], s);
+  s = fma_rn<T>(c.c6, pu[1], s);
+  s = fma_rn<T>(c.c7, pu[lu], s);
+  s = fma_rn<T>(c.c8, pu[lu + 1], s);
+  return s;
+}
+// (pu at U(j, i), pl / pr its neighbours along x across the periodic boundary, pw at W(j-1, i))
+template <typename T>
+__device__ __forceinline__ T vel_dot_u(const RowW<T>& c, const T* pu, const T* pl, const T* pr, const T* pw, int lw) {
+  T s = fma_rn<T>(c.d, pu[0], mul_rn<T>(c.c1, pl[0]));
+  s = fma_rn<T>(c.c2, pr[0], s);
+  s = fma_rn<T>(c.c3, pu[-1], s);
+  s = fma_rn<T>(c.c4, pu[1], s);
+  s = fma_rn<T>(c.c5, pw[0], s);
+  s = fma_rn<T>(c.c6, pw[lw], s);
+  s = fma_rn<T>(c.c7, pw[1], s);
+  s = fma_rn<T>(c.c8, pw[lw + 1], s);
+  return s;
+}
+// ... and the ghost and boundary rows
+__device__ __forceinline__ bool vel_edge_w(const Geo& g, int j, int i) {
+  return i == 0 || i == g.Nx + 1 || j == 0 || j == g.Nz;
+}
+__device__ __forceinline__ bool vel_edge_u(const Geo& g, const OpConst& k, long long u, int j) {
+  return j == 0 || j == g.Nz + 1 || (k.mms && (int)u == k.pin_u);
+}
+template <typename T>
+__device__ __forceinline__ T vel_edge_row_w(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xw,
+                                            const T* xu, long long t, int j, int i, T* dg) {
   const int Nz = g.Nz, Nx = g.Nx, lw = Nz + 1, lu = Nz + 2;
   if (i == 0) { *dg = (T)1; return xw[t] + (T)k.sds * xw[(size_t)Nx * lw + j]; }
   if (i == Nx + 1) { *dg = (T)1; return xw[t] + (T)k.sds * xw[(size_t)1 * lw + j]; }
-  if (j == 0 || j == Nz) {
-    T d;
-    if constexpr (kFly<T>) d = j == 0 ? (T)1 : op.dw[t];
-    else d = op.cw[t];
-    *dg = d;
-    if (j == Nz && k.open_cnv) {   // open bottom: the continuity-like row, no pressure gradient
-      T c1, c5, c7;
-      if constexpr (kFly<T>) {
-        c1 = op.dbot[3 * i]; c5 = op.dbot[3 * i + 1]; c7 = op.dbot[3 * i + 2];
-      } else {
-        c1 = op.cw[g.NW + t]; c5 = op.cw[5 * (size_t)g.NW + t]; c7 = op.cw[7 * (size_t)g.NW + t];
-      }
-      T s = d * xw[t];
-      s += c1 * xw[t - 1];
-      s += c5 * xu[(i - 1) * lu + j];
-      s += c7 * xu[i * lu + j];
-      return s;
+  T d;
+  if constexpr (kFly<T>) d = j == 0 ? (T)1 : op.dw[t];
+  else d = op.cw[t];
+  *dg = d;
+  if (j == Nz && k.open_cnv) {   // open bottom: the continuity-like row, no pressure gradient
+    T c1, c5, c7;
+    if constexpr (kFly<T>) {
+      c1 = op.dbot[3 * i]; c5 = op.dbot[3 * i + 1]; c7 = op.dbot[3 * i + 2];
+    } else {
+      c1 = op.cw[g.NW + t]; c5 = op.cw[5 * (size_t)g.NW + t]; c7 = op.cw[7 * (size_t)g.NW + t];
     }
-    return d * xw[t];
+    T s = d * xw[t];
+    s += c1 * xw[t - 1];
+    s += c5 * xu[(i - 1) * lu + j];
+    s += c7 * xu[i * lu + j];
+    return s;
   }
+  return d * xw[t];
+}
+template <typename T>
+__device__ __forceinline__ T vel_edge_row_u(const Geo& g, const OpConst& k, const T* xu, long long u, int j, T* dg) {
+  *dg = (T)1;
+  if (j == 0) return xu[u] + (T)k.top_cnv * xu[u + 1];
+  if (j == g.Nz + 1) return xu[u] + (T)k.bot_cnv * xu[u - 1];
+  return xu[u];
+}
+template <typename T, bool FULL>
+__device__ __forceinline__ T vel_row_w(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xw,
+                                       const T* xu, const T* xp, long long t, int j, int i, T* dg) {
+  const int lw = g.Nz + 1, lu = g.Nz + 2;
+  if (vel_edge_w(g, j, i)) return vel_edge_row_w<T>(g, k, op, xw, xu, t, j, i, dg);
   const RowW<T> c = w_row<T>(g, op, t, j, i);
   *dg = c.d;
-  const T* pw = xw + t;                          // W(j, i)
-  const T* pu = xu + ((i - 1) * lu + j);         // U(j, i-1)
-  T s = c.d * pw[0];
-  s += c.c1 * pw[-1];
-  s += c.c2 * pw[1];
-  s += c.c3 * pw[-lw];
-  s += c.c4 * pw[lw];
-  s += c.c5 * pu[0];
-  s += c.c6 * pu[1];
-  s += c.c7 * pu[lu];
-  s += c.c8 * pu[lu + 1];
+  T s = vel_dot_w<T>(c, xw + t, xu + ((i - 1) * lu + j), lw, lu);
   if (FULL) {
     const T* pp = xp + (i * lu + j);
     s += geo_invh<T>(g) * (pp[1] - pp[0]);
@@ -386,24 +438,12 @@ __device__ __forceinline__ T vel_row_w(const Geo& g, const OpConst& k, const VOp
 template <typename T, bool FULL>
 __device__ __forceinline__ T vel_row_u(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xw,
                                        const T* xu, const T* xp, long long u, int j, int i, T* dg) {
-  const int Nz = g.Nz, Nx = g.Nx, lw = Nz + 1, lu = Nz + 2;
-  if (j == 0) { *dg = (T)1; return xu[u] + (T)k.top_cnv * xu[u + 1]; }
-  if (j == Nz + 1) { *dg = (T)1; return xu[u] + (T)k.bot_cnv * xu[u - 1]; }
-  if (k.mms && (int)u == k.pin_u) { *dg = (T)1; return xu[u]; }
+  const int Nx = g.Nx, lw = g.Nz + 1, lu = g.Nz + 2;
+  if (vel_edge_u(g, k, u, j)) return vel_edge_row_u<T>(g, k, xu, u, j, dg);
   const int il = (i == 0) ? Nx - 1 : i - 1, ir = (i == Nx) ? 1 : i + 1;
   const RowW<T> c = u_row<T>(g, op, u, j, i);
   *dg = c.d;
-  const T* pu = xu + u;                          // U(j, i)
-  const T* pw = xw + (i * lw + j - 1);           // W(j-1, i)
-  T s = c.d * pu[0];
-  s += c.c1 * xu[il * lu + j];
-  s += c.c2 * xu[ir * lu + j];
-  s += c.c3 * pu[-1];
-  s += c.c4 * pu[1];
-  s += c.c5 * pw[0];
-  s += c.c6 * pw[lw];
-  s += c.c7 * pw[1];
-  s += c.c8 * pw[lw + 1];
+  T s = vel_dot_u<T>(c, xu + u, xu + (il * lu + j), xu + (ir * lu + j), xw + (i * lw + j - 1), lw);
   if (FULL) {
     const T* pp = xp + (i * lu + j);
     s += geo_invh<T>(g) * (pp[lu] - pp[0]);
@@ -495,7 +535,7 @@ __global__ void p_coef_kernel(Geo g, const double* __restrict__ rhow, const doub
 
 // y = S o (LL (S o v)) on the whole unknown vector; t must hold S o v.
 // If b != null: y = b - S o (LL t).  Thread (j, i) of the 2-D grid takes the
-// W, U and P rows at (j, i).
+// W, U and P rows at (j, i), or (three layers, z: small grids) one of them.
 template <typename T>
 __global__ void __launch_bounds__(256) stokes_apply_kernel(Geo g, OpConst k, VOp<T> op, const T* __restrict__ cp,
                                                            const T* __restrict__ scl, const T* __restrict__ tv,
@@ -509,17 +549,18 @@ __global__ void __launch_bounds__(256) stokes_apply_kernel(Geo g, OpConst k, VOp
   const T* xu = tv + g.NW;
   const T* xp = tv + g.NW + g.NU;
   T d;
-  if (j <= Nz) {
+  const int layer = gridDim.z == 1 ? -1 : (int)blockIdx.z;
+  if (j <= Nz && (layer < 0 || layer == 0)) {
     const long long t = (long long)i * (Nz + 1) + j;
     const T v = vel_row_w<T, true>(g, k, op, xw, xu, xp, t, j, i, &d) * scl[t];
     y[t] = b ? b[t] - v : v;
   }
-  if (i <= Nx) {
+  if (i <= Nx && (layer < 0 || layer == 1)) {
     const long long u = (long long)i * (Nz + 2) + j, t = g.NW + u;
     const T v = vel_row_u<T, true>(g, k, op, xw, xu, xp, u, j, i, &d) * scl[t];
     y[t] = b ? b[t] - v : v;
   }
-  {
+  if (layer < 0 || layer == 2) {
     const int pt = i * (Nz + 2) + j;
     const long long t = (long long)g.NW + g.NU + pt;
     const T v = p_row<T>(g, k, cp, xw, xu, xp, pt, j, i) * scl[t];
@@ -563,35 +604,76 @@ __global__ void refine_update_kernel(long long n, const T* __restrict__ dy, cons
 // or of the residual (MODE 2): out = xi + w D^-1 (b - A xi), resp. b - A xi;
 // ghost / boundary rows are relaxed exactly (w = 1)
 template <typename T, int MODE>
+__device__ __forceinline__ void vel_put(const T* xi, const T* b, T* out, T w, int t, T ax, T d, const T* dscl) {
+  if (MODE == 0) out[t] = sdiv<T>(w * b[t], d);
+  else if (MODE == 2) out[t] = b[t] - ax;
+  else if (MODE == 3) out[t] = (xi[t] + sdiv<T>(w * (b[t] - ax), d)) / dscl[t];
+  else out[t] = xi[t] + sdiv<T>(w * (b[t] - ax), d);
+}
+template <typename T, int MODE>
+__device__ __forceinline__ void vel_update_int_w(const Geo& g, const VOp<T>& op, const T* xi, const T* b, T* out,
+                                                 T omega, int t, int j, int i, const T* dscl = nullptr) {
+  const int lw = g.Nz + 1, lu = g.Nz + 2;
+  const RowW<T> c = w_row<T>(g, op, t, j, i);
+  const T ax = MODE == 0 ? (T)0 : vel_dot_w<T>(c, xi + t, xi + (g.NW + (i - 1) * lu + j), lw, lu);
+  vel_put<T, MODE>(xi, b, out, omega, t, ax, c.d, dscl);
+}
+template <typename T, int MODE>
+__device__ __forceinline__ void vel_update_int_u(const Geo& g, const VOp<T>& op, const T* xi, const T* b, T* out,
+                                                 T omega, int u, int j, int i, const T* dscl = nullptr) {
+  const int lw = g.Nz + 1, lu = g.Nz + 2;
+  const RowW<T> c = u_row<T>(g, op, u, j, i);
+  const T* xu = xi + g.NW;
+  const int il = (i == 0) ? g.Nx - 1 : i - 1, ir = (i == g.Nx) ? 1 : i + 1;
+  const T ax =
+      MODE == 0 ? (T)0 : vel_dot_u<T>(c, xu + u, xu + (il * lu + j), xu + (ir * lu + j), xi + (i * lw + j - 1), lw);
+  vel_put<T, MODE>(xi, b, out, omega, g.NW + u, ax, c.d, dscl);
+}
+template <typename T, int MODE>
+__device__ __forceinline__ void vel_update_edge_w(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xi,
+                                                  const T* b, T* out, int t, int j, int i, const T* dscl = nullptr) {
+  T d, ax = 0;
+  if (MODE == 0) d = vel_diag_w<T>(g, op, t, j, i);
+  else ax = vel_edge_row_w<T>(g, k, op, xi, xi + g.NW, t, j, i, &d);
+  vel_put<T, MODE>(xi, b, out, (T)1, t, ax, d, dscl);
+}
+template <typename T, int MODE>
+__device__ __forceinline__ void vel_update_edge_u(const Geo& g, const OpConst& k, const T* xi, const T* b, T* out,
+                                                  int u, int j, const T* dscl = nullptr) {
+  T d = 1, ax = 0;
+  if (MODE != 0) ax = vel_edge_row_u<T>(g, k, xi + g.NW, u, j, &d);
+  vel_put<T, MODE>(xi, b, out, (T)1, g.NW + u, ax, d, dscl);
+}
+template <typename T, int MODE>
 __device__ __forceinline__ void vel_update_w(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xi,
                                              const T* b, T* out, T omega, long long t, int j, int i,
                                              const T* dscl = nullptr) {
-  const bool exact = i == 0 || i == g.Nx + 1 || j == 0 || j == g.Nz;
-  if (MODE == 0) {
-    out[t] = sdiv<T>((exact ? (T)1 : omega) * b[t], vel_diag_w<T>(g, op, t, j, i));
-    return;
-  }
-  T d;
-  const T ax = vel_row_w<T, false>(g, k, op, xi, xi + g.NW, nullptr, t, j, i, &d);
-  if (MODE == 2) out[t] = b[t] - ax;
-  else if (MODE == 3) out[t] = (xi[t] + sdiv<T>((exact ? (T)1 : omega) * (b[t] - ax), d)) / dscl[t];
-  else out[t] = xi[t] + sdiv<T>((exact ? (T)1 : omega) * (b[t] - ax), d);
+  if (vel_edge_w(g, j, i)) vel_update_edge_w<T, MODE>(g, k, op, xi, b, out, (int)t, j, i, dscl);
+  else vel_update_int_w<T, MODE>(g, op, xi, b, out, omega, (int)t, j, i, dscl);
 }
 template <typename T, int MODE>
 __device__ __forceinline__ void vel_update_u(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xi,
                                              const T* b, T* out, T omega, long long u, int j, int i,
                                              const T* dscl = nullptr) {
-  const bool exact = j == 0 || j == g.Nz + 1 || (k.mms && (int)u == k.pin_u);
-  const long long t = g.NW + u;
-  if (MODE == 0) {
-    out[t] = sdiv<T>((exact ? (T)1 : omega) * b[t], vel_diag_u<T>(g, k, op, u, j, i));
-    return;
+  if (vel_edge_u(g, k, u, j)) vel_update_edge_u<T, MODE>(g, k, xi, b, out, (int)u, j, dscl);
+  else vel_update_int_u<T, MODE>(g, op, xi, b, out, omega, (int)u, j, i, dscl);
+}
+// rows of a level in three runs -- interior W, interior U, edges -- so that the
+// lanes of a warp take the same way: row r of run q, in 0 .. count - 1
+__device__ __forceinline__ int vel_edge_count(const Geo& g) { return 2 * (g.Nz + 1) + 4 * g.Nx + 2; }
+template <typename T, int MODE>
+__device__ __forceinline__ void vel_update_edge(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xi,
+                                                const T* b, T* out, int e, const T* dscl = nullptr) {
+  const int Nz = g.Nz, Nx = g.Nx, lw = Nz + 1, nw = 2 * lw + 2 * Nx;
+  if (e < nw) {
+    int j, i;
+    if (e < 2 * lw) { i = e < lw ? 0 : Nx + 1; j = e < lw ? e : e - lw; }
+    else { const int q = e - 2 * lw; j = q < Nx ? 0 : Nz; i = 1 + (q < Nx ? q : q - Nx); }
+    vel_update_edge_w<T, MODE>(g, k, op, xi, b, out, i * lw + j, j, i, dscl);
+  } else {
+    const int q = e - nw, j = q <= Nx ? 0 : Nz + 1, i = q <= Nx ? q : q - Nx - 1;
+    vel_update_edge_u<T, MODE>(g, k, xi, b, out, i * (Nz + 2) + j, j, dscl);
   }
-  T d;
-  const T ax = vel_row_u<T, false>(g, k, op, xi, xi + g.NW, nullptr, u, j, i, &d);
-  if (MODE == 2) out[t] = b[t] - ax;
-  else if (MODE == 3) out[t] = (xi[t] + sdiv<T>((exact ? (T)1 : omega) * (b[t] - ax), d)) / dscl[t];
-  else out[t] = xi[t] + sdiv<T>((exact ? (T)1 : omega) * (b[t] - ax), d);
 }
 // a level's rows on a 2-D grid: thread (j, i) takes W row (j, i) and U row
 // (j, i) -- no index division, and the two rows share viscosity loads.
@@ -608,6 +690,35 @@ __global__ void __launch_bounds__(256) vel_sweep2d_kernel(Geo g, OpConst k, VOp<
     vel_update_w<T, MODE>(g, k, op, xi, b, out, omega, (long long)i * (g.Nz + 1) + j, j, i, dscl);
   if (j <= g.Nz + 1 && i <= g.Nx)
     vel_update_u<T, MODE>(g, k, op, xi, b, out, omega, (long long)i * (g.Nz + 2) + j, j, i, dscl);
+}
+
+// The same on a small level, whose launch lasts as long as one thread's chain of
+// instructions: a row per thread, z = 0 the interior W rows, 1 the interior U
+// rows, 2 the ghost and boundary rows, which a warp of vel_sweep2d_kernel takes
+// one after the other.  grid2 blocks.  A
+// sweep at 64^2 takes 1.7 us against 2.6 us.  Up to 128^2 cells (kSplitCells): with
+// the line at 512^2 the 512^2 solve measured the same and the 1024^2 step 2.5 %
+// slower, without this kernel 3 to 6 % slower.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256) vel_sweep_split_kernel(Geo g, OpConst k, VOp<T> op, const T* __restrict__ xi,
+                                                              const T* __restrict__ b, T* out, T omega,
+                                                              const T* __restrict__ dscl) {
+  XC_PDL_WAIT();
+  const int j = blockIdx.x * 32 + threadIdx.x + 1, i = blockIdx.y * 8 + threadIdx.y;
+  if (blockIdx.z == 0) {
+    if (j < g.Nz && i >= 1 && i <= g.Nx)
+      vel_update_int_w<T, MODE>(g, op, xi, b, out, omega, i * (g.Nz + 1) + j, j, i, dscl);
+  } else if (blockIdx.z == 1) {
+    const int u = i * (g.Nz + 2) + j;
+    if (j <= g.Nz && i <= g.Nx) {
+      if (vel_edge_u(g, k, u, j)) vel_update_edge_u<T, MODE>(g, k, xi, b, out, u, j, dscl);
+      else vel_update_int_u<T, MODE>(g, op, xi, b, out, omega, u, j, i, dscl);
+    }
+  } else {
+    const int n = vel_edge_count(g), step = gridDim.x * gridDim.y * 256;
+    for (int e = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.y * 32 + threadIdx.x; e < n; e += step)
+      vel_update_edge<T, MODE>(g, k, op, xi, b, out, e, dscl);
+  }
 }
 
 
@@ -680,15 +791,7 @@ __global__ void __launch_bounds__(256) vel_sweep_rb_kernel(Geo g, OpConst k, VOp
         out[t] = sdiv<float>(omega * b[t], c.d);
         continue;
       }
-      float sum = c.d * pw[r];
-      sum += c.c1 * pw[r - 1];
-      sum += c.c2 * pw[r + 1];
-      sum += c.c3 * pw[r - lw];
-      sum += c.c4 * pw[r + lw];
-      sum += c.c5 * pu[r];
-      sum += c.c6 * pu[r + 1];
-      sum += c.c7 * pu[r + lu];
-      sum += c.c8 * pu[r + lu + 1];
+      const float sum = vel_dot_w<float>(c, pw + r, pu + r, lw, lu);
       rb_store<MODE>(out, t, pw[r], b[t], sum, c.d, omega, dscl);
     }
   }
@@ -706,15 +809,7 @@ __global__ void __launch_bounds__(256) vel_sweep_rb_kernel(Geo g, OpConst k, VOp
         out[g.NW + u] = sdiv<float>(omega * b[g.NW + u], c.d);
         continue;
       }
-      float sum = c.d * pu[r];
-      sum += c.c1 * pu[r - lu];
-      sum += c.c2 * pu[r + lu];
-      sum += c.c3 * pu[r - 1];
-      sum += c.c4 * pu[r + 1];
-      sum += c.c5 * pw[r];
-      sum += c.c6 * pw[r + lw];
-      sum += c.c7 * pw[r + 1];
-      sum += c.c8 * pw[r + lw + 1];
+      const float sum = vel_dot_u<float>(c, pu + r, pu + r - lu, pu + r + lu, pw + r, lw);
       rb_store<MODE>(out, g.NW + u, pu[r], b[g.NW + u], sum, c.d, omega, dscl);
     }
   }
@@ -784,16 +879,7 @@ __global__ void __launch_bounds__(kTJ * kTI) vel_sweep_tiled_kernel(Geo g, OpCon
     } else {
       const RowW<float> w = fly_row<float>(sC[a - 1][c], sC[a][c], sE[a - 1][c - 1], sE[a - 1][c], op.dw[t], ih2);
       d = w.d;
-      float s = w.d * sW[a][c];
-      s += w.c1 * sW[a][c - 1];
-      s += w.c2 * sW[a][c + 1];
-      s += w.c3 * sW[a - 1][c];
-      s += w.c4 * sW[a + 1][c];
-      s += w.c5 * sU[a - 1][c];
-      s += w.c6 * sU[a - 1][c + 1];
-      s += w.c7 * sU[a][c];
-      s += w.c8 * sU[a][c + 1];
-      ax = s;
+      ax = vel_dot_w<float>(w, &sW[a][c], &sU[a - 1][c], kTJ + 2, kTJ + 2);
     }
     sweep_store<MODE>(out, t, sW[a][c], b[t], ax, d, exact, omega, dscl);
   }
@@ -807,16 +893,7 @@ __global__ void __launch_bounds__(kTJ * kTI) vel_sweep_tiled_kernel(Geo g, OpCon
     else {
       const RowW<float> w = fly_row<float>(sC[a][c - 1], sC[a][c], sE[a - 1][c - 1], sE[a][c - 1], op.du[u], ih2);
       d = w.d;
-      float s = w.d * sU[a][c];
-      s += w.c1 * sU[a - 1][c];
-      s += w.c2 * sU[a + 1][c];
-      s += w.c3 * sU[a][c - 1];
-      s += w.c4 * sU[a][c + 1];
-      s += w.c5 * sW[a][c - 1];
-      s += w.c6 * sW[a + 1][c - 1];
-      s += w.c7 * sW[a][c];
-      s += w.c8 * sW[a + 1][c];
-      ax = s;
+      ax = vel_dot_u<float>(w, &sU[a][c], &sU[a - 1][c], &sU[a + 1][c], &sW[a][c - 1], kTJ + 2);
     }
     sweep_store<MODE>(out, t, sU[a][c], b[t], ax, d, exact, omega, dscl);
   }
@@ -855,46 +932,42 @@ __device__ __forceinline__ void vel_residual_at(const Geo& g, const OpConst& k, 
 // (J, Ic) and U row (Jr, I) of the coarse level.
 template <typename T>
 __device__ __forceinline__ T vel_restrict_w(const Geo& f, const Geo& c, const T* rw, int J, int Ic) {
+  if (J < 1 || J >= c.Nz || Ic < 1 || Ic > c.Nx) return (T)0;
   const int lwf = f.Nz + 1;
+  // columns 2 Ic - 2 .. 2 Ic + 1, the outer two across the periodic boundary
+  const T* col[4];
+  const T* base = rw + 2 * J;
+  col[0] = base + (Ic == 1 ? f.Nx : 2 * Ic - 2) * lwf;
+  col[1] = base + (2 * Ic - 1) * lwf;
+  col[2] = base + 2 * Ic * lwf;
+  col[3] = base + (Ic == c.Nx ? 1 : 2 * Ic + 1) * lwf;
   T acc = 0;
-  if (J >= 1 && J <= c.Nz - 1 && Ic >= 1 && Ic <= c.Nx) {
-    const int I = Ic - 1;
-    const int ixs[4] = {2 * I - 1, 2 * I, 2 * I + 1, 2 * I + 2};
-    const T wx[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
-    for (int dj = -1; dj <= 1; ++dj) {
-      const T wz = dj == 0 ? (T)1 : (T)0.5;
-      const int j = 2 * J + dj;
-      for (int q = 0; q < 4; ++q) {
-        int ix = ixs[q];
-        ix = ix < 0 ? ix + f.Nx : (ix >= f.Nx ? ix - f.Nx : ix);
-        acc += wz * wx[q] * rw[(ix + 1) * lwf + j];
-      }
-    }
-    acc *= (T)0.25;
+#pragma unroll
+  for (int dj = -1; dj <= 1; ++dj) {
+    const T wz = dj == 0 ? (T)1 : (T)0.5;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc = fma_rn<T>(wz * ((q == 0 || q == 3) ? (T)0.25 : (T)0.75), col[q][dj], acc);
   }
-  return acc;
+  return acc * (T)0.25;
 }
 template <typename T>
 __device__ __forceinline__ T vel_restrict_u(const Geo& f, const Geo& c, const T* ru, int Jr, int I) {
+  if (Jr < 1 || Jr > c.Nz) return (T)0;
   const int luf = f.Nz + 2;
+  // rows 2 Jr - 2 .. 2 Jr + 1 inside 1 .. Nz, columns 2 I - 1 .. 2 I + 1 inside 0 .. Nx
+  const T* base = ru + (2 * I * luf + 2 * Jr - 2);
+  const bool lo = Jr > 1, hi = 2 * Jr < f.Nz, left = I > 0, right = 2 * I < f.Nx;
   T acc = 0;
-  if (Jr >= 1 && Jr <= c.Nz) {
-    const int Jc = Jr - 1;
-    const int jzs[4] = {2 * Jc - 1, 2 * Jc, 2 * Jc + 1, 2 * Jc + 2};
-    const T wz[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
-    for (int q = 0; q < 4; ++q) {
-      const int jz = jzs[q];
-      if (jz < 0 || jz >= f.Nz) continue;
-      for (int di = -1; di <= 1; ++di) {
-        const int i = 2 * I + di;
-        if (i < 0 || i > f.Nx) continue;
-        const T wx = di == 0 ? (T)1 : (T)0.5;
-        acc += wz[q] * wx * ru[i * luf + jz + 1];
-      }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const T wz = (q == 0 || q == 3) ? (T)0.25 : (T)0.75;
+#pragma unroll
+    for (int di = -1; di <= 1; ++di) {
+      const bool in = (q != 0 || lo) && (q != 3 || hi) && (di >= 0 || left) && (di <= 0 || right);
+      if (in) acc = fma_rn<T>(wz * (di == 0 ? (T)1 : (T)0.5), base[di * luf + q], acc);
     }
-    acc *= (T)0.25;
   }
-  return acc;
+  return acc * (T)0.25;
 }
 // flat index over the coarse W then U rows (levels stay below 2^31 unknowns)
 template <typename T>
@@ -907,53 +980,60 @@ __device__ __forceinline__ void vel_restrict_at(const Geo& f, const Geo& c, cons
     bc[t] = vel_restrict_u<T>(f, c, r + f.NW, u % (c.Nz + 2), u / (c.Nz + 2));
   }
 }
-// 2-D grid over the coarse row positions (grid2 of the coarse level)
+// 2-D grid over the coarse row positions (grid2 of the coarse level), in one or
+// two layers as vel_prolong2d_kernel's.  x0 (may be null): the coarse level's
+// first sweep from zero, which is pointwise, made along (operations of
+// vel_update_w / vel_update_u, MODE 0)
 template <typename T>
-__global__ void __launch_bounds__(256) vel_restrict2d_kernel(Geo f, Geo c, const T* __restrict__ r, T* bc) {
+__global__ void __launch_bounds__(256) vel_restrict2d_kernel(Geo f, Geo c, const T* __restrict__ r, T* bc, OpConst kc,
+                                                             VOp<T> opc, T omega, T* x0) {
   XC_PDL_WAIT();
   const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
-  if (j <= c.Nz && i <= c.Nx + 1) bc[i * (c.Nz + 1) + j] = vel_restrict_w<T>(f, c, r, j, i);
-  if (j <= c.Nz + 1 && i <= c.Nx) bc[c.NW + i * (c.Nz + 2) + j] = vel_restrict_u<T>(f, c, r + f.NW, j, i);
+  const bool w = gridDim.z == 1 || blockIdx.z == 0, u = gridDim.z == 1 || blockIdx.z == 1;
+  if (w && j <= c.Nz && i <= c.Nx + 1) {
+    const int t = i * (c.Nz + 1) + j;
+    const T v = vel_restrict_w<T>(f, c, r, j, i);
+    bc[t] = v;
+    if (x0) x0[t] = sdiv<T>((vel_edge_w(c, j, i) ? (T)1 : omega) * v, vel_diag_w<T>(c, opc, t, j, i));
+  }
+  if (u && j <= c.Nz + 1 && i <= c.Nx) {
+    const int q = i * (c.Nz + 2) + j;
+    const T v = vel_restrict_u<T>(f, c, r + f.NW, j, i);
+    bc[c.NW + q] = v;
+    if (x0) x0[c.NW + q] = sdiv<T>((vel_edge_u(c, kc, q, j) ? (T)1 : omega) * v, vel_diag_u<T>(c, kc, opc, q, j, i));
+  }
 }
 
 // x_f += P x_c (bilinear; ghost rows of U follow the reflection rule): the
 // correction of fine W row (j, i) and fine U row (j, i)
+// (no branch on the parity along z, which differs between the lanes of a warp,
+// and no index division)
 template <typename T>
 __device__ __forceinline__ T vel_prolong_w(const Geo& f, const Geo& c, const T* cw, int j, int i) {
   const int lwc = c.Nz + 1;
-  int ix = (i - 1) % f.Nx;
-  if (ix < 0) ix += f.Nx;
-  const int I0 = ix / 2;
-  const int In = (ix % 2 == 0) ? (I0 - 1 + c.Nx) % c.Nx : (I0 + 1) % c.Nx;
-  T v = 0;
-  const int J0 = j / 2;
-  const int nz = (j % 2 == 0) ? 1 : 2;
-  for (int q = 0; q < nz; ++q) {
-    const int J = J0 + q;
-    const T wz = nz == 1 ? (T)1 : (T)0.5;
-    v += wz * ((T)0.75 * cw[(I0 + 1) * lwc + J] + (T)0.25 * cw[(In + 1) * lwc + J]);
-  }
-  return v;
+  const int ix = i == 0 ? f.Nx - 1 : (i > f.Nx ? i - 1 - f.Nx : i - 1);
+  const int I0 = ix >> 1;
+  const int In = (ix & 1) ? (I0 + 1 == c.Nx ? 0 : I0 + 1) : (I0 == 0 ? c.Nx - 1 : I0 - 1);
+  const T* p = cw + (I0 + 1) * lwc;
+  const T* n = cw + (In + 1) * lwc;
+  const int J0 = j >> 1, odd = j & 1, J1 = J0 + odd;
+  const T m0 = fma_rn<T>((T)0.75, p[J0], mul_rn<T>((T)0.25, n[J0]));
+  const T m1 = fma_rn<T>((T)0.75, p[J1], mul_rn<T>((T)0.25, n[J1]));
+  return odd ? fma_rn<T>((T)0.5, m1, mul_rn<T>((T)0.5, m0)) : m0;
 }
 template <typename T>
 __device__ __forceinline__ T vel_prolong_u(const Geo& f, const Geo& c, const OpConst& k, const T* cu, int j, int i) {
   const int luc = c.Nz + 2;
-  auto interior = [&](int jj) -> T {
-    const int jz = jj - 1, J0 = jz / 2;
-    const int Jn = (jz % 2 == 0) ? J0 : J0 + 2;     // coarse row of the 1/4 neighbour (full layout)
-    T v = 0;
-    const int nx = (i % 2 == 0) ? 1 : 2;
-    const int I0 = (i % 2 == 0) ? i / 2 : (i - 1) / 2;
-    for (int q = 0; q < nx; ++q) {
-      const T wx = nx == 1 ? (T)1 : (T)0.5;
-      const int I = I0 + q;
-      v += wx * ((T)0.75 * cu[I * luc + J0 + 1] + (T)0.25 * cu[I * luc + Jn]);
-    }
-    return v;
-  };
-  if (j == 0) return -(T)k.top_cnv * interior(1);
-  if (j == f.Nz + 1) return -(T)k.bot_cnv * interior(f.Nz);
-  return interior(j);
+  const int jj = j == 0 ? 1 : (j > f.Nz ? f.Nz : j);
+  const int jz = jj - 1, J0 = jz >> 1;
+  const int Jn = (jz & 1) ? J0 + 2 : J0;            // coarse row of the 1/4 neighbour (full layout)
+  const int odd = i & 1;
+  const T* p = cu + (i >> 1) * luc;
+  const T* q = p + odd * luc;
+  const T m0 = fma_rn<T>((T)0.75, p[J0 + 1], mul_rn<T>((T)0.25, p[Jn]));
+  const T m1 = fma_rn<T>((T)0.75, q[J0 + 1], mul_rn<T>((T)0.25, q[Jn]));
+  const T v = odd ? fma_rn<T>((T)0.5, m1, mul_rn<T>((T)0.5, m0)) : m0;
+  return j == 0 ? mul_rn<T>(-(T)k.top_cnv, v) : (j > f.Nz ? mul_rn<T>(-(T)k.bot_cnv, v) : v);
 }
 template <typename T>
 __device__ __forceinline__ void vel_prolong_at(const Geo& f, const Geo& c, const OpConst& k, const T* xc, T* xf,
@@ -966,14 +1046,16 @@ __device__ __forceinline__ void vel_prolong_at(const Geo& f, const Geo& c, const
     xf[t] += vel_prolong_u<T>(f, c, k, xc + c.NW, u % (f.Nz + 2), u / (f.Nz + 2));
   }
 }
-// 2-D grid over the fine row positions (grid2 of the fine level)
+// 2-D grid over the fine row positions (grid2 of the fine level); two layers of
+// it (z) have the W and the U rows apart, for the same reason as above
 template <typename T>
 __global__ void __launch_bounds__(256) vel_prolong2d_kernel(Geo f, Geo c, OpConst k, const T* __restrict__ xc,
                                                             T* xf) {
   XC_PDL_WAIT();
   const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
-  if (j <= f.Nz && i <= f.Nx + 1) xf[i * (f.Nz + 1) + j] += vel_prolong_w<T>(f, c, xc, j, i);
-  if (j <= f.Nz + 1 && i <= f.Nx) xf[f.NW + i * (f.Nz + 2) + j] += vel_prolong_u<T>(f, c, k, xc + c.NW, j, i);
+  const bool w = gridDim.z == 1 || blockIdx.z == 0, u = gridDim.z == 1 || blockIdx.z == 1;
+  if (w && j <= f.Nz && i <= f.Nx + 1) xf[i * (f.Nz + 1) + j] += vel_prolong_w<T>(f, c, xc, j, i);
+  if (u && j <= f.Nz + 1 && i <= f.Nx) xf[f.NW + i * (f.Nz + 2) + j] += vel_prolong_u<T>(f, c, k, xc + c.NW, j, i);
 }
 
 // coarse coefficient fields: eta (avg4), etaco (injection), rho (avg4),
@@ -1118,11 +1200,26 @@ __device__ void gj_invert_cta(R* M, int n, int* piv, int* ok, R* fcol, double* r
 template <typename T>
 __device__ void dense_apply_cta(const T* __restrict__ inv, int n, const T* b, T* x) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int r = warp; r < n; r += nw) {
-    T acc = 0;
-    for (int c = lane; c < n; c += 32) acc += inv[r * n + c] * b[c];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) x[r] = acc;
+  static_assert(kDenseMax <= 64, "two columns a lane");
+  const bool c0 = lane < n, c1 = lane + 32 < n;
+  const T b0 = c0 ? b[lane] : (T)0, b1 = c1 ? b[lane + 32] : (T)0;
+  for (int r0 = warp; r0 < n; r0 += 4 * nw) {      // four rows of a warp in flight
+    T acc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 + q * nw;
+      acc[q] = 0;
+      if (r < n) {
+        const T* a = inv + r * n + lane;
+        if (c0) acc[q] = mul_rn<T>(a[0], b0);
+        if (c1) acc[q] = fma_rn<T>(a[32], b1, acc[q]);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = add_rn<T>(acc[q], __shfl_xor_sync(0xffffffffu, acc[q], o));
+    if (lane < 4 && r0 + lane * nw < n) x[r0 + lane * nw] = lane == 0 ? acc[0] : (lane == 1 ? acc[1] : (lane == 2 ? acc[2] : acc[3]));
   }
   __syncthreads();
 }
@@ -1365,15 +1462,137 @@ __global__ void __launch_bounds__(1024) wide_check_kernel(int n, const T* __rest
   if (threadIdx.x == 0) *ok = all && !*bad && !null_mode ? 1 : 0;
 }
 
+// e / rows by a multiplication, for e * rows < 2^32
+inline unsigned stage_div(int rows) { return rows == 1 ? 0u : (unsigned)((1ull << 32) / (unsigned)rows) + 1u; }
+__device__ __forceinline__ int stage_col(int e, unsigned dv) { return dv ? (int)__umulhi((unsigned)e, dv) : e; }
+// a row of a level in registers; the rows are numbered with interior W, interior
+// U and edges in runs of whole warps, so that a warp's lanes take the same way
+template <typename T>
+struct VelRow {
+  int kind;                          // 0 none, 1 interior W, 2 interior U, 3 edge, 4 open bottom
+  int t, o1, o2, o3;                 // index of the row and of the unknowns its weights apply to
+  RowW<T> c;                         // (an edge: its diagonal and the weight of o1)
+  T w;                               // relaxation
+};
+__host__ __device__ __forceinline__ int vel_stage_rows(const Geo& g) {
+  const int nw = ((g.Nz - 1) * g.Nx + 31) & ~31, nu = (g.Nz * (g.Nx + 1) + 31) & ~31;
+  return nw + nu + 2 * (g.Nz + 1) + 4 * g.Nx + 2;
+}
+template <typename T>
+__device__ __forceinline__ VelRow<T> vel_stage_row(const Geo& g, const OpConst& k, const VOp<T>& op, T om, int r,
+                                                   unsigned dvw, unsigned dvu) {
+  const int Nz = g.Nz, Nx = g.Nx, lw = Nz + 1, lu = Nz + 2;
+  const int nw = (Nz - 1) * Nx, u0 = (nw + 31) & ~31, nu = Nz * (Nx + 1), e0 = (u0 + nu + 31) & ~31;
+  VelRow<T> v;
+  v.kind = 0; v.t = 0; v.o1 = v.o2 = v.o3 = 0; v.w = om;
+  v.c.d = (T)1; v.c.c1 = (T)0;
+  if (r < u0) {
+    if (r < nw) {
+      const int c = stage_col(r, dvw), i = c + 1, j = r - c * (Nz - 1) + 1;
+      v.kind = 1;
+      v.t = i * lw + j;
+      v.o1 = g.NW + (i - 1) * lu + j;
+      v.c = w_row<T>(g, op, v.t, j, i);
+    }
+  } else if (r < e0) {
+    r -= u0;
+    if (r < nu) {
+      const int i = stage_col(r, dvu), j = r - i * Nz + 1, u = i * lu + j;
+      v.t = g.NW + u;
+      v.o1 = g.NW + (i == 0 ? Nx - 1 : i - 1) * lu + j;
+      v.o2 = g.NW + (i == Nx ? 1 : i + 1) * lu + j;
+      v.o3 = i * lw + j - 1;
+      if (vel_edge_u(g, k, u, j)) {
+        v.kind = 3;
+        v.w = (T)1;
+      } else {
+        v.kind = 2;
+        v.c = u_row<T>(g, op, u, j, i);
+      }
+    }
+  } else if (r - e0 < vel_edge_count(g)) {
+    r -= e0;
+    v.kind = 3;
+    v.w = (T)1;
+    if (r < 2 * lw) {                // ghost columns of W
+      const int j = r < lw ? r : r - lw, i = r < lw ? 0 : Nx + 1;
+      v.t = i * lw + j;
+      v.o1 = (r < lw ? Nx : 1) * lw + j;
+      v.c.c1 = (T)k.sds;
+    } else if ((r -= 2 * lw) < 2 * Nx) {
+      const bool top = r < Nx;
+      const int i = 1 + (top ? r : r - Nx), j = top ? 0 : Nz;
+      v.t = i * lw + j;
+      v.c.d = vel_diag_w<T>(g, op, v.t, j, i);
+      if (!top && k.open_cnv) {
+        v.kind = 4;
+        v.o1 = j;
+        v.o2 = i;
+      }
+    } else {                         // ghost rows of U
+      r -= 2 * Nx;
+      const bool top = r <= Nx;
+      const int i = top ? r : r - Nx - 1, j = top ? 0 : Nz + 1;
+      v.t = g.NW + i * lu + j;
+      v.o1 = v.t + (top ? 1 : -1);
+      v.c.c1 = (T)(top ? k.top_cnv : k.bot_cnv);
+    }
+  }
+  return v;
+}
+template <typename T>
+__device__ __forceinline__ T vel_stage_apply(const Geo& g, const OpConst& k, const VOp<T>& op, const VelRow<T>& v,
+                                             const T* x) {
+  if (v.kind == 1) return vel_dot_w<T>(v.c, x + v.t, x + v.o1, g.Nz + 1, g.Nz + 2);
+  if (v.kind == 2) return vel_dot_u<T>(v.c, x + v.t, x + v.o1, x + v.o2, x + v.o3, g.Nz + 1);
+  if (v.kind == 3) return fma_rn<T>(v.c.c1, x[v.o1], mul_rn<T>(v.c.d, x[v.t]));
+  T d;
+  return vel_edge_row_w<T>(g, k, op, x, x + g.NW, v.t, v.o1, v.o2, &d);
+}
+template <typename T>
+__device__ __forceinline__ T vel_stage_relax(const VelRow<T>& v, T x, T b, T ax) {
+  return x + rdiv<T>(v.w * (b - ax), v.c.d);
+}
+
+// `sweeps` damped-Jacobi sweeps from x (in place of the calls of vel_jacobi_at,
+// whose operations these are) with R rows a thread: weights, right-hand sides
+// and addresses stay in registers, and from shared memory (x, x2) a row of a
+// sweep is nine loads, the sum and the quotient.  A 25 x 25 level's 200 sweeps
+// took 323 us with the weights formed anew in every sweep and x in global
+// memory, and take 106 us (pressure, p_sweeps_reg: 116 and 29).
+template <typename T, int R>
+__device__ __forceinline__ void vel_sweeps_reg(const Geo& g, const OpConst& k, const VOp<T>& op, T* x, T* x2,
+                                               const T* b, int sweeps, T omega, unsigned dvw, unsigned dvu) {
+  VelRow<T> v[R];
+  T bt[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    v[q] = vel_stage_row<T>(g, k, op, omega, threadIdx.x + q * blockDim.x, dvw, dvu);
+    bt[q] = v[q].kind ? b[v[q].t] : (T)0;
+  }
+  T* a = x;
+  T* o = x2;
+  for (int s = 0; s < sweeps; ++s) {
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+      if (v[q].kind) o[v[q].t] = vel_stage_relax<T>(v[q], a[v[q].t], bt[q], vel_stage_apply<T>(g, k, op, v[q], a));
+    __syncthreads();
+    T* tmp = a; a = o; o = tmp;
+  }
+}
+
 // many damped-Jacobi sweeps on the coarsest velocity level, by one whole CTA.
 // With free slip at top and bottom (top_cnv = bot_cnv = -1) and periodic x, a
 // uniform U shift is a null mode of the viscous rows; where inertia does not
 // lift it (the inertia-free limit of the manufactured solution) the sweeps
 // would let that mode grow with the sweep count, so it is removed from the
 // coarse correction and left to the pinned fine level and the Krylov method.
-template <typename T>
+// R: rows a thread of sweeps in registers (the caller's CTA has a thread per R
+// rows); 0: any CTA
+template <typename T, int R>
 __device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op, T* x, T* x2, const T* b,
-                               int sweeps, T omega, const T* inv, const int* inv_ok, const WideInverse& wide) {
+                               int sweeps, T omega, const T* inv, const int* inv_ok, const WideInverse& wide,
+                               unsigned dvw = 0, unsigned dvu = 0) {
   const long long n = (long long)g.NW + g.NU;
   if (inv && *inv_ok) {
     dense_apply_cta<T>(inv, (int)n, b, x);
@@ -1400,10 +1619,15 @@ __device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op,
   __syncthreads();
   T* a = x;
   T* o = x2;
-  for (int s = 0; s < sweeps; ++s) {
-    for (long long t = threadIdx.x; t < n; t += blockDim.x) vel_jacobi_at<T>(g, k, op, a, b, o, omega, 0, t);
-    __syncthreads();
-    T* tmp = a; a = o; o = tmp;
+  if constexpr (R > 0) {
+    vel_sweeps_reg<T, R>(g, k, op, x, x2, b, sweeps, omega, dvw, dvu);
+    if (sweeps & 1) a = x2;
+  } else {
+    for (int s = 0; s < sweeps; ++s) {
+      for (long long t = threadIdx.x; t < n; t += blockDim.x) vel_jacobi_at<T>(g, k, op, a, b, o, omega, 0, t);
+      __syncthreads();
+      T* tmp = a; a = o; o = tmp;
+    }
   }
   if (a != x)
     for (long long t = threadIdx.x; t < n; t += blockDim.x) x[t] = a[t];
@@ -1430,11 +1654,29 @@ __device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op,
   }
 }
 template <typename T>
-__global__ void vel_coarse_kernel(Geo g, OpConst k, VOp<T> op, T* x, T* x2, const T* __restrict__ b, int sweeps,
-                                  T omega, const T* inv, const int* inv_ok, WideInverse wide, const int* solved) {
+__global__ void __launch_bounds__(1024) vel_coarse_kernel(Geo g, OpConst k, VOp<T> op, T* x, T* x2,
+                                                          const T* __restrict__ b, int sweeps, T omega, const T* inv,
+                                                          const int* inv_ok, WideInverse wide, const int* solved) {
   XC_PDL_WAIT();
   if (solved && *solved) return;     // by the launches of the wide inverse before this one
-  vel_coarse_cta<T>(g, k, op, x, x2, b, sweeps, omega, inv, inv_ok, wide);
+  vel_coarse_cta<T, 0>(g, k, op, x, x2, b, sweeps, omega, inv, inv_ok, wide);
+}
+// of up to 2 kCoarseRegThreads rows: two a thread (72 registers), the iterates in
+// shared memory, 2 (NW + NU) elements
+constexpr int kCoarseRegThreads = 896;
+template <typename T>
+__global__ void __launch_bounds__(kCoarseRegThreads) vel_coarse_reg_kernel(Geo g, OpConst k, VOp<T> op, T* x,
+                                                                           const T* __restrict__ b, int sweeps,
+                                                                           T omega, const T* inv, const int* inv_ok,
+                                                                           WideInverse wide, const int* solved,
+                                                                           unsigned dvw, unsigned dvu) {
+  XC_PDL_WAIT();
+  if (solved && *solved) return;
+  extern __shared__ __align__(16) unsigned char xc_stage[];
+  const int n = g.NW + g.NU;
+  T* sx = reinterpret_cast<T*>(xc_stage);
+  vel_coarse_cta<T, 2>(g, k, op, sx, sx + n, b, sweeps, omega, inv, inv_ok, wide, dvw, dvu);
+  for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = sx[t];
 }
 
 // the inverse of the coarsest velocity level (NW + NU <= kDenseMax), one CTA
@@ -1572,20 +1814,12 @@ __device__ __forceinline__ void p_restrict_at(int Nzc, int Nxc, const T* r, T* b
   size_t a = (size_t)(2 * I) * Nz + 2 * J, b = (size_t)(2 * I + 1) * Nz + 2 * J;
   bc[t] = (T)0.25 * (r[a] + r[a + 1] + r[b] + r[b + 1]);
 }
-template <typename T>
-__global__ void p_restrict_kernel(int Nzc, int Nxc, const T* __restrict__ r, T* bc) {
-  XC_PDL_WAIT();
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= Nzc * Nxc) return;
-  p_restrict_at<T>(Nzc, Nxc, r, bc, t);
-}
-
 // bilinear prolongation of the coarse correction to fine cell (j, i)
 template <typename T>
 __device__ __forceinline__ T p_prolong_val(int Nzc, int Nxc, const T* xc, int j, int i) {
-  int J = j / 2, I = i / 2;
-  int Jn = (j % 2 == 0) ? (J > 0 ? J - 1 : 0) : (J < Nzc - 1 ? J + 1 : Nzc - 1);
-  int In = (i % 2 == 0) ? (I - 1 + Nxc) % Nxc : (I + 1) % Nxc;
+  const int J = j >> 1, I = i >> 1;
+  const int Jn = (j & 1) ? (J < Nzc - 1 ? J + 1 : J) : (J > 0 ? J - 1 : 0);
+  const int In = (i & 1) ? (I + 1 == Nxc ? 0 : I + 1) : (I == 0 ? Nxc - 1 : I - 1);
   T v = add_rn<T>(add_rn<T>(add_rn<T>(mul_rn<T>((T)9, xc[(size_t)I * Nzc + J]), mul_rn<T>((T)3, xc[(size_t)I * Nzc + Jn])),
                             mul_rn<T>((T)3, xc[(size_t)In * Nzc + J])),
                   xc[(size_t)In * Nzc + Jn]);
@@ -1596,14 +1830,6 @@ __device__ __forceinline__ void p_prolong_at(int Nzc, int Nxc, const T* xc, T* x
   const int Nz = 2 * Nzc;
   xf[t] = add_rn<T>(xf[t], p_prolong_val<T>(Nzc, Nxc, xc, t % Nz, t / Nz));
 }
-template <typename T>
-__global__ void p_prolong_kernel(int Nzc, int Nxc, const T* __restrict__ xc, T* xf) {
-  XC_PDL_WAIT();
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 4 * Nzc * Nxc) return;
-  p_prolong_at<T>(Nzc, Nxc, xc, xf, t);
-}
-
 // Fused descent of one pressure level (one thread per coarse cell): the
 // residual b - L x of its four fine cells, restricted.  zero_init: x is the
 // first Jacobi sweep from zero, formed on the fly at the cells the stencils
@@ -1659,6 +1885,109 @@ __global__ void p_up_kernel(int Nz, int Nx, const T* __restrict__ kx, const T* _
   xo[t] = d > (T)0 ? xv(j, i) + sdiv<T>(omega * (b[t] - ax), d) : (T)0;
 }
 
+// The same two fusions from shared-memory tiles of 32 x 8 cells, the default:
+// each value formed once, by a thread per cell of the tile and its halo (340 of
+// 352), so that a small level's launch is as long as one thread's chain.
+// p_down_tile_kernel also makes the coarse level's first sweep from zero (xc0,
+// with the coarse level's coefficients), which is pointwise; above the finest
+// level x arrives with that sweep done.  At 64^2 a
+// level takes 3.5 us down and up, in place of 7.3 us for five launches.
+// (p_down_kernel / p_up_kernel form every neighbour's value anew, five diagonals
+// per cell, and measured no faster than one launch per operation.)
+constexpr int kFJ = 32, kFI = 8, kTileThreads = 352;
+static_assert((kFJ + 2) * (kFI + 2) <= kTileThreads, "a thread per cell of tile and halo");
+template <typename T>
+struct PCoarse {                       // the coarse level's first sweep; x0 null: none
+  T* x0;
+  const T* kx;
+  const T* kz;
+  int pin;
+  T dpin;
+};
+template <typename T>
+__global__ void __launch_bounds__(kTileThreads) p_down_tile_kernel(int Nz, int Nx, const T* __restrict__ kx,
+                                                                   const T* __restrict__ kz, int pin, T dpin, T* x,
+                                                                   const T* __restrict__ b, T* bc, T omega,
+                                                                   int zero_init, PCoarse<T> C) {
+  XC_PDL_WAIT();
+  constexpr int XJ = kFJ + 2, XI = kFI + 2;
+  __shared__ T xs[XI][XJ], rs[kFI][kFJ];
+  const int j0 = blockIdx.x * kFJ, i0 = blockIdx.y * kFI, tid = threadIdx.x;
+  if (tid < XJ * XI) {
+    const int ci = tid / XJ, cj = tid - ci * XJ, j = j0 - 1 + cj;
+    int i = i0 - 1 + ci;
+    const bool own = cj >= 1 && cj <= kFJ && ci >= 1 && ci <= kFI && i < Nx;
+    i = i < 0 ? i + Nx : (i >= Nx ? i - Nx : i);      // beyond Nx only in front of cells outside the grid
+    if (j >= 0 && j < Nz && i < Nx) {
+      T v;
+      if (zero_init) {
+        v = p_jacobi0_val<T>(Nz, Nx, kx, kz, pin, dpin, b, omega, j, i);
+        if (own) x[i * Nz + j] = v;
+      } else {
+        v = x[i * Nz + j];
+      }
+      xs[ci][cj] = v;
+    }
+  }
+  __syncthreads();
+  if (tid < kFJ * kFI) {
+    const int ci = tid / kFJ, cj = tid - ci * kFJ, j = j0 + cj, i = i0 + ci;
+    if (j < Nz && i < Nx) {
+      T d;
+      // the neighbour beside column 0 or Nx - 1 lies beside it in the tile
+      auto pv = [&](int jj, int ii) -> T {
+        const int c = ii - i;
+        return xs[ci + 1 + (c > 1 ? -1 : (c < -1 ? 1 : c))][jj - j0 + 1];
+      };
+      rs[ci][cj] = b[i * Nz + j] - p_apply_fn<T>(Nz, Nx, kx, kz, pin, dpin, pv, j, i, &d);
+    }
+  }
+  __syncthreads();
+  const int cj = tid & (kFJ / 2 - 1), ci = tid / (kFJ / 2), J = j0 / 2 + cj, I = i0 / 2 + ci, Nzc = Nz / 2, Nxc = Nx / 2;
+  if (tid < kFJ * kFI / 4 && J < Nzc && I < Nxc) {
+    const T v = (T)0.25 * (rs[2 * ci][2 * cj] + rs[2 * ci][2 * cj + 1] + rs[2 * ci + 1][2 * cj] +
+                           rs[2 * ci + 1][2 * cj + 1]);
+    const int t = I * Nzc + J;
+    bc[t] = v;
+    if (C.x0) {                        // p_jacobi0_val's operations
+      T d;
+      p_apply_fn<T>(Nzc, Nxc, C.kx, C.kz, C.pin, C.dpin, [](int, int) { return (T)0; }, J, I, &d);
+      C.x0[t] = d > (T)0 ? sdiv<T>(omega * v, d) : (T)0;
+    }
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTileThreads) p_up_tile_kernel(int Nz, int Nx, const T* __restrict__ kx,
+                                                                 const T* __restrict__ kz, int pin, T dpin,
+                                                                 const T* __restrict__ xc, const T* __restrict__ x,
+                                                                 const T* __restrict__ b, T* xo, T omega) {
+  XC_PDL_WAIT();
+  constexpr int XJ = kFJ + 2, XI = kFI + 2;
+  __shared__ T xs[XI][XJ];
+  const int j0 = blockIdx.x * kFJ, i0 = blockIdx.y * kFI, tid = threadIdx.x, Nzc = Nz / 2, Nxc = Nx / 2;
+  if (tid < XJ * XI) {
+    const int ci = tid / XJ, cj = tid - ci * XJ, j = j0 - 1 + cj;
+    int i = i0 - 1 + ci;
+    i = i < 0 ? i + Nx : (i >= Nx ? i - Nx : i);
+    if (j >= 0 && j < Nz && i < Nx) xs[ci][cj] = add_rn<T>(x[i * Nz + j], p_prolong_val<T>(Nzc, Nxc, xc, j, i));
+  }
+  __syncthreads();
+  if (tid < kFJ * kFI) {
+    const int ci = tid / kFJ, cj = tid - ci * kFJ, j = j0 + cj, i = i0 + ci;
+    if (j < Nz && i < Nx) {
+      T d;
+      auto pv = [&](int jj, int ii) -> T {
+        const int c = ii - i;
+        return xs[ci + 1 + (c > 1 ? -1 : (c < -1 ? 1 : c))][jj - j0 + 1];
+      };
+      const int t = i * Nz + j;
+      const T ax = p_apply_fn<T>(Nz, Nx, kx, kz, pin, dpin, pv, j, i, &d);
+      xo[t] = d > (T)0 ? xs[ci + 1][cj + 1] + sdiv<T>(omega * (b[t] - ax), d) : (T)0;
+    }
+  }
+}
+
 template <typename T>
 __global__ void p_coarsen_kernel(int Nzc, int Nxc, const T* __restrict__ kx, const T* __restrict__ kz,
                                  T* kxc, T* kzc) {
@@ -1671,6 +2000,65 @@ __global__ void p_coarsen_kernel(int Nzc, int Nxc, const T* __restrict__ kx, con
     kxc[(size_t)I * Nzc + J] = (kx[(size_t)(2 * I) * Nz + 2 * J] + kx[(size_t)(2 * I) * Nz + 2 * J + 1]) / (T)8;
   kzc[(size_t)I * (Nzc + 1) + J] = (kz[(size_t)(2 * I) * (Nz + 1) + 2 * J] +
                                     kz[(size_t)(2 * I + 1) * (Nz + 1) + 2 * J]) / (T)8;
+}
+
+// a cell's weights and neighbours in registers
+template <typename T>
+struct PRow {
+  int t, tl, tr;                     // -1: no cell
+  bool top, bot, pinned;
+  T kl, kr, kt, kb, d;
+};
+template <typename T>
+__device__ __forceinline__ T p_row_apply(const PRow<T>& v, T dpin, const T* a) {     // p_apply_fn's operations
+  const T pc = a[v.t];
+  T ax = add_rn<T>(mul_rn<T>(v.kl, pc - a[v.tl]), mul_rn<T>(v.kr, pc - a[v.tr]));
+  if (v.top) ax = add_rn<T>(ax, mul_rn<T>(v.kt, pc - a[v.t - 1]));
+  if (v.bot) ax = add_rn<T>(ax, mul_rn<T>(v.kb, pc - a[v.t + 1]));
+  if (v.pinned) ax = add_rn<T>(ax, mul_rn<T>(dpin, pc));
+  return ax;
+}
+template <typename T>
+__device__ __forceinline__ PRow<T> p_row_at(int Nz, int Nx, const T* kx, const T* kz, int pin, T dpin, int j, int i) {
+  PRow<T> v;
+  v.t = i * Nz + j;
+  v.tl = (i == 0 ? Nx - 1 : i - 1) * Nz + j;
+  v.tr = (i == Nx - 1 ? 0 : i + 1) * Nz + j;
+  v.top = j > 0;
+  v.bot = j < Nz - 1;
+  v.pinned = v.t == pin;
+  v.kl = kx[v.t];
+  v.kr = kx[v.tr];
+  v.kt = kz[i * (Nz + 1) + j];
+  v.kb = kz[i * (Nz + 1) + j + 1];
+  v.d = v.kl + v.kr + (v.top ? v.kt : (T)0) + (v.bot ? v.kb : (T)0);
+  if (v.pinned) v.d += dpin;
+  return v;
+}
+template <typename T>
+__device__ __forceinline__ T p_row_relax(const PRow<T>& v, T x, T b, T ax, T om) {
+  return v.d > (T)0 ? x + rdiv<T>(om * (b - ax), v.d) : (T)0;
+}
+
+// the sweeps of vel_sweeps_reg on a pressure level, a thread per cell
+template <typename T>
+__device__ __forceinline__ void p_sweeps_reg(int Nz, int Nx, const T* __restrict__ kx, const T* __restrict__ kz,
+                                             int pin, T dpin, T* x, T* x2, const T* b, int sweeps, T omega) {
+  const int i = threadIdx.x / Nz, j = threadIdx.x - i * Nz;
+  const bool act = i < Nx;
+  PRow<T> v;
+  T bt = 0;
+  if (act) {
+    v = p_row_at<T>(Nz, Nx, kx, kz, pin, dpin, j, i);
+    bt = b[v.t];
+  }
+  T* a = x;
+  T* o = x2;
+  for (int s = 0; s < sweeps; ++s) {
+    if (act) o[v.t] = p_row_relax<T>(v, a[v.t], bt, p_row_apply<T>(v, dpin, a), omega);
+    __syncthreads();
+    T* tmp = a; a = o; o = tmp;
+  }
 }
 
 template <typename T>
@@ -1703,26 +2091,41 @@ __device__ void p_coarse_cta(int Nz, int Nx, const T* __restrict__ kx, const T* 
   __syncthreads();
   T* a = x;
   T* o = x2;
-  for (int s = 0; s < sweeps; ++s) {
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      T d;
-      T ax = p_apply_at<T>(Nz, Nx, kx, kz, pin, dpin, a, t % Nz, t / Nz, &d);
-      o[t] = d > (T)0 ? a[t] + sdiv<T>(omega * (b[t] - ax), d) : (T)0;
+  if (n <= (int)blockDim.x) {
+    p_sweeps_reg<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega);
+    if (sweeps & 1) a = x2;
+  } else {
+    for (int s = 0; s < sweeps; ++s) {
+      for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        T d;
+        T ax = p_apply_at<T>(Nz, Nx, kx, kz, pin, dpin, a, t % Nz, t / Nz, &d);
+        o[t] = d > (T)0 ? a[t] + sdiv<T>(omega * (b[t] - ax), d) : (T)0;
+      }
+      __syncthreads();
+      T* tmp = a; a = o; o = tmp;
     }
-    __syncthreads();
-    T* tmp = a; a = o; o = tmp;
   }
   if (a != x)
     for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = a[t];
   __syncthreads();
 }
 template <typename T>
-__global__ void p_coarse_kernel(int Nz, int Nx, const T* __restrict__ kx, const T* __restrict__ kz, int pin,
-                                T dpin, T* x, T* x2, const T* __restrict__ b, int sweeps, T omega, const T* inv,
-                                const int* inv_ok, WideInverse wide, const int* solved) {
+__global__ void __launch_bounds__(1024) p_coarse_kernel(int Nz, int Nx, const T* __restrict__ kx,
+                                                        const T* __restrict__ kz, int pin, T dpin, T* x, T* x2,
+                                                        const T* __restrict__ b, int sweeps, T omega, const T* inv,
+                                                        const int* inv_ok, WideInverse wide, const int* solved,
+                                                        int staged) {
   XC_PDL_WAIT();
   if (solved && *solved) return;
-  p_coarse_cta<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega, inv, inv_ok, wide);
+  extern __shared__ __align__(16) unsigned char xc_stage[];
+  if (staged) {
+    const int n = Nz * Nx;
+    T* sx = reinterpret_cast<T*>(xc_stage);
+    p_coarse_cta<T>(Nz, Nx, kx, kz, pin, dpin, sx, sx + n, b, sweeps, omega, inv, inv_ok, wide);
+    for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = sx[t];
+  } else {
+    p_coarse_cta<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega, inv, inv_ok, wide);
+  }
 }
 
 // diag^-1 L of a coarsest pressure level, as wide_form_vel_kernel
@@ -1783,11 +2186,11 @@ __global__ void __launch_bounds__(256) p_dense_inv_kernel(int Nz, int Nx, const 
 // Small levels in one CTA.  A level of a few hundred cells is a few hundred
 // unknowns, and each phase of its V-cycle (a smoothing sweep, the residual,
 // the restriction, the prolongation) is bound by launch latency, not by
-// bandwidth.  These kernels run the V-cycle from level l0 down to the coarsest
-// level lc and back up inside one CTA, with CTA barriers between the phases;
-// the level data stays in L1/L2.  Measured at 1024^2 against one launch per
-// phase: handing the levels up to 16x16 to one CTA saves 3% of the solve; up
-// to 64x64 it costs 6% (one CTA then streams too many rows per phase).
+// bandwidth.  One CTA runs the V-cycle from level l0 down to the coarsest level
+// lc and back up, with CTA barriers between the phases: from shared memory
+// (vel_vcycle_stage_kernel, p_vcycle_stage_kernel) where the levels fit it and
+// have at most 1024 rows, else on global memory with the bodies of the
+// per-level launches.
 // ---------------------------------------------------------------------------
 template <typename T>
 struct VelLevels {
@@ -1830,36 +2233,6 @@ __host__ __device__ __forceinline__ OpConst level_const(const OpConst& k, int l)
   return c;
 }
 
-// Shared-memory staging of the one-CTA V-cycles.  The small levels are a few
-// hundred unknowns each, and every sweep of them is a chain of dependent loads
-// separated by CTA barriers: from shared memory instead of L2 each sweep costs
-// a fraction of the latency.  Arrays are carved in a fixed order, each rounded
-// up to 16 bytes; the host sizes the dynamic allocation with the same counts.
-template <typename T>
-__host__ __device__ __forceinline__ long long smem_round(long long c) {
-  constexpr long long q = 16 / sizeof(T);
-  return (c + q - 1) / q * q;
-}
-template <typename T>
-__host__ __device__ inline long long vel_stage_elems(const Geo* gs, int l0, int lc) {
-  long long e = 0;
-  for (int q = l0; q <= lc; ++q) {
-    const Geo& g = gs[q];
-    if (kFly<T>)
-      e += smem_round<T>((long long)g.Nz * g.Nx) + smem_round<T>((long long)(g.Nz + 1) * (g.Nx + 1)) +
-           smem_round<T>(g.NW) + smem_round<T>(g.NU) + smem_round<T>(3LL * (g.Nx + 2));
-    else
-      e += smem_round<T>(10LL * g.NW) + smem_round<T>(10LL * g.NU);
-    e += 4 * smem_round<T>((long long)g.NW + g.NU);
-  }
-  return e;
-}
-template <typename T>
-__device__ __forceinline__ void cta_copy(T* dst, const T* src, long long n) {
-  for (long long t = threadIdx.x; t < n; t += blockDim.x) dst[t] = src[t];
-}
-constexpr size_t kStageMaxBytes = 160 * 1024;
-
 // the V-cycle of levels l0..lc (lc the coarsest) by one CTA: nu sweeps
 // before and after each coarse correction, the coarsest solved directly
 template <typename T>
@@ -1878,7 +2251,7 @@ __device__ void vel_vcycle_cta(const VelLevels<T>& L, const OpConst& kf, int l0,
     for (long long t = threadIdx.x; t < nc; t += blockDim.x) vel_restrict_at<T>(g, c, L.r[l], L.b[l + 1], t);
     __syncthreads();
   }
-  vel_coarse_cta<T>(L.g[lc], level_const(kf, lc), L.op[lc], L.x[lc], L.x2[lc], L.b[lc], csweeps, om, inv, inv_ok,
+  vel_coarse_cta<T, 0>(L.g[lc], level_const(kf, lc), L.op[lc], L.x[lc], L.x2[lc], L.b[lc], csweeps, om, inv, inv_ok,
                     wide);
   for (int l = lc - 1; l >= l0; --l) {
     const OpConst k = level_const(kf, l);
@@ -1892,55 +2265,193 @@ __device__ void vel_vcycle_cta(const VelLevels<T>& L, const OpConst& kf, int l0,
 
 template <typename T>
 __global__ void __launch_bounds__(1024) vel_vcycle_small_kernel(VelLevels<T> Lg, OpConst kf, int l0, int lc, int nu,
-                                                                T om, int csweeps, int staged, const T* inv,
-                                                                const int* inv_ok, WideInverse wide) {
+                                                                T om, int csweeps, const T* inv, const int* inv_ok,
+                                                                WideInverse wide) {
   XC_PDL_WAIT();
-  extern __shared__ __align__(16) unsigned char xc_stage[];
   __shared__ VelLevels<T> L;
-  if (threadIdx.x == 0) {
-    T* p = reinterpret_cast<T*>(xc_stage);
-    for (int q = l0; q <= lc; ++q) {
-      const Geo& g = Lg.g[q];
-      L.g[q] = g; L.op[q] = Lg.op[q];
-      L.x[q] = Lg.x[q]; L.x2[q] = Lg.x2[q]; L.b[q] = Lg.b[q]; L.r[q] = Lg.r[q];
-      if (!staged) continue;
-      if constexpr (kFly<T>) {
-        L.op[q].eta = p; p += smem_round<T>((long long)g.Nz * g.Nx);
-        L.op[q].etaco = p; p += smem_round<T>((long long)(g.Nz + 1) * (g.Nx + 1));
-        L.op[q].dw = p; p += smem_round<T>(g.NW);
-        L.op[q].du = p; p += smem_round<T>(g.NU);
-        L.op[q].dbot = p; p += smem_round<T>(3LL * (g.Nx + 2));
-      } else {
-        L.op[q].cw = p; p += smem_round<T>(10LL * g.NW);
-        L.op[q].cu = p; p += smem_round<T>(10LL * g.NU);
-      }
-      const long long nvv = (long long)g.NW + g.NU;
-      L.x[q] = p; p += smem_round<T>(nvv);
-      L.x2[q] = p; p += smem_round<T>(nvv);
-      L.b[q] = p; p += smem_round<T>(nvv);
-      L.r[q] = p; p += smem_round<T>(nvv);
-    }
-  }
+  if (threadIdx.x == 0) L = Lg;
   __syncthreads();
-  if (staged) {
-    for (int q = l0; q <= lc; ++q) {
-      const Geo& g = L.g[q];
-      if constexpr (kFly<T>) {
-        cta_copy<T>(const_cast<T*>(L.op[q].eta), Lg.op[q].eta, (long long)g.Nz * g.Nx);
-        cta_copy<T>(const_cast<T*>(L.op[q].etaco), Lg.op[q].etaco, (long long)(g.Nz + 1) * (g.Nx + 1));
-        cta_copy<T>(const_cast<T*>(L.op[q].dw), Lg.op[q].dw, g.NW);
-        cta_copy<T>(const_cast<T*>(L.op[q].du), Lg.op[q].du, g.NU);
-        cta_copy<T>(const_cast<T*>(L.op[q].dbot), Lg.op[q].dbot, 3LL * (g.Nx + 2));
+  vel_vcycle_cta<T>(L, kf, l0, lc, nu, om, csweeps, inv, inv_ok, wide);
+}
+
+// ---- the same V-cycle from shared memory -----------------------------------
+// One CTA with everything it touches in shared memory: the coefficients of the
+// levels l0..lc and the dense inverse of the coarsest, copied while the kernel
+// before this one still runs (setup wrote them many launches earlier); the
+// right-hand side comes in and the result leaves through the registers of the
+// first and last operation.  A thread has one row of every level, its weights in
+// registers.  Some ten phases follow each other between CTA barriers, so the
+// length of one thread's instruction chain is the time: with the bodies of the
+// separate kernels on global memory (two 64-bit divisions a row, weights formed
+// anew, loops not unrolled) the levels up to 16 x 16 took 15.3 us a V-cycle, now
+// 6.0 us.  Handing 32 x 32 to it as well saved six launches and measured the
+// same (1.25x against 1.25x of the 64^2 step, 1.29x against 1.30x at 512^2).
+struct StageLevel {
+  int a0, a1, a2, a3, a4;            // eta, etaco, dw, du, dbot (FP64: cw, cu); pressure: kx, kz
+  int x, y, b;                       // two iterates, right-hand side
+  unsigned dv[4];                    // stage_div of Nz - 1, Nz, Nz + 1, Nz + 2 (pressure: [1])
+};
+struct StageMap {
+  StageLevel l[kMaxLevels];
+  int inv;                           // the dense inverse, -1: none
+  int total;                         // elements
+};
+template <typename T>
+struct StageCarve {
+  int at = 0;
+  int take(long long n) {
+    constexpr int q = 16 / (int)sizeof(T);
+    const int o = at;
+    at += (int)((n + q - 1) / q * q);
+    return o;
+  }
+};
+// An array to stage, in 16-byte pieces (the arrays' allocations are whole pieces:
+// stage_bytes); a warp takes a segment, so that the copies of all of them are
+// in flight after a few instructions.
+constexpr int kStageSegs = 64;
+struct StageSeg { const void* src; int dst, n16; };
+struct StageList {
+  StageSeg seg[kStageSegs];
+  int count;
+  void add(const void* src, int dst, long long bytes) {
+    for (long long n16 = (bytes + 15) / 16, o = 0; o < n16; o += 128, ++count)      // (count may pass the end: not staged then)
+      if (count < kStageSegs)
+        seg[count] = {(const char*)src + 16 * o, dst + (int)(16 * o), (int)(n16 - o < 128 ? n16 - o : 128)};
+  }
+};
+inline size_t stage_bytes(size_t b) { return (b + 15) / 16 * 16; }
+__device__ __forceinline__ void stage_piece(unsigned char* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void stage_list(unsigned char* sm, const StageList& S) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int q = threadIdx.x >> 5; q < S.count; q += nw) {
+    const StageSeg g = S.seg[q];
+    for (int t = lane; t < g.n16; t += 32) stage_piece(sm + g.dst + 16 * t, (const char*)g.src + 16 * t);
+  }
+}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <typename T>
+__global__ void __launch_bounds__(1024) vel_vcycle_stage_kernel(const __grid_constant__ VelLevels<T> L,
+                                                                const __grid_constant__ StageMap M,
+                                                                const __grid_constant__ StageList S, OpConst kf, int l0,
+                                                                int lc, int nu, T om, int csweeps, const T* inv, const int* inv_ok,
+                                                                WideInverse wide) {
+  extern __shared__ __align__(16) unsigned char xc_stage[];
+  T* const sm = reinterpret_cast<T*>(xc_stage);
+  // the levels' sizes and offsets, read again in every phase (from the parameter
+  // bank each level's first read would miss)
+  __shared__ Geo sg[kMaxLevels];
+  __shared__ StageLevel sl[kMaxLevels];
+  static_assert(sizeof(Geo) % 4 == 0 && sizeof(StageLevel) % 4 == 0, "copied as words");
+  for (int t = threadIdx.x; t < (int)(lc + 1) * (int)(sizeof(Geo) / 4); t += blockDim.x)
+    reinterpret_cast<int*>(sg)[t] = reinterpret_cast<const int*>(L.g)[t];
+  for (int t = threadIdx.x; t < (int)(lc + 1) * (int)(sizeof(StageLevel) / 4); t += blockDim.x)
+    reinterpret_cast<int*>(sl)[t] = reinterpret_cast<const int*>(M.l)[t];
+  auto level_op = [&](int l) {
+    VOp<T> op = {};
+    if constexpr (kFly<T>) {
+      op.eta = sm + sl[l].a0; op.etaco = sm + sl[l].a1; op.dw = sm + sl[l].a2;
+      op.du = sm + sl[l].a3; op.dbot = sm + sl[l].a4;
+    } else {
+      op.cw = sm + sl[l].a0; op.cu = sm + sl[l].a1;
+    }
+    return op;
+  };
+  stage_list(xc_stage, S);
+  const bool dense = M.inv >= 0 && *inv_ok;
+  stage_wait();
+  __syncthreads();
+  const VelRow<T> top = vel_stage_row<T>(sg[l0], level_const(kf, l0), level_op(l0), om, threadIdx.x, sl[l0].dv[0],
+                                         sl[l0].dv[1]);
+  XC_PDL_WAIT();
+  unsigned in_y = 0;                   // bit l: level l's iterate is in y
+  for (int l = l0; l < lc; ++l) {
+    const Geo& g = sg[l];
+    const Geo& c = sg[l + 1];
+    const OpConst k = level_const(kf, l);
+    const VOp<T> op = level_op(l);
+    const StageLevel& m = sl[l];
+    const StageLevel& mc = sl[l + 1];
+    VelRow<T> v = top;
+    if (l != l0) v = vel_stage_row<T>(g, k, op, om, threadIdx.x, m.dv[0], m.dv[1]);
+    T* a = sm + m.x;
+    T* o = sm + m.y;
+    T b = 0;
+    if (v.kind) {
+      b = l == l0 ? L.b[l0][v.t] : sm[m.b + v.t];
+      if (l == l0) sm[m.b + v.t] = b;
+      a[v.t] = rdiv<T>(v.w * b, v.c.d);
+    }
+    __syncthreads();
+    for (int q = 1; q < nu; ++q) {
+      if (v.kind) o[v.t] = vel_stage_relax<T>(v, a[v.t], b, vel_stage_apply<T>(g, k, op, v, a));
+      __syncthreads();
+      T* tmp = a; a = o; o = tmp;
+      in_y ^= 1u << l;
+    }
+    if (v.kind) o[v.t] = b - vel_stage_apply<T>(g, k, op, v, a);
+    __syncthreads();
+    for (int e = threadIdx.x; e < c.NW + c.NU; e += blockDim.x) {
+      if (e < c.NW) {
+        const int i = stage_col(e, mc.dv[2]), j = e - i * (c.Nz + 1);
+        sm[mc.b + e] = vel_restrict_w<T>(g, c, o, j, i);
       } else {
-        cta_copy<T>(const_cast<T*>(L.op[q].cw), Lg.op[q].cw, 10LL * g.NW);
-        cta_copy<T>(const_cast<T*>(L.op[q].cu), Lg.op[q].cu, 10LL * g.NU);
+        const int q = e - c.NW, i = stage_col(q, mc.dv[3]), j = q - i * (c.Nz + 2);
+        sm[mc.b + e] = vel_restrict_u<T>(g, c, o + g.NW, j, i);
       }
     }
-    cta_copy<T>(L.b[l0], Lg.b[l0], (long long)L.g[l0].NW + L.g[l0].NU);
     __syncthreads();
   }
-  vel_vcycle_cta<T>(L, kf, l0, lc, nu, om, csweeps, inv, inv_ok, wide);
-  if (staged) cta_copy<T>(Lg.x[l0], L.x[l0], (long long)L.g[l0].NW + L.g[l0].NU);
+  {
+    const StageLevel& m = sl[lc];
+    if (dense)
+      dense_apply_cta<T>(sm + M.inv, sg[lc].NW + sg[lc].NU, sm + m.b, sm + m.x);
+    else
+      vel_coarse_cta<T, 1>(sg[lc], level_const(kf, lc), level_op(lc), sm + m.x, sm + m.y, sm + m.b, csweeps, om,
+                           nullptr, inv_ok, wide, m.dv[0], m.dv[1]);
+  }
+  for (int l = lc - 1; l >= l0; --l) {
+    const OpConst k = level_const(kf, l);
+    const VOp<T> op = level_op(l);
+    const StageLevel& m = sl[l];
+    const Geo& g = sg[l];
+    const Geo& c = sg[l + 1];
+    const bool yc = (in_y >> (l + 1)) & 1u, yf = (in_y >> l) & 1u;
+    const T* xc = sm + (yc ? sl[l + 1].y : sl[l + 1].x);
+    T* a = sm + (yf ? m.y : m.x);
+    T* o = sm + (yf ? m.x : m.y);
+    for (int e = threadIdx.x; e < g.NW + g.NU; e += blockDim.x) {
+      if (e < g.NW) {
+        const int i = stage_col(e, m.dv[2]), j = e - i * (g.Nz + 1);
+        a[e] += vel_prolong_w<T>(g, c, xc, j, i);
+      } else {
+        const int q = e - g.NW, i = stage_col(q, m.dv[3]), j = q - i * (g.Nz + 2);
+        a[e] += vel_prolong_u<T>(g, c, k, xc + c.NW, j, i);
+      }
+    }
+    VelRow<T> v = top;
+    if (l != l0) v = vel_stage_row<T>(g, k, op, om, threadIdx.x, m.dv[0], m.dv[1]);
+    const T b = v.kind ? sm[m.b + v.t] : (T)0;
+    __syncthreads();
+    for (int q = 0; q < nu; ++q) {
+      T x = 0;
+      if (v.kind) x = vel_stage_relax<T>(v, a[v.t], b, vel_stage_apply<T>(g, k, op, v, a));
+      if (l == l0 && q == nu - 1) {  // straight to the caller's vector
+        if (v.kind) L.x[l][v.t] = x;
+        return;
+      }
+      if (v.kind) o[v.t] = x;
+      __syncthreads();
+      T* tmp = a; a = o; o = tmp;
+      in_y ^= 1u << l;
+    }
+    if (l == l0)                       // no sweep after the correction
+      for (int t = threadIdx.x; t < g.NW + g.NU; t += blockDim.x) L.x[l][t] = a[t];
+  }
 }
 
 
@@ -2068,46 +2579,12 @@ __device__ void p_smooth_cta(const PLevels<T>& L, int l, T om, int sweeps, bool 
 }
 
 template <typename T>
-__host__ __device__ inline long long p_stage_elems(const int* Nzs, const int* Nxs, int l0, int lc) {
-  long long e = 0;
-  for (int q = l0; q <= lc; ++q) {
-    const long long n = (long long)Nzs[q] * Nxs[q];
-    e += 5 * smem_round<T>(n) + smem_round<T>((long long)(Nzs[q] + 1) * Nxs[q]);
-  }
-  return e;
-}
-template <typename T>
-__global__ void __launch_bounds__(1024) p_vcycle_small_kernel(PLevels<T> Lg, int l0, int lc, int nu, T om,
-                                                              int csweeps, int staged, const T* inv,
-                                                              const int* inv_ok, WideInverse wide) {
+__global__ void __launch_bounds__(1024) p_vcycle_small_kernel(PLevels<T> Lg, int l0, int lc, int nu, T om, int csweeps,
+                                                              const T* inv, const int* inv_ok, WideInverse wide) {
   XC_PDL_WAIT();
-  extern __shared__ __align__(16) unsigned char xc_stage[];
   __shared__ PLevels<T> L;
-  if (threadIdx.x == 0) {
-    T* p = reinterpret_cast<T*>(xc_stage);
-    for (int q = l0; q <= lc; ++q) {
-      L.Nz[q] = Lg.Nz[q]; L.Nx[q] = Lg.Nx[q]; L.pin[q] = Lg.pin[q]; L.dpin[q] = Lg.dpin[q];
-      L.kx[q] = Lg.kx[q]; L.kz[q] = Lg.kz[q];
-      L.x[q] = Lg.x[q]; L.x2[q] = Lg.x2[q]; L.b[q] = Lg.b[q]; L.r[q] = Lg.r[q];
-      if (!staged) continue;
-      const long long n = (long long)Lg.Nz[q] * Lg.Nx[q];
-      L.kx[q] = p; p += smem_round<T>(n);
-      L.kz[q] = p; p += smem_round<T>((long long)(Lg.Nz[q] + 1) * Lg.Nx[q]);
-      L.x[q] = p; p += smem_round<T>(n);
-      L.x2[q] = p; p += smem_round<T>(n);
-      L.b[q] = p; p += smem_round<T>(n);
-      L.r[q] = p; p += smem_round<T>(n);
-    }
-  }
+  if (threadIdx.x == 0) L = Lg;
   __syncthreads();
-  if (staged) {
-    for (int q = l0; q <= lc; ++q) {
-      cta_copy<T>(const_cast<T*>(L.kx[q]), Lg.kx[q], (long long)L.Nz[q] * L.Nx[q]);
-      cta_copy<T>(const_cast<T*>(L.kz[q]), Lg.kz[q], (long long)(L.Nz[q] + 1) * L.Nx[q]);
-    }
-    cta_copy<T>(L.b[l0], Lg.b[l0], (long long)L.Nz[l0] * L.Nx[l0]);
-    __syncthreads();
-  }
   for (int l = l0; l < lc; ++l) {
     const int Nz = L.Nz[l], Nx = L.Nx[l], n = Nz * Nx;
     p_smooth_cta<T>(L, l, om, nu, true);
@@ -2126,7 +2603,120 @@ __global__ void __launch_bounds__(1024) p_vcycle_small_kernel(PLevels<T> Lg, int
     __syncthreads();
     p_smooth_cta<T>(L, l, om, nu, false);
   }
-  if (staged) cta_copy<T>(Lg.x[l0], L.x[l0], (long long)L.Nz[l0] * L.Nx[l0]);
+}
+
+// the same from shared memory, as vel_vcycle_stage_kernel, a cell a thread: 7.1 us
+// a V-cycle of the levels up to 16 x 16 before, 4.1 us now
+// the thread's cell of a staged level, the four cells of a coarse one together
+template <typename T>
+__device__ __forceinline__ PRow<T> p_stage_row(int Nz, int Nx, const T* kx, const T* kz, int pin, T dpin,
+                                               unsigned dvc) {
+  const int tc = threadIdx.x >> 2, q = threadIdx.x & 3, Nzc = Nz / 2;
+  if (tc < Nzc * (Nx / 2)) {
+    const int I = stage_col(tc, dvc), J = tc - I * Nzc;
+    return p_row_at<T>(Nz, Nx, kx, kz, pin, dpin, 2 * J + (q & 1), 2 * I + (q >> 1));
+  }
+  PRow<T> v;
+  v.t = -1;
+  return v;
+}
+template <typename T>
+__global__ void __launch_bounds__(1024) p_vcycle_stage_kernel(const __grid_constant__ PLevels<T> L,
+                                                              const __grid_constant__ StageMap M,
+                                                              const __grid_constant__ StageList S, int l0, int lc,
+                                                              int nu, T om, int csweeps, const T* inv,
+                                                              const int* inv_ok, WideInverse wide) {
+  extern __shared__ __align__(16) unsigned char xc_stage[];
+  T* const sm = reinterpret_cast<T*>(xc_stage);
+  __shared__ StageLevel sl[kMaxLevels];
+  __shared__ int sn[kMaxLevels][3];
+  __shared__ T sd[kMaxLevels];
+  for (int t = threadIdx.x; t < (int)(lc + 1) * (int)(sizeof(StageLevel) / 4); t += blockDim.x)
+    reinterpret_cast<int*>(sl)[t] = reinterpret_cast<const int*>(M.l)[t];
+  if ((int)threadIdx.x <= lc) {
+    sn[threadIdx.x][0] = L.Nz[threadIdx.x];
+    sn[threadIdx.x][1] = L.Nx[threadIdx.x];
+    sn[threadIdx.x][2] = L.pin[threadIdx.x];
+    sd[threadIdx.x] = L.dpin[threadIdx.x];
+  }
+  auto row = [&](int l) {
+    return p_stage_row<T>(sn[l][0], sn[l][1], sm + sl[l].a0, sm + sl[l].a1, sn[l][2], sd[l], sl[l + 1].dv[1]);
+  };
+  stage_list(xc_stage, S);
+  const bool dense = M.inv >= 0 && *inv_ok;
+  stage_wait();
+  __syncthreads();
+  const PRow<T> first = row(l0);
+  XC_PDL_WAIT();
+  unsigned in_y = 0;
+  for (int l = l0; l < lc; ++l) {
+    const StageLevel& m = sl[l];
+    const T dpin = sd[l];
+    PRow<T> v = first;
+    if (l != l0) v = row(l);
+    T* a = sm + m.x;
+    T* o = sm + m.y;
+    T b = 0;
+    if (v.t >= 0) {
+      b = l == l0 ? L.b[l0][v.t] : sm[m.b + v.t];
+      if (l == l0) sm[m.b + v.t] = b;
+      a[v.t] = v.d > (T)0 ? rdiv<T>(om * b, v.d) : (T)0;
+    }
+    __syncthreads();
+    for (int q = 1; q < nu; ++q) {
+      if (v.t >= 0) o[v.t] = p_row_relax<T>(v, a[v.t], b, p_row_apply<T>(v, dpin, a), om);
+      __syncthreads();
+      T* tmp = a; a = o; o = tmp;
+      in_y ^= 1u << l;
+    }
+    // the residual and, in p_down_kernel's order, its restriction
+    T r = 0;
+    if (v.t >= 0) r = b - p_row_apply<T>(v, dpin, a);
+    const T r1 = __shfl_down_sync(0xffffffffu, r, 1), r2 = __shfl_down_sync(0xffffffffu, r, 2),
+            r3 = __shfl_down_sync(0xffffffffu, r, 3);
+    if (v.t >= 0 && (threadIdx.x & 3) == 0) sm[sl[l + 1].b + (threadIdx.x >> 2)] = (T)0.25 * (r + r1 + r2 + r3);
+    __syncthreads();
+  }
+  {
+    const StageLevel& m = sl[lc];
+    if (dense)
+      dense_apply_cta<T>(sm + M.inv, sn[lc][0] * sn[lc][1], sm + m.b, sm + m.x);
+    else
+      p_coarse_cta<T>(sn[lc][0], sn[lc][1], sm + m.a0, sm + m.a1, sn[lc][2], sd[lc], sm + m.x, sm + m.y, sm + m.b,
+                      csweeps, om, nullptr, inv_ok, wide);
+  }
+  for (int l = lc - 1; l >= l0; --l) {
+    const StageLevel& m = sl[l];
+    const T dpin = sd[l];
+    PRow<T> v = first;
+    if (l != l0) v = row(l);
+    const bool yc = (in_y >> (l + 1)) & 1u, yf = (in_y >> l) & 1u;
+    const T* xc = sm + (yc ? sl[l + 1].y : sl[l + 1].x);
+    T* a = sm + (yf ? m.y : m.x);
+    T* o = sm + (yf ? m.x : m.y);
+    T b = 0;
+    if (v.t >= 0) {
+      const int tc = threadIdx.x >> 2, q = threadIdx.x & 3, Nzc = sn[l + 1][0];
+      const int I = stage_col(tc, sl[l + 1].dv[1]), J = tc - I * Nzc;
+      a[v.t] = add_rn<T>(a[v.t], p_prolong_val<T>(Nzc, sn[l + 1][1], xc, 2 * J + (q & 1), 2 * I + (q >> 1)));
+      b = sm[m.b + v.t];
+    }
+    __syncthreads();
+    for (int q = 0; q < nu; ++q) {
+      T x = 0;
+      if (v.t >= 0) x = p_row_relax<T>(v, a[v.t], b, p_row_apply<T>(v, dpin, a), om);
+      if (l == l0 && q == nu - 1) {
+        if (v.t >= 0) L.x[l][v.t] = x;
+        return;
+      }
+      if (v.t >= 0) o[v.t] = x;
+      __syncthreads();
+      T* tmp = a; a = o; o = tmp;
+      in_y ^= 1u << l;
+    }
+    if (l == l0)
+      for (int t = threadIdx.x; t < sn[l][0] * sn[l][1]; t += blockDim.x) L.x[l][t] = a[t];
+  }
 }
 
 // fine-level pressure coefficients from the velocity diagonal (plane 0: full,
@@ -2198,9 +2788,8 @@ __global__ void p_scatter_fused_kernel(Geo g, const T* __restrict__ z, const T* 
                                        int open_bottom, T* zp) {
   XC_PDL_WAIT();
   const int Nz = g.Nz, Nx = g.Nx, lp = Nz + 2;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= lp * (Nx + 2)) return;
-  const int j = t % lp, i = t / lp;
+  const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y, t = i * lp + j;
+  if (j > Nz + 1 || i > Nx + 1) return;
   auto r = [&](int jj, int ii) {
     const size_t o = (size_t)ii * lp + jj;
     return vp[o] / sp[o];
@@ -2302,35 +2891,46 @@ __global__ void __launch_bounds__(KB) multidot_kernel(long long n, int m, const 
     part[(size_t)blockIdx.x * m + threadIdx.x] = s;
   }
 }
-__global__ void multidot_final_kernel(int m, int nb, const double* __restrict__ part, double* out) {
-  XC_PDL_WAIT();
-  int k = blockIdx.x;
+// the CTA's KB values added in halves (t + KB/2, then + KB/4, ...), the last
+// five by shuffles; the sum in thread 0.  A dependent FP64 addition is most of a
+// hundred cycles here, and one launch waits for these eight: with a CTA barrier
+// after each, and the square root and quotient of norm_final_kernel as chains of
+// FP64 operations, the two kernels took 4500 cycles; now 2.0 and 1.5 us in place of
+// 2.6 and 2.8 us.
+__device__ __forceinline__ double halving_sum(double v) {
   __shared__ double sh[KB];
-  double acc = 0;
-  for (int b = threadIdx.x; b < nb; b += KB) acc += part[(size_t)b * m + k];
-  sh[threadIdx.x] = acc;
+  sh[threadIdx.x] = v;
   __syncthreads();
-  for (int s = KB / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+#pragma unroll
+  for (int s = KB / 2; s >= 32; s >>= 1) {
+    if (threadIdx.x < s) {
+      v += sh[threadIdx.x + s];
+      sh[threadIdx.x] = v;
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[k] = sh[0];
+  if (threadIdx.x < 32)
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
+  return v;
+}
+__global__ void multidot_final_kernel(int m, int nb, const double* __restrict__ part, double* out) {
+  XC_PDL_WAIT();
+  const int k = blockIdx.x;
+  double acc = 0;
+  for (int b = threadIdx.x; b < nb; b += KB) acc += part[(size_t)b * m + k];
+  acc = halving_sum(acc);
+  if (threadIdx.x == 0) out[k] = acc;
 }
 // ||v||^2 from one partial column -> *nrm2, and 1/||v|| (1 for a zero norm) -> *inv
 __global__ void norm_final_kernel(int nb, const double* __restrict__ part, double* nrm2, double* inv) {
   XC_PDL_WAIT();
-  __shared__ double sh[KB];
   double acc = 0;
   for (int b = threadIdx.x; b < nb; b += KB) acc += part[b];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = KB / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-    __syncthreads();
-  }
+  acc = halving_sum(acc);
   if (threadIdx.x == 0) {
-    *nrm2 = sh[0];
-    *inv = sh[0] > 0.0 ? 1.0 / sqrt(sh[0]) : 1.0;
+    *nrm2 = acc;
+    *inv = acc > 0.0 ? xc_div(1.0, xc_sqrt(acc)) : 1.0;
   }
 }
 // w -= sum_k h[k] V[k] and ||w||^2 in the same pass: per-CTA partial sums
@@ -2593,7 +3193,11 @@ __global__ void pack_kernel(Geo g, CView W, CView U, CView P, double* x) {
 inline unsigned nblk(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 // 2-D launch over the (Nz + 2) x (Nx + 2) row positions of a level
 inline dim3 blk2() { return dim3(32, 8); }
-inline dim3 grid2(const Geo& g) { return dim3((unsigned)((g.Nz + 2 + 31) / 32), (unsigned)((g.Nx + 2 + 7) / 8)); }
+inline dim3 grid2(const Geo& g, int layers = 1) {
+  return dim3((unsigned)((g.Nz + 2 + 31) / 32), (unsigned)((g.Nx + 2 + 7) / 8), (unsigned)layers);
+}
+constexpr long long kSplitCells = 128 * 128;
+inline bool split_rows(const Geo& g) { return (long long)g.Nz * g.Nx <= kSplitCells; }
 
 }  // namespace
 
@@ -2616,14 +3220,10 @@ struct SolveCfg {
   // velocity diagonal instead (cmass then defaults to 0)
   double cmass = 0.5;
   int kplane = 9;
-  // pressure levels of at most this many cells use the fused descent /
-  // ascent kernels, larger ones one launch per operation (none by default:
-  // measured no faster at any level size, programmatic launch already hides
-  // the launches they save, and 1% slower on the fine levels)
+  // pressure levels of at most this many cells use the kernels that form every
+  // neighbour's value anew (p_down_kernel, p_up_kernel) in place of the tiled ones
   long long pfuse_cells = 0;
-  // one-CTA levels staged in shared memory (off by default: measured 1.5%
-  // slower at 1024^2 -- the small levels' sweeps are bound by instruction
-  // latency on one SM, and their L1-resident loads gain nothing from it)
+  // (accepted; the one-CTA levels run from shared memory wherever they fit it)
   bool stage_small = false;
   // coarsest levels of at most kDenseMax unknowns solved by their inverse
   bool direct_coarse = true;
@@ -2784,18 +3384,18 @@ int alloc_hier(StokesWork* w, Hier<T>& H, int m) {
     H.vg[H.nv] = lg;
     long long nvv = (long long)lg.NW + lg.NU;
     if (kFly<T>) {
-      XC_CUDA_TRY(cudaMalloc(&H.feta[H.nv], sizeof(T) * lg.Nz * lg.Nx));
-      XC_CUDA_TRY(cudaMalloc(&H.fetaco[H.nv], sizeof(T) * (lg.Nz + 1) * (lg.Nx + 1)));
-      XC_CUDA_TRY(cudaMalloc(&H.fdw[H.nv], sizeof(T) * lg.NW));
-      XC_CUDA_TRY(cudaMalloc(&H.fdu[H.nv], sizeof(T) * lg.NU));
-      XC_CUDA_TRY(cudaMalloc(&H.fdbot[H.nv], sizeof(T) * 3 * (lg.Nx + 2)));
+      XC_CUDA_TRY(cudaMalloc(&H.feta[H.nv], stage_bytes(sizeof(T) * lg.Nz * lg.Nx)));
+      XC_CUDA_TRY(cudaMalloc(&H.fetaco[H.nv], stage_bytes(sizeof(T) * (lg.Nz + 1) * (lg.Nx + 1))));
+      XC_CUDA_TRY(cudaMalloc(&H.fdw[H.nv], stage_bytes(sizeof(T) * lg.NW)));
+      XC_CUDA_TRY(cudaMalloc(&H.fdu[H.nv], stage_bytes(sizeof(T) * lg.NU)));
+      XC_CUDA_TRY(cudaMalloc(&H.fdbot[H.nv], stage_bytes(sizeof(T) * 3 * (lg.Nx + 2))));
     } else {
-      XC_CUDA_TRY(cudaMalloc(&H.cw[H.nv], sizeof(T) * 10 * lg.NW));
-      XC_CUDA_TRY(cudaMalloc(&H.cu[H.nv], sizeof(T) * 10 * lg.NU));
+      XC_CUDA_TRY(cudaMalloc(&H.cw[H.nv], stage_bytes(sizeof(T) * 10 * lg.NW)));
+      XC_CUDA_TRY(cudaMalloc(&H.cu[H.nv], stage_bytes(sizeof(T) * 10 * lg.NU)));
     }
     XC_CUDA_TRY(cudaMalloc(&H.vx[H.nv], sizeof(T) * nvv));
     XC_CUDA_TRY(cudaMalloc(&H.vx2[H.nv], sizeof(T) * nvv));
-    XC_CUDA_TRY(cudaMalloc(&H.vb[H.nv], sizeof(T) * nvv));
+    XC_CUDA_TRY(cudaMalloc(&H.vb[H.nv], stage_bytes(sizeof(T) * nvv)));
     XC_CUDA_TRY(cudaMalloc(&H.vr[H.nv], sizeof(T) * nvv));
     H.nv++;
     if (Nz % 2 || Nx % 2 || Nz / 2 < 4 || Nx / 2 < 4) break;
@@ -2812,11 +3412,11 @@ int alloc_hier(StokesWork* w, Hier<T>& H, int m) {
   while (H.np_lv < kMaxLevels) {
     int L = H.np_lv;
     H.pNz[L] = Nz; H.pNx[L] = Nx; H.ppin[L] = px * Nz + pz;
-    XC_CUDA_TRY(cudaMalloc(&H.kx[L], sizeof(T) * Nz * Nx));
-    XC_CUDA_TRY(cudaMalloc(&H.kz[L], sizeof(T) * (Nz + 1) * Nx));
+    XC_CUDA_TRY(cudaMalloc(&H.kx[L], stage_bytes(sizeof(T) * Nz * Nx)));
+    XC_CUDA_TRY(cudaMalloc(&H.kz[L], stage_bytes(sizeof(T) * (Nz + 1) * Nx)));
     XC_CUDA_TRY(cudaMalloc(&H.px[L], sizeof(T) * Nz * Nx));
     XC_CUDA_TRY(cudaMalloc(&H.px2[L], sizeof(T) * Nz * Nx));
-    XC_CUDA_TRY(cudaMalloc(&H.pb[L], sizeof(T) * Nz * Nx));
+    XC_CUDA_TRY(cudaMalloc(&H.pb[L], stage_bytes(sizeof(T) * Nz * Nx)));
     XC_CUDA_TRY(cudaMalloc(&H.pr[L], sizeof(T) * Nz * Nx));
     H.np_lv++;
     if (Nz % 2 || Nx % 2 || Nz / 2 < 2 || Nx / 2 < 2) break;
@@ -2893,7 +3493,13 @@ static bool p_coarsest(const Hier<T>& H, const SolveCfg& cfg, int l) {
   return l == H.np_lv - 1 || 4LL * H.pNz[l] * H.pNx[l] <= cfg.coarse_cells;
 }
 
-// one CTA runs the coarsest level; fewer threads make each sweep's barrier cheaper
+// most shared memory of a one-CTA V-cycle
+constexpr size_t kStageMaxBytes = 200 * 1024;
+// the coarsest level's two iterates are in shared memory up to this size (no
+// opt-in needed: 25 x 25 cells are 11 KB in FP32, 22 KB in FP64)
+constexpr size_t kSweepSmemMax = 48 * 1024 - 1024;
+// one CTA runs the coarsest level; fewer threads make each sweep's barrier cheaper,
+// a thread per position keeps its rows' weights in registers
 static int coarse_threads(long long n) { return n > 512 ? 1024 : (n > 128 ? 256 : 128); }
 
 // ---- velocity V-cycle on level l: solve A x = vb[l] approximately (x := vx[l])
@@ -2913,7 +3519,8 @@ void launch_sweep(const SolveCfg& cfg, const Geo& g, const OpConst& k, const VOp
       return;
     }
   }
-  pdl(PDL_ON, vel_sweep2d_kernel<T, MODE>, grid2(g), blk2(), s, g, k, op, xi, b, out, om, dscl);
+  if (split_rows(g)) pdl(PDL_ON, vel_sweep_split_kernel<T, MODE>, grid2(g, 3), blk2(), s, g, k, op, xi, b, out, om, dscl);
+  else pdl(PDL_ON, vel_sweep2d_kernel<T, MODE>, grid2(g), blk2(), s, g, k, op, xi, b, out, om, dscl);
 }
 
 template <typename T>
@@ -2962,17 +3569,45 @@ int vel_cluster_size() {
 }
 
 template <typename T>
+bool vel_in_cluster(const Hier<T>& H, const SolveCfg& cfg, int l) {
+  const long long cells = (long long)H.vg[l].Nz * H.vg[l].Nx;
+  return l > 0 && cfg.cluster_cells > 0 && cells <= cfg.cluster_cells && cells > cfg.small_cells &&
+         !vel_coarsest(H, cfg, l) && vel_cluster_size<T>() > 0;
+}
+// how a level's part of the V-cycle runs: its coarsest solve, one CTA for it and
+// everything below (levels of up to cfg.small_cells cells, unless the coarsest
+// is a wide product of many unknowns, which belongs to the whole GPU), or
+// launches over the grid
+enum { kRouteGrid, kRouteCta, kRouteCoarsest };
+template <typename T>
+int vel_route(const Hier<T>& H, const SolveCfg& cfg, int l) {
+  if (vel_coarsest(H, cfg, l)) return kRouteCoarsest;
+  int lc = l;
+  while (!vel_coarsest(H, cfg, lc)) ++lc;
+  if (H.vwide_on && H.vg[lc].NW + H.vg[lc].NU > kWideCta) return kRouteGrid;
+  return (long long)H.vg[l].Nz * H.vg[l].Nx <= cfg.small_cells ? kRouteCta : kRouteGrid;
+}
+template <typename T>
+int p_route(const Hier<T>& H, const SolveCfg& cfg, int l) {
+  if (p_coarsest(H, cfg, l)) return kRouteCoarsest;
+  int lc = l;
+  while (!p_coarsest(H, cfg, lc)) ++lc;
+  const long long n = (long long)H.pNz[l] * H.pNx[l];
+  if (H.pwide_on && H.pNz[lc] * H.pNx[lc] > kWideCta) return kRouteGrid;
+  return n <= cfg.small_cells ? kRouteCta : kRouteGrid;
+}
+
+// x0_done: the first sweep from zero was made by the level above
+template <typename T>
 int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaStream_t s, T* final_out = nullptr,
-               const T* final_scl = nullptr, bool* final_done = nullptr) {
+               const T* final_scl = nullptr, bool* final_done = nullptr, bool x0_done = false) {
   const Geo& g = H.vg[l];
   const long long n = (long long)g.NW + g.NU;
   const T om = (T)cfg.omega_v;
   const OpConst k = level_const(kf, l);
-  const long long cells = (long long)g.Nz * g.Nx;
-  if (l > 0 && cfg.cluster_cells > 0 && cells <= cfg.cluster_cells && cells > cfg.small_cells &&
-      !vel_coarsest(H, cfg, l)) {
+  if (vel_in_cluster(H, cfg, l)) {
     const int cs = vel_cluster_size<T>();
-    if (cs > 0) {
+    {
       int ls = l;
       while (!vel_coarsest(H, cfg, ls) && (long long)H.vg[ls].Nz * H.vg[ls].Nx > cfg.small_cells) ++ls;
       int lc = ls;
@@ -3003,26 +3638,71 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
       return XC_OK;
     }
   }
-  int lc_small = l;
-  while (!vel_coarsest(H, cfg, lc_small)) ++lc_small;
-  // a wide product of many unknowns belongs to the whole GPU, not to one CTA
-  const bool grid_coarse = H.vwide_on && H.vg[lc_small].NW + H.vg[lc_small].NU > kWideCta;
-  if (!vel_coarsest(H, cfg, l) && (long long)g.Nz * g.Nx <= cfg.small_cells && !grid_coarse) {
-    const int lc = lc_small;
+  const int route = vel_route(H, cfg, l);
+  if (route == kRouteCta) {
+    int lc = l;
+    while (!vel_coarsest(H, cfg, lc)) ++lc;
     VelLevels<T> L;
     for (int q = 0; q <= lc; ++q) {
       L.g[q] = H.vg[q]; L.op[q] = vop(H, q);
       L.x[q] = H.vx[q]; L.x2[q] = H.vx2[q]; L.b[q] = H.vb[q]; L.r[q] = H.vr[q];
     }
-    const size_t bytes = sizeof(T) * (size_t)vel_stage_elems<T>(H.vg, l, lc);
-    const int staged = cfg.stage_small && bytes <= kStageMaxBytes;
-    pdl_smem(PDL_ON, vel_vcycle_small_kernel<T>, 1, coarse_threads(n), staged ? bytes : 0, s, L, kf, l, lc, cfg.nu,
-             om, coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx), staged, H.vdirect ? H.vinv : nullptr, H.dok,
-             vel_wide(H, lc));
+    StageMap M;
+    StageCarve<T> carve;
+    for (int q = l; q <= lc; ++q) {
+      const Geo& gq = H.vg[q];
+      StageLevel& m = M.l[q];
+      if (kFly<T>) {
+        m.a0 = carve.take((long long)gq.Nz * gq.Nx);
+        m.a1 = carve.take((long long)(gq.Nz + 1) * (gq.Nx + 1));
+        m.a2 = carve.take(gq.NW);
+        m.a3 = carve.take(gq.NU);
+        m.a4 = carve.take(3LL * (gq.Nx + 2));
+      } else {
+        m.a0 = carve.take(10LL * gq.NW);
+        m.a1 = carve.take(10LL * gq.NU);
+      }
+      m.x = carve.take((long long)gq.NW + gq.NU);
+      m.y = carve.take((long long)gq.NW + gq.NU);
+      m.b = carve.take((long long)gq.NW + gq.NU);
+      for (int d = 0; d < 4; ++d) m.dv[d] = stage_div(gq.Nz - 1 + d > 0 ? gq.Nz - 1 + d : 1);
+    }
+    const long long nd = (long long)H.vg[lc].NW + H.vg[lc].NU;
+    M.inv = H.vdirect ? carve.take(nd * nd) : -1;
+    M.total = carve.at;
+    StageList S;
+    S.count = 0;
+    for (int q = l; q <= lc; ++q) {
+      const Geo& gq = H.vg[q];
+      const StageLevel& m = M.l[q];
+      const int e = (int)sizeof(T);
+      if (kFly<T>) {
+        S.add(L.op[q].eta, e * m.a0, (long long)e * gq.Nz * gq.Nx);
+        S.add(L.op[q].etaco, e * m.a1, (long long)e * (gq.Nz + 1) * (gq.Nx + 1));
+        S.add(L.op[q].dw, e * m.a2, (long long)e * gq.NW);
+        S.add(L.op[q].du, e * m.a3, (long long)e * gq.NU);
+        if (k.open_cnv) S.add(L.op[q].dbot, e * m.a4, 3LL * e * (gq.Nx + 2));
+      } else {
+        S.add(L.op[q].cw, e * m.a0, 10LL * e * gq.NW);
+        S.add(L.op[q].cu, e * m.a1, 10LL * e * gq.NU);
+      }
+    }
+    if (H.vdirect) S.add(H.vinv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * nd);
+    const int rows = (std::max(vel_stage_rows(g), 128) + 31) / 32 * 32;
+    if (rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
+      pdl_smem(PDL_ON, vel_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, kf, l,
+               lc, cfg.nu, om, coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx),
+               (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok, vel_wide(H, lc));
+      XC_LAUNCH_CHECK();
+      return XC_OK;
+    }
+    pdl_smem(PDL_ON, vel_vcycle_small_kernel<T>, 1, coarse_threads(n), 0, s, L, kf, l, lc, cfg.nu, om,
+             coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx), (const T*)(H.vdirect ? H.vinv : nullptr),
+             (const int*)H.dok, vel_wide(H, lc));
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
-  if (vel_coarsest(H, cfg, l)) {
+  if (route == kRouteCoarsest) {
     const int* solved = nullptr;
     if (H.vwide_on && n > kWideCta) {
       const WideInverse wi = vel_wide(H, l);
@@ -3033,9 +3713,17 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
       }
       solved = H.dok;
     }
-    pdl(PDL_ON, vel_coarse_kernel<T>, 1, coarse_threads(n), s, g, k, vop(H, l), H.vx[l], H.vx2[l], H.vb[l],
-        coarse_sweeps(cfg, g.Nz, g.Nx), om, (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok,
-        solved ? WideInverse{nullptr, 0} : vel_wide(H, l), solved);
+    const size_t sweep_bytes = 2 * sizeof(T) * (size_t)n;
+    const int rows = vel_stage_rows(g);
+    const WideInverse wi = solved ? WideInverse{nullptr, 0} : vel_wide(H, l);
+    if (rows <= 2 * kCoarseRegThreads && sweep_bytes <= kSweepSmemMax)
+      pdl_smem(PDL_ON, vel_coarse_reg_kernel<T>, 1, std::max(128, (rows + 63) / 64 * 32), sweep_bytes, s, g, k, vop(H, l),
+               H.vx[l], (const T*)H.vb[l], coarse_sweeps(cfg, g.Nz, g.Nx), om, (const T*)(H.vdirect ? H.vinv : nullptr),
+               (const int*)H.dok, wi, solved, stage_div(std::max(1, g.Nz - 1)), stage_div(g.Nz));
+    else
+      pdl(PDL_ON, vel_coarse_kernel<T>, 1, coarse_threads(n), s, g, k, vop(H, l), H.vx[l], H.vx2[l],
+          (const T*)H.vb[l], coarse_sweeps(cfg, g.Nz, g.Nx), om, (const T*)(H.vdirect ? H.vinv : nullptr),
+          (const int*)H.dok, wi, solved);
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
@@ -3045,17 +3733,20 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
   const T* no = nullptr;
   T* a = (cfg.nu - 1) % 2 ? H.vx2[l] : H.vx[l];
   T* o = (cfg.nu - 1) % 2 ? H.vx[l] : H.vx2[l];
-  launch_sweep<T, 0>(cfg, g, k, op, a, H.vb[l], a, om, no, s);
+  if (!x0_done) launch_sweep<T, 0>(cfg, g, k, op, a, H.vb[l], a, om, no, s);
   for (int q = 1; q < cfg.nu; ++q) {
     launch_sweep<T, 1>(cfg, g, k, op, a, H.vb[l], o, om, no, s);
     T* tmp = a; a = o; o = tmp;
   }
   launch_sweep<T, 2>(cfg, g, k, op, H.vx[l], H.vb[l], H.vr[l], om, no, s);
   const Geo& c = H.vg[l + 1];
-  pdl(PDL_ON, vel_restrict2d_kernel<T>, grid2(c), blk2(), s, g, c, H.vr[l], H.vb[l + 1]);
+  const bool x0_next = vel_route(H, cfg, l + 1) == kRouteGrid && !vel_in_cluster(H, cfg, l + 1);
+  T* x0 = x0_next ? ((cfg.nu - 1) % 2 ? H.vx2[l + 1] : H.vx[l + 1]) : nullptr;
+  pdl(PDL_ON, vel_restrict2d_kernel<T>, grid2(c, split_rows(c) ? 2 : 1), blk2(), s, g, c, H.vr[l], H.vb[l + 1],
+      level_const(kf, l + 1), vop(H, l + 1), om, x0);
   XC_LAUNCH_CHECK();
-  XC_TRY(vcycle_vel<T>(H, kf, cfg, l + 1, s));
-  pdl(PDL_ON, vel_prolong2d_kernel<T>, grid2(g), blk2(), s, g, c, k, H.vx[l + 1], H.vx[l]);
+  XC_TRY(vcycle_vel<T>(H, kf, cfg, l + 1, s, nullptr, nullptr, nullptr, x0_next));
+  pdl(PDL_ON, vel_prolong2d_kernel<T>, grid2(g, split_rows(g) ? 2 : 1), blk2(), s, g, c, k, H.vx[l + 1], H.vx[l]);
   a = H.vx[l];
   o = H.vx2[l];
   const int npost = cfg.nu_post;
@@ -3078,31 +3769,61 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
 // ---- pressure V-cycle on level l: solve L x = pb[l] approximately; *res is
 // the buffer holding x (px[l] or px2[l]: the sweeps alternate between the two
 // and no copy is made)
+// x0_done: px[l] holds the first sweep from zero (made by the level above)
 template <typename T>
-int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
+int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res, bool x0_done = false) {
   const int Nz = H.pNz[l], Nx = H.pNx[l], n = Nz * Nx;
   const T om = (T)cfg.omega_p;
   *res = H.px[l];
-  int lc_small = l;
-  while (!p_coarsest(H, cfg, lc_small)) ++lc_small;
-  const bool grid_coarse = H.pwide_on && H.pNz[lc_small] * H.pNx[lc_small] > kWideCta;
-  if (!p_coarsest(H, cfg, l) && (long long)n <= cfg.small_cells && !grid_coarse) {
-    const int lc = lc_small;
+  const int route = p_route(H, cfg, l);
+  if (route == kRouteCta) {
+    int lc = l;
+    while (!p_coarsest(H, cfg, lc)) ++lc;
     PLevels<T> L;
     for (int q = 0; q <= lc; ++q) {
       L.Nz[q] = H.pNz[q]; L.Nx[q] = H.pNx[q]; L.pin[q] = H.ppin[q]; L.dpin[q] = H.pdpin[q];
       L.kx[q] = H.kx[q]; L.kz[q] = H.kz[q];
       L.x[q] = H.px[q]; L.x2[q] = H.px2[q]; L.b[q] = H.pb[q]; L.r[q] = H.pr[q];
     }
-    const size_t bytes = sizeof(T) * (size_t)p_stage_elems<T>(H.pNz, H.pNx, l, lc);
-    const int staged = cfg.stage_small && bytes <= kStageMaxBytes;
-    pdl_smem(PDL_ON, p_vcycle_small_kernel<T>, 1, coarse_threads(n), staged ? bytes : 0, s, L, l, lc, cfg.nu_p, om,
-             coarse_sweeps(cfg, H.pNz[lc], H.pNx[lc]), staged, H.pdirect ? H.pinv : nullptr, H.dok + 1,
-             p_wide(H, lc));
+    StageMap M;
+    StageCarve<T> carve;
+    for (int q = l; q <= lc; ++q) {
+      const long long nq = (long long)H.pNz[q] * H.pNx[q];
+      StageLevel& m = M.l[q];
+      m.a0 = carve.take(nq);
+      m.a1 = carve.take(nq + H.pNx[q]);
+      m.x = carve.take(nq);
+      m.y = carve.take(nq);
+      m.b = carve.take(nq);
+      m.dv[1] = stage_div(H.pNz[q]);
+    }
+    const long long nd = (long long)H.pNz[lc] * H.pNx[lc];
+    M.inv = H.pdirect ? carve.take(nd * nd) : -1;
+    M.total = carve.at;
+    StageList S;
+    S.count = 0;
+    for (int q = l; q <= lc; ++q) {
+      const int e = (int)sizeof(T);
+      const long long nq = (long long)H.pNz[q] * H.pNx[q];
+      S.add(L.kx[q], e * M.l[q].a0, e * nq);
+      S.add(L.kz[q], e * M.l[q].a1, e * (nq + H.pNx[q]));
+    }
+    if (H.pdirect) S.add(H.pinv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * nd);
+    const int rows = (std::max(n, 128) + 31) / 32 * 32;
+    if (rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
+      pdl_smem(PDL_ON, p_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, l, lc,
+               cfg.nu_p, om, coarse_sweeps(cfg, H.pNz[lc], H.pNx[lc]), (const T*)(H.pdirect ? H.pinv : nullptr),
+               (const int*)(H.dok + 1), p_wide(H, lc));
+      XC_LAUNCH_CHECK();
+      return XC_OK;
+    }
+    pdl_smem(PDL_ON, p_vcycle_small_kernel<T>, 1, coarse_threads(n), 0, s, L, l, lc, cfg.nu_p, om,
+             coarse_sweeps(cfg, H.pNz[lc], H.pNx[lc]), (const T*)(H.pdirect ? H.pinv : nullptr),
+             (const int*)(H.dok + 1), p_wide(H, lc));
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
-  if (p_coarsest(H, cfg, l)) {
+  if (route == kRouteCoarsest) {
     const int* solved = nullptr;
     if (H.pwide_on && n > kWideCta) {
       const WideInverse wi = p_wide(H, l);
@@ -3114,32 +3835,40 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
       }
       solved = H.dok + 1;
     }
-    pdl(PDL_ON, p_coarse_kernel<T>, 1, coarse_threads(n), s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], H.px[l],
-        H.px2[l], H.pb[l], coarse_sweeps(cfg, Nz, Nx), om, (const T*)(H.pdirect ? H.pinv : nullptr),
-        (const int*)(H.dok + 1), solved ? WideInverse{nullptr, 0} : p_wide(H, l), solved);
+    const size_t sweep_bytes = 2 * sizeof(T) * (size_t)n;
+    const int in_smem = sweep_bytes <= kSweepSmemMax;
+    pdl_smem(PDL_ON, p_coarse_kernel<T>, 1, coarse_threads(2LL * n), in_smem ? sweep_bytes : 0, s, Nz, Nx, H.kx[l], H.kz[l],
+             H.ppin[l], H.pdpin[l], H.px[l], H.px2[l], H.pb[l], coarse_sweeps(cfg, Nz, Nx), om,
+             (const T*)(H.pdirect ? H.pinv : nullptr), (const int*)(H.dok + 1),
+             solved ? WideInverse{nullptr, 0} : p_wide(H, l), solved, in_smem);
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
   const int Nzc = H.pNz[l + 1], Nxc = H.pNx[l + 1];
   T* ec = nullptr;
   if ((long long)n > cfg.pfuse_cells) {
-    // one launch per operation (same values as the fused path below)
-    pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], H.px[l], H.pb[l],
-                                               H.px[l], om, 1);
+    const dim3 tiles((unsigned)((Nz + kFJ - 1) / kFJ), (unsigned)((Nx + kFI - 1) / kFI));
     T* a = H.px[l];
     T* o = H.px2[l];
+    if (cfg.nu_p > 1 && !x0_done)
+      pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l], a,
+          om, 1);
     for (int q = 1; q < cfg.nu_p; ++q) {
       pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l], o,
-                                                 om, 0);
+          om, 0);
       T* tmp = a; a = o; o = tmp;
     }
-    pdl(PDL_ON, p_residual_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l],
-                                                 H.pr[l]);
-    pdl(PDL_ON, p_restrict_kernel<T>, nblk(Nzc * Nxc), 256, s, Nzc, Nxc, H.pr[l], H.pb[l + 1]);
+    PCoarse<T> C = {};
+    const bool x0_next = p_route(H, cfg, l + 1) == kRouteGrid && (long long)Nzc * Nxc > cfg.pfuse_cells;
+    if (x0_next) C = {H.px[l + 1], H.kx[l + 1], H.kz[l + 1], H.ppin[l + 1], H.pdpin[l + 1]};
+    pdl(PDL_ON, p_down_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+        H.pdpin[l], a, (const T*)H.pb[l], H.pb[l + 1], om, cfg.nu_p > 1 || x0_done ? 0 : 1, C);
     XC_LAUNCH_CHECK();
-    XC_TRY(vcycle_p<T>(H, cfg, l + 1, s, &ec));
-    pdl(PDL_ON, p_prolong_kernel<T>, nblk(n), 256, s, Nzc, Nxc, ec, a);
-    for (int q = 0; q < cfg.nu_p; ++q) {
+    XC_TRY(vcycle_p<T>(H, cfg, l + 1, s, &ec, x0_next));
+    pdl(PDL_ON, p_up_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+        H.pdpin[l], (const T*)ec, (const T*)a, (const T*)H.pb[l], o, om);
+    { T* tmp = a; a = o; o = tmp; }
+    for (int q = 1; q < cfg.nu_p; ++q) {
       pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l], o,
                                                  om, 0);
       T* tmp = a; a = o; o = tmp;
@@ -3196,7 +3925,7 @@ int precond(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, co
   T* px0 = nullptr;
   XC_TRY(vcycle_p<T>(H, cfg, 0, s, &px0));
   T* zp = out + nvv;   // physical z_p written directly into out, rescaled below
-  pdl(PDL_ON, p_scatter_fused_kernel<T>, nblk(g.NP), 256, s, g, (const T*)px0, v + nvv, (const T*)(H.scl + nvv),
+  pdl(PDL_ON, p_scatter_fused_kernel<T>, grid2(g), blk2(), s, g, (const T*)px0, v + nvv, (const T*)(H.scl + nvv),
       (const T*)H.etarho, (T)cfg.cmass, k.open_cnv, zp);
   // velocity: rhs r_v - GG z_p, one V-cycle
   pdl(PDL_ON, sub_grad_kernel<T>, nblk(nvv), 256, s, g, zp, v, H.scl, H.vb[0]);
@@ -3219,7 +3948,7 @@ int apply_scaled(StokesWork* w, Hier<T>& H, const OpConst& k, const T* v, const 
   const Geo& g = w->g;
   const long long n = (long long)g.NW + g.NU + g.NP;
   pdl(PDL_ON, mul_kernel<T>, nblk(n), 256, s, n, v, H.scl, H.t);
-  pdl(PDL_ON, stokes_apply_kernel<T>, grid2(g), blk2(), s, g, k, vop(H, 0), H.cp, H.scl, H.t, b, y);
+  pdl(PDL_ON, stokes_apply_kernel<T>, grid2(g, split_rows(g) ? 3 : 1), blk2(), s, g, k, vop(H, 0), H.cp, H.scl, H.t, b, y);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
@@ -3249,9 +3978,11 @@ void md_grid_init() {
 // the number of partial rows written
 template <typename T>
 int launch_multidot(long long n, int m, const T* V, long long ldv, const T* wv, double* part, cudaStream_t s) {
-  const int* gr = g_md_grid[std::is_same<T, float>::value ? 0 : 1];
-  int nb;
-  nb = gr[0];
+  // no more CTAs than hold an element: the others' partial sums would be zeros
+  const int* all = g_md_grid[std::is_same<T, float>::value ? 0 : 1];
+  const int most = (int)std::min<long long>(KGMAX, (n + KB - 1) / KB);
+  const int gr[3] = {std::min(all[0], most), std::min(all[1], most), std::min(all[2], most)};
+  int nb = gr[0];
   switch (m) {
     case 1: pdl(PDL_ON, multidot_kernel<T, 1, true>, nb, KB, s, n, m, V, ldv, wv, part); return nb;
     case 2: pdl(PDL_ON, multidot_kernel<T, 2, true>, nb, KB, s, n, m, V, ldv, wv, part); return nb;
@@ -3431,7 +4162,7 @@ int arnoldi_launches(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg
   const bool zphys = with_precond && cfg.learned == 0;
   if (with_precond) XC_TRY(apply_precond<T>(w, H, k, cfg, vk, zk, s, zphys));
   if (zphys) {
-    pdl(PDL_ON, stokes_apply_kernel<T>, grid2(g), blk2(), s, g, k, vop(H, 0), (const T*)H.cp, (const T*)H.scl,
+    pdl(PDL_ON, stokes_apply_kernel<T>, grid2(g, split_rows(g) ? 3 : 1), blk2(), s, g, k, vop(H, 0), (const T*)H.cp, (const T*)H.scl,
         (const T*)zk, (const T*)nullptr, wv);
   } else {
     XC_TRY(apply_scaled<T>(w, H, k, zk, nullptr, wv, s));
@@ -4110,10 +4841,10 @@ int stokes_create(xc_ctx* c) {
   }
   std::call_once(g_md_once, md_grid_init);
   // the one-CTA V-cycles stage their levels in up to kStageMaxBytes of shared memory
-  cudaFuncSetAttribute(vel_vcycle_small_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
-  cudaFuncSetAttribute(vel_vcycle_small_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
-  cudaFuncSetAttribute(p_vcycle_small_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
-  cudaFuncSetAttribute(p_vcycle_small_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
+  cudaFuncSetAttribute(vel_vcycle_stage_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
+  cudaFuncSetAttribute(vel_vcycle_stage_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
+  cudaFuncSetAttribute(p_vcycle_stage_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
+  cudaFuncSetAttribute(p_vcycle_stage_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxBytes);
   XC_CUDA_TRY(cudaGetLastError());
   StokesWork* w = new StokesWork();
   std::memset((void*)w, 0, sizeof(StokesWork));
@@ -4458,7 +5189,7 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
     double relres_before = 0.0;
     for (int outer = 0; outer < 50; ++outer) {
       // res = S RR - S LL x (FP64), the operator applied to the physical x
-      pdl(PDL_ON, stokes_apply_kernel<double>, grid2(g), blk2(), s, g, k, vop(w->d, 0), w->d.cp, w->d.scl, w->x,
+      pdl(PDL_ON, stokes_apply_kernel<double>, grid2(g, split_rows(g) ? 3 : 1), blk2(), s, g, k, vop(w->d, 0), w->d.cp, w->d.scl, w->x,
           (const double*)w->r, res);
       XC_LAUNCH_CHECK();
       XC_TRY(dot_self<double>(w, w->d, res, n, 3, s));
