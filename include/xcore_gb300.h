@@ -148,8 +148,9 @@ typedef struct xc_solver_opts {
                               graph whose gate kernel skips it once the cycle has stopped, the
                               host queueing the next step before the current one ends (same
                               iterations; measured 7% slower at 1024^2: an IF node costs more
-                              than the host round trip it removes).  0: on the host, one
-                              synchronisation per Arnoldi step */
+                              than the host round trip it removes).  0: on the host, which reads
+                              every step's outcome but queues the step after it beforehand where
+                              it expects the cycle to go on */
   int cluster_cells;       /* velocity multigrid levels below the finest with more than small_cells
                               and at most this many cells run their part of the V-cycle in one
                               launch of a thread-block cluster (16 CTAs; cluster barriers between

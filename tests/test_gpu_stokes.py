@@ -409,3 +409,30 @@ def test_small_level_kernels_give_the_tiled_results(shape, bc):
     assert out[0][0] == out[1][0]
     for a, b in zip(out[0][1], out[1][1]):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("maxit", [1, 2, 3, 8, 9, 17])
+def test_steps_queued_ahead_do_not_count(maxit):
+    """The host queues an Arnoldi step before it has seen the one before it.  A tolerance at the edge of FP64 ends
+    the solve after exactly maxit steps at every place in a cycle of 8, unless it converges in fewer, and a solve that
+    follows gives the bits of one in a fresh context: no step queued too many is counted or leaves anything behind."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=32, Nx=40, steps=1)
+    coefs = O.time_coefs("bd2im", 2)
+    out = []
+    for stop_first in (True, False):
+        ds = device_state(par, g, sc, st)
+        start = {k: ds[k] for k in ("W", "U", "P", "MFS")}
+        if stop_first:
+            try:
+                its = ds.fluidmech(coefs, dt, solver="fgmres64", rtol=1e-14, maxit=maxit, restart=8)["iterations"]
+                assert its <= maxit, its
+            except xc.NotConverged as e:
+                assert int(str(e).split(" after ")[1].split()[0]) == maxit, str(e)
+            for k, v in start.items():
+                ds[k] = v
+        infos = [ds.fluidmech(coefs, dt, solver=sv, rtol=1e-9, restart=8) for sv in ("fgmres64", "mixed")]
+        out.append(([i["iterations"] for i in infos], [ds[k] for k in ("W", "U", "P")]))
+        ds.close()
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)

@@ -2923,13 +2923,15 @@ __global__ void multidot_final_kernel(int m, int nb, const double* __restrict__ 
   if (threadIdx.x == 0) out[k] = acc;
 }
 // ||v||^2 from one partial column -> *nrm2, and 1/||v|| (1 for a zero norm) -> *inv
-__global__ void norm_final_kernel(int nb, const double* __restrict__ part, double* nrm2, double* inv) {
+// and to the host's mirror (may be null)
+__global__ void norm_final_kernel(int nb, const double* __restrict__ part, double* nrm2, double* inv, double* host) {
   XC_PDL_WAIT();
   double acc = 0;
   for (int b = threadIdx.x; b < nb; b += KB) acc += part[b];
   acc = halving_sum(acc);
   if (threadIdx.x == 0) {
     *nrm2 = acc;
+    if (host) *host = acc;
     *inv = acc > 0.0 ? xc_div(1.0, xc_sqrt(acc)) : 1.0;
   }
 }
@@ -2996,24 +2998,45 @@ __device__ __forceinline__ T combine_sum(const T* ys, int m, const T* zk, long l
   return (a0 + a1) + (a2 + a3);
 }
 // x += sum_k y[k] Z[k], or with dscl: x += (sum_k y[k] Z[k]) / dscl (the
-// basis held in physical variables, Z[k] = S z_k of the scaled system)
+// basis held in physical variables, Z[k] = S z_k of the scaled system).  The
+// coefficients come as a parameter (no copy to wait for).  fresh: x counts as
+// zero.  xr: the refinement update xr += sr x along with it (FP64; sr the scaling)
+struct CombineCoef { double y[kMaxRestart]; };
 template <typename T>
 __global__ void combine_kernel(long long n, int m, const T* __restrict__ Z, long long ldz,
-                               const double* __restrict__ y, T* x, const T* __restrict__ dscl) {
+                               const __grid_constant__ CombineCoef y, T* x, const T* __restrict__ dscl, int fresh,
+                               const double* __restrict__ sr, double* xr) {
   XC_PDL_WAIT();
-  __shared__ T ys[64];
-  if (threadIdx.x < m) ys[threadIdx.x] = (T)y[threadIdx.x];
+  __shared__ T ys[kMaxRestart];
+  if (threadIdx.x < m) ys[threadIdx.x] = (T)y.y[threadIdx.x];
   __syncthreads();
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n) return;
   const T* zk = Z + t;
+  const T x0 = fresh ? (T)0 : x[t];
+  T s;
   if (dscl) {
-    x[t] += combine_sum<T>(ys, m, zk, ldz) / dscl[t];
-    return;
+    s = x0 + combine_sum<T>(ys, m, zk, ldz) / dscl[t];
+  } else {
+    s = x0;
+    for (int k = 0; k < m; ++k, zk += ldz) s += ys[k] * *zk;
   }
-  T s = x[t];
-  for (int k = 0; k < m; ++k, zk += ldz) s += ys[k] * *zk;
   x[t] = s;
+  if (xr) xr[t] += sr[t] * (double)s;
+}
+// the start of an inner solve: its FP32 right-hand side rhs = r and first basis
+// vector v = rhs * inv
+__global__ void inner_start_kernel(long long n, const double* __restrict__ inv, const double* __restrict__ r,
+                                   float* rhs, float* v) {
+  XC_PDL_WAIT();
+  __shared__ float f;
+  if (threadIdx.x == 0) f = (float)__ldg(inv);
+  __syncthreads();
+  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const float a = (float)r[t];
+  rhs[t] = a;
+  v[t] = a * f;
 }
 // v = w * inv with a scale factor computed once elsewhere (a per-CTA FP64
 // reciprocal in front of a barrier stalls every CTA of the grid).  The factor
@@ -3029,10 +3052,14 @@ __global__ void scale_kernel(long long n, const double* __restrict__ inv, const 
   if (t < n) v[t] = w[t] * f;
 }
 // v *= inv (inv = 1/||v|| from norm_final_kernel; 1 on a zero norm, which the
-// host reports as breakdown)
+// host reports as breakdown).  The first CTA also writes the step's scalars,
+// count of them, to their pinned mirror on the host: a copy node behind this
+// kernel took 6 us of every step.
 template <typename T>
-__global__ void normalize_kernel(long long n, const double* __restrict__ inv, T* v) {
+__global__ void normalize_kernel(long long n, const double* __restrict__ inv, T* v, const double* __restrict__ dev,
+                                 double* host, int count) {
   XC_PDL_WAIT();
+  if (host && blockIdx.x == 0 && threadIdx.x < count) host[threadIdx.x] = dev[threadIdx.x];
   __shared__ T f;
   if (threadIdx.x == 0) f = (T)__ldg(inv);
   __syncthreads();
@@ -3330,6 +3357,7 @@ struct Hier {
   KrylovStatus* ks_host;
   KrylovStatus* ks_dev;
   cudaEvent_t kev[2];
+  int expect;         // steps of the last cycle of the solve under way (0: none yet)
   bool cond_broken;   // building a conditional graph failed: host Givens from then on
 };
 
@@ -3348,7 +3376,7 @@ struct StokesWork {
   double* r;      // scaled residual (double)
   double* part;   // multidot partials
   double* hdev;   // device small vectors (2 * kMaxRestart + 8)
-  double* hhost;  // pinned host mirror
+  double* hhost;  // pinned host mirror, twice: steps take turns (step_mirror)
   // momentum advection scratch
   double *fz, *uz, *wz, *fx, *ux, *wx, *advz, *advx;
   double *srcw, *srcu, *srcp;
@@ -3999,11 +4027,17 @@ int launch_multidot(long long n, int m, const T* V, long long ldv, const T* wv, 
   return nb;
 }
 
-// ||v||^2 -> hdev[slot] (device), deterministic; 1/||v|| -> hdev[6]
+// where step kk's scalars arrive on the host; the next step, which may be queued
+// before the host has read them, writes to the other
+constexpr int kMirror = 8 + 2 * kMaxRestart;
+static_assert(kMirror <= 256, "written by one CTA of normalize_kernel");
+inline double* step_mirror(StokesWork* w, int kk) { return w->hhost + (kk & 1) * kMirror; }
+
+// ||v||^2 -> hdev[slot] and hhost[slot], deterministic; 1/||v|| -> hdev[6]
 template <typename T>
 int dot_self(StokesWork* w, Hier<T>& H, const T* v, long long n, int slot, cudaStream_t s) {
   const int nb = launch_multidot<T>(n, 1, v, n, v, w->part, s);
-  pdl(PDL_ON, norm_final_kernel, 1, KB, s, nb, w->part, w->hdev + slot, w->hdev + 6);
+  pdl(PDL_ON, norm_final_kernel, 1, KB, s, nb, w->part, w->hdev + slot, w->hdev + 6, w->hhost + slot);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
@@ -4178,12 +4212,12 @@ int arnoldi_launches(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg
       const int nbn = (int)std::min<long long>(nblk(n), (long long)KGMAX);
       pdl(PDL_ON, multiaxpy_norm_kernel<T>, nbn, KB, s, n, kk + 1, (const T*)H.V, n,
           (const double*)(hd + pass * kMaxRestart), wv, w->part);
-      pdl(PDL_ON, norm_final_kernel, 1, KB, s, nbn, (const double*)w->part, w->hdev + 2, w->hdev + 6);
+      pdl(PDL_ON, norm_final_kernel, 1, KB, s, nbn, (const double*)w->part, w->hdev + 2, w->hdev + 6,
+          (double*)nullptr);
     }
   }
-  pdl(PDL_ON, normalize_kernel<T>, nblk(n), 256, s, n, w->hdev + 6, wv);
-  if (host_copy)
-    XC_CUDA_TRY(cudaMemcpyAsync(w->hhost, w->hdev, sizeof(double) * (8 + 2 * kMaxRestart), cudaMemcpyDeviceToHost, s));
+  pdl(PDL_ON, normalize_kernel<T>, nblk(n), 256, s, n, (const double*)(w->hdev + 6), wv, (const double*)w->hdev,
+      host_copy ? step_mirror(w, kk) : (double*)nullptr, kMirror);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
@@ -4474,35 +4508,49 @@ struct HessLS {
 // solve whose caller forms the exact FP64 residual anyway).
 constexpr int FG_ZERO_GUESS = 1;
 constexpr int FG_TRUST_EST = 2;
+constexpr int FG_STARTED = 4;
 
 // Right-preconditioned FGMRES(m) on the scaled system S LL S y = rhs, from the
 // initial guess in H.y (updated in place).  *its_out = iterations used,
 // *relres_out = ||rhs - A y|| / ||rhs|| of the true residual at the last restart
 // (the estimate under FG_TRUST_EST).
-// rhs_norm2 >= 0 (with FG_ZERO_GUESS): ||rhs||^2 is known on the host and its
-// reciprocal root already sits in hdev[6] (the FP64 norm of the residual the
-// FP32 rhs was rounded from), so no reduction or synchronisation is needed
+// rhs_norm2 >= 0 (with FG_ZERO_GUESS): ||rhs||^2 is known on the host and V[0] =
+// rhs / ||rhs|| already formed.
+// FG_STARTED: step 0 is queued too, its end in H.kev[0].
+// tail (may be null): the FP64 refinement update of a solve that ends with its
+// first cycle goes along with the combine, tail->done says so.
+//
+// A step's outcome takes the host some 12 us to read and answer, in which the
+// GPU would stand idle.  So the host queues the step after one it has not seen
+// yet where it expects the cycle to go on: as many steps as the cycle before
+// took, or while the estimate, falling as it did and half again as fast, stays
+// above the tolerance.  A step too many leaves nothing behind (its vectors are
+// not combined); at 512^2 and below it costs less than two waits.
+struct RefineTail {
+  const double* scl;
+  double* x;
+  bool done;
+};
 template <typename T>
 int fgmres(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, const T* rhs, double rtol,
-           int maxit, int* its_out, double* relres_out, cudaStream_t s, int flags = 0, double rhs_norm2 = -1.0) {
+           int maxit, int* its_out, double* relres_out, cudaStream_t s, int flags = 0, double rhs_norm2 = -1.0,
+           RefineTail* tail = nullptr) {
   const Geo& g = w->g;
   const long long n = (long long)g.NW + g.NU + g.NP;
   const int m = H.m;
   double* hh = w->hhost;
   const bool zero = (flags & FG_ZERO_GUESS) != 0;
   const bool known = zero && rhs_norm2 >= 0.0;
-  if (!known) XC_TRY(dot_self<T>(w, H, rhs, n, 0, s));
-  if (zero) {
-    XC_CUDA_TRY(cudaMemsetAsync(H.y, 0, sizeof(T) * n, s));
-    // V[0] = rhs / ||rhs|| with the reciprocal left on the device
-    scale_kernel<T><<<nblk(n), 256, 0, s>>>(n, w->hdev + 6, rhs, H.V); xc_count_launch();
-  }
   double rhs2 = rhs_norm2;
   if (!known) {
-    XC_CUDA_TRY(cudaMemcpyAsync(hh, w->hdev, sizeof(double), cudaMemcpyDeviceToHost, s));
+    XC_TRY(dot_self<T>(w, H, rhs, n, 0, s));
+    // V[0] = rhs / ||rhs|| with the reciprocal left on the device
+    if (zero) { scale_kernel<T><<<nblk(n), 256, 0, s>>>(n, w->hdev + 6, rhs, H.V); xc_count_launch(); }
     XC_CUDA_TRY(cudaStreamSynchronize(s));
     rhs2 = hh[0];
   }
+  bool fresh = zero;       // y still counts as zero
+  int launched = (flags & FG_STARTED) ? 1 : 0;
   const double bnorm = std::sqrt(rhs2) > 0 ? std::sqrt(rhs2) : 1.0;
   int its = 0;
   double relres = 1.0;
@@ -4512,12 +4560,14 @@ int fgmres(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, con
     if (zero && cycle == 0) {
       beta = std::sqrt(rhs2);
       relres = beta > 0 ? 1.0 : 0.0;
-      if (!(relres > rtol) || its >= maxit) break;
+      if (!(relres > rtol) || its >= maxit) {
+        XC_CUDA_TRY(cudaMemsetAsync(H.y, 0, sizeof(T) * n, s));
+        break;
+      }
     } else {
       // r = rhs - A y  -> V[0]
       XC_TRY(apply_scaled<T>(w, H, k, H.y, rhs, H.V, s));
       XC_TRY(dot_self<T>(w, H, H.V, n, 0, s));
-      XC_CUDA_TRY(cudaMemcpyAsync(hh, w->hdev, sizeof(double), cudaMemcpyDeviceToHost, s));
       XC_CUDA_TRY(cudaStreamSynchronize(s));
       beta = std::sqrt(hh[0]);
       relres = beta / bnorm;
@@ -4526,6 +4576,8 @@ int fgmres(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, con
       scale_kernel<T><<<nblk(n), 256, 0, s>>>(n, w->hdev + 6, H.V, H.V); xc_count_launch();
     }
     if (cfg.device_givens && !H.cond_broken) {
+      if (fresh) XC_CUDA_TRY(cudaMemsetAsync(H.y, 0, sizeof(T) * n, s));
+      fresh = false;
       // the cycle with the least-squares problem on the device: the host
       // queues step kk + 1 before it looks at step kk's outcome, so the GPU
       // never waits for it; a step queued after the cycle stopped is skipped
@@ -4572,26 +4624,50 @@ int fgmres(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, con
     }
     ls.start(beta);
     int kk = 0;
+    double before = beta / bnorm;      // the estimate before the last known one
     for (; kk < m && its < maxit; ++kk) {
       // z_k = M v_k, v_{k+1} = A z_k orthogonalised and normalised, H column
-      // copied to pinned host memory -- one CUDA graph launch per iteration
-      XC_TRY(arnoldi_step<T>(w, H, k, cfg, kk, s));
-      XC_CUDA_TRY(cudaStreamSynchronize(s));
+      // written to pinned host memory -- one CUDA graph launch per iteration
+      if (launched == kk) {
+        XC_TRY(arnoldi_step<T>(w, H, k, cfg, kk, s));
+        XC_CUDA_TRY(cudaEventRecord(H.kev[kk & 1], s));
+        ++launched;
+      }
+      const bool falling = kk >= 2 && relres * (relres / before) * 0.5 > rtol;
+      if (kk + 1 < m && its + 1 < maxit && (kk + 1 < H.expect || falling)) {
+        XC_TRY(arnoldi_step<T>(w, H, k, cfg, kk + 1, s));
+        XC_CUDA_TRY(cudaEventRecord(H.kev[(kk + 1) & 1], s));
+        ++launched;
+      }
+      XC_CUDA_TRY(cudaEventSynchronize(H.kev[kk & 1]));
       XC_LAUNCH_CHECK();
-      const double hn = std::sqrt(hh[2]);
+      const double* hs = step_mirror(w, kk);
+      const double hn = std::sqrt(hs[2]);
       ++its;
-      relres = ls.add(kk, hh + 8, cfg.gs_passes > 1 ? hh + 8 + kMaxRestart : nullptr, hn) / bnorm;
-      if (!std::isfinite(relres)) { xc_set_error("fgmres: breakdown"); return XC_NAN; }
+      before = relres;
+      relres = ls.add(kk, hs + 8, cfg.gs_passes > 1 ? hs + 8 + kMaxRestart : nullptr, hn) / bnorm;
+      if (!std::isfinite(relres)) {
+        XC_CUDA_TRY(cudaStreamSynchronize(s));
+        xc_set_error("fgmres: breakdown");
+        return XC_NAN;
+      }
       if (relres <= rtol * 0.5 || hn == 0.0) { ++kk; break; }
     }
+    launched = 0;
+    H.expect = kk;
     // back substitution and update y += Z yv
     ls.solve(kk);
-    XC_CUDA_TRY(cudaMemcpyAsync(w->hdev + 8, ls.yv.data(), sizeof(double) * kk, cudaMemcpyHostToDevice, s));
-    combine_kernel<T><<<nblk(n), 256, 0, s>>>(n, kk, H.Z, n, w->hdev + 8, H.y,
-                                              cfg.learned == 0 ? (const T*)H.scl : nullptr);
+    CombineCoef coef;
+    std::copy(ls.yv.begin(), ls.yv.begin() + kk, coef.y);
+    const bool last = (flags & FG_TRUST_EST) && (relres <= rtol || its >= maxit);
+    const bool refine = last && tail && cycle == 0;
+    combine_kernel<T><<<nblk(n), 256, 0, s>>>(n, kk, H.Z, n, coef, H.y, cfg.learned == 0 ? (const T*)H.scl : nullptr,
+                                              fresh ? 1 : 0, refine ? tail->scl : nullptr, refine ? tail->x : nullptr);
     xc_count_launch();
     XC_LAUNCH_CHECK();
-    if ((flags & FG_TRUST_EST) && (relres <= rtol || its >= maxit)) break;
+    fresh = false;
+    if (refine) tail->done = true;
+    if (last) break;
   }
   *its_out = its;
   *relres_out = relres;
@@ -4613,7 +4689,6 @@ int fgmres_outer(StokesWork* w, const OpConst& k, const SolveCfg& cfg, const Sol
   const int m = H.m;
   double* hh = w->hhost;
   XC_TRY(dot_self<double>(w, H, rhs, n, 0, s));
-  XC_CUDA_TRY(cudaMemcpyAsync(hh, w->hdev, sizeof(double), cudaMemcpyDeviceToHost, s));
   XC_CUDA_TRY(cudaStreamSynchronize(s));
   const double bnorm = std::sqrt(hh[0]) > 0 ? std::sqrt(hh[0]) : 1.0;
   int its = 0, outer = 0;
@@ -4623,7 +4698,6 @@ int fgmres_outer(StokesWork* w, const OpConst& k, const SolveCfg& cfg, const Sol
   while (status == XC_OK) {
     XC_TRY(apply_scaled<double>(w, H, k, H.y, rhs, H.V, s));
     XC_TRY(dot_self<double>(w, H, H.V, n, 0, s));
-    XC_CUDA_TRY(cudaMemcpyAsync(hh, w->hdev, sizeof(double), cudaMemcpyDeviceToHost, s));
     XC_CUDA_TRY(cudaStreamSynchronize(s));
     const double beta = std::sqrt(hh[0]);
     relres = beta / bnorm;
@@ -4646,8 +4720,9 @@ int fgmres_outer(StokesWork* w, const OpConst& k, const SolveCfg& cfg, const Sol
       XC_TRY(arnoldi_launches<double>(w, H, k, cfg, kk, s, false));
       XC_CUDA_TRY(cudaStreamSynchronize(s));
       XC_LAUNCH_CHECK();
-      const double hn = std::sqrt(hh[2]);
-      relres = ls.add(kk, hh + 8, cfg.gs_passes > 1 ? hh + 8 + kMaxRestart : nullptr, hn) / bnorm;
+      const double* hs = step_mirror(w, kk);
+      const double hn = std::sqrt(hs[2]);
+      relres = ls.add(kk, hs + 8, cfg.gs_passes > 1 ? hs + 8 + kMaxRestart : nullptr, hn) / bnorm;
       if (!std::isfinite(relres)) { xc_set_error("mixed solver: breakdown"); status = XC_NAN; ++kk; break; }
       // the FP64 Arnoldi relation makes the estimate accurate far below rtol;
       // the true residual above confirms it
@@ -4655,8 +4730,10 @@ int fgmres_outer(StokesWork* w, const OpConst& k, const SolveCfg& cfg, const Sol
     }
     if (status != XC_OK) break;
     ls.solve(kk);
-    XC_CUDA_TRY(cudaMemcpyAsync(w->hdev + 8, ls.yv.data(), sizeof(double) * kk, cudaMemcpyHostToDevice, s));
-    combine_kernel<double><<<nblk(n), 256, 0, s>>>(n, kk, H.Z, n, w->hdev + 8, H.y, (const double*)nullptr);
+    CombineCoef coef;
+    std::copy(ls.yv.begin(), ls.yv.begin() + kk, coef.y);
+    combine_kernel<double><<<nblk(n), 256, 0, s>>>(n, kk, H.Z, n, coef, H.y, (const double*)nullptr, 0,
+                                                   (const double*)nullptr, (double*)nullptr);
     xc_count_launch();
     XC_LAUNCH_CHECK();
   }
@@ -4866,7 +4943,7 @@ int stokes_create(xc_ctx* c) {
   XC_CUDA_TRY(cudaMalloc(&w->r, sizeof(double) * n));
   XC_CUDA_TRY(cudaMalloc(&w->part, sizeof(double) * KGMAX * (kMaxRestart + 1)));
   XC_CUDA_TRY(cudaMalloc(&w->hdev, sizeof(double) * (8 + 2 * kMaxRestart)));
-  XC_CUDA_TRY(cudaMallocHost(&w->hhost, sizeof(double) * (8 + 2 * kMaxRestart + kMaxRestart)));
+  XC_CUDA_TRY(cudaMallocHost(&w->hhost, sizeof(double) * 2 * (8 + 2 * kMaxRestart)));
   const int Nz = g.Nz, Nx = g.Nx;
   XC_CUDA_TRY(cudaMalloc(&w->fz, sizeof(double) * (Nz - 1) * Nx));
   XC_CUDA_TRY(cudaMalloc(&w->uz, sizeof(double) * (Nz - 1) * (Nx + 1)));
@@ -5165,6 +5242,7 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
   int status = XC_OK;
   // scaled rhs S RR -> r (double)
   mul_kernel<double><<<nblk(n), 256, 0, s>>>(n, w->RR, w->d.scl, w->r); xc_count_launch();
+  w->d.expect = w->f.expect = 0;
   if (o.kind == XC_SOLVER_MIXED) {
     if (!w->f_alloc) { XC_TRY(alloc_hier<float>(w, w->f, 30)); w->f_alloc = true; }
     XC_TRY(setup_hier<float>(w, w->f, k, cfg, c, s));
@@ -5178,7 +5256,6 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
     } else {
     // plain refinement: FP64 norm of the scaled rhs
     XC_TRY(dot_self<double>(w, w->d, w->r, n, 3, s));
-    XC_CUDA_TRY(cudaMemcpyAsync(w->hhost, w->hdev, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
     XC_CUDA_TRY(cudaStreamSynchronize(s));
     const double bn = std::sqrt(w->hhost[3]) > 0 ? std::sqrt(w->hhost[3]) : 1.0;
     // the FP64 operator reuses d.V[0] as residual storage
@@ -5187,14 +5264,26 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
     // least halve the FP64 residual; the multigrid takes the rest of the solve
     bool learned_on = o.learned != 0, judge = false;
     double relres_before = 0.0;
+    double expect = 1.0;     // the last pass's reduction
     for (int outer = 0; outer < 50; ++outer) {
       // res = S RR - S LL x (FP64), the operator applied to the physical x
       pdl(PDL_ON, stokes_apply_kernel<double>, grid2(g, split_rows(g) ? 3 : 1), blk2(), s, g, k, vop(w->d, 0), w->d.cp, w->d.scl, w->x,
           (const double*)w->r, res);
       XC_LAUNCH_CHECK();
       XC_TRY(dot_self<double>(w, w->d, res, n, 3, s));
-      XC_CUDA_TRY(cudaMemcpyAsync(w->hhost, w->hdev, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
-      XC_CUDA_TRY(cudaStreamSynchronize(s));
+      // the inner solve's first step is queued before the residual is known
+      // where the last pass is expected to have left more to do
+      bool started = false;
+      if (outer > 0 && !learned_on && relres * expect > 2.0 * o.rtol && its < o.maxit) {
+        XC_CUDA_TRY(cudaEventRecord(w->f.kev[1], s));
+        inner_start_kernel<<<nblk(n), 256, 0, s>>>(n, w->hdev + 6, res, w->f.w, w->f.V); xc_count_launch();
+        XC_TRY(arnoldi_step<float>(w, w->f, k, icfg, 0, s));
+        XC_CUDA_TRY(cudaEventRecord(w->f.kev[0], s));
+        started = true;
+        XC_CUDA_TRY(cudaEventSynchronize(w->f.kev[1]));
+      } else {
+        XC_CUDA_TRY(cudaStreamSynchronize(s));
+      }
       relres = std::sqrt(w->hhost[3]) / bn;
       if (judge) {
         judge = false;
@@ -5212,19 +5301,24 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
       // inner FP32 solve of S LL S dy = res from dy = 0.  Its right-hand side
       // lives in f.w, which the FP32 Krylov and multigrid code never writes
       // (f.t is the operator's scratch, f.V / f.Z the basis).
-      convert_kernel<double, float><<<nblk(n), 256, 0, s>>>(n, res, w->f.w); xc_count_launch();
+      if (!started) {
+        inner_start_kernel<<<nblk(n), 256, 0, s>>>(n, w->hdev + 6, res, w->f.w, w->f.V); xc_count_launch();
+      }
       const float* frhs = w->f.w;
       int iits = 0;
       double irr = 1.0;
       const double rn2 = w->hhost[3];
+      RefineTail tail{w->d.scl, w->x, false};
       if (learned_on) {
         XC_CUDA_TRY(cudaMemcpyAsync(w->nn_xprev, w->x, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
         relres_before = relres;
         judge = true;
       }
       XC_TRY(fgmres<float>(w, w->f, k, learned_on ? icfg_nn : icfg, frhs, o.inner_rtol, o.inner_maxit, &iits,
-                           &irr, s, FG_ZERO_GUESS | FG_TRUST_EST, rn2));
+                           &irr, s, FG_ZERO_GUESS | FG_TRUST_EST | (started ? FG_STARTED : 0), rn2,
+                           learned_on ? nullptr : &tail));
       its += iits;
+      expect = irr;
       if (learned_on && !(irr <= o.inner_rtol)) {
         // the learned inner solve missed its reduction: the multigrid
         // preconditioner redoes this pass from zero and takes the rest of
@@ -5237,7 +5331,9 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
                              FG_ZERO_GUESS | FG_TRUST_EST, -1.0));
         its += iits;
       }
-      refine_update_kernel<float><<<nblk(n), 256, 0, s>>>(n, w->f.y, w->d.scl, w->x); xc_count_launch();
+      if (!tail.done) {
+        refine_update_kernel<float><<<nblk(n), 256, 0, s>>>(n, w->f.y, w->d.scl, w->x); xc_count_launch();
+      }
       XC_LAUNCH_CHECK();
     }
     }
@@ -5251,7 +5347,6 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
       XC_TRY(apply_scaled<double>(w, w->d, k, w->d.y, w->r, w->d.V, s));
       XC_TRY(dot_self<double>(w, w->d, w->d.V, n, 3, s));
       XC_TRY(dot_self<double>(w, w->d, w->r, n, 4, s));
-      XC_CUDA_TRY(cudaMemcpyAsync(w->hhost, w->hdev, sizeof(double) * 5, cudaMemcpyDeviceToHost, s));
       XC_CUDA_TRY(cudaStreamSynchronize(s));
       relres = std::sqrt(w->hhost[3]) / (std::sqrt(w->hhost[4]) > 0 ? std::sqrt(w->hhost[4]) : 1.0);
     }
