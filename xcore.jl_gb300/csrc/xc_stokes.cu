@@ -1944,9 +1944,9 @@ __global__ void p_up_kernel(int Nz, int Nx, const T* __restrict__ kx, const T* _
 // The same two fusions from shared-memory tiles of 32 x 8 cells, the default:
 // each value formed once, by a thread per cell of the tile and its halo (340 of
 // 352), so that a small level's launch is as long as one thread's chain.
-// p_down_tile_kernel also makes the coarse level's first sweep from zero (xc0,
-// with the coarse level's coefficients), which is pointwise; above the finest
-// level x arrives with that sweep done.  At 64^2 a
+// p_down_tile_kernel also makes the coarse level's first sweep from zero (C.x0),
+// which is pointwise; x arrives with its own done, the finest level's by
+// p_gather_fused_kernel.  At 64^2 a
 // level takes 3.5 us down and up, in place of 7.3 us for five launches.
 // (p_down_kernel / p_up_kernel form every neighbour's value anew, five diagonals
 // per cell, and measured no faster than one launch per operation.)
@@ -1962,9 +1962,9 @@ struct PCoarse {                       // the coarse level's first sweep; x0 nul
 };
 template <typename T>
 __global__ void __launch_bounds__(kTileThreads) p_down_tile_kernel(int Nz, int Nx, const T* __restrict__ kx,
-                                                                   const T* __restrict__ kz, int pin, T dpin, T* x,
-                                                                   const T* __restrict__ b, T* bc, T omega,
-                                                                   int zero_init, PCoarse<T> C) {
+                                                                   const T* __restrict__ kz, int pin, T dpin,
+                                                                   const T* __restrict__ x, const T* __restrict__ b,
+                                                                   T* bc, T omega, PCoarse<T> C) {
   XC_PDL_WAIT();
   constexpr int XJ = kFJ + 2, XI = kFI + 2;
   __shared__ T xs[XI][XJ], rs[kFI][kFJ];
@@ -1972,18 +1972,8 @@ __global__ void __launch_bounds__(kTileThreads) p_down_tile_kernel(int Nz, int N
   if (tid < XJ * XI) {
     const int ci = tid / XJ, cj = tid - ci * XJ, j = j0 - 1 + cj;
     int i = i0 - 1 + ci;
-    const bool own = cj >= 1 && cj <= kFJ && ci >= 1 && ci <= kFI && i < Nx;
     i = i < 0 ? i + Nx : (i >= Nx ? i - Nx : i);      // beyond Nx only in front of cells outside the grid
-    if (j >= 0 && j < Nz && i < Nx) {
-      T v;
-      if (zero_init) {
-        v = p_jacobi0_val<T>(Nz, Nx, kx, kz, pin, dpin, b, omega, j, i);
-        if (own) x[i * Nz + j] = v;
-      } else {
-        v = x[i * Nz + j];
-      }
-      xs[ci][cj] = v;
-    }
+    if (j >= 0 && j < Nz && i < Nx) xs[ci][cj] = x[i * Nz + j];
   }
   __syncthreads();
   if (tid < kFJ * kFI) {
@@ -2825,34 +2815,41 @@ __global__ void p_kcoef_kernel(Geo g, const double* __restrict__ rhow, const dou
 // the interior or ghost-column value it copies with the same operations (the
 // ghost rows of columns 0 and Nx+1 read ghost-column values).
 template <typename T>
-__global__ void p_gather_fused_kernel(Geo g, const T* __restrict__ kx, const T* __restrict__ kr,
-                                      const T* __restrict__ vp, const T* __restrict__ sp, T* rin) {
+__global__ void __launch_bounds__(256) p_gather_fused_kernel(Geo g, const T* __restrict__ kr, const T* __restrict__ vp,
+                                                             const T* __restrict__ sp, const T* __restrict__ inv,
+                                                             T* rin, T omega, PCoarse<T> C) {
   XC_PDL_WAIT();
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
   const int Nz = g.Nz, Nx = g.Nx, lp = Nz + 2;
-  if (t >= Nz * Nx) return;
-  int j = t % Nz, i = t / Nz;
-  const size_t o = (size_t)(i + 1) * lp + j + 1;
-  T v = vp[o] / sp[o];
-  if (i == 0) v += kx[j] * (vp[j + 1] / sp[j + 1]);
+  if (j >= Nz || i >= Nx) return;
+  const T f = inv ? *inv : (T)1;       // v comes unnormalised: the basis vector is v * f
+  const int o = (i + 1) * lp + j + 1, t = i * Nz + j;
+  T v = mul_rn<T>(vp[o], f) / sp[o];
+  if (i == 0) v += C.kx[j] * (mul_rn<T>(vp[j + 1], f) / sp[j + 1]);
   if (i == Nx - 1) {
-    const size_t q = (size_t)(Nx + 1) * lp + j + 1;
-    v += kr[j] * (vp[q] / sp[q]);
+    const int q = (Nx + 1) * lp + j + 1;
+    v += kr[j] * (mul_rn<T>(vp[q], f) / sp[q]);
   }
   rin[t] = v;
+  if (C.x0) {                          // the first sweep from zero, p_jacobi0_val's operations
+    T d;
+    p_apply_fn<T>(Nz, Nx, C.kx, C.kz, C.pin, C.dpin, [](int, int) { return (T)0; }, j, i, &d);
+    C.x0[t] = d > (T)0 ? sdiv<T>(omega * v, d) : (T)0;
+  }
 }
 
 template <typename T>
 __global__ void p_scatter_fused_kernel(Geo g, const T* __restrict__ z, const T* __restrict__ vp,
-                                       const T* __restrict__ sp, const T* __restrict__ etarho, T cmass,
-                                       int open_bottom, T* zp) {
+                                       const T* __restrict__ sp, const T* __restrict__ inv,
+                                       const T* __restrict__ etarho, T cmass, int open_bottom, T* zp) {
   XC_PDL_WAIT();
   const int Nz = g.Nz, Nx = g.Nx, lp = Nz + 2;
   const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y, t = i * lp + j;
   if (j > Nz + 1 || i > Nx + 1) return;
+  const T f = inv ? *inv : (T)1;
   auto r = [&](int jj, int ii) {
-    const size_t o = (size_t)ii * lp + jj;
-    return vp[o] / sp[o];
+    const int o = ii * lp + jj;
+    return mul_rn<T>(vp[o], f) / sp[o];
   };
   auto zint = [&](int jj, int ii) {   // interior cell (1..Nz, 1..Nx)
     const int c = (ii - 1) * Nz + (jj - 1);
@@ -2872,23 +2869,45 @@ __global__ void p_scatter_fused_kernel(Geo g, const T* __restrict__ z, const T* 
 
 // velocity right-hand side of the preconditioner: rv = S^-1 v - GG z_p on the
 // interior velocity rows (fluidmech.jl:343-356), S^-1 v elsewhere -- the
-// unscaling of the residual fused with the gradient of the pressure part
+// unscaling of the residual fused with the gradient of the pressure part, and
+// with what else is pointwise here: the first sweep from zero of the finest
+// level (x0, may be null; MODE 0 of vel_update_w / vel_update_u), and where v
+// comes unnormalised (inv) the normalisation of the whole basis vector, which
+// the pressure kernels before this one read as it was.  At 1024^2 the three
+// separate launches took 13.3, 10.7 and 8.7 us; this one takes 16.8 us.
+// 2-D grid over the (Nz + 2, Nx + 2) box, layers as stokes_apply_kernel.
 template <typename T>
-__global__ void sub_grad_kernel(Geo g, const T* __restrict__ zp, const T* __restrict__ v,
-                                const T* __restrict__ scl, T* rv) {
+__global__ void __launch_bounds__(256) vel_rhs_kernel(Geo g, OpConst k, VOp<T> op, const T* __restrict__ zp, T* v,
+                                                      const T* __restrict__ scl, const T* __restrict__ inv, T* rv,
+                                                      T omega, T* x0) {
   XC_PDL_WAIT();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
   const int Nz = g.Nz, Nx = g.Nx, lw = Nz + 1, lu = Nz + 2;
-  if (t >= g.NW + g.NU) return;
-  T r = v[t] / scl[t];
-  if (t < g.NW) {
-    const int j = t % lw, i = t / lw;
+  if (j > Nz + 1 || i > Nx + 1) return;
+  const int layer = gridDim.z == 1 ? -1 : (int)blockIdx.z;
+  const T f = inv ? *inv : (T)1;
+  if (j <= Nz && (layer < 0 || layer == 0)) {
+    const int t = i * lw + j;
+    T r = v[t];
+    if (inv) { r = mul_rn<T>(r, f); v[t] = r; }
+    r = r / scl[t];
     if (j >= 1 && j <= Nz - 1 && i >= 1 && i <= Nx) r -= geo_invh<T>(g) * (zp[i * lu + j + 1] - zp[i * lu + j]);
-  } else {
-    const int u = t - g.NW, j = u % lu, i = u / lu;
-    if (j >= 1 && j <= Nz) r -= geo_invh<T>(g) * (zp[(i + 1) * lu + j] - zp[i * lu + j]);
+    rv[t] = r;
+    if (x0) x0[t] = sdiv<T>((vel_edge_w(g, j, i) ? (T)1 : omega) * r, vel_diag_w<T>(g, op, t, j, i));
   }
-  rv[t] = r;
+  if (i <= Nx && (layer < 0 || layer == 1)) {
+    const int u = i * lu + j, t = g.NW + u;
+    T r = v[t];
+    if (inv) { r = mul_rn<T>(r, f); v[t] = r; }
+    r = r / scl[t];
+    if (j >= 1 && j <= Nz) r -= geo_invh<T>(g) * (zp[(i + 1) * lu + j] - zp[i * lu + j]);
+    rv[t] = r;
+    if (x0) x0[t] = sdiv<T>((vel_edge_u(g, k, u, j) ? (T)1 : omega) * r, vel_diag_u<T>(g, k, op, u, j, i));
+  }
+  if (inv && (layer < 0 || layer == 2)) {
+    const int t = g.NW + g.NU + i * lu + j;
+    v[t] = mul_rn<T>(v[t], f);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2983,8 +3002,10 @@ __global__ void multidot_final_kernel(int m, int nb, const double* __restrict__ 
   if (threadIdx.x == 0) out[k] = acc;
 }
 // ||v||^2 from one partial column -> *nrm2, and 1/||v|| (1 for a zero norm) -> *inv
-// and to the host's mirror (may be null)
-__global__ void norm_final_kernel(int nb, const double* __restrict__ part, double* nrm2, double* inv, double* host) {
+// (in FP64, and behind it in FP32) and to the host (may be null); then count
+// scalars from dev to their mirror there (may be null)
+__global__ void norm_final_kernel(int nb, const double* __restrict__ part, double* nrm2, double* inv, double* host,
+                                  const double* dev, double* mirror, int count) {
   XC_PDL_WAIT();
   double acc = 0;
   for (int b = threadIdx.x; b < nb; b += KB) acc += part[b];
@@ -2992,8 +3013,13 @@ __global__ void norm_final_kernel(int nb, const double* __restrict__ part, doubl
   if (threadIdx.x == 0) {
     *nrm2 = acc;
     if (host) *host = acc;
-    *inv = acc > 0.0 ? xc_div(1.0, xc_sqrt(acc)) : 1.0;
+    const double f = acc > 0.0 ? xc_div(1.0, xc_sqrt(acc)) : 1.0;
+    *inv = f;
+    *reinterpret_cast<float*>(inv + 1) = (float)f;
   }
+  if (!mirror) return;
+  __syncthreads();
+  if (threadIdx.x < count) mirror[threadIdx.x] = dev[threadIdx.x];
 }
 // w -= sum_k h[k] V[k] and ||w||^2 in the same pass: per-CTA partial sums
 // (working precision per thread and warp, FP64 across warps) to part[blk],
@@ -3684,8 +3710,14 @@ int p_route(const Hier<T>& H, const SolveCfg& cfg, int l) {
   if (H.pwide_on && H.pNz[lc] * H.pNx[lc] > kWideCta) return kRouteGrid;
   return n <= cfg.small_cells ? kRouteCta : kRouteGrid;
 }
+// launches over the grid, from tiles: the first sweep from zero is made by the
+// level above, the finest level's by p_gather_fused_kernel
+template <typename T>
+bool p_tiled(const Hier<T>& H, const SolveCfg& cfg, int l) {
+  return p_route(H, cfg, l) == kRouteGrid && (long long)H.pNz[l] * H.pNx[l] > cfg.pfuse_cells;
+}
 
-// x0_done: the first sweep from zero was made by the level above
+// x0_done: the first sweep from zero was made by the launch before
 template <typename T>
 int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaStream_t s, T* final_out = nullptr,
                const T* final_scl = nullptr, bool* final_done = nullptr, bool x0_done = false) {
@@ -3857,9 +3889,9 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
 // ---- pressure V-cycle on level l: solve L x = pb[l] approximately; *res is
 // the buffer holding x (px[l] or px2[l]: the sweeps alternate between the two
 // and no copy is made)
-// x0_done: px[l] holds the first sweep from zero (made by the level above)
+// (where p_tiled, px[l] holds the first sweep from zero already)
 template <typename T>
-int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res, bool x0_done = false) {
+int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
   const int Nz = H.pNz[l], Nx = H.pNx[l], n = Nz * Nx;
   const T om = (T)cfg.omega_p;
   *res = H.px[l];
@@ -3938,21 +3970,17 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res, bo
     const dim3 tiles((unsigned)((Nz + kFJ - 1) / kFJ), (unsigned)((Nx + kFI - 1) / kFI));
     T* a = H.px[l];
     T* o = H.px2[l];
-    if (cfg.nu_p > 1 && !x0_done)
-      pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l], a,
-          om, 1);
     for (int q = 1; q < cfg.nu_p; ++q) {
       pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l], o,
           om, 0);
       T* tmp = a; a = o; o = tmp;
     }
     PCoarse<T> C = {};
-    const bool x0_next = p_route(H, cfg, l + 1) == kRouteGrid && (long long)Nzc * Nxc > cfg.pfuse_cells;
-    if (x0_next) C = {H.px[l + 1], H.kx[l + 1], H.kz[l + 1], H.ppin[l + 1], H.pdpin[l + 1]};
+    if (p_tiled(H, cfg, l + 1)) C = {H.px[l + 1], H.kx[l + 1], H.kz[l + 1], H.ppin[l + 1], H.pdpin[l + 1]};
     pdl(PDL_ON, p_down_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
-        H.pdpin[l], a, (const T*)H.pb[l], H.pb[l + 1], om, cfg.nu_p > 1 || x0_done ? 0 : 1, C);
+        H.pdpin[l], (const T*)a, (const T*)H.pb[l], H.pb[l + 1], om, C);
     XC_LAUNCH_CHECK();
-    XC_TRY(vcycle_p<T>(H, cfg, l + 1, s, &ec, x0_next));
+    XC_TRY(vcycle_p<T>(H, cfg, l + 1, s, &ec));
     pdl(PDL_ON, p_up_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
         H.pdpin[l], (const T*)ec, (const T*)a, (const T*)H.pb[l], o, om);
     { T* tmp = a; a = o; o = tmp; }
@@ -3997,36 +4025,39 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res, bo
 
 // out = M^-1 v for the scaled system: out = S^-1 M_phys (S^-1 v)
 // phys_out: out = M_phys (S^-1 v) in physical variables, without the final
-// S^-1 (the caller applies the operator to it directly)
+// S^-1 (the caller applies the operator to it directly).  inv: v is the basis
+// vector before its normalisation, which is made along (v := v * *inv)
 template <typename T>
-int precond(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, const T* v, T* out,
-            cudaStream_t s, bool phys_out = false) {
+int precond(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, T* v, T* out, cudaStream_t s,
+            bool phys_out = false, const T* inv = nullptr) {
   const Geo& g = w->g;
-  const long long n = (long long)g.NW + g.NU + g.NP;
   const long long nvv = (long long)g.NW + g.NU;
-  // physical residual r = S^-1 v: pressure part into rp here, velocity part
-  // into vb[0] by sub_grad_kernel below
+  // physical residual r = S^-1 v: pressure part into pb[0], velocity part into
+  // vb[0] by vel_rhs_kernel below
   // pressure: interior solve with ghost elimination
-  pdl(PDL_ON, p_gather_fused_kernel<T>, nblk(g.Nz * g.Nx), 256, s, g, (const T*)H.kx[0], (const T*)H.kr,
-      v + nvv, (const T*)(H.scl + nvv), H.pb[0]);
+  PCoarse<T> C = {p_tiled(H, cfg, 0) ? H.px[0] : nullptr, H.kx[0], H.kz[0], H.ppin[0], H.pdpin[0]};
+  pdl(PDL_ON, p_gather_fused_kernel<T>, grid2(g), blk2(), s, g, (const T*)H.kr, (const T*)(v + nvv),
+      (const T*)(H.scl + nvv), inv, H.pb[0], (T)cfg.omega_p, C);
   XC_LAUNCH_CHECK();
   T* px0 = nullptr;
   XC_TRY(vcycle_p<T>(H, cfg, 0, s, &px0));
   T* zp = out + nvv;   // physical z_p written directly into out, rescaled below
-  pdl(PDL_ON, p_scatter_fused_kernel<T>, grid2(g), blk2(), s, g, (const T*)px0, v + nvv, (const T*)(H.scl + nvv),
-      (const T*)H.etarho, (T)cfg.cmass, k.open_cnv, zp);
+  pdl(PDL_ON, p_scatter_fused_kernel<T>, grid2(g), blk2(), s, g, (const T*)px0, (const T*)(v + nvv),
+      (const T*)(H.scl + nvv), inv, (const T*)H.etarho, (T)cfg.cmass, k.open_cnv, zp);
   // velocity: rhs r_v - GG z_p, one V-cycle
-  pdl(PDL_ON, sub_grad_kernel<T>, nblk(nvv), 256, s, g, zp, v, H.scl, H.vb[0]);
+  const bool x0 = vel_route(H, cfg, 0) == kRouteGrid;
+  pdl(PDL_ON, vel_rhs_kernel<T>, grid2(g, split_rows(g) ? 3 : 1), blk2(), s, g, level_const(k, 0), vop(H, 0),
+      (const T*)zp, v, (const T*)H.scl, inv, H.vb[0], (T)cfg.omega_v,
+      x0 ? ((cfg.nu - 1) % 2 ? H.vx2[0] : H.vx[0]) : (T*)nullptr);
   XC_LAUNCH_CHECK();
   bool done = false;
-  XC_TRY(vcycle_vel<T>(H, k, cfg, 0, s, out, phys_out ? nullptr : H.scl, &done));
+  XC_TRY(vcycle_vel<T>(H, k, cfg, 0, s, out, phys_out ? nullptr : H.scl, &done, x0));
   if (!done) {
     if (phys_out) XC_CUDA_TRY(cudaMemcpyAsync(out, H.vx[0], sizeof(T) * nvv, cudaMemcpyDeviceToDevice, s));
     else pdl(PDL_ON, div_kernel<T>, nblk(nvv), 256, s, nvv, H.vx[0], H.scl, out);
   }
   if (!phys_out) pdl(PDL_ON, div_kernel<T>, nblk(g.NP), 256, s, g.NP, zp, H.scl + nvv, zp);
   XC_LAUNCH_CHECK();
-  (void)n;
   return XC_OK;
 }
 
@@ -4097,7 +4128,8 @@ inline double* step_mirror(StokesWork* w, int kk) { return w->hhost + (kk & 1) *
 template <typename T>
 int dot_self(StokesWork* w, Hier<T>& H, const T* v, long long n, int slot, cudaStream_t s) {
   const int nb = launch_multidot<T>(n, 1, v, n, v, w->part, s);
-  pdl(PDL_ON, norm_final_kernel, 1, KB, s, nb, w->part, w->hdev + slot, w->hdev + 6, w->hhost + slot);
+  pdl(PDL_ON, norm_final_kernel, 1, KB, s, nb, w->part, w->hdev + slot, w->hdev + 6, w->hhost + slot,
+      (const double*)nullptr, (double*)nullptr, 0);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
@@ -4196,8 +4228,8 @@ __global__ void nn_target_kernel(Geo g, const double* __restrict__ y, float* out
 
 // z = M v for the configured preconditioner
 template <typename T>
-int apply_precond(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, const T* v, T* out,
-                  cudaStream_t s, bool phys_out = false) {
+int apply_precond(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, T* v, T* out, cudaStream_t s,
+                  bool phys_out = false, const T* inv = nullptr) {
   if constexpr (std::is_same<T, float>::value) {
     if (cfg.learned != 0) {
       const Geo& g = w->g;
@@ -4234,7 +4266,7 @@ int apply_precond(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& c
       return XC_OK;
     }
   }
-  return precond<T>(w, H, k, cfg, v, out, s, phys_out);
+  return precond<T>(w, H, k, cfg, v, out, s, phys_out, inv);
 }
 
 // The launches of one Arnoldi step k: z_k = M v_k; w = A z_k; two classical
@@ -4254,7 +4286,10 @@ int arnoldi_launches(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg
   // cycle's update applies S^-1 once, instead of an S^-1 pass after every
   // preconditioner and an S pass before every operator
   const bool zphys = with_precond && cfg.learned == 0;
-  if (with_precond) XC_TRY(apply_precond<T>(w, H, k, cfg, vk, zk, s, zphys));
+  // and v_k is normalised by the preconditioner's kernels as they read it (v_0
+  // comes normalised)
+  const T* inv = reinterpret_cast<const T*>(w->hdev + (std::is_same<T, float>::value ? 7 : 6));
+  if (with_precond) XC_TRY(apply_precond<T>(w, H, k, cfg, vk, zk, s, zphys, zphys && kk > 0 ? inv : nullptr));
   if (zphys) {
     pdl(PDL_ON, stokes_apply_kernel<T>, grid2(g, split_rows(g) ? 3 : 1), blk2(), s, g, k, vop(H, 0), (const T*)H.cp, (const T*)H.scl,
         (const T*)zk, (const T*)nullptr, wv);
@@ -4273,11 +4308,12 @@ int arnoldi_launches(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg
       pdl(PDL_ON, multiaxpy_norm_kernel<T>, nbn, KB, s, n, kk + 1, (const T*)H.V, n,
           (const double*)(hd + pass * kMaxRestart), wv, w->part);
       pdl(PDL_ON, norm_final_kernel, 1, KB, s, nbn, (const double*)w->part, w->hdev + 2, w->hdev + 6,
-          (double*)nullptr);
+          (double*)nullptr, (const double*)w->hdev, zphys && host_copy ? step_mirror(w, kk) : (double*)nullptr, kMirror);
     }
   }
-  pdl(PDL_ON, normalize_kernel<T>, nblk(n), 256, s, n, (const double*)(w->hdev + 6), wv, (const double*)w->hdev,
-      host_copy ? step_mirror(w, kk) : (double*)nullptr, kMirror);
+  if (!zphys)
+    pdl(PDL_ON, normalize_kernel<T>, nblk(n), 256, s, n, (const double*)(w->hdev + 6), wv, (const double*)w->hdev,
+        host_copy ? step_mirror(w, kk) : (double*)nullptr, kMirror);
   XC_LAUNCH_CHECK();
   return XC_OK;
 }
