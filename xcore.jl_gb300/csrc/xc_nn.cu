@@ -23,6 +23,7 @@
 
 #include <cuda_bf16.h>
 
+#define XC_PDL_EARLY     // the next grid may be scheduled while this one runs (see xc_nn_conv.cu)
 #include "xc_internal.cuh"
 #include "xc_nn.cuh"
 
