@@ -108,3 +108,46 @@ def test_integer_functions_against_the_processor(tmp_path):
                     str(exe)], check=True, capture_output=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+PRODUCTS = PROBE[:PROBE.index("int main() {")] + r"""
+static bool same(double a, double b) { return xc_bits(a) == xc_bits(b) || (a != a && b != b); }
+static long check(double a, double b) {
+  long bad = !same(xc_mul(a, b), a * b) + !same(xc_sqr(a), a * a);
+  return bad + !same(xc_mul_small<3>(a), 3 * a) + !same(xc_mul_small<5>(a), 5 * a) + !same(xc_mul_small<6>(a), 6 * a) +
+         !same(xc_mul_small<7>(a), 7 * a) + !same(xc_mul_small<11>(a), 11 * a);
+}
+int main() {
+  std::mt19937_64 g(21);
+  long bad = 0;
+  const double edge[] = {0.0, -0.0, 1.0, -1.5, 5e-324, 0x1p-1022, 0x1.fffffffffffffp-1023, 0x1.fffffffffffffp1023, INFINITY,
+                         -INFINITY, NAN, 0x1p-511, 0x1.fffffffffffffp-512, 0x1p512, 0x1.fffffffffffffp511};
+  for (double a : edge)
+    for (double b : edge) bad += check(a, b);
+  for (long i = 0; i < 8000000; ++i) {
+    const int wide = i % 4 == 0 ? 2048 : (i % 4 == 1 ? 80 : 1100), low = i % 4 == 3 ? 948 : (i % 4 == 1 ? 983 : 0);
+    auto draw = [&] {
+      return xc_from_bits((g() & (1ull << 63)) | ((uint64_t)(low + g() % wide) << 52) | significand(g(), g() % 5));
+    };
+    const double a = draw(), b = draw();
+    bad += check(a, b);
+  }
+  std::printf("bad %ld\n", bad);
+  return bad != 0;
+}
+"""
+
+
+def test_integer_products_against_the_processor(tmp_path):
+    """xc_mul, xc_sqr and xc_mul_small: the processor's bits for all kinds of significands and all exponents, through
+    both ends of the range, and for zeros, infinities and NaN."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not available")
+    src = tmp_path / "products.cpp"
+    src.write_text(PRODUCTS)
+    exe = tmp_path / "products"
+    subprocess.run([gxx, "-O2", "-std=c++17", "-ffp-contract=off", "-I", os.path.join(ROOT, "xcore.jl_gb300", "csrc"),
+                    str(src), "-o", str(exe)], check=True, capture_output=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout

@@ -135,6 +135,23 @@ def test_stencil_tiles_bitwise(scheme, shape, bcs):
         np.testing.assert_array_equal(_host(got), want)
 
 
+def test_large_advection_tile_bitwise():
+    """A grid just above the line between the two advection tiles (18 * 152 * 512 cells), an odd number of rows and
+    columns: the reference's bits, subnormal and zero fields included."""
+    Nz, Nx = 1187, 1183
+    rng = np.random.default_rng(5)
+    f = rng.random((Nz, Nx))
+    f[:200] = 0.0
+    f[200:400] *= 1e-310
+    u, w = rng.standard_normal((Nz, Nx + 1)), rng.standard_normal((Nz + 1, Nx))
+    d = [torch.zeros(s, dtype=torch.float64, device="cuda") for s in ((Nx, Nz), (Nx + 1, Nz + 2), (Nx + 2, Nz + 1))]
+    ref = O.advect_centered_with_flux(f, u, w, 0.37, "weno5", "periodic", "closed")
+    xc.advect_centered_with_flux(*d, _dev(f), _dev(u), _dev(w), 0.37, "weno5", "periodic", "closed")
+    torch.cuda.synchronize()
+    for got, want in zip(d, ref):
+        np.testing.assert_array_equal(_host(got), want)
+
+
 def test_ghosts_halo3_both_closed():
     Nz, Nx, g = 9, 6, 3
     f = np.random.default_rng(1).random((Nz, Nx))

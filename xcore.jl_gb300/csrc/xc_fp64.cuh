@@ -124,6 +124,70 @@ XC_HD double xc_div(double a, double b) {
   return a / b;
 }
 
+// a b, correctly rounded (a multiplication occupies the FP64 unit for 64 cycles; this is some 40 integer
+// instructions: worth it where the FP64 unit is what a kernel waits for).  The 106-bit product of the significands
+// is rounded to nearest even; a zero factor gives its zero, and whatever else leaves the normal range takes the FP64
+// unit's product, in a call so that it is not issued otherwise.
+#ifdef __CUDACC__
+__host__ __device__ __noinline__ inline double xc_mul_any(double a, double b) { return a * b; }
+#else
+inline double xc_mul_any(double a, double b) { return a * b; }
+#endif
+XC_HD double xc_mul_edge(double a, double b) {
+  const uint64_t ua = xc_bits(a), ub = xc_bits(b), inf = 0x7ffull << 53;
+  if ((!(ua << 1) && (ub << 1) < inf) || (!(ub << 1) && (ua << 1) < inf)) return xc_from_bits((ua ^ ub) & (1ull << 63));
+  return xc_mul_any(a, b);
+}
+// 63 bits h, the leading one at 62 or 61, and whether any below them is set -> the rounded product; e the biased
+// exponent for a leading one at 61
+XC_HD uint64_t xc_round63(uint64_t h, uint32_t sticky, int e, uint32_t sign) {
+  const int up = (int)(h >> 62);
+  h = up ? h : h << 1;
+  h |= sticky ? 1u : 0u;
+  const uint64_t r = (h + 0x1ff + ((uint32_t)(h >> 10) & 1u)) >> 10;    // with its leading bit, which adds one to the exponent
+  return ((uint64_t)(sign & 0x80000000u) << 32) + ((uint64_t)(uint32_t)(e + up - 1) << 52) + r;
+}
+XC_HD double xc_mul(double a, double b) {
+  const uint64_t ua = xc_bits(a), ub = xc_bits(b);
+  const uint32_t ha = (uint32_t)(ua >> 32), hb = (uint32_t)(ub >> 32);
+  const int ea = (int)((ha >> 20) & 0x7ffu), eb = (int)((hb >> 20) & 0x7ffu), e = ea + eb - 1023;
+  if ((unsigned)(ea - 1) < 2046u && (unsigned)(eb - 1) < 2046u && (unsigned)(e - 1) < 2044u) {
+    const uint32_t al = (uint32_t)ua, bl = (uint32_t)ub, ah = (ha & 0xfffffu) | 0x100000u, bh = (hb & 0xfffffu) | 0x100000u;
+    const uint64_t p = xc_mulwide(al, bl);
+    const uint64_t m = xc_mulwide(ah, bl) + (xc_mulwide(al, bh) + (p >> 32));
+    const uint64_t h = xc_mulwide(ah, bh) + (m >> 32);
+    return xc_from_bits(xc_round63((h << 21) | ((uint32_t)m >> 11), ((uint32_t)m << 21) | (uint32_t)p, e, ha ^ hb));
+  }
+  return xc_mul_edge(a, b);
+}
+XC_HD double xc_sqr(double a) {
+  const uint64_t ua = xc_bits(a);
+  const uint32_t ha = (uint32_t)(ua >> 32);
+  const int ea = (int)((ha >> 20) & 0x7ffu), e = 2 * ea - 1023;
+  if ((unsigned)(e - 1) < 2044u) {
+    const uint32_t al = (uint32_t)ua, ah = (ha & 0xfffffu) | 0x100000u;
+    const uint64_t p = xc_mulwide(al, al);
+    const uint64_t m = 2 * xc_mulwide(al, ah) + (p >> 32);
+    const uint64_t h = xc_mulwide(ah, ah) + (m >> 32);
+    return xc_from_bits(xc_round63((h << 21) | ((uint32_t)m >> 11), ((uint32_t)m << 21) | (uint32_t)p, e, 0));
+  }
+  return xc_mul_edge(a, a);
+}
+// K a for a small odd K: the product of the significand is exact in 64 bits
+template <int K>
+XC_HD double xc_mul_small(double a) {
+  constexpr int L = K < 4 ? 1 : (K < 8 ? 2 : 3);              // K in [2^L, 2^(L+1))
+  static_assert(K >= 2 && K < 16, "small factors");
+  const uint64_t ua = xc_bits(a);
+  const uint32_t ha = (uint32_t)(ua >> 32);
+  const int e = (int)((ha >> 20) & 0x7ffu) + L;
+  if ((unsigned)(e - L - 1) < 2040u) {
+    const uint64_t m = xc_mulwide((uint32_t)ua, K) + ((uint64_t)(((ha & 0xfffffu) | 0x100000u) * K) << 32);
+    return xc_from_bits(xc_round63(m << (9 - L), 0, e, ha));
+  }
+  return xc_mul_edge((double)K, a);
+}
+
 // sqrt(a), correctly rounded
 XC_HD double xc_sqrt(double a) {
   const uint64_t ua = xc_bits(a);

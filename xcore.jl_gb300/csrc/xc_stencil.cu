@@ -14,10 +14,13 @@
 // What bounds it: sm_103a's FP64 unit takes one warp instruction per 64 cycles
 // and sub-partition, so the stencils cost their FP64 instructions and little
 // else.  Products by 2, 4 and 1/4 are exact and go into the following sum as an
-// FMA (the same rounding, one instruction instead of two), quotients run on
-// the integer pipe (xc_fp64.cuh), signs are tested on the bits.  WENO5 in the
-// reference's form takes 60 FP64 instructions per face instead of 110: 237 us
-// for one 1024^2 field with its fluxes instead of 443; QUICK 7.3 us at 400^2 instead of 21.
+// FMA (the same rounding, one instruction instead of two), quotients and most
+// other products run on the integer pipe (xc_fp64.cuh), signs are tested on
+// the bits: what is left for the FP64 unit are the sums.  WENO5 in the
+// reference's form takes 27 FP64 instructions per face, and some 1400 integer
+// ones beside them that issue in about their time.  One 1024^2 field with its
+// fluxes: 443 us with everything on the FP64 unit, 237 us with the quotients
+// taken off it, 156 us with the products off it too.
 #include "xc_internal.cuh"
 
 namespace {
@@ -27,17 +30,18 @@ namespace {
 // index space, so that a small tile's faces (280 of 16 x 8) are one round of
 // its threads: the time of a small grid is that round.  The larger tile
 // evaluates 2.09 faces per cell instead of 2.19 and reads less halo, but its
-// last wave is emptier.  Measured, small against large tile, WENO5: 7.0 / 22.4
-// us at 100^2, 42 / 54 at 400^2, 117 / 120 at 700^2, 171 / 171 at 850^2, 239 /
-// 237 at 1024^2, 513 / 498 at 1500^2; diffusion, which is read and write: 7.6
-// / 8.2 at 400^2, 11.1 / 10.4 at 512^2, 39 / 31 at 1024^2.  The lines lie at
-// nine and at three waves of the larger tile (152 of 512 cells each).
+// last wave is emptier.  Measured, small against large tile, WENO5: 6.9 / 23.3
+// us at 100^2, 29 / 40 at 400^2, 77 / 84 at 700^2, 111 / 117 at 850^2, 156 /
+// 160 at 1024^2, 334 / 330 at 1500^2; diffusion, which is read and write: 6.6
+// / 8.6 at 400^2, 8.6 / 9.9 at 512^2, 14.2 / 14.6 at 700^2, 27.0 / 24.5 at
+// 1024^2.  The lines lie at 18 and at 7 waves of the larger tile (152 of 512
+// cells each).
 template <int Z, int X, int T> struct TileShape {
   static constexpr int TZ = Z, TX = X, NT = T;
 };
 using SmallTile = TileShape<16, 8, 288>;
 using LargeTile = TileShape<32, 16, 256>;
-constexpr long long kSmallAdvect = 9LL * kNumSMs * 512, kSmallDiffus = 3LL * kNumSMs * 512;
+constexpr long long kSmallAdvect = 18LL * kNumSMs * 512, kSmallDiffus = 7LL * kNumSMs * 512;
 
 // ---------------------------------------------------------------------------
 // face reconstructions (advect.jl:35-53, 216-229, 275-283)
@@ -46,22 +50,23 @@ __device__ __forceinline__ double weno5_poly(double fmm, double fm, double fc, d
                                              double fpp) {
   const double sixth = 1.0 / 6.0, quarter = 0.25, c1312 = 13.0 / 12.0;
   const double eps_val = XC_EPS;
-  const double p1 = sixth * (__fma_rn(2.0, fmm, -(7.0 * fm)) + 11.0 * fc);
-  const double p2 = sixth * __fma_rn(2.0, fp, 5.0 * fc - fm);
-  const double p3 = sixth * (__fma_rn(2.0, fc, 5.0 * fp) - fpp);
-  double t = __fma_rn(-2.0, fm, fmm) + fc, s = __fma_rn(-4.0, fm, fmm) + 3.0 * fc;
-  const double b1 = __fma_rn(quarter, s * s, c1312 * (t * t));
+  const double p1 = xc_mul(__fma_rn(2.0, fmm, -xc_mul_small<7>(fm)) + xc_mul_small<11>(fc), sixth);
+  const double p2 = xc_mul(__fma_rn(2.0, fp, xc_mul_small<5>(fc) - fm), sixth);
+  const double p3 = xc_mul(__fma_rn(2.0, fc, xc_mul_small<5>(fp)) - fpp, sixth);
+  const double fc3 = xc_mul_small<3>(fc);
+  double t = __fma_rn(-2.0, fm, fmm) + fc, s = __fma_rn(-4.0, fm, fmm) + fc3;
+  const double b1 = __fma_rn(quarter, xc_sqr(s), xc_mul(xc_sqr(t), c1312));
   t = __fma_rn(-2.0, fc, fm) + fp;
   s = fm - fp;
-  const double b2 = __fma_rn(quarter, s * s, c1312 * (t * t));
+  const double b2 = __fma_rn(quarter, xc_sqr(s), xc_mul(xc_sqr(t), c1312));
   t = __fma_rn(-2.0, fp, fc) + fpp;
-  s = __fma_rn(-4.0, fp, 3.0 * fc) + fpp;
-  const double b3 = __fma_rn(quarter, s * s, c1312 * (t * t));
+  s = __fma_rn(-4.0, fp, fc3) + fpp;
+  const double b3 = __fma_rn(quarter, xc_sqr(s), xc_mul(xc_sqr(t), c1312));
   const double e1 = b1 + eps_val, e2 = b2 + eps_val, e3 = b3 + eps_val;
-  const double w1 = xc_div(0.1, e1 * e1);
-  const double w2 = xc_div(0.6, e2 * e2);
-  const double w3 = xc_div(0.3, e3 * e3);
-  return xc_div((w1 * p1 + w2 * p2) + w3 * p3, (w1 + w2) + w3);
+  const double w1 = xc_div(0.1, xc_sqr(e1));
+  const double w2 = xc_div(0.6, xc_sqr(e2));
+  const double w3 = xc_div(0.3, xc_sqr(e3));
+  return xc_div((xc_mul(w1, p1) + xc_mul(w2, p2)) + xc_mul(w3, p3), (w1 + w2) + w3);
 }
 
 // The same reconstruction with the weights over a common denominator: with
@@ -76,30 +81,30 @@ __device__ __forceinline__ double weno5_poly(double fmm, double fm, double fc, d
 __device__ __forceinline__ double weno5_poly_onediv(double fmm, double fm, double fc, double fp,
                                                     double fpp) {
   const double c133 = 4.0 * (13.0 / 12.0), eps4 = 4.0 * XC_EPS;
-  const double p1 = __fma_rn(11.0, fc, __fma_rn(-7.0, fm, 2.0 * fmm));
+  const double p1 = __fma_rn(11.0, fc, __fma_rn(-7.0, fm, xc_scale2<1>(fmm)));
   const double p2 = __fma_rn(2.0, fp, __fma_rn(5.0, fc, -fm));
   const double p3 = __fma_rn(2.0, fc, __fma_rn(5.0, fp, -fpp));
   double t = __fma_rn(-2.0, fm, fmm) + fc, s = __fma_rn(3.0, fc, __fma_rn(-4.0, fm, fmm));
-  const double e1 = __fma_rn(c133 * t, t, s * s) + eps4;
+  const double e1 = __fma_rn(xc_mul(t, c133), t, xc_sqr(s)) + eps4;
   t = __fma_rn(-2.0, fc, fm) + fp;
   s = fm - fp;
-  const double e2 = __fma_rn(c133 * t, t, s * s) + eps4;
+  const double e2 = __fma_rn(xc_mul(t, c133), t, xc_sqr(s)) + eps4;
   t = __fma_rn(-2.0, fp, fc) + fpp;
   s = __fma_rn(3.0, fc, __fma_rn(-4.0, fp, fpp));
-  const double e3 = __fma_rn(c133 * t, t, s * s) + eps4;
-  const double q1 = e1 * e1, q2 = e2 * e2, q3 = e3 * e3;
-  const double n1 = q2 * q3, n2 = 6.0 * (q1 * q3), n3 = 3.0 * (q1 * q2);
-  return (1.0 / 6.0) * xc_div(__fma_rn(n1, p1, __fma_rn(n2, p2, n3 * p3)), (n1 + n2) + n3);
+  const double e3 = __fma_rn(xc_mul(t, c133), t, xc_sqr(s)) + eps4;
+  const double q1 = xc_sqr(e1), q2 = xc_sqr(e2), q3 = xc_sqr(e3);
+  const double n1 = xc_mul(q2, q3), n2 = xc_mul_small<6>(xc_mul(q1, q3)), n3 = xc_mul_small<3>(xc_mul(q1, q2));
+  return xc_mul(xc_div(__fma_rn(n1, p1, __fma_rn(n2, p2, xc_mul(n3, p3))), (n1 + n2) + n3), 1.0 / 6.0);
 }
 
 __device__ __forceinline__ double weno3_poly(double fm, double fc, double fp) {
-  const double half = 0.5, eps_val = 1e-6;
-  double p1 = half * (fc + fp);
-  double p2 = half * (3.0 * fc - fm);
+  const double eps_val = 1e-6;
+  double p1 = xc_half(fc + fp);
+  double p2 = xc_half(xc_mul_small<3>(fc) - fm);
   double d1 = fp - fc, d2 = fc - fm;
-  double w1 = xc_div(1.0 / 3.0, d1 * d1 + eps_val);
-  double w2 = xc_div(2.0 / 3.0, d2 * d2 + eps_val);
-  return xc_div(w1 * p1 + w2 * p2, w1 + w2);
+  double w1 = xc_div(1.0 / 3.0, xc_sqr(d1) + eps_val);
+  double w2 = xc_div(2.0 / 3.0, xc_sqr(d2) + eps_val);
+  return xc_div(xc_mul(w1, p1) + xc_mul(w2, p2), w1 + w2);
 }
 
 __device__ __forceinline__ double tvd_flux(double fm, double fc, double fp, double vm, double vp) {
@@ -136,7 +141,8 @@ __device__ __forceinline__ double face_flux(double s0, double s1, double s2, dou
     if (finite_bits(s1) && finite_bits(s2) && finite_bits(s3) && finite_bits(s4) && finite_bits(v)) {
       const bool up = !sign_bit(v);
       const double a1 = up ? s1 : s4, a2 = up ? s2 : s3, a3 = up ? s3 : s2;
-      return v * (S == XC_QUICK ? sixth * (__fma_rn(2.0, a3, 5.0 * a2) - a1) : __fma_rn(0.25, a3 - a1, a2));
+      return xc_mul(v, S == XC_QUICK ? xc_mul(__fma_rn(2.0, a3, xc_mul_small<5>(a2)) - a1, sixth)
+                                     : __fma_rn(0.25, a3 - a1, a2));
     }
     double pos, neg;
     if (S == XC_QUICK) {
@@ -161,7 +167,7 @@ __device__ __forceinline__ double face_flux(double s0, double s1, double s2, dou
     const double p = S == XC_WENO5        ? weno5_poly(a0, a1, a2, a3, a4)
                      : S == kWeno5OneDiv ? weno5_poly_onediv(a0, a1, a2, a3, a4)
                                          : weno3_poly(a1, a2, a3);
-    return zero_bits(v) ? v : v * p;
+    return zero_bits(v) ? v : xc_mul(v, p);
   } else {  // XC_TVDIM
     double cpos = vpos(v), cneg = vneg(v);
     double pos = tvd_flux(s1, s2, s3, vpos(vl), cpos);
@@ -307,7 +313,8 @@ __device__ __forceinline__ void advect_tile(TileSmem<T, Halo<S>::G>& sm, const F
     int jj = idx % TZ, ii = idx / TZ;
     int j = j0 + jj, i = i0 + ii;
     if (j < Nz && i < Nx)
-      AT(a.out, j, i) = (((sm.q[idx + TZ] - sm.q[idx]) + qz[ii * (TZ + 1) + jj + 1]) - qz[ii * (TZ + 1) + jj]) * invh;
+      AT(a.out, j, i) =
+          xc_mul(((sm.q[idx + TZ] - sm.q[idx]) + qz[ii * (TZ + 1) + jj + 1]) - qz[ii * (TZ + 1) + jj], invh);
   }
 }
 
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(T::NT) advect_tile_kernel(FluxArgs a, int Nz, 
 // (k_L + k_R)(f_R - f_L) is formed once: the divergence takes it from both
 // sides, and the face flux -(k_L + k_R)/2 (f_R - f_L)/h is the same product
 // halved and negated, which is exact (subnormal products aside, far below any
-// flux).  12 FP64 instructions per cell instead of 28.
+// flux).  7 FP64 instructions per cell instead of 28.
 // ---------------------------------------------------------------------------
 template <class T, bool HALOD>
 __device__ __forceinline__ void diffus_tile(TileSmem<T, 1>& sm, double* sk, const FluxArgs& a, int Nz, int Nx, int xBC,
@@ -347,7 +354,7 @@ __device__ __forceinline__ void diffus_tile(TileSmem<T, 1>& sm, double* sk, cons
     if (in) {
       fv = a.f[o];
       kv = a.k1[o];
-      if (a.k2) kv = kv * a.k2[o];
+      if (a.k2) kv = xc_mul(kv, a.k2[o]);
     }
     sm.f[idx] = fv;
     sk[idx] = kv;
@@ -360,14 +367,14 @@ __device__ __forceinline__ void diffus_tile(TileSmem<T, 1>& sm, double* sk, cons
     const int ii = xf ? k / TZ : k / (TZ + 1), jj = k - ii * (xf ? TZ : TZ + 1);
     const int j = j0 + jj, i = i0 + ii;
     const int c = (ii + 1) * HZ + jj + 1, b = c - (xf ? HZ : 1);
-    const double q = (sk[c] + sk[b]) * (sm.f[c] - sm.f[b]);
+    const double q = xc_mul(sk[c] + sk[b], sm.f[c] - sm.f[b]);
     sm.q[idx] = q;
     if (xf) {
       if (a.qx.p && j < Nz && i <= Nx && (ii < TX || i == Nx))
-        put_qx(a.qx, j, i, q * mhalf_invh, Nz, zBC, pad);
+        put_qx(a.qx, j, i, xc_mul(q, mhalf_invh), Nz, zBC, pad);
     } else {
       if (a.qz.p && j <= Nz && i < Nx && (jj < TZ || j == Nz))
-        put_qz(a.qz, j, i, q * mhalf_invh, Nx, xBC, pad);
+        put_qz(a.qz, j, i, xc_mul(q, mhalf_invh), Nx, xBC, pad);
     }
   }
   if (!a.out.p) return;
@@ -379,7 +386,7 @@ __device__ __forceinline__ void diffus_tile(TileSmem<T, 1>& sm, double* sk, cons
     int j = j0 + jj, i = i0 + ii;
     if (j < Nz && i < Nx)
       AT(a.out, j, i) =
-          hih2 * (((sm.q[idx + TZ] - sm.q[idx]) + qz[ii * (TZ + 1) + jj + 1]) - qz[ii * (TZ + 1) + jj]);
+          xc_mul(((sm.q[idx + TZ] - sm.q[idx]) + qz[ii * (TZ + 1) + jj + 1]) - qz[ii * (TZ + 1) + jj], hih2);
   }
 }
 
@@ -434,17 +441,17 @@ __global__ void phsevo_tail_kernel(int Nz, int Nx, double a1, double a2, double 
     if (j >= Nz || i >= Nx) return;
     double aX = AT(advn_X, j, i);
     AT(advn_rho, j, i) = aX + AT(advn_M, j, i);
-    double gx = (G0 * (1.0 - AT(x, j, i))) * AT(bndshape, j, i);
+    double gx = xc_mul(xc_mul(1.0 - AT(x, j, i), G0), AT(bndshape, j, i));
     AT(Gx, j, i) = gx;
     double dxdt = (-aX + AT(dffn_X, j, i)) + gx;
     AT(dXdt, j, i) = dxdt;
     double Xc = AT(X, j, i);
-    double res = ((a1 * Xc - a2 * AT(Xo, j, i)) - a3 * AT(Xoo, j, i)) -
-                 (((b1 * dxdt + b2 * AT(dXdto, j, i)) + b3 * AT(dXdtoo, j, i)) * dt);
-    double upd = xc_div((-alpha) * res, a1);
+    double res = ((xc_mul(Xc, a1) - xc_mul(AT(Xo, j, i), a2)) - xc_mul(AT(Xoo, j, i), a3)) -
+                 xc_mul((xc_mul(dxdt, b1) + xc_mul(AT(dXdto, j, i), b2)) + xc_mul(AT(dXdtoo, j, i), b3), dt);
+    double upd = xc_div(xc_mul(res, -alpha), a1);
     double Xn = Xc + upd;
     double r = AT(rho, j, i);
-    double lo = r * XC_EPS, hi = r * (1.0 - XC_EPS);
+    double lo = xc_mul(r, XC_EPS), hi = xc_mul(r, 1.0 - XC_EPS);
     Xn = Xn > hi ? hi : (Xn < lo ? lo : Xn);
     AT(X, j, i) = Xn;
     double Mn = r - Xn;
