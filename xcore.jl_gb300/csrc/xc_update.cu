@@ -233,36 +233,39 @@ __device__ __forceinline__ void for_corner_tiles(int Nz, int Nx, double (&sq)[9]
 }
 
 // update_kinematics! (update.jl:202-280): exz on corners, the rest on cells.
-// 34 FP64 instructions per cell instead of 120: at 1024^2 226 -> 78 us.
+// 23 FP64 instructions per cell instead of 120: at 1024^2 226 us with everything
+// on the FP64 unit, 78 us without quotients and roots, 59 us without products.
+// (volfrac_rheology, viscblend and the blends keep their products there: they are
+// bound by integer issue already, and took 5 to 40 % longer with them moved.)
 __global__ void kinematics_kernel(int Nz, int Nx, double invh, CView W, CView U, CView wx,
                                   CView wm, DView exz, DView exx, DView ezz, DView Div_V,
                                   DView eII, DView V, DView vx, DView vm) {
   XC_PDL_WAIT();
   __shared__ double sq[9][33];
   for_corner_tiles(Nz, Nx, sq, [&](int j, int i, bool own) {
-    double dUdz = (AT(U, j + 1, i) - AT(U, j, i)) * invh;
-    double dWdx = (AT(W, j, i + 1) - AT(W, j, i)) * invh;
+    double dUdz = xc_mul(AT(U, j + 1, i) - AT(U, j, i), invh);
+    double dWdx = xc_mul(AT(W, j, i + 1) - AT(W, j, i), invh);
     const double e = xc_half(dUdz + dWdx);
     if (own) AT(exz, j, i) = e;
-    return e * e;
+    return xc_sqr(e);
   }, [&](int j, int i, double exz_sq) {
     const double Ua = AT(U, j + 1, i), Ub = AT(U, j + 1, i + 1), Wa = AT(W, j, i + 1), Wb = AT(W, j + 1, i + 1);
-    double Ux_c = (Ub - Ua) * invh;
-    double Wz_c = (Wb - Wa) * invh;
+    double Ux_c = xc_mul(Ub - Ua, invh);
+    double Wz_c = xc_mul(Wb - Wa, invh);
     double div = Ux_c + Wz_c;
     AT(Div_V, j, i) = div;
     const double d3 = xc_div(div, 3.0);
     double ex = Ux_c - d3, ez = Wz_c - d3;
     AT(exx, j, i) = ex;
     AT(ezz, j, i) = ez;
-    AT(eII, j, i) = xc_sqrt((XC_EPS + xc_half(ex * ex + ez * ez)) + exz_sq);
+    AT(eII, j, i) = xc_sqrt((XC_EPS + xc_half(xc_sqr(ex) + xc_sqr(ez))) + exz_sq);
     double wc = avg(Wa, Wb);
     double uc = avg(Ua, Ub);
-    AT(V, j, i) = xc_sqrt(wc * wc + uc * uc);
+    AT(V, j, i) = xc_sqrt(xc_sqr(wc) + xc_sqr(uc));
     double t = avg(AT(wx, j, i + 1), AT(wx, j + 1, i + 1));
-    AT(vx, j, i) = xc_sqrt(t * t + XC_EPS);
+    AT(vx, j, i) = xc_sqrt(xc_sqr(t) + XC_EPS);
     t = avg(AT(wm, j, i + 1), AT(wm, j + 1, i + 1));
-    AT(vm, j, i) = xc_sqrt(t * t + XC_EPS);
+    AT(vm, j, i) = xc_sqrt(xc_sqr(t) + XC_EPS);
   });
 }
 
@@ -367,15 +370,15 @@ __global__ void stress_kernel(int Nz, int Nx, double D0, CView etaco, CView exz,
   XC_PDL_WAIT();
   __shared__ double sq[9][33];
   for_corner_tiles(Nz, Nx, sq, [&](int j, int i, bool own) {
-    const double t = AT(etaco, j, i) * AT(exz, j, i);
+    const double t = xc_mul(AT(etaco, j, i), AT(exz, j, i));
     if (own) AT(txz, j, i) = t;
-    return t * t;
+    return xc_sqr(t);
   }, [&](int j, int i, double txz_sq) {
     double e = AT(eta, j, i);
-    double tx = e * AT(exx, j, i), tz = e * AT(ezz, j, i);
+    double tx = xc_mul(e, AT(exx, j, i)), tz = xc_mul(e, AT(ezz, j, i));
     AT(txx, j, i) = tx;
     AT(tzz, j, i) = tz;
-    AT(tII, j, i) = xc_sqrt((XC_EPS + xc_half(tx * tx + tz * tz)) + txz_sq);
+    AT(tII, j, i) = xc_sqrt((XC_EPS + xc_half(xc_sqr(tx) + xc_sqr(tz))) + txz_sq);
     AT(Ra, j, i) = xc_div(AT(V, j, i) * D0, AT(kx, j, i));
   });
 }
@@ -395,17 +398,17 @@ __global__ void phase_velocities_kernel(int Nz, int Nx, int xBC, int zBC, double
       // the ghost columns copy the tapered interior columns periodically
       // (store.jl:272-273 applies the copy for every xBC)
       int is = (i == 0) ? Nx : (i == Nx + 1 ? 1 : i);
-      double w = (xc_div(d0 * d0, AT(etasw, j, is - 1)) * AT(Drhox, j, is - 1)) * g0;
-      w = w * AT(bndtaperw, j, is);
+      double w = xc_mul(xc_mul(xc_div(xc_sqr(d0), AT(etasw, j, is - 1)), AT(Drhox, j, is - 1)), g0);
+      w = xc_mul(w, AT(bndtaperw, j, is));
       AT(wx, j, i) = w;
       int ci = icx_at(i, Nx, xBC);
       const double xm = xc_div(AT(x_w, j, ci), xc_max_pos(AT(m_w, j, ci), XC_EPS));
-      double wmv = (-xm) * w;
+      double wmv = xc_mul(-xm, w);
       AT(wm, j, i) = wmv;
       double sx = AT(xisw, j, i) + AT(xixw, j, i);
       double Wv = AT(W, j, i), xe_w = AT(xiew, j, i);
       AT(Wx, j, i) = ((Wv + w) + sx) + xe_w;
-      AT(Wm, j, i) = ((Wv + wmv) - (xm * sx)) + xe_w;
+      AT(Wm, j, i) = ((Wv + wmv) - xc_mul(xm, sx)) + xe_w;
     }
     if (i <= Nx) {   // U-shaped (Nz+2, Nx+1)
       int cj = icz_at(j, Nz, zBC);
@@ -413,7 +416,7 @@ __global__ void phase_velocities_kernel(int Nz, int Nx, int xBC, int zBC, double
       double sx = AT(xisu, j, i) + AT(xixu, j, i);
       double Uv = AT(U, j, i), xe_u = AT(xieu, j, i);
       AT(Ux, j, i) = (Uv + sx) + xe_u;
-      AT(Um, j, i) = (Uv + ((-xm) * sx)) + xe_u;
+      AT(Um, j, i) = (Uv + xc_mul(-xm, sx)) + xe_u;
     }
   });
 }
