@@ -114,6 +114,8 @@ PRODUCTS = PROBE[:PROBE.index("int main() {")] + r"""
 static bool same(double a, double b) { return xc_bits(a) == xc_bits(b) || (a != a && b != b); }
 static long check(double a, double b) {
   long bad = !same(xc_mul(a, b), a * b) + !same(xc_sqr(a), a * a);
+  const float f = (float)a, r = xc_to_float(a);
+  bad += std::memcmp(&f, &r, 4) != 0 && f == f;
   return bad + !same(xc_mul_small<3>(a), 3 * a) + !same(xc_mul_small<5>(a), 5 * a) + !same(xc_mul_small<6>(a), 6 * a) +
          !same(xc_mul_small<7>(a), 7 * a) + !same(xc_mul_small<11>(a), 11 * a);
 }
@@ -139,7 +141,7 @@ int main() {
 
 
 def test_integer_products_against_the_processor(tmp_path):
-    """xc_mul, xc_sqr and xc_mul_small: the processor's bits for all kinds of significands and all exponents, through
+    """xc_mul, xc_sqr, xc_mul_small and the conversion to float: the processor's bits for all kinds of significands and all exponents, through
     both ends of the range, and for zeros, infinities and NaN."""
     gxx = shutil.which("g++")
     if gxx is None:

@@ -188,6 +188,32 @@ XC_HD double xc_mul_small(double a) {
   return xc_mul_edge((double)K, a);
 }
 
+// a rounded to a float (a conversion is on the FP64 unit too); results outside its normal range by the compiler's
+// conversion, in a call
+#ifdef __CUDACC__
+__host__ __device__ __noinline__ inline float xc_to_float_any(double a) { return (float)a; }
+#else
+inline float xc_to_float_any(double a) { return (float)a; }
+#endif
+XC_HD float xc_from_float_bits(uint32_t u) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float x;
+  std::memcpy(&x, &u, 4);
+  return x;
+#endif
+}
+XC_HD float xc_to_float(double a) {
+  const uint64_t u = xc_bits(a);
+  const uint32_t h = (uint32_t)(u >> 32), sign = h & 0x80000000u;
+  const int e = (int)((h >> 20) & 0x7ffu) - 896;
+  if ((unsigned)(e - 1) < 253u) {
+    const uint64_t m = (u & ((1ull << 52) - 1)) + 0xfffffffull + ((uint32_t)(u >> 29) & 1u);
+    return xc_from_float_bits(sign | (((uint32_t)e << 23) + (uint32_t)(m >> 29)));
+  }
+  return u << 1 ? xc_to_float_any(a) : xc_from_float_bits(sign);
+}
 // sqrt(a), correctly rounded
 XC_HD double xc_sqrt(double a) {
   const uint64_t ua = xc_bits(a);
