@@ -1198,7 +1198,7 @@ __device__ void gj_invert_cta(R* M, int n, int* piv, int* ok, R* fcol, double* r
 
 // x = inv b by one CTA (a warp per row); ends with a barrier
 template <typename T>
-__device__ void dense_apply_cta(const T* __restrict__ inv, int n, const T* b, T* x) {
+__device__ void dense_apply_cta(const T* __restrict__ inv, int n, int ld, const T* b, T* x) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   static_assert(kDenseMax <= 64, "two columns a lane");
   const bool c0 = lane < n, c1 = lane + 32 < n;
@@ -1210,7 +1210,7 @@ __device__ void dense_apply_cta(const T* __restrict__ inv, int n, const T* b, T*
       const int r = r0 + q * nw;
       acc[q] = 0;
       if (r < n) {
-        const T* a = inv + r * n + lane;
+        const T* a = inv + r * ld + lane;
         if (c0) acc[q] = mul_rn<T>(a[0], b0);
         if (c1) acc[q] = fma_rn<T>(a[32], b1, acc[q]);
       }
@@ -1651,7 +1651,7 @@ __device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op,
                                unsigned dvw = 0, unsigned dvu = 0) {
   const long long n = (long long)g.NW + g.NU;
   if (inv && *inv_ok) {
-    dense_apply_cta<T>(inv, (int)n, b, x);
+    dense_apply_cta<T>(inv, (int)n, (int)n, b, x);
     return;
   }
   if (wide.inv && *inv_ok) {
@@ -2113,7 +2113,7 @@ __device__ void p_coarse_cta(int Nz, int Nx, const T* __restrict__ kx, const T* 
                              const int* inv_ok, const WideInverse& wide) {
   const int n = Nz * Nx;
   if (inv && *inv_ok) {
-    dense_apply_cta<T>(inv, n, b, x);
+    dense_apply_cta<T>(inv, n, n, b, x);
     return;
   }
   if (wide.inv && *inv_ok) {
@@ -2343,7 +2343,7 @@ struct StageLevel {
 };
 struct StageMap {
   StageLevel l[kMaxLevels];
-  int inv;                           // the dense inverse, -1: none
+  int inv, ld;                       // the coarsest level's inverse (-1: not staged) and its row length
   int total;                         // elements
 };
 template <typename T>
@@ -2459,7 +2459,7 @@ __global__ void __launch_bounds__(1024) vel_vcycle_stage_kernel(const __grid_con
   {
     const StageLevel& m = sl[lc];
     if (dense)
-      dense_apply_cta<T>(sm + M.inv, sg[lc].NW + sg[lc].NU, sm + m.b, sm + m.x);
+      dense_apply_cta<T>(sm + M.inv, sg[lc].NW + sg[lc].NU, M.ld, sm + m.b, sm + m.x);
     else
       vel_coarse_cta<T, 1>(sg[lc], level_const(kf, lc), level_op(lc), sm + m.x, sm + m.y, sm + m.b, csweeps, om,
                            nullptr, inv_ok, wide, m.dv[0], m.dv[1]);
@@ -2730,7 +2730,7 @@ __global__ void __launch_bounds__(1024) p_vcycle_stage_kernel(const __grid_const
   {
     const StageLevel& m = sl[lc];
     if (dense)
-      dense_apply_cta<T>(sm + M.inv, sn[lc][0] * sn[lc][1], sm + m.b, sm + m.x);
+      dense_apply_cta<T>(sm + M.inv, sn[lc][0] * sn[lc][1], M.ld, sm + m.b, sm + m.x);
     else
       p_coarse_cta<T>(sn[lc][0], sn[lc][1], sm + m.a0, sm + m.a1, sn[lc][2], sd[lc], sm + m.x, sm + m.y, sm + m.b,
                       csweeps, om, nullptr, inv_ok, wide);
@@ -3794,8 +3794,13 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
       m.b = carve.take((long long)gq.NW + gq.NU);
       for (int d = 0; d < 4; ++d) m.dv[d] = stage_div(gq.Nz - 1 + d > 0 ? gq.Nz - 1 + d : 1);
     }
+    // the coarsest level's inverse: the dense one, or a wide one of as many
+    // unknowns, whose FP32 product is the same sum
     const long long nd = (long long)H.vg[lc].NW + H.vg[lc].NU;
-    M.inv = H.vdirect ? carve.take(nd * nd) : -1;
+    const WideInverse wi = vel_wide(H, lc);
+    const bool wide64 = kFly<T> && wi.inv && nd <= kDenseMax;
+    M.ld = wide64 ? wi.np : (int)nd;
+    M.inv = H.vdirect || wide64 ? carve.take(nd * M.ld) : -1;
     M.total = carve.at;
     StageList S;
     S.count = 0;
@@ -3814,12 +3819,12 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
         S.add(L.op[q].cu, e * m.a1, 10LL * e * gq.NU);
       }
     }
-    if (H.vdirect) S.add(H.vinv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * nd);
+    if (M.inv >= 0) S.add(H.vdirect ? (const void*)H.vinv : wi.inv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * M.ld);
     const int rows = (std::max(vel_stage_rows(g), 128) + 31) / 32 * 32;
     if (rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
       pdl_smem(PDL_ON, vel_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, kf, l,
                lc, cfg.nu, om, coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx),
-               (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok, vel_wide(H, lc));
+               (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok, wi);
       XC_LAUNCH_CHECK();
       return XC_OK;
     }
@@ -3925,7 +3930,10 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
       m.dv[1] = stage_div(H.pNz[q]);
     }
     const long long nd = (long long)H.pNz[lc] * H.pNx[lc];
-    M.inv = H.pdirect ? carve.take(nd * nd) : -1;
+    const WideInverse wi = p_wide(H, lc);
+    const bool wide64 = kFly<T> && wi.inv && nd <= kDenseMax;
+    M.ld = wide64 ? wi.np : (int)nd;
+    M.inv = H.pdirect || wide64 ? carve.take(nd * M.ld) : -1;
     M.total = carve.at;
     StageList S;
     S.count = 0;
@@ -3935,7 +3943,7 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
       S.add(L.kx[q], e * M.l[q].a0, e * nq);
       S.add(L.kz[q], e * M.l[q].a1, e * (nq + H.pNx[q]));
     }
-    if (H.pdirect) S.add(H.pinv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * nd);
+    if (M.inv >= 0) S.add(H.pdirect ? (const void*)H.pinv : wi.inv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * M.ld);
     const int rows = (std::max(n, 128) + 31) / 32 * 32;
     if (rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
       pdl_smem(PDL_ON, p_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, l, lc,
