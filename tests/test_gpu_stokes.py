@@ -436,3 +436,22 @@ def test_steps_queued_ahead_do_not_count(maxit):
     assert out[0][0] == out[1][0]
     for a, b in zip(out[0][1], out[1][1]):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("shape", [(130, 130), (256, 68), (134, 256)])
+@pytest.mark.parametrize("solver", ["mixed", "fgmres64"])
+def test_large_pressure_levels_give_the_per_cell_results(shape, solver):
+    """Pressure levels of more than 128^2 cells take their descent and ascent with a thread per 2 x 2 cells; the kernels
+    that form every neighbour's value anew (fused_pressure_cells) have the same operations: equal bits, for numbers of
+    coarse rows and columns that fill neither a block nor a warp."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=shape[0], Nx=shape[1], steps=1)
+    coefs = O.time_coefs("bd2im", 2)
+    out = []
+    for fuse in (1 << 30, -1):
+        ds = device_state(par, g, sc, st)
+        info = ds.fluidmech(coefs, dt, solver=solver, rtol=1e-9, maxit=2000, fused_pressure_cells=fuse)
+        out.append((info["iterations"], [ds[k] for k in ("W", "U", "P")]))
+        ds.close()
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)

@@ -2034,6 +2034,131 @@ __global__ void __launch_bounds__(kTileThreads) p_up_tile_kernel(int Nz, int Nx,
   }
 }
 
+// The same two on large levels, which are bound by instruction issue: a thread
+// per coarse cell takes its 2 x 2 fine ones, whose values, coefficients and
+// prolongations it shares between them, in pairs along z (Nz is even), without
+// a halo formed twice.  From which size on matters little (1024^2 step with the
+// line at 64^2, 128^2, 256^2 cells: 1.602x, 1.608x, 1.592x of the original,
+// without them 1.499x; 512^2 solve 1.573x, 1.560x, 1.581x and 1.536x).
+template <typename T>
+struct Pair { T a, b; };
+template <typename T>
+__device__ __forceinline__ Pair<T> ld_pair(const T* p) {
+  if constexpr (kFly<T>) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    return {v.x, v.y};
+  } else {
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    return {v.x, v.y};
+  }
+}
+template <typename T>
+__device__ __forceinline__ void st_pair(T* p, T a, T b) {
+  if constexpr (kFly<T>) *reinterpret_cast<float2*>(p) = make_float2(a, b);
+  else *reinterpret_cast<double2*>(p) = make_double2(a, b);
+}
+// (L p) of one cell from its value and neighbours, p_apply_fn's operations
+template <typename T>
+__device__ __forceinline__ T p_quad_apply(T pc, T pl, T pr, T pt, T pb, T kl, T kr, T kt, T kb, bool top, bool bot,
+                                          bool pinned, T dpin) {
+  T s = add_rn<T>(mul_rn<T>(kl, pc - pl), mul_rn<T>(kr, pc - pr));
+  if (top) s = add_rn<T>(s, mul_rn<T>(kt, pc - pt));
+  if (bot) s = add_rn<T>(s, mul_rn<T>(kb, pc - pb));
+  if (pinned) s = add_rn<T>(s, mul_rn<T>(dpin, pc));
+  return s;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) p_down_quad_kernel(int Nz, int Nx, const T* __restrict__ kx,
+                                                          const T* __restrict__ kz, int pin, T dpin,
+                                                          const T* __restrict__ x, const T* __restrict__ b, T* bc,
+                                                          T omega, PCoarse<T> C) {
+  XC_PDL_WAIT();
+  const int Nzc = Nz / 2, Nxc = Nx / 2;
+  const int J = blockIdx.x * 32 + threadIdx.x, I = blockIdx.y * 8 + threadIdx.y;
+  if (J >= Nzc || I >= Nxc) return;
+  const int j = 2 * J, i0 = 2 * I, i1 = i0 + 1, il = i0 == 0 ? Nx - 1 : i0 - 1, ir = i1 == Nx - 1 ? 0 : i1 + 1;
+  const bool top = j > 0, bot = j + 2 < Nz;
+  const int o0 = i0 * Nz + j, o1 = i1 * Nz + j, ol = il * Nz + j, orr = ir * Nz + j;
+  const Pair<T> xl = ld_pair(x + ol), xa = ld_pair(x + o0), xb = ld_pair(x + o1), xr = ld_pair(x + orr);
+  const T ta = top ? x[o0 - 1] : (T)0, tb = top ? x[o1 - 1] : (T)0;
+  const T ba = bot ? x[o0 + 2] : (T)0, bb = bot ? x[o1 + 2] : (T)0;
+  const Pair<T> kl = ld_pair(kx + o0), km = ld_pair(kx + o1), kr = ld_pair(kx + orr);
+  const T* za = kz + i0 * (Nz + 1) + j;
+  const T* zb = za + Nz + 1;
+  const T a0 = za[0], a1 = za[1], a2 = za[2], b0 = zb[0], b1 = zb[1], b2 = zb[2];
+  const Pair<T> ra = ld_pair(b + o0), rb = ld_pair(b + o1);
+  const T r00 = ra.a - p_quad_apply<T>(xa.a, xl.a, xb.a, ta, xa.b, kl.a, km.a, a0, a1, top, true, o0 == pin, dpin);
+  const T r10 = ra.b - p_quad_apply<T>(xa.b, xl.b, xb.b, xa.a, ba, kl.b, km.b, a1, a2, true, bot, o0 + 1 == pin, dpin);
+  const T r01 = rb.a - p_quad_apply<T>(xb.a, xa.a, xr.a, tb, xb.b, km.a, kr.a, b0, b1, top, true, o1 == pin, dpin);
+  const T r11 = rb.b - p_quad_apply<T>(xb.b, xa.b, xr.b, xb.a, bb, km.b, kr.b, b1, b2, true, bot, o1 + 1 == pin, dpin);
+  const T v = (T)0.25 * (r00 + r10 + r01 + r11);
+  const int t = I * Nzc + J;
+  bc[t] = v;
+  if (C.x0) {                          // p_jacobi0_val's operations
+    T d;
+    p_apply_fn<T>(Nzc, Nxc, C.kx, C.kz, C.pin, C.dpin, [](int, int) { return (T)0; }, J, I, &d);
+    C.x0[t] = d > (T)0 ? sdiv<T>(omega * v, d) : (T)0;
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) p_up_quad_kernel(int Nz, int Nx, const T* __restrict__ kx,
+                                                        const T* __restrict__ kz, int pin, T dpin,
+                                                        const T* __restrict__ xc, const T* __restrict__ x,
+                                                        const T* __restrict__ b, T* xo, T omega) {
+  XC_PDL_WAIT();
+  const int Nzc = Nz / 2, Nxc = Nx / 2;
+  const int J = blockIdx.x * 32 + threadIdx.x, I = blockIdx.y * 8 + threadIdx.y;
+  if (J >= Nzc || I >= Nxc) return;
+  const int j = 2 * J, i0 = 2 * I, i1 = i0 + 1, il = i0 == 0 ? Nx - 1 : i0 - 1, ir = i1 == Nx - 1 ? 0 : i1 + 1;
+  const bool top = j > 0, bot = j + 2 < Nz;
+  const int o0 = i0 * Nz + j, o1 = i1 * Nz + j, ol = il * Nz + j, orr = ir * Nz + j;
+  // the coarse cells around (J, I): rows clamped, columns periodic
+  const int Jm = J > 0 ? J - 1 : 0, Jp = J < Nzc - 1 ? J + 1 : J;
+  const T* cm = xc + (I == 0 ? Nxc - 1 : I - 1) * Nzc;
+  const T* c0 = xc + I * Nzc;
+  const T* cp = xc + (I + 1 == Nxc ? 0 : I + 1) * Nzc;
+  const T mm = cm[Jm], m0 = cm[J], mp = cm[Jp], zm = c0[Jm], z0 = c0[J], zp = c0[Jp], pm = cp[Jm], p0 = cp[J], pp = cp[Jp];
+  // p_prolong_val from a cell's own coarse value, the one along z, along x, and across
+  auto pro = [](T own, T along, T side, T cross) {
+    return mul_rn<T>(add_rn<T>(add_rn<T>(add_rn<T>(mul_rn<T>((T)9, own), mul_rn<T>((T)3, along)), mul_rn<T>((T)3, side)),
+                               cross), (T)0.0625);
+  };
+  const Pair<T> fl = ld_pair(x + ol), fa = ld_pair(x + o0), fb = ld_pair(x + o1), fr = ld_pair(x + orr);
+  const T xa0 = add_rn<T>(fa.a, pro(z0, zm, m0, mm)), xa1 = add_rn<T>(fa.b, pro(z0, zp, m0, mp));
+  const T xb0 = add_rn<T>(fb.a, pro(z0, zm, p0, pm)), xb1 = add_rn<T>(fb.b, pro(z0, zp, p0, pp));
+  const T xl0 = add_rn<T>(fl.a, pro(m0, mm, z0, zm)), xl1 = add_rn<T>(fl.b, pro(m0, mp, z0, zp));
+  const T xr0 = add_rn<T>(fr.a, pro(p0, pm, z0, zm)), xr1 = add_rn<T>(fr.b, pro(p0, pp, z0, zp));
+  T ta = 0, tb = 0, ba = 0, bb = 0;
+  if (top) {
+    ta = add_rn<T>(x[o0 - 1], pro(zm, z0, mm, m0));
+    tb = add_rn<T>(x[o1 - 1], pro(zm, z0, pm, p0));
+  }
+  if (bot) {
+    ba = add_rn<T>(x[o0 + 2], pro(zp, z0, mp, m0));
+    bb = add_rn<T>(x[o1 + 2], pro(zp, z0, pp, p0));
+  }
+  const Pair<T> kl = ld_pair(kx + o0), km = ld_pair(kx + o1), kr = ld_pair(kx + orr);
+  const T* za = kz + i0 * (Nz + 1) + j;
+  const T* zb = za + Nz + 1;
+  const T a0 = za[0], a1 = za[1], a2 = za[2], b0 = zb[0], b1 = zb[1], b2 = zb[2];
+  const Pair<T> ra = ld_pair(b + o0), rb = ld_pair(b + o1);
+  auto relax = [&](T xv, T bv, T ax, T k0, T k1, T k2, T k3, bool t, bool u, bool pinned) {
+    T d = k0 + k1 + (t ? k2 : (T)0) + (u ? k3 : (T)0);
+    if (pinned) d += dpin;
+    return d > (T)0 ? xv + sdiv<T>(omega * (bv - ax), d) : (T)0;
+  };
+  const T y00 = relax(xa0, ra.a, p_quad_apply<T>(xa0, xl0, xb0, ta, xa1, kl.a, km.a, a0, a1, top, true, o0 == pin, dpin),
+                      kl.a, km.a, a0, a1, top, true, o0 == pin);
+  const T y10 = relax(xa1, ra.b, p_quad_apply<T>(xa1, xl1, xb1, xa0, ba, kl.b, km.b, a1, a2, true, bot, o0 + 1 == pin, dpin),
+                      kl.b, km.b, a1, a2, true, bot, o0 + 1 == pin);
+  const T y01 = relax(xb0, rb.a, p_quad_apply<T>(xb0, xa0, xr0, tb, xb1, km.a, kr.a, b0, b1, top, true, o1 == pin, dpin),
+                      km.a, kr.a, b0, b1, top, true, o1 == pin);
+  const T y11 = relax(xb1, rb.b, p_quad_apply<T>(xb1, xa1, xr1, xb0, bb, km.b, kr.b, b1, b2, true, bot, o1 + 1 == pin, dpin),
+                      km.b, kr.b, b1, b2, true, bot, o1 + 1 == pin);
+  st_pair(xo + o0, y00, y10);
+  st_pair(xo + o1, y01, y11);
+}
+
 template <typename T>
 __global__ void p_coarsen_kernel(int Nzc, int Nxc, const T* __restrict__ kx, const T* __restrict__ kz,
                                  T* kxc, T* kzc) {
@@ -3317,6 +3442,7 @@ inline dim3 grid2(const Geo& g, int layers = 1) {
   return dim3((unsigned)((g.Nz + 2 + 31) / 32), (unsigned)((g.Nx + 2 + 7) / 8), (unsigned)layers);
 }
 constexpr long long kSplitCells = 128 * 128;
+constexpr long long kQuadCells = 128 * 128;
 inline bool split_rows(const Geo& g) { return (long long)g.Nz * g.Nx <= kSplitCells; }
 
 }  // namespace
@@ -3992,12 +4118,22 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
     }
     PCoarse<T> C = {};
     if (p_tiled(H, cfg, l + 1)) C = {H.px[l + 1], H.kx[l + 1], H.kz[l + 1], H.ppin[l + 1], H.pdpin[l + 1]};
-    pdl(PDL_ON, p_down_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
-        H.pdpin[l], (const T*)a, (const T*)H.pb[l], H.pb[l + 1], om, C);
+    const bool quads = (long long)n > kQuadCells;
+    const dim3 qgrid((unsigned)((Nzc + 31) / 32), (unsigned)((Nxc + 7) / 8));
+    if (quads)
+      pdl(PDL_ON, p_down_quad_kernel<T>, qgrid, blk2(), s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+          H.pdpin[l], (const T*)a, (const T*)H.pb[l], H.pb[l + 1], om, C);
+    else
+      pdl(PDL_ON, p_down_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+          H.pdpin[l], (const T*)a, (const T*)H.pb[l], H.pb[l + 1], om, C);
     XC_LAUNCH_CHECK();
     XC_TRY(vcycle_p<T>(H, cfg, l + 1, s, &ec));
-    pdl(PDL_ON, p_up_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
-        H.pdpin[l], (const T*)ec, (const T*)a, (const T*)H.pb[l], o, om);
+    if (quads)
+      pdl(PDL_ON, p_up_quad_kernel<T>, qgrid, blk2(), s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+          H.pdpin[l], (const T*)ec, (const T*)a, (const T*)H.pb[l], o, om);
+    else
+      pdl(PDL_ON, p_up_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+          H.pdpin[l], (const T*)ec, (const T*)a, (const T*)H.pb[l], o, om);
     { T* tmp = a; a = o; o = tmp; }
     for (int q = 1; q < cfg.nu_p; ++q) {
       pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l], o,
