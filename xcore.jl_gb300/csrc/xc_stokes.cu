@@ -2037,25 +2037,19 @@ __global__ void __launch_bounds__(kTileThreads) p_up_tile_kernel(int Nz, int Nx,
 // The same two on large levels, which are bound by instruction issue: a thread
 // per coarse cell takes its 2 x 2 fine ones, whose values, coefficients and
 // prolongations it shares between them, in pairs along z (Nz is even), without
-// a halo formed twice.  From which size on matters little (1024^2 step with the
+// a halo formed twice.  FP32 only: in FP64 the ascent's twelve prolongations cost
+// more of the FP64 unit than the tile's (1024^2 step of the FP64 solver 106 against
+// 103 ms).  From which size on matters little (1024^2 step with the
 // line at 64^2, 128^2, 256^2 cells: 1.602x, 1.608x, 1.592x of the original,
 // without them 1.499x; 512^2 solve 1.573x, 1.560x, 1.581x and 1.536x).
 template <typename T>
 struct Pair { T a, b; };
-template <typename T>
-__device__ __forceinline__ Pair<T> ld_pair(const T* p) {
-  if constexpr (kFly<T>) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    return {v.x, v.y};
-  } else {
-    const double2 v = *reinterpret_cast<const double2*>(p);
-    return {v.x, v.y};
-  }
+__device__ __forceinline__ Pair<float> ld_pair(const float* p) {
+  const float2 v = *reinterpret_cast<const float2*>(p);
+  return {v.x, v.y};
 }
-template <typename T>
-__device__ __forceinline__ void st_pair(T* p, T a, T b) {
-  if constexpr (kFly<T>) *reinterpret_cast<float2*>(p) = make_float2(a, b);
-  else *reinterpret_cast<double2*>(p) = make_double2(a, b);
+__device__ __forceinline__ void st_pair(float* p, float a, float b) {
+  *reinterpret_cast<float2*>(p) = make_float2(a, b);
 }
 // (L p) of one cell from its value and neighbours, p_apply_fn's operations
 template <typename T>
@@ -4118,22 +4112,26 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
     }
     PCoarse<T> C = {};
     if (p_tiled(H, cfg, l + 1)) C = {H.px[l + 1], H.kx[l + 1], H.kz[l + 1], H.ppin[l + 1], H.pdpin[l + 1]};
-    const bool quads = (long long)n > kQuadCells;
+    const bool quads = kFly<T> && (long long)n > kQuadCells;
     const dim3 qgrid((unsigned)((Nzc + 31) / 32), (unsigned)((Nxc + 7) / 8));
-    if (quads)
-      pdl(PDL_ON, p_down_quad_kernel<T>, qgrid, blk2(), s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+    if (quads) {
+      if constexpr (kFly<T>)
+        pdl(PDL_ON, p_down_quad_kernel<T>, qgrid, blk2(), s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
           H.pdpin[l], (const T*)a, (const T*)H.pb[l], H.pb[l + 1], om, C);
-    else
+    } else {
       pdl(PDL_ON, p_down_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
           H.pdpin[l], (const T*)a, (const T*)H.pb[l], H.pb[l + 1], om, C);
+    }
     XC_LAUNCH_CHECK();
     XC_TRY(vcycle_p<T>(H, cfg, l + 1, s, &ec));
-    if (quads)
-      pdl(PDL_ON, p_up_quad_kernel<T>, qgrid, blk2(), s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
+    if (quads) {
+      if constexpr (kFly<T>)
+        pdl(PDL_ON, p_up_quad_kernel<T>, qgrid, blk2(), s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
           H.pdpin[l], (const T*)ec, (const T*)a, (const T*)H.pb[l], o, om);
-    else
+    } else {
       pdl(PDL_ON, p_up_tile_kernel<T>, tiles, kTileThreads, s, Nz, Nx, (const T*)H.kx[l], (const T*)H.kz[l], H.ppin[l],
           H.pdpin[l], (const T*)ec, (const T*)a, (const T*)H.pb[l], o, om);
+    }
     { T* tmp = a; a = o; o = tmp; }
     for (int q = 1; q < cfg.nu_p; ++q) {
       pdl(PDL_ON, p_jacobi_kernel<T>, nblk(n), 256, s, Nz, Nx, H.kx[l], H.kz[l], H.ppin[l], H.pdpin[l], a, H.pb[l], o,
