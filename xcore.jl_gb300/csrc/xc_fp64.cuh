@@ -121,6 +121,8 @@ XC_HD double xc_div(double a, double b) {
     const uint64_t mant = (q + 1) >> 1;                      // with its leading bit, which adds one to the exponent
     return xc_from_bits(((uint64_t)((ha ^ hb) & 0x80000000u) << 32) + ((uint64_t)(uint32_t)(e0 - lt - 1) << 52) + mant);
   }
+  // a field that is zero where it has not started to move takes this way in every cell
+  if (!(ua << 1) && (ub << 1) - 1 < (0x7ffull << 53) - 1) return xc_from_bits((ua ^ ub) & (1ull << 63));
   return a / b;
 }
 
@@ -238,6 +240,7 @@ XC_HD double xc_sqrt(double a) {
     const uint64_t mant = (S + 1) >> 1;
     return xc_from_bits(((uint64_t)(uint32_t)((e + 1023 - odd) >> 1) << 52) + (mant - (1ull << 52)));
   }
+  if (!(ua << 1)) return a;
   return std::sqrt(a);
 }
 
