@@ -484,7 +484,7 @@ long long xc_launch_count(void);
    together exceed twice the L2).  which: 0 WENO5/QUICK advect-with-flux of X (phsevo!),
    1 FP64 Stokes operator apply, 2 FP32 velocity Jacobi sweep (finest level,
    one row per thread as the mixed solver runs it), 3 FP64 velocity Jacobi
-   sweep, 4 FFT line filter (z pass of psie), 5 the FP32 sweep with four rows
+   sweep, 4 filter pass along z of psie (sums or FFT, as noise! has it), 5 the FP32 sweep with four rows
    per thread (row_block_sweep).
    out = {ms per launch, algorithmic bytes per
    launch, algorithmic flops per launch, units per launch}.  Kernels 1-3 need
