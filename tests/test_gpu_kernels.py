@@ -104,8 +104,8 @@ def test_diffus_and_ghosts_bitwise():
     np.testing.assert_array_equal(_host(d_dff), dff)
 
 
-# edges of the 16 x 8 tile of small grids and the 32 x 16 tile of grids above
-# 3 * 152 * 512 (diffusion) and 9 * 152 * 512 cells (advection)
+# edges of the 16 x 8 tile of small grids and the 32 x 16 tile of large ones
+# (diffusion above 7 * 152 * 512 cells; advection in the test below)
 @pytest.mark.parametrize("scheme", ["weno5", "quick", "fromm"])
 @pytest.mark.parametrize("shape", [(16, 8), (17, 9), (15, 7), (3, 130), (569, 547), (863, 833)])
 @pytest.mark.parametrize("bcs", [("periodic", "closed"), ("closed", "periodic")])
