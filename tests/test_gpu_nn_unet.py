@@ -123,6 +123,27 @@ def test_unet_gradients_match_torch_autograd():
     net.close()
 
 
+@pytest.mark.parametrize("B,N", [(1, 128), (8, 256), (4, 512)])
+def test_output_bias_gradient_against_64_bits(B, N):
+    """The output layer's bias gradient is the sum of dY = 2 (out - target) / pixels in BF16 over all pixels, which
+    the forward pass gives exactly.  It is added in FP32: at most 8 terms of a lane in a tile, 241 tiles of a CTA and
+    some ten more roundings of 2^-24 each, which add up like a random walk to 1e-6 of sum |dY|; twice that here."""
+    net = Net(N, N, B, seed=4)
+    x, t = _inputs(B, N, N, net.cin, net.cout, seed=6)
+    x, t = x.cuda(), (t + 0.3).cuda().contiguous()
+    out = torch.empty((B, N, N, net.cout), device="cuda")
+    loss = ctypes.c_float()
+    torch.cuda.synchronize()
+    assert xc.lib().xc_nn_forward(net.h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()), None) == xc.XC_OK
+    assert xc.lib().xc_nn_loss_grad(net.h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(t.data_ptr()),
+                                    ctypes.byref(loss), None) == xc.XC_OK
+    db = net.layer(net.grads(), 14)[1][:net.cout].astype(np.float64)
+    d = (2.0 * (out - t) * (1.0 / (B * N * N))).to(torch.bfloat16).double().reshape(-1, net.cout)
+    err = np.abs(db - d.sum(0).cpu().numpy()) / d.abs().sum(0).cpu().numpy()
+    assert err.max() <= 2e-6, err
+    net.close()
+
+
 def test_unet_forward_matches_torch():
     B, H, W = 1, 256, 256
     net = Net(H, W, B, seed=5)

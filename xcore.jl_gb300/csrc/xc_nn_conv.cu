@@ -20,7 +20,8 @@
 // for the tensor core, so tiles of 128 pixels are operands as they lie in
 // memory.  M holds several taps at once: 128 / Cin tiles of Cin channels each
 // (they lie one after another, the descriptor's leading offset steps from one
-// to the next), N is Cout; a tile of ones gives sum_p dY, the bias gradient.  FP32 partial sums per CTA, reduced over CTAs
+// to the next), N is Cout.  The bias gradient sum_p dY is added in FP32 by warps
+// of its own from the same tiles.  FP32 partial sums per CTA, reduced over CTAs
 // in a fixed order (deterministic).
 #include <algorithm>
 #include <cstring>
@@ -442,12 +443,12 @@ bool tile_shape(int H, int W, int* bw, int* bh) {
 // weight gradient
 // ---------------------------------------------------------------------------
 // A CTA takes one row of taps (blockIdx.y: dy) over the tiles blockIdx.x,
-// + gridDim.x, ...  A step is one tile: the three taps' X tiles, a tile of ones
-// behind them (its sums are the bias gradient) and dY's tile.  The rows of A
-// are 128 / Cin of these tiles at a time (16 and 32 channels: all of them, 64:
-// two and two, 128: one by one), so one pass over A serves several taps; rows
-// beyond the fourth tile (16 channels) read what lies behind and are not
-// stored.  Operands come in as the forward's pixels do.  It was bound by two-byte transposing stores and by nine passes over dY with M
+// + gridDim.x, ...  A step is one tile: the three taps' X tiles, a tile of zeros
+// behind them where 128 rows of A reach beyond the third, and dY's tile.  The rows
+// of A are 128 / Cin of these tiles at a time (16 and 32 channels: all of them,
+// 64: two and two, 128: one by one), so one pass over A serves several taps; rows
+// beyond the fourth tile (16 channels) read what lies behind, and no row but
+// the taps' is stored.  Operands come in as the forward's pixels do.  It was bound by two-byte transposing stores and by nine passes over dY with M
 // mostly zero rows: 16 x 16 channels at 8 x 256 x 256 pixels 154 us, with the
 // bias gradient's own two kernels 220; now 62 and 3 for the reduction.  What
 // bounds it is the rate of the MMAs themselves (eight per tile and CTA, about
@@ -455,30 +456,54 @@ bool tile_shape(int H, int W, int* bw, int* bh) {
 struct WgradArgs {
   const __nv_bfloat16* x;    // NHWC [B][H][W][Cin]
   const __nv_bfloat16* dy;   // NHWC [B][H][W][Cout]
-  float* partial;            // [gridDim.x][9][Cin][Cout], then [gridDim.x][Cout]
+  float* partial;            // [gridDim.x][9][Cin][Cout], then [gridDim.x][kBiasWarps][Cout]
+  int bias;                  // 1: the bias gradient's partial sums too
   int B, H, W, bw, bh, tiles;
   int* err;
 };
 
-constexpr int kWgThreads = 160;           // four loading warps, one issuing
+constexpr int kBiasWarps = 2;
+constexpr int kWgThreads = 160 + 32 * kBiasWarps;   // four loading warps, one issuing, those of the bias gradient
 constexpr int kWgMaxStages = 8;
 
 template <int CIN, int COUT>
 struct WgCfg {
   static constexpr uint32_t kX = 128u * CIN * 2u, kY = 128u * COUT * 2u;
-  // tile of ones: as large as a tap's where it shares rows with taps, else a
-  // 4 KB block that every K step reads
-  static constexpr uint32_t kOnes = CIN == 128 ? 4096u : kX;
-  static constexpr uint32_t kStage = 3u * kX + kOnes + kY;
+  static constexpr uint32_t kZeros = CIN == 128 ? 0u : kX;        // the fourth tile of A's rows
+  static constexpr uint32_t kStage = 3u * kX + kZeros + kY;
   static constexpr uint32_t kRoom = 200u * 1024u;
   static constexpr int kStages = kRoom / kStage > kWgMaxStages ? kWgMaxStages : (int)(kRoom / kStage);
-  // rows beyond the ones tile (16 channels: four more tiles' worth) stay inside the allocation
+  // rows beyond the fourth tile (16 channels: four more tiles' worth) stay inside the allocation
   static constexpr uint32_t kTail = CIN == 16 ? 4u * kX : 0u;
   static constexpr uint32_t kSmem = kStages * kStage + kTail + 1024u;
   static constexpr int kSlots = 128 / CIN;                       // tiles per group of A rows
-  static constexpr int kGroups = CIN == 16 || CIN == 32 ? 1 : (CIN == 64 ? 2 : 4);
+  static constexpr int kGroups = CIN == 16 || CIN == 32 ? 1 : (CIN == 64 ? 2 : 3);
   static constexpr uint32_t kTmemCols = tmem_cols_for(kGroups * COUT);
 };
+
+// sum over the 128 pixels of a dY tile by the kBiasWarps warps, thread t of
+// them the 8 channels of chunk t % (COUT / 8) of every (32 kBiasWarps / CH)th
+// pixel, added to acc
+template <int COUT>
+__device__ __forceinline__ void bias_add_tile(const uint8_t* tile, int t, float (&acc)[8]) {
+  constexpr int CH = COUT / 8, STEP = 32 * kBiasWarps / CH, KY = COUT < 64 ? COUT : 64;
+  constexpr uint32_t RB = KY * 2u;
+  const int c = t % CH;
+  const uint8_t* part = tile + (uint32_t)(c / (KY / 8)) * 128u * RB;
+  float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int m = t / CH; m < 128; m += STEP) {
+    const uint4 q = *reinterpret_cast<const uint4*>(part + swz_chunk<RB>((uint32_t)m, (uint32_t)(c % (KY / 8))));
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sum[2 * j] += __uint_as_float(w[j] << 16);
+      sum[2 * j + 1] += __uint_as_float(w[j] & 0xffff0000u);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] += sum[j];
+}
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap tmX,
@@ -501,14 +526,20 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_kernel(const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
   const int dy = (int)blockIdx.y - 1;
 
+  // The bias gradient's own warps in one row of CTAs: added in FP32, a tile's
+  // sum apart from the running one.  As a row of ones in the MMAs it comes at no
+  // cost, but the tensor core truncates its running sum: up to 2e-5 of sum |dY|
+  // off (4 x 512^2 pixels), here up to 1.2e-7, in launches of its own 6e-7.  U-Net
+  // gradient at 8 x 256^2 with ones 1181 us, two warps 1187, one 1210, four 1209.
+  const bool bias = a.bias != 0 && dy == 0;
+
   for (int s = 0; s < NS; ++s)
-    for (uint32_t o = tid * 16u; o < Cfg::kOnes; o += kWgThreads * 16u)
-      *reinterpret_cast<uint4*>(gbase + s * Cfg::kStage + 3u * Cfg::kX + o) =
-          make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+    for (uint32_t o = tid * 16u; o < Cfg::kZeros; o += kWgThreads * 16u)
+      *reinterpret_cast<uint4*>(gbase + s * Cfg::kStage + 3u * Cfg::kX + o) = make_uint4(0, 0, 0, 0);
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) {
       mbar_init(smem_u32(&bar_full[s]), (TX && TY ? 0 : 128) + (TX || TY ? 1 : 0));
-      mbar_init(smem_u32(&bar_empty[s]), 1);
+      mbar_init(smem_u32(&bar_empty[s]), bias ? 1 + kBiasWarps : 1);
     }
     mbar_init(smem_u32(&bar_done), 1);
     s_fail = 0;
@@ -538,7 +569,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_kernel(const __gr
           break;
         }
         const ImageTile tile = tile_at(t, a.W, a.H, a.bw, a.bh);
-        const uint32_t sx = base + s * Cfg::kStage, sy = sx + 3u * Cfg::kX + Cfg::kOnes, full = smem_u32(&bar_full[s]);
+        const uint32_t sx = base + s * Cfg::kStage, sy = sx + 3u * Cfg::kX + Cfg::kZeros, full = smem_u32(&bar_full[s]);
         if (tid == 0 && (TX || TY)) {
           mbar_expect_tx(full, (TX ? 3u * Cfg::kX : 0u) + (TY ? Cfg::kY : 0u));
           if (TX) {
@@ -563,6 +594,35 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_kernel(const __gr
     // TMA loads still in flight (only after a wait ran out) end before the CTA does
     if (tid == 0 && (TX || TY))
       for (int q = it - NS > 0 ? it - NS : 0; q < it; ++q) mbar_wait(smem_u32(&bar_full[q % NS]), (q / NS) & 1);
+  } else if (warp >= 5) {
+    if (bias) {
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      bool ok = true;
+      int it = 0;
+      for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, ++it) {
+        const int s = it % NS;
+        ok = true;
+        if (lane == 0) ok = mbar_wait(smem_u32(&bar_full[s]), (it / NS) & 1);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (lane == 0) flag_error(a.err, 11);
+          s_fail = 1;
+          break;
+        }
+        bias_add_tile<COUT>(gbase + s * Cfg::kStage + 3u * Cfg::kX + Cfg::kZeros, tid - 160, acc);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
+      }
+      constexpr int CH = COUT / 8;
+#pragma unroll
+      for (int o = CH; o < 32; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+      float* dst = a.partial + (size_t)gridDim.x * 9 * CIN * COUT + ((size_t)blockIdx.x * kBiasWarps + (warp - 5)) * COUT;
+      if (ok && lane < CH)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dst[lane * 8 + j] = acc[j];
+    }
   } else if (lane == 0) {
     int it = 0;
     bool ok = true;
@@ -576,19 +636,14 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_kernel(const __gr
       }
       if (!(TX && TY)) fence_async_shared();
       tc_fence_after();
-      const uint32_t sx = base + s * Cfg::kStage, ones = sx + 3u * Cfg::kX, sy = ones + Cfg::kOnes;
+      const uint32_t sx = base + s * Cfg::kStage, sy = sx + 3u * Cfg::kX + Cfg::kZeros;
 #pragma unroll
-      for (int g = 0; g < Cfg::kGroups; ++g) {
-        if (CIN == 128 && g == 3 && dy != 0) continue;       // its own group: the bias of one row of CTAs
+      for (int g = 0; g < Cfg::kGroups; ++g)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint64_t ad = CIN == 128 && g == 3
-                                  ? smem_desc_mn(ones, 2048u, 1024u, kLayoutSW128)
-                                  : smem_desc_mn(sx + g * Cfg::kSlots * Cfg::kX + k * 16 * RBX, TILEX, 8u * RBX, LX);
-          umma_bf16(tmem + (uint32_t)(g * COUT), ad, smem_desc_mn(sy + k * 16 * RBY, TILEY, 8u * RBY, LY), IDESC,
-                    (it | k) != 0 ? 1u : 0u);
-        }
-      }
+        for (int k = 0; k < 8; ++k)
+          umma_bf16(tmem + (uint32_t)(g * COUT),
+                    smem_desc_mn(sx + g * Cfg::kSlots * Cfg::kX + k * 16 * RBX, TILEX, 8u * RBX, LX),
+                    smem_desc_mn(sy + k * 16 * RBY, TILEY, 8u * RBY, LY), IDESC, (it | k) != 0 ? 1u : 0u);
       umma_commit(smem_u32(&bar_empty[s]));
     }
     if (ok) umma_commit(smem_u32(&bar_done));
@@ -605,11 +660,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_kernel(const __gr
     const int m = warp * 32 + lane;
 #pragma unroll
     for (int g = 0; g < Cfg::kGroups; ++g) {
-      const int slot = g * Cfg::kSlots + m / CIN;              // 0..2 taps, 3 the ones
-      if (CIN == 128 && g == 3 && dy != 0) continue;
-      const bool live = slot < 3 || (slot == 3 && m % CIN == 0 && dy == 0);
-      float* dst = slot < 3 ? a.partial + (((size_t)blockIdx.x * 9 + 3 * blockIdx.y + slot) * CIN + m % CIN) * COUT
-                            : a.partial + (size_t)gridDim.x * 9 * CIN * COUT + (size_t)blockIdx.x * COUT;
+      const int slot = g * Cfg::kSlots + m / CIN;              // 0..2 taps
+      const bool live = slot < 3;
+      float* dst = a.partial + (((size_t)blockIdx.x * 9 + 3 * blockIdx.y + (live ? slot : 0)) * CIN + m % CIN) * COUT;
 #pragma unroll
       for (int c0 = 0; c0 < COUT; c0 += 16) {
         uint32_t r[16];
@@ -645,11 +698,12 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
   const int n = 9 * Cin * Cout;
   const int q = threadIdx.x >> 5, i = blockIdx.x * 32 + (threadIdx.x & 31);
   float v = 0.0f;
-  if (i < n + Cout) {
+  if (i < n || (db && i < n + Cout)) {
     const float* p = i < n ? partial + i : partial + (size_t)nblk * n + (i - n);
     const size_t st = i < n ? n : Cout;
+    const int nb = i < n ? nblk : nblk * kBiasWarps;
 #pragma unroll 4
-    for (int k = q; k < nblk; k += 8) v += p[(size_t)k * st];
+    for (int k = q; k < nb; k += 8) v += p[(size_t)k * st];
   }
   sh[q][threadIdx.x & 31] = v;
   __syncthreads();
@@ -731,7 +785,7 @@ int nn_conv3x3_fwd(const void* x, const void* w, const float* bias, void* y, flo
 }
 
 long long nn_wgrad_scratch(int B, int H, int W, int Cin, int Cout) {
-  return std::min<long long>((long long)B * H * W / 128, kWgBlocks) * (9 * Cin + 1) * Cout;
+  return std::min<long long>((long long)B * H * W / 128, kWgBlocks) * (9 * Cin + kBiasWarps) * Cout;
 }
 
 int nn_conv3x3_wgrad(const void* x, const void* dy, float* dw, float* db, float* partial, int B, int H, int W,
@@ -757,7 +811,7 @@ int nn_conv3x3_wgrad(const void* x, const void* dy, float* dw, float* db, float*
   std::memset(&ty, 0, sizeof(ty));
   if (Cin >= 64) XC_TRY(make_act_map(&tx, x, B, H, W, Cin, bw, bh));
   if (Cout >= 64) XC_TRY(make_act_map(&ty, dy, B, H, W, Cout, bw, bh));
-  WgradArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, partial, B, H, W, bw, bh, tiles, err};
+  WgradArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, partial, db ? 1 : 0, B, H, W, bw, bh, tiles, err};
   switch (Cin) {
     case 16: XC_TRY(launch_wgrad_n<16>(Cout, tx, ty, a, nx, s)); break;
     case 32: XC_TRY(launch_wgrad_n<32>(Cout, tx, ty, a, nx, s)); break;
