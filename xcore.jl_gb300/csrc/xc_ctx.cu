@@ -7,6 +7,8 @@
 #include <unordered_map>
 #include <mutex>
 
+#include <cuda.h>
+
 #include "xc_internal.cuh"
 
 namespace {
@@ -47,6 +49,25 @@ void xc_set_error(const char* fmt, ...) {
 }
 
 extern "C" const char* xc_last_error(void) { return g_err; }
+
+int xc_context_id(unsigned long long* id) {
+  typedef CUresult (*Fn)(CUcontext, unsigned long long*);
+  static Fn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+                   q == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<Fn>(p)
+               : nullptr;
+  }();
+  if (fn && fn(nullptr, id) == CUDA_SUCCESS) return XC_OK;
+  XC_CUDA_TRY(cudaFree(nullptr));      // the runtime's first call makes the context
+  if (!fn || fn(nullptr, id) != CUDA_SUCCESS) {
+    xc_set_error("cuCtxGetId is not available from the driver");
+    return XC_CUDA;
+  }
+  return XC_OK;
+}
 
 unsigned persistent_grid(const void* kernel, int rows, int cols) {
   static std::mutex mu;

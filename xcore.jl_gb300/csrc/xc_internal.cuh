@@ -99,6 +99,10 @@ void xc_set_error(const char* fmt, ...);
 
 #define XC_LAUNCH_CHECK() XC_CUDA_TRY(cudaGetLastError())
 
+// the calling thread's current context (the device's primary one where none is
+// current yet): an id that no other context has, also none after a reset
+int xc_context_id(unsigned long long* id);
+
 // number of kernels this library has launched (host side): process-wide, and
 // per host thread for the bookkeeping of stream capture (contexts may be
 // driven from several threads at once)

@@ -10,7 +10,7 @@
 struct ErrFlag {
   int* dev = nullptr;
   int* host = nullptr;
-  int slot = -1;
+  bool* used = nullptr;      // its place in the context's page (null: allocated for itself)
   ErrFlag() = default;
   ErrFlag(const ErrFlag&) = delete;
   ErrFlag& operator=(const ErrFlag&) = delete;

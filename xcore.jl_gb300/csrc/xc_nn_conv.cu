@@ -36,6 +36,7 @@
 #define XC_PDL_EARLY
 #include "xc_internal.cuh"
 #include "xc_nn.cuh"
+#include "xc_once.h"
 #include "xc_nn_tc.cuh"
 
 using namespace xcnn;
@@ -391,6 +392,17 @@ __global__ void __launch_bounds__(kFwdThreads) conv3x3_fwd_kernel(const __grid_c
   }
 }
 
+// the shared memory a kernel opts into, once per context
+int opt_in_smem(xc::PerKey<char>& done, const void* kernel, size_t bytes) {
+  unsigned long long id = 0;
+  XC_TRY(xc_context_id(&id));
+  char* set = nullptr;
+  return done.get(id, &set, [&](char*) -> int {
+    XC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return XC_OK;
+  });
+}
+
 template <int KC, int NOUT, bool RES>
 int launch_fwd_res(const CUtensorMap& ta, const CUtensorMap& tb, const ConvArgs& a, cudaStream_t s) {
   using Cfg = FwdCfg<KC, NOUT>;
@@ -400,13 +412,8 @@ int launch_fwd_res(const CUtensorMap& ta, const CUtensorMap& tb, const ConvArgs&
   const int per_sm = w + 4u * Cfg::kStage(RES) + 1024u <= kMost / 2 && Cfg::kTmemCols <= 256 ? 2 : 1;
   int stages = (int)((kMost / per_sm - 1024u - w) / Cfg::kStage(RES));
   if (stages > kMaxStages) stages = kMaxStages;
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(conv3x3_fwd_kernel<KC, NOUT, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kMost);
-  });
-  XC_CUDA_TRY(attr);
+  static xc::PerKey<char> smem;
+  XC_TRY(opt_in_smem(smem, (const void*)conv3x3_fwd_kernel<KC, NOUT, RES>, kMost));
   const int grid = a.tiles < per_sm * kNumSMs ? a.tiles : per_sm * kNumSMs;
   xc_launch(conv3x3_fwd_kernel<KC, NOUT, RES>, grid, kFwdThreads, w + stages * Cfg::kStage(RES) + 1024u, s, ta, tb,
             a, stages);
@@ -722,13 +729,8 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
 template <int CIN, int COUT>
 int launch_wgrad(const CUtensorMap& tx, const CUtensorMap& ty, const WgradArgs& a, int nx, cudaStream_t s) {
   using Cfg = WgCfg<CIN, COUT>;
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(conv3x3_wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)Cfg::kSmem);
-  });
-  XC_CUDA_TRY(attr);
+  static xc::PerKey<char> smem;
+  XC_TRY(opt_in_smem(smem, (const void*)conv3x3_wgrad_kernel<CIN, COUT>, Cfg::kSmem));
   xc_launch(conv3x3_wgrad_kernel<CIN, COUT>, dim3(nx, 3), kWgThreads, Cfg::kSmem, s, tx, ty, a);
   XC_LAUNCH_CHECK();
   return XC_OK;
@@ -826,30 +828,39 @@ int nn_conv3x3_wgrad(const void* x, const void* dy, float* dw, float* db, float*
 }
 
 // Error flags of the kernels' bounded waits: ints of one page of pinned host
-// memory that every device can write, taken for the length of a call (or of a
-// network's life).  Nothing is allocated, cleared or copied per call: a kernel
-// writes its flag only when a wait ran out, and the host reads it after it has
-// waited for the stream.  The page is allocated on first use and kept; with all
-// kFlagSlots taken a flag is allocated for itself.
+// memory per context, taken for the length of a call (or of a network's life).
+// Nothing is allocated, cleared or copied per call: a kernel writes its flag only
+// when a wait ran out, and the host reads it after it has waited for the stream.
+// A page is allocated on first use and kept; with all kFlagSlots taken a flag is
+// allocated for itself.
 namespace {
 constexpr int kFlagSlots = 256;
-std::mutex g_flag_mu;
-int* g_flags = nullptr;
-bool g_flag_used[kFlagSlots];
+struct FlagPage {
+  int* host = nullptr;
+  bool used[kFlagSlots] = {};
+};
+std::mutex g_flag_mu;                                       // of the pages' `used`
+auto& g_flag_pages = *new xc::PerKey<FlagPage>();           // (outlives every flag)
 }  // namespace
 
 int ErrFlag::init() {
-  std::lock_guard<std::mutex> lock(g_flag_mu);
-  if (!g_flags)
-    XC_CUDA_TRY(cudaHostAlloc((void**)&g_flags, sizeof(int) * kFlagSlots, cudaHostAllocPortable | cudaHostAllocMapped));
-  for (int q = 0; q < kFlagSlots && slot < 0; ++q)
-    if (!g_flag_used[q]) slot = q;
-  if (slot >= 0) {
-    g_flag_used[slot] = true;
-    host = g_flags + slot;
-  } else {
-    XC_CUDA_TRY(cudaHostAlloc((void**)&host, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+  unsigned long long id = 0;
+  XC_TRY(xc_context_id(&id));
+  FlagPage* p = nullptr;
+  XC_TRY(g_flag_pages.get(id, &p, [](FlagPage* f) -> int {
+    XC_CUDA_TRY(cudaHostAlloc((void**)&f->host, sizeof(int) * kFlagSlots, cudaHostAllocMapped));
+    return XC_OK;
+  }));
+  {
+    std::lock_guard<std::mutex> lock(g_flag_mu);
+    for (int q = 0; q < kFlagSlots && !used; ++q)
+      if (!p->used[q]) {
+        used = &p->used[q];
+        *used = true;
+        host = p->host + q;
+      }
   }
+  if (!used) XC_CUDA_TRY(cudaHostAlloc((void**)&host, sizeof(int), cudaHostAllocMapped));
   *host = 0;
   XC_CUDA_TRY(cudaHostGetDevicePointer((void**)&dev, host, 0));
   return XC_OK;
@@ -864,9 +875,9 @@ int ErrFlag::check(cudaStream_t s, const char* what) {
   return XC_OK;
 }
 ErrFlag::~ErrFlag() {
-  if (slot >= 0) {
+  if (used) {
     std::lock_guard<std::mutex> lock(g_flag_mu);
-    g_flag_used[slot] = false;
+    *used = false;
   } else if (host) {
     cudaFreeHost(host);
   }
@@ -876,26 +887,23 @@ namespace {
 // stream-ordered scratch of one call from a pool that keeps up to 32 MB (with
 // the default pool every call that waits for its stream gives the memory back
 // to the system and maps it again)
-cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev >= 64) return cudaMallocAsync(p, bytes, s);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!pools[dev]) {
-      cudaMemPoolProps props = {};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
-      if ((e = cudaMemPoolCreate(&pools[dev], &props)) != cudaSuccess) return e;
-      unsigned long long keep = 32ull << 20;
-      cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
-    }
-  }
-  return cudaMallocFromPoolAsync(p, bytes, pools[dev], s);
+int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+  static xc::PerKey<cudaMemPool_t> pools;
+  unsigned long long id = 0;
+  XC_TRY(xc_context_id(&id));
+  cudaMemPool_t* pool = nullptr;
+  XC_TRY(pools.get(id, &pool, [](cudaMemPool_t* q) -> int {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    XC_CUDA_TRY(cudaGetDevice(&props.location.id));
+    XC_CUDA_TRY(cudaMemPoolCreate(q, &props));
+    unsigned long long keep = 32ull << 20;
+    cudaMemPoolSetAttribute(*q, cudaMemPoolAttrReleaseThreshold, &keep);
+    return XC_OK;
+  }));
+  XC_CUDA_TRY(cudaMallocFromPoolAsync(p, bytes, *pool, s));
+  return XC_OK;
 }
 }  // namespace
 
@@ -919,7 +927,7 @@ extern "C" int xc_nn_conv3x3_wgrad(const void* x, const void* dy, float* dw, int
   XC_TRY(e.init());
   float* partial = nullptr;
   if (Cin >= 16 && Cin <= 128 && Cout >= 16 && Cout <= 128 && B > 0 && H > 0 && W > 0)
-    XC_CUDA_TRY(scratch_alloc((void**)&partial, sizeof(float) * (size_t)nn_wgrad_scratch(B, H, W, Cin, Cout), s));
+    XC_TRY(scratch_alloc((void**)&partial, sizeof(float) * (size_t)nn_wgrad_scratch(B, H, W, Cin, Cout), s));
   const int st = nn_conv3x3_wgrad(x, dy, dw, nullptr, partial, B, H, W, Cin, Cout, 1.0f, 0, e.dev, s);
   if (partial) cudaFreeAsync(partial, s);
   if (st == XC_BAD_ARG) return st;
