@@ -346,6 +346,23 @@ def test_device_givens_respects_the_iteration_cap():
         assert its == maxit, (maxit, str(e.value))
 
 
+def test_device_givens_queues_no_step_of_the_host_path():
+    """Refinement passes of one inner iteration each: with the least-squares update on the device every pass makes the
+    same launches, and none for a step of the host path queued ahead and done again."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=48, Nx=48, steps=1)
+    total = []
+    for maxit in range(5):
+        ds = device_state(par, g, sc, st)
+        before = xc.lib().xc_launch_count()
+        with pytest.raises(xc.NotConverged):
+            ds.fluidmech(O.time_coefs("bd2im", 2), dt, solver="mixed", rtol=1e-15, maxit=maxit, inner_rtol=1e-3,
+                         inner_maxit=1, device_givens=True)
+        total.append(xc.lib().xc_launch_count() - before)
+        ds.close()
+    per_pass = np.diff(total)
+    assert per_pass[0] > 0 and (per_pass == per_pass[0]).all(), per_pass
+
+
 @pytest.mark.parametrize("N", [128, 200, 256])
 def test_cluster_vcycle_matches_the_per_level_launches(N):
     """cluster_cells: the velocity levels between the one-CTA size and 128^2

@@ -4830,19 +4830,19 @@ int fgmres(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, con
       krylov_start_kernel<<<1, 32, 0, s>>>(H.kd, beta, bnorm, rtol * 0.5, maxit, its);
       xc_count_launch();
       const int its0 = its;
-      int launched = 0, st = XC_OK;
+      int queued = 0, st = XC_OK;
       for (int kk = 0; kk < m; ++kk) {
         st = cond_step<T>(w, H, k, cfg, kk, s);
         if (st != XC_OK) break;
         XC_CUDA_TRY(cudaEventRecord(H.kev[kk & 1], s));
-        ++launched;
+        ++queued;
         if (kk >= 1) {
           XC_CUDA_TRY(cudaEventSynchronize(H.kev[(kk - 1) & 1]));
           const volatile KrylovStatus* ks = H.ks_host;
           if (ks->done || ks->its >= maxit) break;
         }
       }
-      if (st != XC_OK && launched == 0 && its == its0) {
+      if (st != XC_OK && queued == 0 && its == its0) {
         // no conditional graph could be built (nothing ran): host Givens
         // for this hierarchy from now on
         H.cond_broken = true;
@@ -4864,6 +4864,7 @@ int fgmres(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, con
         relres = ks->relres;
         if (ks->bad) { xc_set_error("fgmres: breakdown"); *its_out = its; *relres_out = relres; return XC_NAN; }
         if ((flags & FG_TRUST_EST) && (relres <= rtol || its >= maxit)) break;
+        launched = 0;
         continue;
       }
     }
@@ -5520,9 +5521,11 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
       XC_LAUNCH_CHECK();
       XC_TRY(dot_self<double>(w, w->d, res, n, 3, s));
       // the inner solve's first step is queued before the residual is known
-      // where the last pass is expected to have left more to do
+      // where the last pass is expected to have left more to do (a solve whose
+      // least-squares problem is on the device queues its own steps)
+      const bool host_steps = !icfg.device_givens || w->f.cond_broken;
       bool started = false;
-      if (outer > 0 && !learned_on && relres * expect > 2.0 * o.rtol && its < o.maxit) {
+      if (outer > 0 && !learned_on && host_steps && relres * expect > 2.0 * o.rtol && its < o.maxit) {
         XC_CUDA_TRY(cudaEventRecord(w->f.kev[1], s));
         inner_start_kernel<<<nblk(n, 256 * kVecRows), 256, 0, s>>>(n, w->hdev + 6, res, w->f.w, w->f.V); xc_count_launch();
         XC_TRY(arnoldi_step<float>(w, w->f, k, icfg, 0, s));
