@@ -644,19 +644,53 @@ __device__ __forceinline__ void vel_update_edge_u(const Geo& g, const OpConst& k
   if (MODE != 0) ax = vel_edge_row_u<T>(g, k, xi + g.NW, u, j, &d);
   vel_put<T, MODE>(xi, b, out, (T)1, g.NW + u, ax, d, dscl);
 }
+// Rows of mixed kinds.  In FP64 the two ways meet again before the quotient, which
+// is most of such a row: a warp that holds both kinds then takes it once (one
+// CTA's sweeps on a 75 x 75 level, whose every second warp holds an edge: a 300^2
+// FP64 solve 2.05 s, with a quotient in either way 2.30 s).  An FP32 quotient is
+// cheaper than the selects (1024^2 mixed step 34.3 ms, with one quotient 36.4).
 template <typename T, int MODE>
 __device__ __forceinline__ void vel_update_w(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xi,
                                              const T* b, T* out, T omega, long long t, int j, int i,
                                              const T* dscl = nullptr) {
-  if (vel_edge_w(g, j, i)) vel_update_edge_w<T, MODE>(g, k, op, xi, b, out, (int)t, j, i, dscl);
-  else vel_update_int_w<T, MODE>(g, op, xi, b, out, omega, (int)t, j, i, dscl);
+  if constexpr (kFly<T>) {
+    if (vel_edge_w(g, j, i)) vel_update_edge_w<T, MODE>(g, k, op, xi, b, out, (int)t, j, i, dscl);
+    else vel_update_int_w<T, MODE>(g, op, xi, b, out, omega, (int)t, j, i, dscl);
+    return;
+  }
+  T d, ax = 0, w = omega;
+  if (vel_edge_w(g, j, i)) {
+    if (MODE == 0) d = vel_diag_w<T>(g, op, t, j, i);
+    else ax = vel_edge_row_w<T>(g, k, op, xi, xi + g.NW, t, j, i, &d);
+    w = (T)1;
+  } else {
+    const RowW<T> c = w_row<T>(g, op, t, j, i);
+    if (MODE != 0) ax = vel_dot_w<T>(c, xi + t, xi + (g.NW + (i - 1) * (g.Nz + 2) + j), g.Nz + 1, g.Nz + 2);
+    d = c.d;
+  }
+  vel_put<T, MODE>(xi, b, out, w, (int)t, ax, d, dscl);
 }
 template <typename T, int MODE>
 __device__ __forceinline__ void vel_update_u(const Geo& g, const OpConst& k, const VOp<T>& op, const T* xi,
                                              const T* b, T* out, T omega, long long u, int j, int i,
                                              const T* dscl = nullptr) {
-  if (vel_edge_u(g, k, u, j)) vel_update_edge_u<T, MODE>(g, k, xi, b, out, (int)u, j, dscl);
-  else vel_update_int_u<T, MODE>(g, op, xi, b, out, omega, (int)u, j, i, dscl);
+  if constexpr (kFly<T>) {
+    if (vel_edge_u(g, k, u, j)) vel_update_edge_u<T, MODE>(g, k, xi, b, out, (int)u, j, dscl);
+    else vel_update_int_u<T, MODE>(g, op, xi, b, out, omega, (int)u, j, i, dscl);
+    return;
+  }
+  const T* xu = xi + g.NW;
+  T d = 1, ax = 0, w = omega;
+  if (vel_edge_u(g, k, u, j)) {
+    if (MODE != 0) ax = vel_edge_row_u<T>(g, k, xu, u, j, &d);
+    w = (T)1;
+  } else {
+    const RowW<T> c = u_row<T>(g, op, u, j, i);
+    const int lu = g.Nz + 2, il = (i == 0) ? g.Nx - 1 : i - 1, ir = (i == g.Nx) ? 1 : i + 1;
+    if (MODE != 0) ax = vel_dot_u<T>(c, xu + u, xu + (il * lu + j), xu + (ir * lu + j), xi + (i * (g.Nz + 1) + j - 1), g.Nz + 1);
+    d = c.d;
+  }
+  vel_put<T, MODE>(xi, b, out, w, g.NW + (int)u, ax, d, dscl);
 }
 // rows of a level in three runs -- interior W, interior U, edges -- so that the
 // lanes of a warp take the same way: row r of run q, in 0 .. count - 1
