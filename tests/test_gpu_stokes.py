@@ -363,6 +363,32 @@ def test_device_givens_queues_no_step_of_the_host_path():
     assert per_pass[0] > 0 and (per_pass == per_pass[0]).all(), per_pass
 
 
+def test_long_steps_are_not_queued_ahead():
+    """On a grid whose coarsest level (31x47 cells) one CTA sweeps for milliseconds a mixed solve makes the launches of
+    its refinement passes and of the steps it counts, and none for a step queued too many.  A pass's and a step's own
+    launches come from solves that their caps stop after none or one pass of one or two steps."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=62, Nx=94, steps=1)
+    coefs = O.time_coefs("bd2im", 2)
+
+    def launches(rtol, maxit, inner_rtol, inner_maxit):
+        ds = device_state(par, g, sc, st)
+        before, info = xc.lib().xc_launch_count(), None
+        try:
+            info = ds.fluidmech(coefs, dt, solver="mixed", rtol=rtol, maxit=maxit, inner_rtol=inner_rtol,
+                                inner_maxit=inner_maxit)
+        except xc.NotConverged:
+            pass
+        n = xc.lib().xc_launch_count() - before
+        ds.close()
+        return n, info
+    none, one, two = (launches(1e-15, m, 1e-15, max(m, 1))[0] for m in (0, 1, 2))
+    step, per_pass = two - one, one - none - (two - one)
+    assert step > 0 and per_pass > 0
+    for inner_rtol in (0.1, 5e-2, 1e-2, 1e-3):
+        n, info = launches(1e-9, 600, inner_rtol, 30)
+        assert n == none + per_pass * info["refinements"] + step * info["iterations"], (inner_rtol, info, n, none, step)
+
+
 @pytest.mark.parametrize("N", [128, 200, 256])
 def test_cluster_vcycle_matches_the_per_level_launches(N):
     """cluster_cells: the velocity levels between the one-CTA size and 128^2

@@ -3605,6 +3605,7 @@ struct Hier {
   KrylovStatus* ks_dev;
   cudaEvent_t kev[2];
   int expect;         // steps of the last cycle of the solve under way (0: none yet)
+  bool ahead;         // steps may be queued before the one before them is known (fgmres)
   bool cond_broken;   // building a conditional graph failed: host Givens from then on
 };
 
@@ -4804,7 +4805,13 @@ constexpr int FG_STARTED = 4;
 // yet where it expects the cycle to go on: as many steps as the cycle before
 // took, or while the estimate, falling as it did and half again as fast, stays
 // above the tolerance.  A step too many leaves nothing behind (its vectors are
-// not combined); at 512^2 and below it costs less than two waits.
+// not combined), but costs its time, in about one cycle of two with FP32's short
+// cycles: a time step with and without queueing 3.97 and 4.13 ms at 64^2, 26.4 and
+// 26.7 at 576^2, 17.9 and 17.8 at 640^2, 22.3 and 21.9 at 768^2, 70.8 and 68.3 at
+// 1536^2.  FP64 cycles are longer and gain at every size (192^2 12.8 and 13.0 ms,
+// 1024^2 123.7 and 124.5).  Where one CTA's sweeps make a step last milliseconds
+// queueing loses with both (100 x 202 mixed, 50 x 101 cells swept: 160 and 146 ms;
+// 78 x 82, 39 x 41: 115.5 and 112.8; 400^2, 25 x 25: 31.5 and 31.8).
 struct RefineTail {
   const double* scl;
   double* x;
@@ -4914,7 +4921,7 @@ int fgmres(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, con
         ++launched;
       }
       const bool falling = kk >= 2 && relres * (relres / before) * 0.5 > rtol;
-      if (kk + 1 < m && its + 1 < maxit && (kk + 1 < H.expect || falling)) {
+      if (H.ahead && kk + 1 < m && its + 1 < maxit && (kk + 1 < H.expect || falling)) {
         XC_TRY(arnoldi_step<T>(w, H, k, cfg, kk + 1, s));
         XC_CUDA_TRY(cudaEventRecord(H.kev[(kk + 1) & 1], s));
         ++launched;
@@ -5175,6 +5182,10 @@ int setup_hier(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg,
   const bool wide = cfg.direct_coarse && !k.mms && (np <= kDenseMax || sweeps_c >= (kFly<T> ? 0.0125 : 0.01));
   H.vwide_on = wide && !H.vdirect && nv <= kWideMax;
   H.pwide_on = wide && !H.pdirect && np <= kWideMax;
+  // steps are queued ahead up to 2^20 unknowns (FP32) and 2^20 row sweeps of one CTA
+  const long long swept = (H.vdirect || H.vwide_on ? 0 : nv * coarse_sweeps(cfg, H.vg[lv].Nz, H.vg[lv].Nx)) +
+                          (H.pdirect || H.pwide_on ? 0 : np * coarse_sweeps(cfg, H.pNz[lp], H.pNx[lp]));
+  H.ahead = swept <= (1 << 20) && (!kFly<T> || n <= (1 << 20));
   if (H.vwide_on || H.pwide_on) XC_TRY(wide_inverses<T>(H, k, cfg, lv, lp, s));
   if (H.vdirect) {
     vel_dense_inv_kernel<T><<<1, 256, 0, s>>>(H.vg[lv], level_const(k, lv), vop(H, lv), H.vinv, H.dok);
@@ -5559,7 +5570,7 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
       // least-squares problem is on the device queues its own steps)
       const bool host_steps = !icfg.device_givens || w->f.cond_broken;
       bool started = false;
-      if (outer > 0 && !learned_on && host_steps && relres * expect > 2.0 * o.rtol && its < o.maxit) {
+      if (outer > 0 && !learned_on && host_steps && w->f.ahead && relres * expect > 2.0 * o.rtol && its < o.maxit) {
         XC_CUDA_TRY(cudaEventRecord(w->f.kev[1], s));
         inner_start_kernel<<<nblk(n, 256 * kVecRows), 256, 0, s>>>(n, w->hdev + 6, res, w->f.w, w->f.V); xc_count_launch();
         XC_TRY(arnoldi_step<float>(w, w->f, k, icfg, 0, s));
