@@ -1680,31 +1680,9 @@ __device__ __forceinline__ void vel_sweeps_reg(const Geo& g, const OpConst& k, c
 // R: rows a thread of sweeps in registers (the caller's CTA has a thread per R
 // rows); 0: any CTA
 template <typename T, int R>
-__device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op, T* x, T* x2, const T* b,
-                               int sweeps, T omega, const T* inv, const int* inv_ok, const WideInverse& wide,
-                               unsigned dvw = 0, unsigned dvu = 0) {
+__device__ __forceinline__ void vel_coarse_sweeps(const Geo& g, const OpConst& k, const VOp<T>& op, T* x, T* x2,
+                                                  const T* b, int sweeps, T omega, unsigned dvw = 0, unsigned dvu = 0) {
   const long long n = (long long)g.NW + g.NU;
-  if (inv && *inv_ok) {
-    dense_apply_cta<T>(inv, (int)n, (int)n, b, x);
-    return;
-  }
-  if (wide.inv && *inv_ok) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int pass = 0; pass < (kFly<T> ? 1 : 2); ++pass) {
-      const T* rhs = b;
-      if (pass == 1) {       // one step of refinement in FP64, the residual in x2
-        for (long long t = threadIdx.x; t < n; t += blockDim.x) vel_residual_at<T>(g, k, op, x, b, x2, t);
-        __syncthreads();
-        rhs = x2;
-      }
-      for (int r = warp; r < n; r += nw) {
-        const float v = wide_row<T>(wide, (int)n, rhs, r, lane);
-        if (lane == 0) x[r] = pass == 1 ? x[r] + (T)v : (T)v;
-      }
-      __syncthreads();
-    }
-    return;
-  }
   for (long long t = threadIdx.x; t < n; t += blockDim.x) x[t] = 0;
   __syncthreads();
   T* a = x;
@@ -1743,13 +1721,48 @@ __device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op,
     __syncthreads();
   }
 }
+// the level's solve: by its inverse, dense or wide, or by the sweeps
+template <typename T, int R>
+__device__ void vel_coarse_cta(const Geo& g, const OpConst& k, const VOp<T>& op, T* x, T* x2, const T* b,
+                               int sweeps, T omega, const T* inv, const int* inv_ok, const WideInverse& wide,
+                               unsigned dvw = 0, unsigned dvu = 0) {
+  const long long n = (long long)g.NW + g.NU;
+  if (inv && *inv_ok) {
+    dense_apply_cta<T>(inv, (int)n, (int)n, b, x);
+    return;
+  }
+  if (wide.inv && *inv_ok) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int pass = 0; pass < (kFly<T> ? 1 : 2); ++pass) {
+      const T* rhs = b;
+      if (pass == 1) {       // one step of refinement in FP64, the residual in x2
+        for (long long t = threadIdx.x; t < n; t += blockDim.x) vel_residual_at<T>(g, k, op, x, b, x2, t);
+        __syncthreads();
+        rhs = x2;
+      }
+      for (int r = warp; r < n; r += nw) {
+        const float v = wide_row<T>(wide, (int)n, rhs, r, lane);
+        if (lane == 0) x[r] = pass == 1 ? x[r] + (T)v : (T)v;
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  vel_coarse_sweeps<T, R>(g, k, op, x, x2, b, sweeps, omega, dvw, dvu);
+}
+// Sweeps alone, of levels too large for the kernel below, which have neither a
+// dense inverse nor a wide one inside a CTA (with the code for those beside them
+// the sweeps were 1 % slower, the pressure's 12 %).  They last milliseconds, so the
+// next grid is not let in early: its blocks would share the one busy SM (120 x 250
+// mixed solve 566 and 596 ms).
+__device__ __forceinline__ void wait_only() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename T>
 __global__ void __launch_bounds__(1024) vel_coarse_kernel(Geo g, OpConst k, VOp<T> op, T* x, T* x2,
-                                                          const T* __restrict__ b, int sweeps, T omega, const T* inv,
-                                                          const int* inv_ok, WideInverse wide, const int* solved) {
-  XC_PDL_WAIT();
+                                                          const T* __restrict__ b, int sweeps, T omega,
+                                                          const int* solved) {
+  wait_only();
   if (solved && *solved) return;     // by the launches of the wide inverse before this one
-  vel_coarse_cta<T, 0>(g, k, op, x, x2, b, sweeps, omega, inv, inv_ok, wide);
+  vel_coarse_sweeps<T, 0>(g, k, op, x, x2, b, sweeps, omega);
 }
 // of up to 2 kCoarseRegThreads rows: two a thread (72 registers), the iterates in
 // shared memory, 2 (NW + NU) elements
@@ -2260,6 +2273,28 @@ __device__ __forceinline__ void p_sweeps_reg(int Nz, int Nx, const T* __restrict
   }
 }
 
+// `sweeps` damped-Jacobi sweeps from zero by one CTA
+template <typename T>
+__device__ __forceinline__ void p_coarse_sweeps(int Nz, int Nx, const T* __restrict__ kx, const T* __restrict__ kz,
+                                                int pin, T dpin, T* x, T* x2, const T* b, int sweeps, T omega) {
+  const int n = Nz * Nx;
+  for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = 0;
+  __syncthreads();
+  T* a = x;
+  T* o = x2;
+  for (int s = 0; s < sweeps; ++s) {
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+      T d;
+      T ax = p_apply_at<T>(Nz, Nx, kx, kz, pin, dpin, a, t % Nz, t / Nz, &d);
+      o[t] = d > (T)0 ? a[t] + sdiv<T>(omega * (b[t] - ax), d) : (T)0;
+    }
+    __syncthreads();
+    T* tmp = a; a = o; o = tmp;
+  }
+  if (a != x)
+    for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = a[t];
+  __syncthreads();
+}
 template <typename T>
 __device__ void p_coarse_cta(int Nz, int Nx, const T* __restrict__ kx, const T* __restrict__ kz, int pin,
                              T dpin, T* x, T* x2, const T* b, int sweeps, T omega, const T* inv,
@@ -2286,44 +2321,35 @@ __device__ void p_coarse_cta(int Nz, int Nx, const T* __restrict__ kx, const T* 
     }
     return;
   }
+  if (n > (int)blockDim.x) {
+    p_coarse_sweeps<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega);
+    return;
+  }
   for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = 0;
   __syncthreads();
-  T* a = x;
-  T* o = x2;
-  if (n <= (int)blockDim.x) {
-    p_sweeps_reg<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega);
-    if (sweeps & 1) a = x2;
-  } else {
-    for (int s = 0; s < sweeps; ++s) {
-      for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        T d;
-        T ax = p_apply_at<T>(Nz, Nx, kx, kz, pin, dpin, a, t % Nz, t / Nz, &d);
-        o[t] = d > (T)0 ? a[t] + sdiv<T>(omega * (b[t] - ax), d) : (T)0;
-      }
-      __syncthreads();
-      T* tmp = a; a = o; o = tmp;
-    }
-  }
-  if (a != x)
-    for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = a[t];
+  p_sweeps_reg<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega);
+  if (sweeps & 1)
+    for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = x2[t];
   __syncthreads();
 }
-template <typename T>
+// (STAGED: the iterates in shared memory; levels too large for it have no inverse
+// inside a CTA either)
+template <typename T, bool STAGED>
 __global__ void __launch_bounds__(1024) p_coarse_kernel(int Nz, int Nx, const T* __restrict__ kx,
                                                         const T* __restrict__ kz, int pin, T dpin, T* x, T* x2,
                                                         const T* __restrict__ b, int sweeps, T omega, const T* inv,
-                                                        const int* inv_ok, WideInverse wide, const int* solved,
-                                                        int staged) {
-  XC_PDL_WAIT();
+                                                        const int* inv_ok, WideInverse wide, const int* solved) {
+  if (STAGED) XC_PDL_WAIT();
+  else wait_only();
   if (solved && *solved) return;
-  extern __shared__ __align__(16) unsigned char xc_stage[];
-  if (staged) {
+  if constexpr (STAGED) {
+    extern __shared__ __align__(16) unsigned char xc_stage[];
     const int n = Nz * Nx;
     T* sx = reinterpret_cast<T*>(xc_stage);
     p_coarse_cta<T>(Nz, Nx, kx, kz, pin, dpin, sx, sx + n, b, sweeps, omega, inv, inv_ok, wide);
     for (int t = threadIdx.x; t < n; t += blockDim.x) x[t] = sx[t];
   } else {
-    p_coarse_cta<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega, inv, inv_ok, wide);
+    p_coarse_sweeps<T>(Nz, Nx, kx, kz, pin, dpin, x, x2, b, sweeps, omega);
   }
 }
 
@@ -4009,8 +4035,7 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
                (const int*)H.dok, wi, solved, stage_div(std::max(1, g.Nz - 1)), stage_div(g.Nz));
     else
       pdl(PDL_ON, vel_coarse_kernel<T>, 1, coarse_threads(n), s, g, k, vop(H, l), H.vx[l], H.vx2[l],
-          (const T*)H.vb[l], coarse_sweeps(cfg, g.Nz, g.Nx), om, (const T*)(H.vdirect ? H.vinv : nullptr),
-          (const int*)H.dok, wi, solved);
+          (const T*)H.vb[l], coarse_sweeps(cfg, g.Nz, g.Nx), om, solved);
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
@@ -4126,11 +4151,12 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
       solved = H.dok + 1;
     }
     const size_t sweep_bytes = 2 * sizeof(T) * (size_t)n;
-    const int in_smem = sweep_bytes <= kSweepSmemMax;
-    pdl_smem(PDL_ON, p_coarse_kernel<T>, 1, coarse_threads(2LL * n), in_smem ? sweep_bytes : 0, s, Nz, Nx, H.kx[l], H.kz[l],
+    const bool in_smem = sweep_bytes <= kSweepSmemMax;
+    pdl_smem(PDL_ON, in_smem ? p_coarse_kernel<T, true> : p_coarse_kernel<T, false>, 1, coarse_threads(2LL * n),
+             in_smem ? sweep_bytes : 0, s, Nz, Nx, H.kx[l], H.kz[l],
              H.ppin[l], H.pdpin[l], H.px[l], H.px2[l], H.pb[l], coarse_sweeps(cfg, Nz, Nx), om,
              (const T*)(H.pdirect ? H.pinv : nullptr), (const int*)(H.dok + 1),
-             solved ? WideInverse{nullptr, 0} : p_wide(H, l), solved, in_smem);
+             solved ? WideInverse{nullptr, 0} : p_wide(H, l), solved);
     XC_LAUNCH_CHECK();
     return XC_OK;
   }
