@@ -152,6 +152,30 @@ def test_large_advection_tile_bitwise():
         np.testing.assert_array_equal(_host(got), want)
 
 
+@pytest.mark.parametrize("scheme,Nz,Nx", [("quick", 2, 524280), ("quick", 2, 524281), ("centr", 1, 1048560)])
+def test_thin_fields_of_many_columns_bitwise(scheme, Nz, Nx):
+    """Rows on both sides of the most columns that 65535 blocks of the small tile cover (8 each), and the most that the
+    large one covers."""
+    rng = np.random.default_rng(Nx % 97)
+    f, u, w = rng.random((Nz, Nx)), rng.standard_normal((Nz, Nx + 1)), rng.standard_normal((Nz + 1, Nx))
+    d = [torch.zeros(s, dtype=torch.float64, device="cuda") for s in ((Nx, Nz), (Nx + 1, Nz + 2), (Nx + 2, Nz + 1))]
+    xc.advect_centered_with_flux(*d, _dev(f), _dev(u), _dev(w), 0.37, scheme, "periodic", "closed")
+    torch.cuda.synchronize()
+    for got, want in zip(d, O.advect_centered_with_flux(f, u, w, 0.37, scheme, "periodic", "closed")):
+        np.testing.assert_array_equal(_host(got), want)
+
+
+@pytest.mark.parametrize("Nx", [524280, 530000])
+def test_thin_diffusion_of_many_columns_bitwise(Nx):
+    rng = np.random.default_rng(3)
+    f, k = rng.random((1, Nx)), rng.random((1, Nx))
+    fh, kh = O.embed_halo(f, 1, "closed", "periodic"), O.embed_halo(k, 1, "closed", "periodic")
+    d = torch.zeros((Nx, 1), dtype=torch.float64, device="cuda")
+    xc.diffus(d, _dev(fh), _dev(kh), 0.2)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(_host(d), O.diffus_halo(fh, kh, 0.2))
+
+
 def test_ghosts_halo3_both_closed():
     Nz, Nx, g = 9, 6, 3
     f = np.random.default_rng(1).random((Nz, Nx))

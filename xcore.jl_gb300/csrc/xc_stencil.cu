@@ -42,6 +42,11 @@ template <int Z, int X, int T> struct TileShape {
 using SmallTile = TileShape<16, 8, 288>;
 using LargeTile = TileShape<32, 16, 256>;
 constexpr long long kSmallAdvect = 18LL * kNumSMs * 512, kSmallDiffus = 7LL * kNumSMs * 512;
+// (a grid has at most 65535 blocks along x: rows of more than 8 times as many
+// columns, fields one or two cells high, take the larger tile's 16 columns too)
+inline bool small_tile(long long most, int Nz, int Nx) {
+  return (long long)Nz * Nx <= most && (Nx + SmallTile::TX - 1) / SmallTile::TX <= 65535;
+}
 
 // ---------------------------------------------------------------------------
 // face reconstructions (advect.jl:35-53, 216-229, 275-283)
@@ -478,7 +483,7 @@ void launch_advect_tile(const FluxArgs& a, bool halod, int Nz, int Nx, int xBC, 
 template <int S>
 int launch_advect(const FluxArgs& a, bool halod, int Nz, int Nx, int xBC, int zBC, double invh, bool pad,
                   cudaStream_t s) {
-  if ((long long)Nz * Nx <= kSmallAdvect)
+  if (small_tile(kSmallAdvect, Nz, Nx))
     launch_advect_tile<SmallTile, S>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
   else
     launch_advect_tile<LargeTile, S>(a, halod, Nz, Nx, xBC, zBC, invh, pad, s);
@@ -488,7 +493,7 @@ int launch_advect(const FluxArgs& a, bool halod, int Nz, int Nx, int xBC, int zB
 
 template <int S>
 int launch_phsevo_fluxes(const PhsevoFluxes& p, int Nz, int Nx, int xBC, int zBC, double invh, cudaStream_t s) {
-  if ((long long)Nz * Nx <= kSmallAdvect)
+  if (small_tile(kSmallAdvect, Nz, Nx))
     xc_launch(phsevo_flux_kernel<SmallTile, S>, tile_grid<SmallTile>(Nz, Nx, 3), SmallTile::NT, 0, s, p, Nz, Nx, xBC,
               zBC, invh);
   else
@@ -542,7 +547,7 @@ static int diffus_launch(const double* f, const double* k, int ld, int Nz, int N
                          DView dff, DView qx, DView qz, bool pad, cudaStream_t s) {
   const FluxArgs a{f, ld, CView{nullptr, 0}, CView{nullptr, 0}, k, nullptr, dff, qx, qz};
   const double invh = 1.0 / h;
-  if ((long long)Nz * Nx <= kSmallDiffus)
+  if (small_tile(kSmallDiffus, Nz, Nx))
     xc_launch(diffus_tile_kernel<SmallTile, true>, tile_grid<SmallTile>(Nz, Nx), SmallTile::NT, 0, s, a, Nz, Nx, xBC,
               zBC, invh, pad);
   else
