@@ -110,6 +110,41 @@ def test_integer_functions_against_the_processor(tmp_path):
     assert r.returncode == 0, r.stdout
 
 
+SQUARES = PROBE[:PROBE.index("int main() {")] + r"""
+int main() {
+  std::mt19937_64 g(22);
+  long bad = 0;
+  const double edge[] = {0.0, -0.0, 1.0, -1.5, 5e-324, 0x1p-1022, 0x1.fffffffffffffp1023, INFINITY, -INFINITY, NAN,
+                         0x1p-511, 0x1p-507, 0x1.fffffffffffffp-508, 0x1p515, 0x1.fffffffffffffp515, 0x1p516};
+  auto check = [&](double a) {
+    const double q = xc_sqr<8>(a), r = (a * 0.0625) * (a * 0.0625);
+    if (xc_bits(q) != xc_bits(r) && !(q != q && r != r)) { if (bad++ < 5) std::printf("%a: %a not %a\n", a, q, r); }
+  };
+  for (double a : edge) check(a);
+  for (long i = 0; i < 4000000; ++i) {       // all exponents whose quotient by 16 is normal
+    const uint64_t e = i % 2 ? 983 + g() % 80 : 5 + g() % 2042;
+    check(xc_from_bits((g() & (1ull << 63)) | (e << 52) | significand(g(), g() % 5)));
+  }
+  std::printf("bad %ld\n", bad);
+  return bad != 0;
+}
+"""
+
+
+def test_scaled_squares_against_the_processor(tmp_path):
+    """xc_sqr<K>: the bits of the square of a 2^(-K/2), through both ends of the range, zeros, infinities and NaN."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not available")
+    src = tmp_path / "squares.cpp"
+    src.write_text(SQUARES)
+    exe = tmp_path / "squares"
+    subprocess.run([gxx, "-O2", "-std=c++17", "-ffp-contract=off", "-I", os.path.join(ROOT, "xcore.jl_gb300", "csrc"),
+                    str(src), "-o", str(exe)], check=True, capture_output=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
 PRODUCTS = PROBE[:PROBE.index("int main() {")] + r"""
 static bool same(double a, double b) { return xc_bits(a) == xc_bits(b) || (a != a && b != b); }
 static long check(double a, double b) {

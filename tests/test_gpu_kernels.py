@@ -215,6 +215,20 @@ def test_phsevo_weno5_one_division_weights(ADVN):
     ds.close()
 
 
+def test_weno5_common_denominator_for_large_fields():
+    """The products of the common denominator grow as the ninth power of the field.  Of values 0 and A, the weights
+    0.1, 0.6, 0.3 of indicators up to 8.4 A^2 times polynomials up to 2 A reach 5800 A^9: finite for A = 6e33."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=40, Nx=36, ADVN="weno5")
+    ds = device_state(par, g, sc, st, weno_weights=1)
+    X = 6e33 * rng.integers(0, 2, (g.Nz, g.Nx)).astype(np.float64)
+    ds["X"] = X
+    ds.phsevo(O.time_coefs("bd2im", 3), dt, ADVN="weno5")
+    adv, qx, qz = O.advect_centered_with_flux(X, ds["Ux"][1:-1], ds["Wx"][:, 1:-1], g.h, "weno5")
+    for name, want in (("advn_X", adv), ("qx_advn_X", qx), ("qz_advn_X", qz)):
+        assert np.isfinite(want).all() and rel_err(ds[name], want) <= 1e-12, (name, rel_err(ds[name], want))
+    ds.close()
+
+
 def test_store_and_phase_velocities_bitwise():
     par, g, sc, ns, st, dt, rng = realistic_state()
     ds = device_state(par, g, sc, st)

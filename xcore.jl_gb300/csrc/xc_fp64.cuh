@@ -162,10 +162,18 @@ XC_HD double xc_mul(double a, double b) {
   }
   return xc_mul_edge(a, b);
 }
+// a^2 2^-K, K even: the power of two costs nothing here
+#ifdef __CUDACC__
+__host__ __device__ __noinline__ inline double xc_sqr_any(double a, double scale) { return (a * scale) * (a * scale); }
+#else
+inline double xc_sqr_any(double a, double scale) { return (a * scale) * (a * scale); }
+#endif
+template <int K = 0>
 XC_HD double xc_sqr(double a) {
+  static_assert(K >= 0 && K % 2 == 0 && K < 100, "the scale's root is a power of two");
   const uint64_t ua = xc_bits(a);
   const uint32_t ha = (uint32_t)(ua >> 32);
-  const int ea = (int)((ha >> 20) & 0x7ffu), e = 2 * ea - 1023;
+  const int ea = (int)((ha >> 20) & 0x7ffu), e = 2 * ea - 1023 - K;
   if ((unsigned)(e - 1) < 2044u) {
     const uint32_t al = (uint32_t)ua, ah = (ha & 0xfffffu) | 0x100000u;
     const uint64_t p = xc_mulwide(al, al);
@@ -173,7 +181,7 @@ XC_HD double xc_sqr(double a) {
     const uint64_t h = xc_mulwide(ah, ah) + (m >> 32);
     return xc_from_bits(xc_round63((h << 21) | ((uint32_t)m >> 11), ((uint32_t)m << 21) | (uint32_t)p, e, 0));
   }
-  return xc_mul_edge(a, a);
+  return ua << 1 ? xc_sqr_any(a, xc_from_bits((uint64_t)(1023 - K / 2) << 52)) : 0.0;
 }
 // K a for a small odd K: the product of the significand is exact in 64 bits
 template <int K>

@@ -77,12 +77,14 @@ __device__ __forceinline__ double weno5_poly(double fmm, double fm, double fc, d
 // The same reconstruction with the weights over a common denominator: with
 // q_k = (eps + b_k)^2 the weights d_k / q_k are proportional to
 // n_1 = q_2 q_3, n_2 = 6 q_1 q_3, n_3 = 3 q_1 q_2, so the weighted mean needs
-// one division instead of four.  Each q_k lies in [eps^2, (eps + b_k)^2]: the
-// products stay normal and finite for fields below about 1e70.  The
-// smoothness indicators are taken four times as large (a power of two, which
-// leaves the weights as they are) and the common factor 1/6 of the three
-// polynomials is applied once: 46 FP64 instructions per reconstruction
-// (within a few ulps).
+// one division instead of four.  The smoothness indicators are formed four
+// times as large and the q_k a sixteenth of their size (powers of two, which
+// leave the weights as they are), and the common factor 1/6 of the three
+// polynomials is applied once (within a few ulps).  The products n_k p_k grow as
+// the ninth power of the field and are finite up to some 1e34; each q_k is at
+// least (4 eps)^2 / 256, far from underflow.  27 FP64 instructions per
+// reconstruction, as many as the reference's form takes: the products and the
+// quotients are integer ones.
 __device__ __forceinline__ double weno5_poly_onediv(double fmm, double fm, double fc, double fp,
                                                     double fpp) {
   const double c133 = 4.0 * (13.0 / 12.0), eps4 = 4.0 * XC_EPS;
@@ -97,7 +99,7 @@ __device__ __forceinline__ double weno5_poly_onediv(double fmm, double fm, doubl
   t = __fma_rn(-2.0, fp, fc) + fpp;
   s = __fma_rn(3.0, fc, __fma_rn(-4.0, fp, fpp));
   const double e3 = __fma_rn(xc_mul(t, c133), t, xc_sqr(s)) + eps4;
-  const double q1 = xc_sqr(e1), q2 = xc_sqr(e2), q3 = xc_sqr(e3);
+  const double q1 = xc_sqr<8>(e1), q2 = xc_sqr<8>(e2), q3 = xc_sqr<8>(e3);
   const double n1 = xc_mul(q2, q3), n2 = xc_mul_small<6>(xc_mul(q1, q3)), n3 = xc_mul_small<3>(xc_mul(q1, q2));
   return xc_mul(xc_div(__fma_rn(n1, p1, __fma_rn(n2, p2, xc_mul(n3, p3))), (n1 + n2) + n3), 1.0 / 6.0);
 }
