@@ -188,3 +188,18 @@ def test_integer_products_against_the_processor(tmp_path):
                     str(src), "-o", str(exe)], check=True, capture_output=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.parametrize("call", ["xc_exp(0.5)", "(double)xc_log2_fixed(0.5)", "xc_exp2_product(1ull << 58, 5)"])
+def test_table_functions_do_not_compile_for_the_host_under_nvcc(tmp_path, call):
+    """Their tables are in device memory: a host call in a .cu file is an error, not a wrong number."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    for body, ok in ((f"__global__ void k(double* y) {{ *y = {call}; }}", True), (f"double h() {{ return {call}; }}", False)):
+        src = tmp_path / "call.cu"
+        src.write_text('#include "xc_fp64.cuh"\n' + body + "\n")
+        r = subprocess.run([nvcc, "-std=c++17", "--expt-relaxed-constexpr", "-gencode", "arch=compute_103a,code=sm_103a",
+                            "-I", os.path.join(ROOT, "xcore.jl_gb300", "csrc"), "-c", str(src), "-o",
+                            str(tmp_path / "call.o")], capture_output=True, text=True)
+        assert (r.returncode == 0) == ok, r.stderr

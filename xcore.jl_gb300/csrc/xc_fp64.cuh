@@ -610,19 +610,25 @@ XC_TABLE uint64_t xc_log_tab[256] = {
     0x01f98946c4e51d34ull, 0x01faf7be53ad9b7eull, 0x01fc66ec0d05314eull, 0x01fdd6d0a66103dcull,
 };
 
-#if defined(__CUDA_ARCH__)
+// (the tables are in device memory where nvcc compiles, so what reads them is
+// device code alone there)
+#ifdef __CUDACC__
 #define XC_TAB(t, i) __ldg(&t[i])
-XC_HD uint64_t xc_mulhi64(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
-#elif defined(__CUDACC__)
-#define XC_TAB(t, i) 0
-XC_HD uint64_t xc_mulhi64(uint64_t a, uint64_t b) { return (uint64_t)(((unsigned __int128)a * b) >> 64); }
+#define XC_TAB_FN __device__ __forceinline__
 #else
 #define XC_TAB(t, i) t[i]
-XC_HD uint64_t xc_mulhi64(uint64_t a, uint64_t b) { return (uint64_t)(((unsigned __int128)a * b) >> 64); }
+#define XC_TAB_FN inline
 #endif
+XC_HD uint64_t xc_mulhi64(uint64_t a, uint64_t b) {
+#ifdef __CUDA_ARCH__
+  return __umul64hi(a, b);
+#else
+  return (uint64_t)(((unsigned __int128)a * b) >> 64);
+#endif
+}
 
 // 2^(k + f / 2^64), |k| <= 1000
-XC_HD double xc_exp2_fixed(int k, uint64_t f) {
+XC_TAB_FN double xc_exp2_fixed(int k, uint64_t f) {
   const uint64_t t = XC_TAB(xc_exp2_tab, (uint32_t)(f >> 54));
   const uint64_t Y = xc_mulhi64(f << 10, 0xb17217f7d1cf79abull);   // y 2^74, y = r ln 2 < 2^-10.5
   const uint32_t yh = (uint32_t)(Y >> 32);
@@ -635,7 +641,7 @@ XC_HD double xc_exp2_fixed(int k, uint64_t f) {
   return xc_from_bits(((uint64_t)(uint32_t)(k + 1022) << 52) + (R >> 11) + ((R >> 10) & 1));
 }
 
-XC_HD double xc_exp(double x) {
+XC_TAB_FN double xc_exp(double x) {
   const uint64_t u = xc_bits(x);
   const uint32_t h = (uint32_t)(u >> 32) & 0x7fffffffu;
   if (h < 0x3f100000u) {                                           // |x| < 2^-14: four terms, errors of 2^-75
@@ -670,7 +676,7 @@ XC_HD double xc_exp(double x) {
 
 // log2(x) 2^57 of a normal x in [2^-62, 2^62], to within 2^-56
 XC_HD bool xc_log2_ok(double x) { return (uint32_t)(xc_bits(x) >> 52) - 961u <= 123u; }
-XC_HD int64_t xc_log2_fixed(double x) {
+XC_TAB_FN int64_t xc_log2_fixed(double x) {
   const uint64_t u = xc_bits(x);
   const int k = (int)(u >> 52) - 1023;
   const uint32_t i = (uint32_t)(u >> 44) & 255u;
@@ -687,7 +693,7 @@ XC_HD int64_t xc_log2_fixed(double x) {
 }
 
 // 2^(c 2^-58 l 2^-57), l signed: the power of a logarithm above
-XC_HD double xc_exp2_product(uint64_t c, int64_t l) {
+XC_TAB_FN double xc_exp2_product(uint64_t c, int64_t l) {
   const uint64_t a = l < 0 ? 0 - (uint64_t)l : (uint64_t)l;
   const uint64_t H = xc_mulhi64(a, c), L = a * c;                  // scale 2^115
   int64_t k = (int64_t)(H >> 51);
