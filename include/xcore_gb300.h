@@ -127,8 +127,9 @@ typedef struct xc_solver_opts {
                                (ascent) as one launch each, from shared-memory tiles; levels of at
                                most this many cells form every neighbour's value from global memory
                                instead (same results either way; default and -1: none) */
-  int stage_small_levels;  /* no longer chooses anything: the one-CTA V-cycles of the small levels run
-                              from shared memory wherever they fit it (same results) */
+  int stage_small_levels;  /* the one-CTA V-cycles of the small levels run from shared memory wherever
+                              they fit it (0, 1); -1: on global memory (same results; the velocity
+                              levels up to 16 x 16 in 15.3 us instead of 6.0) */
   int jacobi_coarse;       /* 1: Jacobi sweeps (coarse_sweeps) on the coarsest levels even where they
                               have at most 64 unknowns, which by default are solved with their
                               dense inverse (formed and inverted on the device once per solve) */

@@ -435,6 +435,33 @@ def test_staged_vcycle_gives_the_generic_results(shape, kw):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("solver", ["mixed", "fgmres64"])
+@pytest.mark.parametrize("shape,bc,kw", [
+    ((48, 40), {}, {}),                                              # 6x5 velocity cells (wide or swept), 3x5 pressure
+    ((64, 64), {}, dict(smooth_sweeps=2, post_sweeps=2, pressure_sweeps=1)),   # dense coarsest levels
+    ((64, 64), {}, dict(smooth_sweeps=3, pressure_sweeps=3)),        # an odd number of sweeps after each correction
+    ((44, 44), dict(open_cnv=True), dict(pressure_sweeps=1)),        # 11x11: wide inverse inside the CTA
+    ((56, 24), dict(top_cnv=-1, bot_cnv=-1), dict(jacobi_coarse=True)),        # sweeps inside the CTA, free slip
+    ((16, 256), {}, dict(pressure_sweeps=1)),                        # long levels
+])
+def test_staged_levels_give_the_generic_results(solver, shape, bc, kw):
+    """The one-CTA V-cycles of velocity and pressure from shared memory against the generic bodies on global memory
+    (stage_small_levels = -1): the same operations in the same order, so equal bits and iterations."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=shape[0], Nx=shape[1], steps=1)
+    coefs = O.time_coefs("bd2im", 2)
+    out = []
+    for stage in (0, -1):
+        ds = xc.State(product_params(par), grid=xc.Grid(Nx=g.Nx, Nz=g.Nz, h=g.h, D=g.D, L=g.L), scales=sc, **bc)
+        upload_all(ds, st)
+        info = ds.fluidmech(coefs, dt, solver=solver, rtol=1e-9, maxit=2000, inner_rtol=5e-2, stage_small_levels=stage,
+                            **kw)
+        out.append((info["iterations"], [ds[k] for k in ("W", "U", "P")]))
+        ds.close()
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("shape", [(66, 34), (128, 128), (130, 128)])
 @pytest.mark.parametrize("bc", [{}, dict(open_cnv=True)])
 def test_small_level_kernels_give_the_tiled_results(shape, bc):

@@ -99,7 +99,7 @@ class SolverOpts(ctypes.Structure):
                    int(coarse_cells), int(coarse_sweeps), int(small_cells), int(pressure_sweeps),
                    int(inner_gs_passes), int(bool(serial_launch)), int(coarse_viscosity_mean),
                    int(bool(tiled_sweep)), int(post_sweeps), int(outer_solver),
-                   int(fused_pressure_cells), int(bool(stage_small_levels)),
+                   int(fused_pressure_cells), int(stage_small_levels),
                    int(bool(jacobi_coarse)), int(bool(row_block_sweep)), int(learned), int(bool(device_givens)),
                    int(cluster_cells))
 

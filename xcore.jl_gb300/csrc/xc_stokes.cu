@@ -3523,8 +3523,8 @@ struct SolveCfg {
   // pressure levels of at most this many cells use the kernels that form every
   // neighbour's value anew (p_down_kernel, p_up_kernel) in place of the tiled ones
   long long pfuse_cells = 0;
-  // (accepted; the one-CTA levels run from shared memory wherever they fit it)
-  bool stage_small = false;
+  // one-CTA V-cycles from shared memory wherever their levels fit it
+  bool stage_small = true;
   // coarsest levels of at most kDenseMax unknowns solved by their inverse
   bool direct_coarse = true;
   // FP32 inner solves: 0 multigrid preconditioner, 1 the learned network in
@@ -4002,7 +4002,7 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
     }
     if (M.inv >= 0) S.add(H.vdirect ? (const void*)H.vinv : wi.inv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * M.ld);
     const int rows = (std::max(vel_stage_rows(g), 128) + 31) / 32 * 32;
-    if (rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
+    if (cfg.stage_small && rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
       pdl_smem(PDL_ON, vel_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, kf, l,
                lc, cfg.nu, om, coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx),
                (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok, wi);
@@ -4125,7 +4125,7 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
     }
     if (M.inv >= 0) S.add(H.pdirect ? (const void*)H.pinv : wi.inv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * M.ld);
     const int rows = (std::max(n, 128) + 31) / 32 * 32;
-    if (rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
+    if (cfg.stage_small && rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
       pdl_smem(PDL_ON, p_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, l, lc,
                cfg.nu_p, om, coarse_sweeps(cfg, H.pNz[lc], H.pNx[lc]), (const T*)(H.pdirect ? H.pinv : nullptr),
                (const int*)(H.dok + 1), p_wide(H, lc));
@@ -5516,7 +5516,7 @@ int fluidmech_impl(xc_ctx* c, const double coefs[6], double dt, const xc_solver_
   cfg.row_block = o.row_block_sweep != 0;
   cfg.device_givens = o.device_givens != 0;
   cfg.cluster_cells = o.cluster_cells < 0 ? 0 : (o.cluster_cells > 0 ? o.cluster_cells : 0);
-  cfg.stage_small = o.stage_small_levels != 0;
+  cfg.stage_small = o.stage_small_levels >= 0;
   cfg.direct_coarse = !o.jacobi_coarse;
   if (o.fused_pressure_cells != 0) cfg.pfuse_cells = o.fused_pressure_cells < 0 ? 0 : o.fused_pressure_cells;
   g_xc_pdl = cfg.pdl;
