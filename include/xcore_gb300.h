@@ -103,9 +103,8 @@ typedef struct xc_solver_opts {
   int schur_full_diagonal; /* 1: pressure Laplacian from the full velocity diagonal, no mass term */
   int coarse_cells;        /* a velocity level of at most this many cells is the coarsest, a pressure
                               level of a quarter of it (16; 256 for MMS) */
-  int coarse_sweeps;       /* Jacobi sweeps on a coarsest level that is not solved with its dense
-                              inverse (above 64 unknowns, or jacobi_coarse): 4 (Nz + Nx), at
-                              least 32; 200 for MMS */
+  int coarse_sweeps;       /* Jacobi sweeps on a coarsest level that is not solved with an inverse
+                              (jacobi_coarse): 4 (Nz + Nx), at least 32; 200 for MMS */
   int small_cells;         /* levels of at most this many cells run their V-cycle in one CTA
                               (256; -1: none) */
   int pressure_sweeps;     /* pressure-multigrid Jacobi sweeps before and after each coarse
@@ -130,9 +129,13 @@ typedef struct xc_solver_opts {
   int stage_small_levels;  /* the one-CTA V-cycles of the small levels run from shared memory wherever
                               they fit it (0, 1); -1: on global memory (same results; the velocity
                               levels up to 16 x 16 in 15.3 us instead of 6.0) */
-  int jacobi_coarse;       /* 1: Jacobi sweeps (coarse_sweeps) on the coarsest levels even where they
-                              have at most 64 unknowns, which by default are solved with their
-                              dense inverse (formed and inverted on the device once per solve) */
+  int jacobi_coarse;       /* 1: Jacobi sweeps (coarse_sweeps) on the coarsest levels even where these
+                              are solved with their inverse by default, formed on the device once
+                              per solve: up to 64 unknowns of the FP64 solver in FP64; up to 2048
+                              (and all of the mixed solver's) in FP32, the FP64 solver adding one
+                              refinement with the level's FP64 rows.  An inverse that does not
+                              reproduce a known vector to 1e-2 is not used, and grids whose sweeps
+                              leave the pressure's constant mode undetermined keep the sweeps. */
   int row_block_sweep;     /* 1: FP32 velocity sweeps with four consecutive rows along z per thread
                               and an interior path without boundary tests (same operations as the
                               default one row per thread; measured 20% slower at 1024^2: the
@@ -491,6 +494,13 @@ long long xc_launch_count(void);
    launch, algorithmic flops per launch, units per launch}.  Kernels 1-3 need
    a previous xc_fluidmech call (2 needs the mixed solver). */
 int xc_bench_kernel(xc_ctx* ctx, int which, int iters, double out[4]);
+
+/* How the last xc_fluidmech solved its small multigrid levels.  out = {the
+   coarsest velocity level, the coarsest pressure level: 0 Jacobi sweeps, 1 dense
+   inverse, 2 wide FP32 inverse; 1 where that inverse passed its check (else the
+   sweeps served in its place), velocity and pressure; 1 where the one-CTA
+   V-cycles ran from shared memory, velocity and pressure}.  Synchronises. */
+int xc_stokes_routes(xc_ctx* ctx, int out[6]);
 
 /* Last error message of the calling thread ("" when none). */
 const char* xc_last_error(void);

@@ -100,6 +100,84 @@ def test_wide_coarse_inverse_matches_lu(shape, solver):
     ds.close()
 
 
+def _expected_routes(shape, solver, dt0_h2, jacobi):
+    """The rule of the coarse solves: dense up to 64 unknowns (FP64), wide up to 2048 where the pressure level has at
+    most 64 cells or its sweeps determine the constant mode at the scales' first step."""
+    def coarsest(least):
+        a, b = shape
+        while a % 2 == 0 and b % 2 == 0 and a // 2 >= least and b // 2 >= least and (
+                a * b > 16 if least == 4 else 4 * a * b > 16):
+            a, b = a // 2, b // 2
+        return a, b
+    (a, b), (pa, pb) = coarsest(4), coarsest(2)
+    nv, n = (a + 1) * (b + 2) + (a + 2) * (b + 1), pa * pb
+    c = max(32, 4 * (pa + pb)) * 0.8 / (4 * n * dt0_h2)
+    wide = n <= 64 or c >= (0.01 if solver == "fgmres64" else 0.0125)
+    return ["sweeps" if jacobi else "dense" if solver == "fgmres64" and u <= 64 else
+            "wide" if wide and u <= 2048 else "sweeps" for u in (nv, n)]
+
+
+@pytest.mark.parametrize("solver", ["fgmres64", "mixed"])
+@pytest.mark.parametrize("shape,limit", [((32, 32), 0), ((44, 44), 0), ((50, 50), 0), ((30, 31), 0), ((31, 34), 0),
+                                         ((58, 54), -1), ((76, 84), -1), ((100, 100), -1)])
+def test_coarse_routes_match_lu(shape, limit, solver):
+    """Which way the coarsest levels are solved, dense, wide or by sweeps, on both sides of the lines between them
+    (limit -1: sweeps that leave the pressure's constant mode undetermined), and each way the sparse-LU solution."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=shape[0], Nx=shape[1], steps=1)
+    coefs = O.time_coefs("bd2im", 3)
+    ds = device_state(par, g, sc, st)
+    O.fluidmech(st, g, par, coefs, dt)
+    for jacobi in (False, True):
+        if jacobi:
+            upload_all(ds, start)
+        else:
+            import copy
+            start = copy.deepcopy(st)
+            for k in ("W", "U", "P", "MFS"):
+                setattr(start, k, ds[k])
+        ds.fluidmech(coefs, dt, solver=solver, rtol=1e-12, maxit=2000, inner_rtol=5e-2, jacobi_coarse=jacobi)
+        r, want = ds.solver_routes(), _expected_routes(shape, solver, sc["dt0"] / g.h ** 2, jacobi)
+        assert [r["velocity"], r["pressure"]] == want, (r, want)
+        assert r["velocity_ok"] == (want[0] != "sweeps") and r["pressure_ok"] == (want[1] != "sweeps"), r
+        if limit < 0:
+            assert want[0] == "sweeps", want
+        for k in ("W", "U", "P"):
+            assert _maxrel(ds[k], getattr(st, k)) <= 1e-8, (k, _maxrel(ds[k], getattr(st, k)))
+    ds.close()
+
+
+@pytest.mark.parametrize("solver,shape", [("mixed", (28, 32))] + [(s, n) for s in ("fgmres64", "mixed")
+                                                                  for n in ((44, 44), (52, 48), (50, 50))])
+def test_refused_wide_inverse_gives_the_sweeps(solver, shape):
+    """Coarsest levels whose wide inverse fails its check on the device: with free slip at both walls and next to no
+    inertia the velocity has an unlifted uniform mode, and the pressure matrix of so long a step (k = dt / h^2 = 2e7)
+    is too ill conditioned for FP32.  The sweeps then serve both levels, inside the one-CTA V-cycle (28x32), in the
+    coarse kernel (44: 11x11 cells) and behind the launches over the grid: the bits of jacobi_coarse."""
+    par, g, sc, ns, st, dt, rng = realistic_state(N=shape[0], Nx=shape[1], steps=1)
+    out = []
+    for jacobi in (False, True):
+        ds = xc.State(product_params(par), grid=xc.Grid(Nx=g.Nx, Nz=g.Nz, h=g.h, D=g.D, L=g.L), scales=sc, sds=-1,
+                      top_cnv=-1, bot_cnv=-1)
+        upload_all(ds, st)
+        for k in ("rho", "rhow", "rhou"):
+            ds[k] = np.full(ds[k].shape, 2800.0)
+        for k in ("eta", "etaco"):
+            ds[k] = 1e5 * (1 + 0.5 * np.random.default_rng(1).random(ds[k].shape))
+        try:
+            ds.fluidmech(O.time_coefs("bd2im", 1), 2e7 * g.h ** 2, solver=solver, rtol=1e-14, maxit=12, inner_rtol=1e-2,
+                         inner_maxit=6, jacobi_coarse=jacobi)
+        except xc.NotConverged:
+            pass
+        r = ds.solver_routes()
+        want = "sweeps" if jacobi else "wide"
+        assert r["velocity"] == r["pressure"] == want and not r["velocity_ok"] and not r["pressure_ok"], r
+        out.append([ds[k] for k in ("W", "U", "P")])
+        assert all(np.isfinite(a).all() for a in out[-1]) and np.abs(out[-1][0]).max() > 0
+        ds.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("bc", [dict(sds=-1, top_cnv=-1, bot_cnv=-1), dict(sds=-1, top_cnv=-1, bot_cnv=1),
                                 dict(sds=1, top_cnv=1, bot_cnv=1)])
 def test_fluidmech_boundary_variants_match_lu(bc):
@@ -440,9 +518,9 @@ def test_staged_vcycle_gives_the_generic_results(shape, kw):
     ((48, 40), {}, {}),                                              # 6x5 velocity cells (wide or swept), 3x5 pressure
     ((64, 64), {}, dict(smooth_sweeps=2, post_sweeps=2, pressure_sweeps=1)),   # dense coarsest levels
     ((64, 64), {}, dict(smooth_sweeps=3, pressure_sweeps=3)),        # an odd number of sweeps after each correction
-    ((44, 44), dict(open_cnv=True), dict(pressure_sweeps=1)),        # 11x11: wide inverse inside the CTA
-    ((56, 24), dict(top_cnv=-1, bot_cnv=-1), dict(jacobi_coarse=True)),        # sweeps inside the CTA, free slip
-    ((16, 256), {}, dict(pressure_sweeps=1)),                        # long levels
+    ((28, 32), dict(open_cnv=True), dict(pressure_sweeps=1)),        # 14x16, 7x8: wide inverse inside the CTA
+    ((56, 32), dict(top_cnv=-1, bot_cnv=-1), dict(jacobi_coarse=True)),        # sweeps inside the CTA, free slip
+    ((32, 128), {}, dict(pressure_sweeps=1)),                        # 8x32, 4x16: long levels
 ])
 def test_staged_levels_give_the_generic_results(solver, shape, bc, kw):
     """The one-CTA V-cycles of velocity and pressure from shared memory against the generic bodies on global memory
@@ -456,6 +534,8 @@ def test_staged_levels_give_the_generic_results(solver, shape, bc, kw):
         info = ds.fluidmech(coefs, dt, solver=solver, rtol=1e-9, maxit=2000, inner_rtol=5e-2, stage_small_levels=stage,
                             **kw)
         out.append((info["iterations"], [ds[k] for k in ("W", "U", "P")]))
+        routes = ds.solver_routes()
+        assert routes["velocity_staged"] == routes["pressure_staged"] == (stage == 0), routes
         ds.close()
     assert out[0][0] == out[1][0]
     for a, b in zip(out[0][1], out[1][1]):

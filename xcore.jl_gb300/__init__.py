@@ -183,6 +183,7 @@ def lib():
             "xc_stream": (vp, [vp]),
             "xc_launch_count": (ctypes.c_longlong, []),
             "xc_bench_kernel": (ip, [vp, ip, ip, D6]),
+            "xc_stokes_routes": (ip, [vp, vp]),
             "xc_update_dt_noalloc": (ip, [vp, vp, vp, vp, vp, ip, ip, dp, dp, dp, dp, vp, vp]),
             "xc_nn_conv3x3": (ip, [vp, vp, vp, vp, vp, ip, ip, ip, ip, ip, ip, vp]),
             "xc_nn_conv3x3_wgrad": (ip, [vp, vp, vp, ip, ip, ip, ip, ip, vp]),
@@ -452,6 +453,16 @@ class State:
         out = (ctypes.c_double * 4)()
         _check(lib().xc_bench_kernel(self._h, int(which), int(iters), out))
         return tuple(out)
+
+    def solver_routes(self):
+        """How the last fluidmech solved its small multigrid levels: the coarsest
+        velocity and pressure level by "sweeps", "dense" or "wide" inverse, whether
+        the inverses passed their check, whether the one-CTA V-cycles were staged."""
+        out = (ctypes.c_int * 6)()
+        _check(lib().xc_stokes_routes(self._h, out))
+        kind = ("sweeps", "dense", "wide")
+        return dict(velocity=kind[out[0]], pressure=kind[out[1]], velocity_ok=bool(out[2]), pressure_ok=bool(out[3]),
+                    velocity_staged=bool(out[4]), pressure_staged=bool(out[5]))
 
 
     # -- the reference's functions ------------------------------------------

@@ -532,6 +532,12 @@ thread_local long long g_xc_thread_launches = 0;
 extern "C" void* xc_stream(xc_ctx* c) { return c ? (void*)c->stream : nullptr; }
 extern "C" long long xc_launch_count(void) { return g_xc_launches.load(); }
 
+extern "C" int xc_stokes_routes(xc_ctx* c, int out[6]) {
+  XC_TRY(check_ctx(c));
+  if (!out) { xc_set_error("xc_stokes_routes: null argument"); return XC_BAD_ARG; }
+  return stokes_routes(c, out);
+}
+
 int noise_bench_zpass(xc_ctx* c, int iters, double out[4]);
 
 extern "C" int xc_bench_kernel(xc_ctx* c, int which, int iters, double out[4]) {

@@ -331,6 +331,7 @@ int stokes_create(xc_ctx* c);
 void stokes_destroy(xc_ctx* c);
 struct MmsData { const double *src_W, *src_U, *src_P, *W_exact, *U_exact, *P_exact; };
 int stokes_bench(xc_ctx* c, int which, int iters, double out[4]);
+int stokes_routes(xc_ctx* c, int out[6]);
 // before_solve (may be null) is called once on the host after the solve's
 // right-hand side and setup have been enqueued and before its iterations:
 // the step forks noise! there, so that it runs beside the latency-bound

@@ -3602,6 +3602,7 @@ struct Hier {
   int* wbad;
   int vwide_np, pwide_np;      // allocated sizes
   bool vwide_on, pwide_on;     // in use by the current solve
+  bool vstaged, pstaged;       // the last one-CTA V-cycles launched or captured ran from shared memory
   T* cp;          // DM coefficient planes (fine level)
   T* scl;         // scaling vector
   T* etarho;      // eta/rho on interior cells
@@ -4002,7 +4003,8 @@ int vcycle_vel(Hier<T>& H, const OpConst& kf, const SolveCfg& cfg, int l, cudaSt
     }
     if (M.inv >= 0) S.add(H.vdirect ? (const void*)H.vinv : wi.inv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * M.ld);
     const int rows = (std::max(vel_stage_rows(g), 128) + 31) / 32 * 32;
-    if (cfg.stage_small && rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
+    H.vstaged = cfg.stage_small && rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes;
+    if (H.vstaged) {
       pdl_smem(PDL_ON, vel_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, kf, l,
                lc, cfg.nu, om, coarse_sweeps(cfg, H.vg[lc].Nz, H.vg[lc].Nx),
                (const T*)(H.vdirect ? H.vinv : nullptr), (const int*)H.dok, wi);
@@ -4125,7 +4127,8 @@ int vcycle_p(Hier<T>& H, const SolveCfg& cfg, int l, cudaStream_t s, T** res) {
     }
     if (M.inv >= 0) S.add(H.pdirect ? (const void*)H.pinv : wi.inv, (int)sizeof(T) * M.inv, (long long)sizeof(T) * nd * M.ld);
     const int rows = (std::max(n, 128) + 31) / 32 * 32;
-    if (cfg.stage_small && rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes) {
+    H.pstaged = cfg.stage_small && rows <= 1024 && S.count <= kStageSegs && sizeof(T) * (size_t)M.total <= kStageMaxBytes;
+    if (H.pstaged) {
       pdl_smem(PDL_ON, p_vcycle_stage_kernel<T>, 1, rows, sizeof(T) * (size_t)M.total, s, L, M, S, l, lc,
                cfg.nu_p, om, coarse_sweeps(cfg, H.pNz[lc], H.pNx[lc]), (const T*)(H.pdirect ? H.pinv : nullptr),
                (const int*)(H.dok + 1), p_wide(H, lc));
@@ -4634,7 +4637,10 @@ __global__ void combine_dev_kernel(long long n, const KrylovDev* __restrict__ kd
   x[t] = s;
 }
 
-unsigned long long graph_key(const OpConst& k, const SolveCfg& cfg) {
+// what a captured step's launches depend on: the options, the boundary rows and how
+// the coarsest levels are solved
+template <typename T>
+unsigned long long graph_key(const Hier<T>& H, const OpConst& k, const SolveCfg& cfg) {
   unsigned long long h = 1469598103934665603ULL;
   auto mix = [&](double v) {
     unsigned long long b;
@@ -4642,6 +4648,7 @@ unsigned long long graph_key(const OpConst& k, const SolveCfg& cfg) {
     h = (h ^ b) * 1099511628211ULL;
   };
   mix(cfg.omega_v); mix(cfg.omega_p); mix(cfg.nu); mix(cfg.nu_post); mix(cfg.coarse_sweeps); mix(cfg.coarse_cells); mix(cfg.small_cells); mix(cfg.nu_p); mix(cfg.gs_passes); mix(cfg.pdl ? 1.0 : 0.0); mix(cfg.tiled ? 1.0 : 0.0); mix(cfg.cmass); mix(cfg.kplane); mix((double)cfg.pfuse_cells); mix(cfg.stage_small ? 1.0 : 0.0); mix(cfg.direct_coarse ? 1.0 : 0.0); mix((double)cfg.learned); mix(cfg.row_block ? 1.0 : 0.0); mix((double)cfg.cluster_cells);
+  mix(H.vdirect); mix(H.pdirect); mix(H.vwide_on); mix(H.pwide_on);
   mix(k.mms); mix(k.pin_u); mix(k.pin_p); mix(k.open_cnv); mix(k.sds); mix(k.top_cnv); mix(k.bot_cnv);
   return h | 1ULL;
 }
@@ -4659,7 +4666,7 @@ void drop_graphs(Hier<T>& H, int e) {
 // per context, so a graph stays valid across solves while the key holds)
 template <typename T>
 int arnoldi_step(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, int kk, cudaStream_t s) {
-  const unsigned long long key = graph_key(k, cfg);
+  const unsigned long long key = graph_key(H, k, cfg);
   int e = H.gkey[0] == key ? 0 : (H.gkey[1] == key ? 1 : -1);
   if (e < 0) {
     e = 1 - H.glast;   // replace the set used less recently
@@ -4753,7 +4760,7 @@ int build_cond_step(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg&
 // the conditional graph of step kk for this configuration, built on first use
 template <typename T>
 int cond_step(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg, int kk, cudaStream_t s) {
-  const unsigned long long key = graph_key(k, cfg);
+  const unsigned long long key = graph_key(H, k, cfg);
   int e = H.gkey[0] == key ? 0 : (H.gkey[1] == key ? 1 : -1);
   if (e < 0) {
     e = 1 - H.glast;
@@ -5194,15 +5201,19 @@ int setup_hier(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg,
   // inertia-free limit of the manufactured solution stays with its sweeps.
   H.vdirect = cfg.direct_coarse && nv <= kDenseMax && (!kFly<T> || k.mms);
   H.pdirect = cfg.direct_coarse && np <= kDenseMax && (!kFly<T> || k.mms);
-  // And where a coarsest pressure level is too large for its dense inverse,
-  // its sweeps must determine the pressure's slowest mode, the constant lifted
-  // by the pin alone, well enough that both ways end in the same digits: with
-  // k = dt / h^2 the mode decays as (1 - omega / (4 n k))^sweeps, c being that
-  // exponent at the scales' first time step.  Measured over 60 grids, P of the
-  // two ways differs by at most 2.5e-10 for c >= 0.01 (FP64 to a residual of
-  // 1e-12; the 100^2 box: c = 0.011, a step in 15 ms instead of 233) and c >=
-  // 0.0125 (mixed to 1e-13), but by 1e-9 to 2e-8 below, all of it the sweeps'
-  // error: there the results stay those of the sweeps.
+  // Where a coarsest pressure level is too large for its dense inverse, both levels
+  // keep their sweeps unless those determine the pressure's slowest mode, the
+  // constant lifted by the pin alone: with k = dt / h^2 it decays as
+  // (1 - omega / (4 n k))^sweeps, c being that exponent.  Up to c = 0.01 (FP64) and
+  // 0.0125 (mixed) the two ways' P over a time step differ by 1e-9 to 2e-8, above by
+  // at most 2.5e-10: the line keeps the results that such grids have had.  It is
+  // no bound of the inverse, which wide_check_kernel tests in every solve and which
+  // is the nearer way: against the sparse LU at 100^2 to 272^2, c from 0.001 to
+  // 0.03, P is off by 2e-11 to 6e-9 with it and by 6e-11 to 2e-5 with the sweeps
+  // (mixed to 1e-9; FP64 to 1e-10: 3e-11 to 3e-9 and 1e-11 to 5e-8), W and U
+  // likewise, and a 200^2 FP64 solve takes 5 ms in place of 35.  c is taken at the
+  // scales' first step, once for a context, and not at each solve's dt, which
+  // grows to 2.6 dt0 within four steps: a run keeps one way throughout.
   const double k0 = c->p.dt0 / (w->g.h * w->g.h);
   const double sweeps_c = coarse_sweeps(cfg, H.pNz[lp], H.pNx[lp]) * cfg.omega_p / (4.0 * (double)np * k0);
   const bool wide = cfg.direct_coarse && !k.mms && (np <= kDenseMax || sweeps_c >= (kFly<T> ? 0.0125 : 0.01));
@@ -5778,6 +5789,23 @@ int sweep_bench(cudaStream_t s, const Geo& g, const OpConst& k, const Hier<T>& H
   for (auto& v : cp)
     for (void* p : v) cudaFree(p);
   return st;
+}
+
+int stokes_routes(xc_ctx* c, int out[6]) {
+  StokesWork* w = c->stokes;
+  if (!w || !w->have_k) { xc_set_error("xc_stokes_routes: run xc_fluidmech first"); return XC_BAD_ARG; }
+  auto fill = [&](const auto& H) -> int {
+    int ok[2] = {0, 0};
+    XC_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    XC_CUDA_TRY(cudaMemcpy(ok, H.dok, sizeof(ok), cudaMemcpyDeviceToHost));
+    out[0] = H.vdirect ? 1 : (H.vwide_on ? 2 : 0);
+    out[1] = H.pdirect ? 1 : (H.pwide_on ? 2 : 0);
+    for (int q = 0; q < 2; ++q) out[2 + q] = out[q] ? ok[q] : 0;
+    out[4] = H.vstaged;
+    out[5] = H.pstaged;
+    return XC_OK;
+  };
+  return w->last_fp64_mg ? fill(w->d) : fill(w->f);
 }
 
 int stokes_bench(xc_ctx* c, int which, int iters, double out[4]) {
