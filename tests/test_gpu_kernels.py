@@ -176,6 +176,26 @@ def test_thin_diffusion_of_many_columns_bitwise(Nx):
     np.testing.assert_array_equal(_host(d), O.diffus_halo(fh, kh, 0.2))
 
 
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("scale", [1e-310, 3e-308, 1e-300])
+def test_subnormal_fields_bitwise(scheme, scale):
+    """Advection and diffusion of fields at the lower end of the range, whose halves and quarters round."""
+    Nz, Nx = 33, 29
+    rng = np.random.default_rng(9)
+    f, k = scale * rng.standard_normal((Nz, Nx)), rng.random((Nz, Nx))
+    u, w = rng.standard_normal((Nz, Nx + 1)), rng.standard_normal((Nz + 1, Nx))
+    d = [torch.zeros(s, dtype=torch.float64, device="cuda") for s in ((Nx, Nz), (Nx + 1, Nz + 2), (Nx + 2, Nz + 1))]
+    xc.advect_centered_with_flux(*d, _dev(f), _dev(u), _dev(w), 0.37, scheme)
+    torch.cuda.synchronize()
+    for got, want in zip(d, O.advect_centered_with_flux(f, u, w, 0.37, scheme)):
+        np.testing.assert_array_equal(_host(got), want)
+    fh, kh = O.embed_halo(f, 1, "closed", "periodic"), O.embed_halo(k, 1, "closed", "periodic")
+    xc.diffus_with_flux(*d, _dev(fh), _dev(kh), 0.37)
+    torch.cuda.synchronize()
+    for got, want in zip(d, O.diffus_centered_with_flux(f, k, 0.37)):
+        np.testing.assert_array_equal(_host(got), want)
+
+
 def test_ghosts_halo3_both_closed():
     Nz, Nx, g = 9, 6, 3
     f = np.random.default_rng(1).random((Nz, Nx))

@@ -14,7 +14,8 @@
 // What bounds it: sm_103a's FP64 unit takes one warp instruction per 64 cycles
 // and sub-partition, so the stencils cost their FP64 instructions and little
 // else.  Products by 2, 4 and 1/4 are exact and go into the following sum as an
-// FMA (the same rounding, one instruction instead of two), quotients and most
+// FMA (the same rounding, one instruction instead of two; WENO5's quarters of
+// squares, where a subnormal one is far below the sum), quotients and most
 // other products run on the integer pipe (xc_fp64.cuh), signs are tested on
 // the bits: what is left for the FP64 unit are the sums.  WENO5 in the
 // reference's form takes 27 FP64 instructions per face, and some 1400 integer
@@ -149,7 +150,7 @@ __device__ __forceinline__ double face_flux(double s0, double s1, double s2, dou
       const bool up = !sign_bit(v);
       const double a1 = up ? s1 : s4, a2 = up ? s2 : s3, a3 = up ? s3 : s2;
       return xc_mul(v, S == XC_QUICK ? xc_mul(__fma_rn(2.0, a3, xc_mul_small<5>(a2)) - a1, sixth)
-                                     : __fma_rn(0.25, a3 - a1, a2));
+                                     : a2 + xc_scale2<-2>(a3 - a1));   // (a quarter of a subnormal rounds)
     }
     double pos, neg;
     if (S == XC_QUICK) {
@@ -337,9 +338,15 @@ __global__ void __launch_bounds__(T::NT) advect_tile_kernel(FluxArgs a, int Nz, 
 // diffusion of one tile (diffus.jl:9-31, 68-91).  A face's product
 // (k_L + k_R)(f_R - f_L) is formed once: the divergence takes it from both
 // sides, and the face flux -(k_L + k_R)/2 (f_R - f_L)/h is the same product
-// halved and negated, which is exact (subnormal products aside, far below any
-// flux).  7 FP64 instructions per cell instead of 28.
+// halved and negated, which is exact but for subnormal products.  7 FP64
+// instructions per cell instead of 28.
 // ---------------------------------------------------------------------------
+__device__ __noinline__ double diffus_flux_any(double k, double df, double invh) { return (((-k) * 0.5) * df) * invh; }
+__device__ __forceinline__ double diffus_flux(double q, double mhalf_invh, double k, double df, double invh) {
+  const uint64_t u = xc_bits(q) << 1;
+  if (u - 1 < (3ull << 53) - 1) return diffus_flux_any(k, df, invh);     // not zero, below 2^-1020
+  return xc_mul(q, mhalf_invh);
+}
 template <class T, bool HALOD>
 __device__ __forceinline__ void diffus_tile(TileSmem<T, 1>& sm, double* sk, const FluxArgs& a, int Nz, int Nx, int xBC,
                                             int zBC, double invh, bool pad) {
@@ -374,14 +381,14 @@ __device__ __forceinline__ void diffus_tile(TileSmem<T, 1>& sm, double* sk, cons
     const int ii = xf ? k / TZ : k / (TZ + 1), jj = k - ii * (xf ? TZ : TZ + 1);
     const int j = j0 + jj, i = i0 + ii;
     const int c = (ii + 1) * HZ + jj + 1, b = c - (xf ? HZ : 1);
-    const double q = xc_mul(sk[c] + sk[b], sm.f[c] - sm.f[b]);
+    const double ks = sk[c] + sk[b], df = sm.f[c] - sm.f[b], q = xc_mul(ks, df);
     sm.q[idx] = q;
     if (xf) {
       if (a.qx.p && j < Nz && i <= Nx && (ii < TX || i == Nx))
-        put_qx(a.qx, j, i, xc_mul(q, mhalf_invh), Nz, zBC, pad);
+        put_qx(a.qx, j, i, diffus_flux(q, mhalf_invh, ks, df, invh), Nz, zBC, pad);
     } else {
       if (a.qz.p && j <= Nz && i < Nx && (jj < TZ || j == Nz))
-        put_qz(a.qz, j, i, xc_mul(q, mhalf_invh), Nx, xBC, pad);
+        put_qz(a.qz, j, i, diffus_flux(q, mhalf_invh, ks, df, invh), Nx, xBC, pad);
     }
   }
   if (!a.out.p) return;
