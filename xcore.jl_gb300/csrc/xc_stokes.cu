@@ -2085,10 +2085,10 @@ __global__ void __launch_bounds__(kTileThreads) p_up_tile_kernel(int Nz, int Nx,
 // per coarse cell takes its 2 x 2 fine ones, whose values, coefficients and
 // prolongations it shares between them, in pairs along z (Nz is even), without
 // a halo formed twice.  FP32 only: in FP64 the ascent's twelve prolongations cost
-// more of the FP64 unit than the tile's (1024^2 step of the FP64 solver 106 against
-// 103 ms).  From which size on matters little (1024^2 step with the
-// line at 64^2, 128^2, 256^2 cells: 1.602x, 1.608x, 1.592x of the original,
-// without them 1.499x; 512^2 solve 1.573x, 1.560x, 1.581x and 1.536x).
+// more of the FP64 unit than the tile's (1024^2 step of the FP64 solver 109 against
+// 106 ms).  From which size on matters little (1024^2 mixed step with the line at
+// 64^2, 128^2, 256^2 cells: 34.5, 34.3, 34.7 ms, without them 36.8; 512^2 solve
+// 4.29, 4.33, 4.27 and 4.39 ms).
 template <typename T>
 struct Pair { T a, b; };
 __device__ __forceinline__ Pair<float> ld_pair(const float* p) {
@@ -5208,10 +5208,10 @@ int setup_hier(StokesWork* w, Hier<T>& H, const OpConst& k, const SolveCfg& cfg,
   // 0.0125 (mixed) the two ways' P over a time step differ by 1e-9 to 2e-8, above by
   // at most 2.5e-10: the line keeps the results that such grids have had.  It is
   // no bound of the inverse, which wide_check_kernel tests in every solve and which
-  // is the nearer way: against the sparse LU at 100^2 to 272^2, c from 0.001 to
-  // 0.03, P is off by 2e-11 to 6e-9 with it and by 6e-11 to 2e-5 with the sweeps
-  // (mixed to 1e-9; FP64 to 1e-10: 3e-11 to 3e-9 and 1e-11 to 5e-8), W and U
-  // likewise, and a 200^2 FP64 solve takes 5 ms in place of 35.  c is taken at the
+  // is mostly the nearer way: against the sparse LU in 30 solves at 72 x 104 to 272^2,
+  // c from 0.001 to 0.1, P is off by 7e-10 (median; 2e-8 at most) with it and by 2e-8
+  // (2e-5) with the sweeps (mixed to 1e-9; FP64 to 1e-10: 2e-10 (3e-9) and 5e-10
+  // (5e-8)), and a 200^2 FP64 solve takes 5 ms in place of 35.  c is taken at the
   // scales' first step, once for a context, and not at each solve's dt, which
   // grows to 2.6 dt0 within four steps: a run keeps one way throughout.
   const double k0 = c->p.dt0 / (w->g.h * w->g.h);

@@ -12,9 +12,10 @@
 // twenty.  Quotients, roots, exponentials, logarithms, halvings and
 // comparisons run on the integer pipe instead (correctly rounded quotients
 // and roots: the same bits), which leaves a few additions and products per
-// cell on the FP64 unit.  At 1024^2: volfrac_rheology 468 -> 76 us, kinematics
-// 226 -> 78, blend_segvisc 154 -> 50, stress 83 -> 40, viscblend 76 -> 26,
-// corner_eta 59 -> 20, interp 51 -> 33, etas_blend 49 -> 17.
+// cell on the FP64 unit.  A call at 1024^2 1093 -> 267 us; of it, as single
+// launches with a cold cache: volfrac_rheology 468 -> 78 us, kinematics 226 -> 67,
+// blend_segvisc 154 -> 40, stress 83 -> 36, viscblend 76 -> 25, corner_eta 59 ->
+// 22, interp 51 -> 34, etas_blend 49 -> 19.
 #include <cmath>
 
 #include "xc_internal.cuh"
@@ -233,8 +234,9 @@ __device__ __forceinline__ void for_corner_tiles(int Nz, int Nx, double (&sq)[9]
 }
 
 // update_kinematics! (update.jl:202-280): exz on corners, the rest on cells.
-// 23 FP64 instructions per cell instead of 120: at 1024^2 226 us with everything
-// on the FP64 unit, 78 us without quotients and roots, 59 us without products.
+// 22 FP64 instructions per cell instead of 120: at 1024^2 226 us with everything
+// on the FP64 unit, 67 us now (single launches with a cold cache; within a call 78
+// us without quotients and roots, 59 us without products).
 // (volfrac_rheology, viscblend and the blends keep their products there: they are
 // bound by integer issue already, and took 5 to 40 % longer with them moved.)
 __global__ void kinematics_kernel(int Nz, int Nx, double invh, CView W, CView U, CView wx,
