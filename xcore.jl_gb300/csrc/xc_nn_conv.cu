@@ -455,11 +455,12 @@ bool tile_shape(int H, int W, int* bw, int* bh) {
 // of A are 128 / Cin of these tiles at a time (16 and 32 channels: all of them,
 // 64: two and two, 128: one by one), so one pass over A serves several taps; rows
 // beyond the fourth tile (16 channels) read what lies behind, and no row but
-// the taps' is stored.  Operands come in as the forward's pixels do.  It was bound by two-byte transposing stores and by nine passes over dY with M
-// mostly zero rows: 16 x 16 channels at 8 x 256 x 256 pixels 154 us, with the
-// bias gradient's own two kernels 220; now 62 and 3 for the reduction.  What
-// bounds it is the rate of the MMAs themselves (eight per tile and CTA, about
-// 110 clocks each; a second accumulator for every other tile changes nothing).
+// the taps' is stored.  Operands come in as the forward's pixels do.  It was bound
+// by two-byte transposing stores and by nine passes over dY with M mostly zero
+// rows: 16 x 16 channels at 8 x 256 x 256 pixels 154 us, with the bias gradient's
+// own two kernels 220; now 62 and 3 for the reduction.  What bounds it is the rate
+// of the MMAs themselves (eight per tile and CTA, about 110 clocks each; a second
+// accumulator for every other tile changes nothing).
 struct WgradArgs {
   const __nv_bfloat16* x;    // NHWC [B][H][W][Cin]
   const __nv_bfloat16* dy;   // NHWC [B][H][W][Cout]
